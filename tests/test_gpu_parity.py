@@ -608,6 +608,24 @@ def test_prefill_shapes_full_size(ctx, oracle, pkg, name, g, M):
     assert np.array_equal(got.view(np.uint16), want.view(np.uint16))
 
 
+@pytest.mark.parametrize("g", [64, 128, 256])
+@pytest.mark.parametrize("bt,form", [(32, "SINGLE"), (64, "SINGLE"), (96, "SINGLE"), (128, "SINGLE"), (192, "PAIR"), (256, "PAIR")])
+@pytest.mark.parametrize("M,N,K", [(1, 136, 256), (257, 272, 1280), (383, 40, 768)])
+def test_gemm_tcgen05_tile_widths(ctx, oracle, pkg, monkeypatch, M, N, K, bt, form, g):
+    """Every token width of a tile: one token, tiles that end one past or one short of a width, rows that end inside a
+    warp's 32, K of 2, 6 and 10 stages (the ring of stages and the ring of scale chunks wrap at other places than the
+    tiles do), an odd and an even number of groups. Bit for bit the oracle's."""
+    monkeypatch.setenv("W8A8_GEMM_BT", str(bt))
+    X, W, ws = synth.linear_case(M + N + K + bt, M, N, K, g)
+    Xq, Xs = oracle.quantize(X, g)
+    buf, dY = guarded((M, N), torch.float16, 99.0)
+    ctx.linear_q(dev(W), dev(ws), g, dev(Xq), dev(Xs), dY, M, N, K, kernel=getattr(pkg, "KERNEL_GEMM_" + form))
+    torch.cuda.synchronize()
+    ctx.check_device_status()
+    assert guards_intact(buf, 99.0)
+    assert np.array_equal(dY.cpu().numpy().view(np.uint16), oracle.linear_q(W, ws, Xq, Xs, g).view(np.uint16))
+
+
 @pytest.mark.parametrize("split_k", [1, 2, 3, 4, 5, 8])
 def test_gemv_split_k_is_deterministic_and_correct(ctx, oracle, pkg, split_k):
     M, N, K, g = 16, 320, 2560, 256
