@@ -40,6 +40,26 @@ __device__ __forceinline__ float warp_max(float v) {
     return v;
 }
 
+// Eight int8 codes (int8_gemm.cu:201-210), packed two at a time by the saturating pack instruction. A scale made from the
+// group's own maximum gives no code below -127, so only a static scale (STATIC) needs the lower clamp. (At prefill sizes the
+// row kernels are bound by instructions as much as by bytes; shifts and masks per code were half of them.)
+__device__ __forceinline__ uint2 codes8(const float (&v)[8], float inv_scale, bool is_static) {
+    int q[8];
+#pragma unroll
+    for (int e = 0; e < 8; ++e) q[e] = __float2int_rn(v[e] * inv_scale);
+    if (is_static) {
+#pragma unroll
+        for (int e = 0; e < 8; ++e) q[e] = max(-127, q[e]);
+    }
+    uint32_t w[2];
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+        asm("cvt.pack.sat.s8.s32.b32 %0, %1, %2, %3;" : "=r"(w[h]) : "r"(q[4 * h + 3]), "r"(q[4 * h + 2]), "r"(0));
+        asm("cvt.pack.sat.s8.s32.b32 %0, %1, %2, %3;" : "=r"(w[h]) : "r"(q[4 * h + 1]), "r"(q[4 * h]), "r"(w[h]));
+    }
+    return make_uint2(w[0], w[1]);
+}
+
 __global__ void __launch_bounds__(1024) rowquant_kernel(const RowQuantParams p) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     __half* row = reinterpret_cast<__half*>(smem_raw);
@@ -400,88 +420,209 @@ __global__ void __launch_bounds__(256) rowquant_compact_kernel(const RowQuantPar
         float scale = amax / 127.0f;
         if (scale < 1e-8f) scale = 1e-8f;
         if ((lane & (LANES - 1)) == 0) p.Xs[static_cast<size_t>(row) * G + (c8 * 8) / GM] = scale;
-        const float inv_scale = 1.0f / scale;
-        uint32_t lo = 0, hi = 0;
-#pragma unroll
-        for (int e = 0; e < 8; ++e) {
-            int q = __float2int_rn(v[e] * inv_scale);
-            q = max(-127, min(127, q));
-            if (e < 4) lo |= (static_cast<uint32_t>(q) & 0xffu) << (8 * e);
-            else hi |= (static_cast<uint32_t>(q) & 0xffu) << (8 * (e - 4));
-        }
-        *reinterpret_cast<uint2*>(p.Xq + base + c8 * 8) = make_uint2(lo, hi);
+        *reinterpret_cast<uint2*>(p.Xq + base + c8 * 8) = codes8(v, 1.0f / scale, false);
     }
     W8A8_TRACE_END(2u);
 }
 
-// The quantiser alone (int8_gemm.cu:147-211) for g in {64, 128, 256}: no shared memory, no block
-// barrier. A thread owns 8 consecutive activations (one 128-bit load), the g/8 threads of a group
-// find the absmax with shuffles, and each thread stores its 8 codes as one 64-bit word. At decode
-// sizes the whole activation matrix is a few KB, so what counts is the length of the dependency
-// chain (one load, log2(g/8) shuffles, one divide, one store), not bandwidth.
-template <int LANES>  // threads per group = g / 8
+// [residual add] -> RMSNorm -> [group quantiser] for many rows (prefill): a WARP per row, the row in registers from the
+// load to the codes, no shared memory and no barrier; K a multiple of 256, 512 < K <= 256 * KI, g in {64, 128, 256}.
+// Lane l owns the 16-byte pieces l + 32 i of its row, i.e. elements e = 8 l + j + 256 i (j < 8): these are ALL the elements
+// of the reference's virtual threads vt = 8 l + j + 256 (i mod 4) of its 1024-thread launch (rms_norm.cu:23-27), which sum
+// e = vt, vt + 1024, ... in that order, so its sum of squares can be taken in exactly the reference's order.
+// A row kernel at these sizes is bandwidth: what counts is loads in flight. A CTA per row (rowquant_compact_kernel) has
+// two 16-byte loads per thread and four barriers: 8192 x 2560 took 40 us (1.6 TB/s); ten per lane and no barrier: 19 us.
+template <int GM, int KI>
+__global__ void __launch_bounds__(128, KI > 10 ? 4 : 5) rownorm_warp_kernel(const RowQuantParams p, int M) {
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    const int lane = threadIdx.x & 31, row = blockIdx.x * 4 + (threadIdx.x >> 5);
+    if (row >= M) return;
+    const int K = p.K, iters = K / 256;
+    const size_t base = static_cast<size_t>(row) * K;
+    const __half* res = p.residual ? p.residual + base : nullptr;
+    uint4 v[KI];
+#pragma unroll
+    for (int i = 0; i < KI; ++i)
+        if (i < iters) v[i] = reinterpret_cast<const uint4*>(p.x_in + base)[lane + 32 * i];
+    if (res) {
+#pragma unroll
+        for (int i0 = 0; i0 < KI; i0 += 5) {  // five residual pieces in flight at a time
+            uint4 r[5];
+#pragma unroll
+            for (int i = 0; i < 5; ++i)
+                if (i0 + i < KI && i0 + i < iters) r[i] = reinterpret_cast<const uint4*>(res)[lane + 32 * (i0 + i)];
+#pragma unroll
+            for (int i = 0; i < 5; ++i)
+                if (i0 + i < KI && i0 + i < iters) {
+                    __half* hv = reinterpret_cast<__half*>(&v[i0 + i < KI ? i0 + i : 0]);
+                    const __half* hr = reinterpret_cast<const __half*>(&r[i]);
+#pragma unroll
+                    for (int e = 0; e < 8; ++e) hv[e] = __float2half(__half2float(hv[e]) + __half2float(hr[e]));
+                }
+        }
+        if (p.x_out) {  // (may be x_in: every load of the row is above)
+#pragma unroll
+            for (int i = 0; i < KI; ++i)
+                if (i < iters) reinterpret_cast<uint4*>(p.x_out + base)[lane + 32 * i] = v[i];
+        }
+    }
+    float ls[4][8];  // per virtual thread (r, j): its elements i = r, r + 4, r + 8, ... ascending
+#pragma unroll
+    for (int r = 0; r < 4; ++r)
+#pragma unroll
+        for (int j = 0; j < 8; ++j) ls[r][j] = 0.0f;
+#pragma unroll
+    for (int i = 0; i < KI; ++i)
+        if (i < iters) {
+            const __half* hv = reinterpret_cast<const __half*>(&v[i]);
+#pragma unroll
+            for (int j = 0; j < 8; ++j) {
+                const float val = __half2float(hv[j]);
+                ls[i & 3][j] += val * val;
+            }
+        }
+    // The reference's shuffle-down tree over a virtual warp: virtual warp (r, l / 4) is made of the virtual lanes
+    // 8 (l % 4) + j; offsets 16 and 8 cross real lanes (l + 2, l + 1), offsets 4, 2, 1 stay inside the lane's eight j. Only
+    // virtual lane 0 is used afterwards, and it takes exactly the reference's operands in the reference's order.
+    float wsum[4];
+#pragma unroll
+    for (int r = 0; r < 4; ++r) {
+        float b8[8];
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+            float local_sum = ls[r][j];
+            local_sum += __shfl_down_sync(0xffffffffu, local_sum, 2);
+            local_sum += __shfl_down_sync(0xffffffffu, local_sum, 1);
+            b8[j] = local_sum;
+        }
+#pragma unroll
+        for (int j = 0; j < 4; ++j) b8[j] += b8[j + 4];
+        b8[0] += b8[2];
+        b8[1] += b8[3];
+        wsum[r] = b8[0] + b8[1];
+    }
+    // second tree (rms_norm.cu:36-42): lane w takes the sum of virtual warp w = 8 r + q, which lives in lane 4 q
+    float total_sum = 0.0f;
+#pragma unroll
+    for (int r = 0; r < 4; ++r) {
+        const float t = __shfl_sync(0xffffffffu, wsum[r], 4 * (lane & 7));
+        if ((lane >> 3) == r) total_sum = t;
+    }
+    for (int offset = 16; offset > 0; offset /= 2) total_sum += __shfl_down_sync(0xffffffffu, total_sum, offset);
+    total_sum = __shfl_sync(0xffffffffu, total_sum, 0);
+    const float rms = rsqrtf(total_sum / K + p.eps);
+    constexpr int LANES = GM / 8;
+#pragma unroll
+    for (int i = 0; i < KI; ++i)
+        if (i < iters) {
+            const int c8 = lane + 32 * i;
+            const uint4 w = __ldg(reinterpret_cast<const uint4*>(p.norm_weight) + c8);
+            __half* hv = reinterpret_cast<__half*>(&v[i]);
+            const __half* hw = reinterpret_cast<const __half*>(&w);
+            float f[8], amax = 0.0f;
+#pragma unroll
+            for (int e = 0; e < 8; ++e) {
+                const float val = __half2float(hv[e]) * rms;
+                hv[e] = __float2half(val * __half2float(hw[e]));
+                f[e] = __half2float(hv[e]);
+                amax = fmaxf(amax, fabsf(f[e]));
+            }
+            if (p.normed_out) reinterpret_cast<uint4*>(p.normed_out + base)[c8] = v[i];
+            if (p.Xq) {
+#pragma unroll
+                for (int o = LANES / 2; o > 0; o >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, o));
+                float scale = amax / 127.0f;
+                if (scale < 1e-8f) scale = 1e-8f;
+                if ((lane & (LANES - 1)) == 0) p.Xs[static_cast<size_t>(row) * p.G + (c8 * 8) / GM] = scale;
+                *reinterpret_cast<uint2*>(p.Xq + base + c8 * 8) = codes8(f, 1.0f / scale, false);
+            }
+        }
+}
+
+// The quantiser alone (int8_gemm.cu:147-211) for g in {64, 128, 256}, K a multiple of g: no shared memory, no block
+// barrier. A thread owns 8 consecutive activations (one 128-bit load), the g/8 threads of a group find the absmax with
+// shuffles, and each thread stores its 8 codes as one 64-bit word. The groups of all rows lie one after another ([M, K] and
+// [M, G] are contiguous and K is a multiple of g), so the whole matrix is one flat run of pieces. At decode sizes it is a
+// few KB, and what counts is the length of the dependency chain (one load, log2(g/8) shuffles, one divide, one store): one
+// piece per thread (U = 1). At prefill sizes it is bandwidth: four loads in flight per thread (8192 x 9728: 86 -> 37 us, 6.5 TB/s).
+template <int LANES, int U>  // LANES: threads per group = g / 8
 __global__ void __launch_bounds__(128) groupquant_kernel(const __half* __restrict__ X,
                                                          const __half* __restrict__ smooth_inv,
                                                          const __half* __restrict__ act_scale,
-                                                         int8_t* __restrict__ Xq, float* __restrict__ Xs, int K,
-                                                         int G) {
+                                                         int8_t* __restrict__ Xq, float* __restrict__ Xs, unsigned pieces,
+                                                         unsigned K8) {
     W8A8_TRACE_SCOPE();
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     asm volatile("griddepcontrol.wait;" ::: "memory");
     W8A8_TRACE_WAITED();
-    const int m = blockIdx.y;
-    const int e = (blockIdx.x * 128 + threadIdx.x) * 8;
-    const bool live = e < K;
-    float v[8];
-    float amax = 0.0f;
-    if (live) {
-        const uint4 u = *reinterpret_cast<const uint4*>(X + static_cast<size_t>(m) * K + e);
-        const __half* h = reinterpret_cast<const __half*>(&u);
-        uint4 su = make_uint4(0, 0, 0, 0);
-        if (smooth_inv) su = *reinterpret_cast<const uint4*>(smooth_inv + e);
-        const __half* sh = reinterpret_cast<const __half*>(&su);
+    const unsigned p0 = blockIdx.x * (128u * U) + threadIdx.x;
+    uint4 u[U];
 #pragma unroll
-        for (int i = 0; i < 8; ++i) {
-            v[i] = __half2float(h[i]);
-            if (smooth_inv) v[i] *= __half2float(sh[i]);
-            amax = fmaxf(amax, fabsf(v[i]));
+    for (int k = 0; k < U; ++k)  // (a whole group is live or not: pieces is a multiple of LANES)
+        u[k] = p0 + k * 128u < pieces ? *(reinterpret_cast<const uint4*>(X) + p0 + k * 128u) : make_uint4(0, 0, 0, 0);
+#pragma unroll
+    for (int k = 0; k < U; ++k) {
+        const unsigned pc = p0 + k * 128u;
+        const bool live = pc < pieces;
+        const __half* h = reinterpret_cast<const __half*>(&u[k]);
+        float v[8], amax = 0.0f;
+#pragma unroll
+        for (int i = 0; i < 8; ++i) v[i] = __half2float(h[i]);
+        const unsigned c8 = (smooth_inv || act_scale) ? pc % K8 : 0u;  // piece inside its row
+        if (smooth_inv) {
+            const uint4 su = __ldg(reinterpret_cast<const uint4*>(smooth_inv) + c8);
+            const __half* sh = reinterpret_cast<const __half*>(&su);
+#pragma unroll
+            for (int i = 0; i < 8; ++i) v[i] *= __half2float(sh[i]);
         }
-    }
 #pragma unroll
-    for (int o = LANES / 2; o > 0; o >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, o));
-    if (!live) return;
-    const int j = e / (LANES * 8);
-    float scale = act_scale ? __half2float(act_scale[j]) : amax / 127.0f;
-    if (scale < 1e-8f) scale = 1e-8f;
-    if ((threadIdx.x & (LANES - 1)) == 0) Xs[static_cast<size_t>(m) * G + j] = scale;
-    const float inv_scale = 1.0f / scale;
-    uint32_t lo = 0, hi = 0;
+        for (int i = 0; i < 8; ++i) amax = fmaxf(amax, fabsf(v[i]));
 #pragma unroll
-    for (int i = 0; i < 8; ++i) {
-        int q = __float2int_rn(v[i] * inv_scale);
-        q = max(-127, min(127, q));
-        if (i < 4) lo |= (static_cast<uint32_t>(q) & 0xffu) << (8 * i);
-        else hi |= (static_cast<uint32_t>(q) & 0xffu) << (8 * (i - 4));
+        for (int o = LANES / 2; o > 0; o >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, o));
+        if (!live) continue;
+        float scale = act_scale ? __half2float(act_scale[c8 / LANES]) : amax / 127.0f;
+        if (scale < 1e-8f) scale = 1e-8f;
+        if ((threadIdx.x & (LANES - 1)) == 0) Xs[pc / LANES] = scale;
+        *reinterpret_cast<uint2*>(Xq + static_cast<size_t>(pc) * 8) = codes8(v, 1.0f / scale, act_scale != nullptr);
     }
-    *reinterpret_cast<uint2*>(Xq + static_cast<size_t>(m) * K + e) = make_uint2(lo, hi);
     W8A8_TRACE_END(3u);
 }
 
-template <int LANES>
-int launch_groupquant(const __half* X, const __half* smooth_inv, const __half* act_scale, int8_t* Xq, float* Xs,
-                      int M, int K, int G, cudaStream_t stream) {
+template <typename... Params, typename... Args>
+int launch_row_kernel(const char* what, void (*kernel)(Params...), unsigned blocks, unsigned threads, size_t smem, cudaStream_t stream,
+                      Args... args) {
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((K + 1023) / 1024, M, 1);
-    cfg.blockDim = dim3(128, 1, 1);
+    cfg.gridDim = dim3(blocks, 1, 1);
+    cfg.blockDim = dim3(threads, 1, 1);
+    cfg.dynamicSmemBytes = smem;
     cfg.stream = stream;
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
     cfg.numAttrs = pdl_enabled(kPdlRow) ? 1 : 0;
-    cudaError_t e = cudaLaunchKernelEx(&cfg, groupquant_kernel<LANES>, X, smooth_inv, act_scale, Xq, Xs, K, G);
-    if (e != cudaSuccess) return fail(W8A8_ERR_CUDA, "groupquant launch: %s", cudaGetErrorString(e));
+    cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, args...);
+    if (e != cudaSuccess) return fail(W8A8_ERR_CUDA, "%s launch: %s", what, cudaGetErrorString(e));
     return W8A8_OK;
+}
+
+template <int LANES>
+int launch_groupquant(const __half* X, const __half* smooth_inv, const __half* act_scale, int8_t* Xq, float* Xs,
+                      unsigned pieces, unsigned K8, cudaStream_t stream) {
+    // four pieces per thread once the single-piece form would fill every SM with more than two rounds of threads
+    if (pieces > 148u * 2048u * 2u)
+        return launch_row_kernel("groupquant", groupquant_kernel<LANES, 4>, (pieces + 511) / 512, 128, 0, stream, X, smooth_inv,
+                                 act_scale, Xq, Xs, pieces, K8);
+    return launch_row_kernel("groupquant", groupquant_kernel<LANES, 1>, (pieces + 127) / 128, 128, 0, stream, X, smooth_inv, act_scale,
+                             Xq, Xs, pieces, K8);
+}
+
+template <int GM>
+int launch_rownorm_warp(const RowQuantParams& p, int M, cudaStream_t stream) {
+    const unsigned blocks = (M + 3) / 4;
+    if (p.K <= 2560) return launch_row_kernel("rownorm_warp", rownorm_warp_kernel<GM, 10>, blocks, 128, 0, stream, p, M);
+    return launch_row_kernel("rownorm_warp", rownorm_warp_kernel<GM, 16>, blocks, 128, 0, stream, p, M);
 }
 
 }  // namespace
@@ -491,15 +632,15 @@ int launch_rowquant(const __half* x_in, __half* x_out, const __half* residual,
                     const __half* act_scale, int M, int K, int g, int act_mode, __half* normed_out,
                     int8_t* Xq, float* Xs, cudaStream_t stream) {
     if (M == 0) return W8A8_OK;
-    {   // the quantiser alone, common group sizes: the barrier-free kernel
+    {   // the quantiser alone, common group sizes: the barrier-free kernel (pieces are counted in 32 bits)
         const int gn = norm_group(K, g);
         if (!residual && !norm_weight && !normed_out && Xq && act_mode == W8A8_ACT_PER_TOKEN_GROUP &&
-            (gn == 64 || gn == 128 || gn == 256) && K % gn == 0 && M <= 65535 && aligned16(x_in) &&
+            (gn == 64 || gn == 128 || gn == 256) && K % gn == 0 && static_cast<long long>(M) * K / 8 < (1ll << 31) && aligned16(x_in) &&
             (reinterpret_cast<uintptr_t>(Xq) & 7u) == 0 && (!smooth_inv || aligned16(smooth_inv))) {
-            const int G = K / gn;
-            if (gn == 64) return launch_groupquant<8>(x_in, smooth_inv, act_scale, Xq, Xs, M, K, G, stream);
-            if (gn == 128) return launch_groupquant<16>(x_in, smooth_inv, act_scale, Xq, Xs, M, K, G, stream);
-            return launch_groupquant<32>(x_in, smooth_inv, act_scale, Xq, Xs, M, K, G, stream);
+            const unsigned pieces = static_cast<unsigned>(static_cast<long long>(M) * K / 8), K8 = static_cast<unsigned>(K / 8);
+            if (gn == 64) return launch_groupquant<8>(x_in, smooth_inv, act_scale, Xq, Xs, pieces, K8, stream);
+            if (gn == 128) return launch_groupquant<16>(x_in, smooth_inv, act_scale, Xq, Xs, pieces, K8, stream);
+            return launch_groupquant<32>(x_in, smooth_inv, act_scale, Xq, Xs, pieces, K8, stream);
         }
     }
     RowQuantParams p;
@@ -533,38 +674,22 @@ int launch_rowquant(const __half* x_in, __half* x_out, const __half* residual,
         const char* v = std::getenv("W8A8_ROW_COMPACT");
         return v ? (*v && *v != '0') : true;
     }();
-    if (compact_ok && norm_weight && threads >= 256 && K % 256 == 0 && K <= 4096 && !smooth_inv && !act_scale && !p.per_token &&
-        (p.g == 64 || p.g == 128 || p.g == 256) && p.vec_ok && aligned16(norm_weight) &&
+    // (without codes to make, the group size does not matter)
+    const int gm = Xq ? p.g : 256;
+    if (compact_ok && norm_weight && threads >= 256 && K % 256 == 0 && K <= 4096 && !smooth_inv && !act_scale && (!p.per_token || !Xq) &&
+        (gm == 64 || gm == 128 || gm == 256) && p.vec_ok && aligned16(norm_weight) &&
         (!normed_out || aligned16(normed_out)) && (!Xq || (reinterpret_cast<uintptr_t>(Xq) & 7u) == 0)) {
-        cudaLaunchConfig_t cfg = {};
-        cfg.gridDim = dim3(M, 1, 1);
-        cfg.blockDim = dim3(256, 1, 1);
-        cfg.stream = stream;
-        cudaLaunchAttribute attr[1];
-        attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-        attr[0].val.programmaticStreamSerializationAllowed = 1;
-        cfg.attrs = attr;
-        cfg.numAttrs = pdl_enabled(kPdlRow) ? 1 : 0;
-        cudaError_t e = p.g == 64    ? cudaLaunchKernelEx(&cfg, rowquant_compact_kernel<64>, p, threads)
-                        : p.g == 128 ? cudaLaunchKernelEx(&cfg, rowquant_compact_kernel<128>, p, threads)
-                                     : cudaLaunchKernelEx(&cfg, rowquant_compact_kernel<256>, p, threads);
-        if (e != cudaSuccess) return fail(W8A8_ERR_CUDA, "rowquant_compact launch: %s", cudaGetErrorString(e));
-        return W8A8_OK;
+        // A CTA per row has the shorter chain, a warp per row more bytes in flight: the line is where the CTAs no longer all
+        // fit the chip at once (eight per SM). At 150 rows a warp per row leaves three SMs of four idle: 8 us against 5.
+        if (threads == 1024 && M > 148 * 8)
+            return gm == 64 ? launch_rownorm_warp<64>(p, M, stream) : gm == 128 ? launch_rownorm_warp<128>(p, M, stream)
+                                                                                : launch_rownorm_warp<256>(p, M, stream);
+        return launch_row_kernel("rowquant_compact", gm == 64    ? rowquant_compact_kernel<64>
+                                                     : gm == 128 ? rowquant_compact_kernel<128>
+                                                                 : rowquant_compact_kernel<256>, M, 256, 0, stream, p, threads);
     }
-    if (norm_weight && threads >= 32 && K <= kFastElems * threads && p.g % 32 == 0 && p.G <= 160) {
-        cudaLaunchConfig_t cfg = {};
-        cfg.gridDim = dim3(M, 1, 1);
-        cfg.blockDim = dim3(threads, 1, 1);
-        cfg.stream = stream;
-        cudaLaunchAttribute attr[1];
-        attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-        attr[0].val.programmaticStreamSerializationAllowed = 1;
-        cfg.attrs = attr;
-        cfg.numAttrs = pdl_enabled(kPdlRow) ? 1 : 0;
-        cudaError_t e = cudaLaunchKernelEx(&cfg, rowquant_fast_kernel, p);
-        if (e != cudaSuccess) return fail(W8A8_ERR_CUDA, "rowquant_fast launch: %s", cudaGetErrorString(e));
-        return W8A8_OK;
-    }
+    if (norm_weight && threads >= 32 && K <= kFastElems * threads && p.g % 32 == 0 && p.G <= 160)
+        return launch_row_kernel("rowquant_fast", rowquant_fast_kernel, M, threads, 0, stream, p);
     size_t smem = ((static_cast<size_t>(K) * 2 + 15) & ~size_t(15)) + static_cast<size_t>(p.G) * 4;
     if (smem > 200 * 1024) return fail(W8A8_ERR_UNSUPPORTED, "row of K=%d does not fit shared memory", K);
     if (smem > 48 * 1024) {
@@ -572,19 +697,7 @@ int launch_rowquant(const __half* x_in, __half* x_out, const __half* residual,
                                              static_cast<int>(smem));
         if (e != cudaSuccess) return fail(W8A8_ERR_CUDA, "cudaFuncSetAttribute: %s", cudaGetErrorString(e));
     }
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(M, 1, 1);
-    cfg.blockDim = dim3(threads, 1, 1);
-    cfg.dynamicSmemBytes = smem;
-    cfg.stream = stream;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = pdl_enabled(kPdlRow) ? 1 : 0;
-    cudaError_t e = cudaLaunchKernelEx(&cfg, rowquant_kernel, p);
-    if (e != cudaSuccess) return fail(W8A8_ERR_CUDA, "rowquant launch: %s", cudaGetErrorString(e));
-    return W8A8_OK;
+    return launch_row_kernel("rowquant", rowquant_kernel, M, threads, smem, stream, p);
 }
 
 }  // namespace w8a8

@@ -220,6 +220,49 @@ def test_elementwise(ctx, oracle, n):
         assert torch.equal(ra, dr)
 
 
+@pytest.mark.parametrize("M,K,g", [(1185, 768, 256), (1186, 2560, 64), (1187, 2816, 128), (1200, 4096, 256), (1185, 4096, 64)])
+@pytest.mark.parametrize("with_residual", [False, True])
+def test_rmsnorm_quantize_many_rows(ctx, oracle, M, K, g, with_residual):
+    """More rows than eight per SM: the warp-per-row form (its shortest row, the last row count that fills a CTA of four and the ones
+    that do not, the widths at which its register rows end). The sum of squares follows the reference's order; the device's
+    rsqrtf may move a normed value by one fp16 ulp against the oracle's, and codes are compared on the device's own norm."""
+    rng = np.random.default_rng(M + K)
+    x = synth.activations(rng, M, K)
+    w = rng.uniform(0.8, 1.2, K).astype(np.float16)
+    r = rng.standard_normal((M, K)).astype(np.float16) if with_residual else None
+    dx, dn = dev(x), torch.empty((M, K), dtype=torch.float16, device="cuda")
+    dq = torch.empty((M, K), dtype=torch.int8, device="cuda")
+    ds = torch.empty((M, K // g), dtype=torch.float32, device="cuda")
+    ctx.rmsnorm_quantize(dx, dev(w), 1e-6, M, K, g, dq, ds, residual=dev(r) if with_residual else None, normed_out=dn)
+    torch.cuda.synchronize()
+    want_x = oracle.residual_add(x, r) if with_residual else x
+    assert np.array_equal(dx.cpu().numpy(), want_x)
+    normed = dn.cpu().numpy()
+    assert oracle.ulp_distance_fp16(normed, oracle.rms_norm(want_x, w, 1e-6)).max() <= 1
+    wq, wsc = oracle.quantize(normed, g)
+    assert np.array_equal(dq.cpu().numpy(), wq) and np.array_equal(ds.cpu().numpy(), wsc)
+    alone = torch.empty_like(dn)
+    ctx.rms_norm(dev(want_x), dev(w), alone, M, K, 1e-6)
+    torch.cuda.synchronize()
+    assert torch.equal(alone, dn)
+
+
+@pytest.mark.parametrize("M,K,g", [(613, 9728, 64), (1901, 2560, 256), (947, 5120, 128)])
+@pytest.mark.parametrize("mode", ["dynamic", "smooth", "static"])
+def test_quantize_flat_form(ctx, oracle, M, K, g, mode):
+    """Enough activations for the four-pieces-per-thread form of the quantiser, the last block partly filled."""
+    rng = np.random.default_rng(M)
+    X = synth.activations(rng, M, K)
+    smooth = rng.uniform(0.5, 2.0, K).astype(np.float16) if mode != "dynamic" else None
+    act = rng.uniform(5e-3, 2e-2, K // g).astype(np.float16) if mode == "static" else None
+    wq, wsc = oracle.quantize(X, g, smooth_inv=smooth, act_scale=act)
+    dq = torch.empty((M, K), dtype=torch.int8, device="cuda")
+    ds = torch.empty((M, K // g), dtype=torch.float32, device="cuda")
+    ctx.quantize(dev(X), M, K, g, dq, ds, smooth_inv=None if smooth is None else dev(smooth), act_scale=None if act is None else dev(act))
+    torch.cuda.synchronize()
+    assert np.array_equal(dq.cpu().numpy(), wq) and np.array_equal(ds.cpu().numpy(), wsc)
+
+
 # ---------------------------------------------------------------- linear (A3-A8)
 def run_linear(ctx, oracle, M, N, K, g, seed=0, fused_quant=True, **kw):
     X, W, ws = synth.linear_case(seed, M, N, K, g)
