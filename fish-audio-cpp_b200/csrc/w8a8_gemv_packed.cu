@@ -21,10 +21,11 @@
 // shared loads, and finds the scales in the same stage — no strided access, no separate scale
 // traffic, no tensor map. Rows past N are stored as zeros, so no tail handling is needed on loads.
 // A row tile cut by a run boundary is always cut between warps of one CTA: its fp32 partial tiles meet in
-// shared memory and the warp that arrives last adds them in ascending-K order. (An earlier form cut one
-// global range over all warps of the grid and fixed cut tiles up through global scratch and L2 atomics:
-// perfectly balanced, but two to three L2 round trips at the tail of every launch; measured 2 us slower
-// per launch on the decode shapes than the at most one-tile imbalance of this form.)
+// shared memory, and once the CTA has streamed its blocks all its threads add them up in ascending-K order. (One
+// warp, the last to arrive, used to do that, with two divisions per contributor: 2300 clocks of a 6400-clock launch
+// of 2560 x 4096. An earlier form still cut one global range over all warps of the grid and fixed cut tiles up
+// through global scratch and L2 atomics: perfectly balanced, but two to three L2 round trips at the tail of every
+// launch; measured 2 us slower per launch on the decode shapes than the at most one-tile imbalance of this form.)
 //
 // Launched with programmatic dependent launch: the first kStages blocks are requested before
 // griddepcontrol.wait. Every mbarrier wait is bounded; on expiry the warp records an error word.
@@ -41,10 +42,13 @@ constexpr int kWarps = 8;
 constexpr int kThreads = kWarps * 32;
 constexpr int kBlockW = 16 * 256;        // weight bytes of a block
 constexpr int kStagePitch = kBlockW + 128;  // room for the largest scale tail, keeps stages 128-byte aligned
-constexpr int kLocalTiles = 128;  // row tiles per CTA whose arrival counters live in shared memory
 // How the activations arrive (template parameter PRO):
 enum { kProCodes = 0,   // int8 codes + fp32 scales made by an earlier launch (Xq, Xs)
        kProNorm = 1 };  // fp16 rows: every CTA does [x + residual] -> RMSNorm -> quantiser itself, in its prologue
+
+// Forms of the kernel, by 8-token B tiles and group size class (reasons: see the consumer loop).
+constexpr bool in_place(int mt, int gm) { return mt == 4 || (mt == 2 && gm != 64); }
+constexpr bool two_per_sm(int mt, int gm) { return mt == 1 || (mt == 2 && gm != 64); }
 
 struct GemvPackedParams {
     LinearArgs a;
@@ -87,12 +91,6 @@ __device__ __forceinline__ uint32_t lds16(uint32_t addr) {
 __device__ __forceinline__ uint4 ld_cg16(const __half* p) {
     uint4 v;
     asm volatile("ld.global.cg.v4.u32 {%0,%1,%2,%3}, [%4];\n" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p));
-    return v;
-}
-
-__device__ __forceinline__ float ld_cg(const float* p) {
-    float v;
-    asm volatile("ld.global.cg.f32 %0, [%1];\n" : "=f"(v) : "l"(p));
     return v;
 }
 
@@ -327,8 +325,10 @@ __device__ __forceinline__ void tail_group_quant(const LinearArgs& a, int ct0, i
 // the GPU idle, and the trip of its results through L2.
 // ST: stages of a warp's ring (3; 2 for kProNorm so that two CTAs fit an SM beside the code rows).
 // KI: kProNorm only, the 16-byte pieces of a row a lane holds (K <= 256 * KI): 10 for the stack's K = 2560, else 16.
-template <int MT, int GM, int PRO, int ST, int KI>
-__global__ void __launch_bounds__(kThreads, (PRO == kProNorm || MT == 1) ? 2 : 1)
+// EXTRA: the call wants the group sums dumped or has a tail. An instance of its own: the check per promote alone cost 0.1-1.1 us
+// per launch.
+template <int MT, int GM, int PRO, int ST, int KI, bool EXTRA>
+__global__ void __launch_bounds__(kThreads, two_per_sm(MT, GM) ? 2 : 1)
 gemv_packed_kernel(const GemvPackedParams p) {
     constexpr bool FUSED = PRO == kProNorm;
     constexpr int kStages = ST;
@@ -347,10 +347,9 @@ gemv_packed_kernel(const GemvPackedParams p) {
 
     // ---- this warp's contiguous range of units; the eight ranges of a CTA are neighbours, so that most row
     // tiles cut by a range boundary are cut between warps of ONE CTA and can be added up in shared memory ----
-    __shared__ float red_s[kWarps][2][MT * 4 * 32];
-    __shared__ int cnt_s[kLocalTiles];
-    for (int i = threadIdx.x; i < kLocalTiles; i += kThreads) cnt_s[i] = 0;
-    __syncthreads();
+    __shared__ float red_s[kWarps][MT * 4 * 32];  // a warp's part of the tile its run begins in (slot 0)
+    __shared__ int cut_s[kWarps][3];  // per boundary between two warps' runs: the row tile it cuts (-1: none, or counted with
+                                      // the boundary before it), the slot of its first contributor, its last contributor
     // Whole 16-row tiles per CTA (tile t of `tiles` goes to CTA t * C / tiles), the CTA's units in equal contiguous
     // runs to its warps (none with an empty run): a tile cut by a run boundary is always cut between warps of
     // this CTA.
@@ -364,6 +363,25 @@ gemv_packed_kernel(const GemvPackedParams p) {
         u1 = cu0 + (warp + 1) * n_cta / nw_cta;
     }
     const int T = static_cast<int>(u1 - u0) * p.bpu;  // blocks
+    // The row tiles cut by run boundaries, worked out while nothing is waited for: a division costs a lone warp some forty
+    // clocks, and this used to sit between a tile's last block and its store.
+    if (threadIdx.x < kWarps) {
+        const int w = threadIdx.x;
+        auto start = [&](int i) { return cu0 + i * n_cta / nw_cta; };
+        int tile = -1, slot = 0, last = 0;
+        if (w + 1 < static_cast<int>(nw_cta)) {
+            const unsigned b = start(w + 1), t = b / p.upt;
+            if (b != t * p.upt && (w == 0 || start(w) <= t * p.upt)) {  // inside tile t, and no boundary before it is
+                tile = static_cast<int>(t);
+                slot = start(w) / p.upt == t ? 0 : 1;
+                last = w + 1;
+                while (last + 1 < static_cast<int>(nw_cta) && start(last + 1) < (t + 1) * p.upt) ++last;
+            }
+        }
+        cut_s[w][0] = tile;
+        cut_s[w][1] = slot;
+        cut_s[w][2] = last;
+    }
 
     const uint32_t ring = ((ptx::smem_u32(smem_raw) + 127u) & ~127u) + warp * kRingBytes;
     uint64_t* bar = bars[warp];
@@ -626,50 +644,23 @@ gemv_packed_kernel(const GemvPackedParams p) {
         }
     };
 
-    auto warp_of_unit = [&](unsigned u) -> unsigned {  // the warp of this CTA whose run holds unit u
-        return ((u - cu0 + 1) * nw_cta - 1) / n_cta;
-    };
-    const int cta_rt0 = static_cast<int>(ct0);
-
-    // Called when the warp has added its last unit of row tile rt into acc. A cut tile: the fp32 partial goes to
-    // the warp's slot in shared memory, the arrival is counted, and whichever warp arrives last adds the
-    // partials in ascending-K order and stores. Nothing waits; nothing leaves the SM.
+    // Slot 1, a warp's part of the tile its run ends in, lies in the warp's own ring: it is written after the run's last block.
+    static_assert(MT * 4 * 32 * sizeof(float) <= kRingBytes, "a partial tile fits a warp's ring");
+    float* const ring0 = reinterpret_cast<float*>(smem_raw + (ring - warp * kRingBytes - ptx::smem_u32(smem_raw)));
+    auto slot1 = [&](int w) { return ring0 + w * (kRingBytes / 4); };
+    // Called when the warp has added its last unit of row tile rt into acc. A tile that lies inside the warp's run is stored;
+    // of a cut tile the fp32 partial goes to the warp's slot in shared memory (0: the tile its run begins in, 1: the tile it
+    // ends in) and is added up when the whole CTA has streamed its blocks (below).
     auto finish_tile = [&](int rt) {
         const unsigned t_lo = static_cast<unsigned>(rt) * p.upt, t_hi = t_lo + p.upt;  // [t_lo, t_hi)
         if ((u0 <= t_lo && t_hi <= u1) || W8A8_ABLATED(8)) {
             store_tile(rt, acc);
         } else {
-            const unsigned first = warp_of_unit(t_lo), last = warp_of_unit(t_hi - 1);
-            const int my_slot = (static_cast<int>(u0 / p.upt) == rt) ? 0 : 1;
-            float* mine = red_s[warp][my_slot];
+            float* mine = u0 < t_hi && u0 >= t_lo ? red_s[warp] : slot1(warp);
 #pragma unroll
             for (int nt = 0; nt < MT; ++nt)
 #pragma unroll
                 for (int r = 0; r < 4; ++r) mine[(nt * 4 + r) * 32 + lane] = acc[nt][r];
-            __syncwarp();
-            int old = 0;
-            if (lane == 0) {
-                __threadfence_block();
-                old = atomicAdd(&cnt_s[rt - cta_rt0], 1);
-            }
-            old = __shfl_sync(0xffffffffu, old, 0);
-            if (old == static_cast<int>(last - first)) {
-                __threadfence_block();
-                float sum[MT][4];
-#pragma unroll
-                for (int nt = 0; nt < MT; ++nt)
-#pragma unroll
-                    for (int r = 0; r < 4; ++r) sum[nt][r] = 0.0f;
-                for (unsigned ww = first; ww <= last; ++ww) {
-                    const unsigned wu0 = cu0 + ww * n_cta / nw_cta;
-                    const float* src = red_s[ww][(static_cast<int>(wu0 / p.upt) == rt) ? 0 : 1];
-#pragma unroll
-                    for (int nt = 0; nt < MT; ++nt)
-#pragma unroll
-                        for (int r = 0; r < 4; ++r) sum[nt][r] += src[(nt * 4 + r) * 32 + lane];
-                }
-                store_tile(rt, sum);
-            }
         }
 #pragma unroll
         for (int nt = 0; nt < MT; ++nt)
@@ -684,7 +675,7 @@ gemv_packed_kernel(const GemvPackedParams p) {
             const float x0 = xsv[nt][0], x1 = xsv[nt][1];
 #pragma unroll
             for (int r = 0; r < 4; ++r) { P[nt][r] += Q[nt][r]; Q[nt][r] = 0; }
-            if (a.dump) {
+            if (EXTRA && a.dump) {
                 const int t0 = nt * 8 + 2 * c, rA = rt * 16 + gq;
                 const size_t NG = static_cast<size_t>(a.N) * a.G;
 #pragma unroll
@@ -703,52 +694,55 @@ gemv_packed_kernel(const GemvPackedParams p) {
 
     // ---- consumer loop: one packed block (16 rows x 256 bytes of K, plus its scales) per step ----
     // Activation codes and scales are a few KB shared by the whole grid, but each warp touches a
-    // given piece only once, so these reads mostly miss L1 and cost an L2 round trip. They are
-    // requested one block ahead (registers xn / xsn) and never sit on the critical path.
+    // given piece only once, so these reads mostly miss L1 and cost an L2 round trip. They are requested a block
+    // ahead, into a second set of registers; or (kInPlace) the registers of a 64-byte chunk are refilled as soon as
+    // its MMAs have been issued, a little later but in half the registers: for M > 16, and for M = 9..16 where it lets
+    // two CTAs share an SM (w2 at M = 16, g = 256: 11.3 -> 9.4 us; at g = 64 the second CTA gains less than the
+    // later request costs; at M <= 8 two CTAs fit either way, and a run is often just two blocks long).
     int si = 0;
     int ub = static_cast<int>(u0 % p.upt), rt = static_cast<int>(u0 / p.upt);
     bool ok = true;
-    uint4 xc[4][MT], xn[4][MT];
-    float xsc[GPU][MT][2], xsn[GPU][MT][2];
-    auto load_x = [&](int kbase, uint4 (&dst)[4][MT]) {
+    constexpr bool kInPlace = in_place(MT, GM) && !FUSED;
+    constexpr int NX = kInPlace ? 1 : 2;
+    uint4 x[NX][4][MT];
+    float xs[NX][GPU][MT][2];
+    auto load_x = [&](int kbase, int ch, int buf) {
 #pragma unroll
-        for (int ch = 0; ch < 4; ++ch)
-#pragma unroll
-            for (int nt = 0; nt < MT; ++nt) {
-                if constexpr (FUSED) dst[ch][nt] = lds128(xq_s + kbase + ch * 64);
-                else if (W8A8_ABLATED(1)) dst[ch][nt] = make_uint4(0x01010101u, 0x01010101u, 0x01010101u, 0x01010101u);
-                else dst[ch][nt] = __ldg(reinterpret_cast<const uint4*>(xq[nt] + kbase + ch * 64));
-            }
+        for (int nt = 0; nt < MT; ++nt) {
+            if constexpr (FUSED) x[buf][ch][nt] = lds128(xq_s + kbase + ch * 64);
+            else if (W8A8_ABLATED(1)) x[buf][ch][nt] = make_uint4(0x01010101u, 0x01010101u, 0x01010101u, 0x01010101u);
+            else x[buf][ch][nt] = __ldg(reinterpret_cast<const uint4*>(xq[nt] + kbase + ch * 64));
+        }
     };
-    auto load_xs = [&](int unit_b, float (&dst)[GPU][MT][2]) {
+    auto load_xs = [&](int unit_b, int q, int buf) {
 #pragma unroll
-        for (int q = 0; q < GPU; ++q)
+        for (int nt = 0; nt < MT; ++nt)
 #pragma unroll
-            for (int nt = 0; nt < MT; ++nt) {
-                if constexpr (FUSED) {
-                    dst[q][nt][0] = xsp_s[0][unit_b * GPU + q];
-                    dst[q][nt][1] = xsp_s[1][unit_b * GPU + q];
-                } else if (W8A8_ABLATED(2)) {
-                    dst[q][nt][0] = 1.0f;
-                    dst[q][nt][1] = 1.0f;
-                } else {
-                    dst[q][nt][0] = __ldg(xsp[nt][0] + unit_b * GPU + q);
-                    dst[q][nt][1] = __ldg(xsp[nt][1] + unit_b * GPU + q);
-                }
+            for (int e = 0; e < 2; ++e) {
+                if constexpr (FUSED) xs[buf][q][nt][e] = xsp_s[e][unit_b * GPU + q];
+                else if (W8A8_ABLATED(2)) xs[buf][q][nt][e] = 1.0f;
+                else xs[buf][q][nt][e] = __ldg(xsp[nt][e] + unit_b * GPU + q);
             }
     };
     if (T > 0) {
-        load_x(ub * p.bpu * 256, xc);
-        load_xs(ub, xsc);
+#pragma unroll
+        for (int ch = 0; ch < 4; ++ch) load_x(ub * p.bpu * 256, ch, 0);
+#pragma unroll
+        for (int q = 0; q < GPU; ++q) load_xs(ub, q, 0);
     }
     for (int t = 0; t < T; ++t) {
         const int slot = t % kStages;
         // position of the next block (the same row tile or the next one: K restarts at 0)
         int nsi = si + 1, nub = ub;
         if (nsi == p.bpu) { nsi = 0; if (++nub == p.upt) nub = 0; }
-        if (t + 1 < T) {
-            load_x((nub * p.bpu + nsi) * 256, xn);
-            if (nsi == 0) load_xs(nub, xsn);
+        const int nkb = (nub * p.bpu + nsi) * 256;
+        if (!kInPlace && t + 1 < T) {
+#pragma unroll
+            for (int ch = 0; ch < 4; ++ch) load_x(nkb, ch, NX - 1);
+            if (nsi == 0) {
+#pragma unroll
+                for (int q = 0; q < GPU; ++q) load_xs(nub, q, NX - 1);
+            }
         }
         if (!ptx::mbar_wait_bounded(&bar[slot], (t / kStages) & 1)) {
             if (lane == 0) atomicExch(p.status, 600 + slot);
@@ -769,39 +763,56 @@ gemv_packed_kernel(const GemvPackedParams p) {
             const uint4 wa = lds128(fa), wb = lds128(fa + 512);
 #pragma unroll
             for (int nt = 0; nt < MT; ++nt) {
-                mma_s8(P[nt], wa.x, wb.x, wa.y, wb.y, xc[ch][nt].x, xc[ch][nt].y);
-                mma_s8(Q[nt], wa.z, wb.z, wa.w, wb.w, xc[ch][nt].z, xc[ch][nt].w);
+                mma_s8(P[nt], wa.x, wb.x, wa.y, wb.y, x[0][ch][nt].x, x[0][ch][nt].y);
+                mma_s8(Q[nt], wa.z, wb.z, wa.w, wb.w, x[0][ch][nt].z, x[0][ch][nt].w);
             }
-            if (GM == 64) promote(rt, ub * 4 + ch, sa[ch % GPU], sb[ch % GPU], xsc[ch % GPU]);
-            if (GM == 128 && (ch & 1))
-                promote(rt, ub * 2 + (ch >> 1), sa[(ch >> 1) % GPU], sb[(ch >> 1) % GPU], xsc[(ch >> 1) % GPU]);
+            if (kInPlace) load_x(nkb, ch, 0);  // (after the range's last block: a block of the same rows, read for nothing)
+            if (GM == 64) {
+                promote(rt, ub * 4 + ch, sa[ch % GPU], sb[ch % GPU], xs[0][ch % GPU]);
+                if (kInPlace) load_xs(nub, ch % GPU, 0);
+            }
+            if (GM == 128 && (ch & 1)) {
+                promote(rt, ub * 2 + (ch >> 1), sa[(ch >> 1) % GPU], sb[(ch >> 1) % GPU], xs[0][(ch >> 1) % GPU]);
+                if (kInPlace) load_xs(nub, (ch >> 1) % GPU, 0);
+            }
         }
         // The block's bytes are in registers: the slot may be refilled.
         __syncwarp();
-        // (No proxy fence: the shared-memory reads above have returned their data — the MMAs consumed it —
-        // before the copy that overwrites the slot is even issued.)
-        if (lane == 0 && pt < T) issue();
+        // The fence orders the reads of the slot before the copy that overwrites it. Without it the compiler may sink the
+        // scales' loads down to their use in the promote, past the copy: it did in the M = 9..16 form (128 registers), and
+        // a group's promote then took the next block's scales now and then.
+        if (lane == 0 && pt < T) {
+            ptx::fence_proxy_async();
+            issue();
+        }
 #ifdef W8A8_TAIL_TIMELINE
         if (t == 0) W8A8_STAMP(6);
 #endif
         if (++si == p.bpu) {
             si = 0;
-            if (GM == 256) promote(rt, ub, sa[0], sb[0], xsc[0]);
+            if (GM == 256) {
+                promote(rt, ub, sa[0], sb[0], xs[0][0]);
+                if (kInPlace) load_xs(nub, 0, 0);
+            }
             // one call site for the tile end: the row tile is complete, or the range ends inside it
             ++ub;
             if (ub == p.upt || t + 1 == T) {
                 finish_tile(rt);
                 if (ub == p.upt) { ub = 0; ++rt; }
             }
+            if (!kInPlace) {
 #pragma unroll
-            for (int q = 0; q < GPU; ++q)
+                for (int q = 0; q < GPU; ++q)
 #pragma unroll
-                for (int nt = 0; nt < MT; ++nt) { xsc[q][nt][0] = xsn[q][nt][0]; xsc[q][nt][1] = xsn[q][nt][1]; }
+                    for (int nt = 0; nt < MT; ++nt) { xs[0][q][nt][0] = xs[NX - 1][q][nt][0]; xs[0][q][nt][1] = xs[NX - 1][q][nt][1]; }
+            }
         }
+        if (!kInPlace) {
 #pragma unroll
-        for (int ch = 0; ch < 4; ++ch)
+            for (int ch = 0; ch < 4; ++ch)
 #pragma unroll
-            for (int nt = 0; nt < MT; ++nt) xc[ch][nt] = xn[ch][nt];
+                for (int nt = 0; nt < MT; ++nt) x[0][ch][nt] = x[NX - 1][ch][nt];
+        }
     }
     if (!ok) {
         // Leave only once every requested block has landed (or a second bounded wait ran out): a TMA write
@@ -810,13 +821,53 @@ gemv_packed_kernel(const GemvPackedParams p) {
         for (int s = 0; s < kStages; ++s)
             if (pt > s) ptx::mbar_wait_bounded(&bar[s], ((pt - 1 - s) / kStages) & 1, 1u << 16);
     }
+    // ---- cut tiles: all warps add the partials up, in ascending-K order, a token's pair of rows per item ----
+    __syncthreads();
+#pragma unroll 1
+    for (int i = threadIdx.x; i < (kWarps - 1) * MT * 64; i += kThreads) {
+        const int w = i / (MT * 64), rt_cut = cut_s[w][0];
+        if (rt_cut < 0) continue;
+        const int f = i % (MT * 64), nt = f >> 6, e = (f >> 5) & 1, fl = f & 31, last = cut_s[w][2];
+        const float* src = (cut_s[w][1] ? slot1(w) : red_s[w]) + (nt * 4 + e) * 32 + fl;
+        float v[2] = {0.0f + src[0], 0.0f + src[64]};
+        for (int ww = w + 1; ww <= last; ++ww) {
+            const float* more = red_s[ww] + (nt * 4 + e) * 32 + fl;
+            v[0] += more[0];
+            v[1] += more[64];
+        }
+        const int tok = nt * 8 + 2 * (fl & 3) + e, rA = rt_cut * 16 + (fl >> 2);
+        if (tok >= a.M) continue;
+        if (a.epilogue == W8A8_EPI_SWIGLU) {
+            if (rA + 8 < a.N) {
+                const float g16 = __half2float(__float2half(v[0]));
+                const __half s16 = __float2half(g16 / (1.0f + expf(-g16)));
+                const float u16 = __half2float(__float2half(v[1]));
+                a.Y[static_cast<size_t>(tok) * (a.N / 2) + rt_cut * 8 + (fl >> 2)] = __float2half(__half2float(s16) * u16);
+            }
+            continue;
+        }
+#pragma unroll 1
+        for (int row = rA; row <= rA + 8 && row < a.N; row += 8) {
+            const size_t o = static_cast<size_t>(tok) * a.N + row;
+            const float val = row == rA ? v[0] : v[1];
+            if (a.tp.world > 0) {
+                const size_t word = (static_cast<size_t>((tp_ep & 1) * a.tp.world + a.tp.rank) * a.tp.max_tokens + tok) * a.N + row;
+                const uint2 wd = make_uint2(__float_as_uint(val), static_cast<unsigned>(tp_ep));
+                for (int r = 0; r < a.tp.world; ++r) reinterpret_cast<uint2*>(a.tp.peers[r])[word] = wd;
+            }
+            if (!a.Y || W8A8_ABLATED(4)) continue;
+            __half y = __float2half(val);
+            if (a.epilogue == W8A8_EPI_RESIDUAL) y = __float2half(__half2float(y) + __half2float(a.residual[o]));
+            a.Y[o] = y;
+        }
+    }
 #ifdef W8A8_TAIL_TIMELINE
     if (a.tail_kind == kTailNone && a.tail_counters) {
         W8A8_STAMP(7);
         W8A8_STAMP_FLUSH(a.tail_counters, blockIdx.x == gridDim.x - 1);
     }
 #endif
-    if constexpr (PRO == kProCodes && MT == 1) {
+    if constexpr (EXTRA && PRO == kProCodes && MT == 1) {
         if (a.tail_kind != kTailNone) {
             // every copy this CTA asked for has been consumed: the rings are free to serve as the tail's scratch
             W8A8_STAMP(7);  // this thread's own warp is done
@@ -920,14 +971,13 @@ bool make_plan(const LinearArgs& a, Plan& pl) {
     pl.block_bytes = kBlockW + 32 * (a.g >= 256 ? 1 : 256 / a.g);
     pl.tiles = (a.N + 15) / 16;
     pl.U = static_cast<long long>(pl.tiles) * pl.upt;
-    // Up to two CTAs per SM at M <= 8 (their registers and shared memory fit twice), never more CTAs than row tiles.
-    pl.ctas = gemv_packed_ctas(pl.tiles, num_sms(), pl.MT == 1);
+    // Up to two CTAs per SM where their registers and shared memory fit twice, never more CTAs than row tiles.
+    pl.ctas = gemv_packed_ctas(pl.tiles, num_sms(), two_per_sm(pl.MT, pl.GM));
     if ((pl.U + 1) * static_cast<long long>(pl.ctas) * kWarps >= (1ll << 32)) return false;  // 32-bit range math
-    if (pl.tiles / pl.ctas + 2 > kLocalTiles) return false;  // arrival counters of a CTA's tiles sit in shared memory
     return true;
 }
 
-template <int MT, int GM, int PRO, int ST, int KI>
+template <int MT, int GM, int PRO, int ST, int KI, bool EXTRA>
 int launch_variant(const LinearArgs& a, const Plan& pl, int* status, cudaStream_t stream) {
     GemvPackedParams p;
     p.a = a;
@@ -943,7 +993,7 @@ int launch_variant(const LinearArgs& a, const Plan& pl, int* status, cudaStream_
         p.ablate = v ? std::atoi(v) : 0;
     }
 #endif
-    auto kern = gemv_packed_kernel<MT, GM, PRO, ST, KI>;
+    auto kern = gemv_packed_kernel<MT, GM, PRO, ST, KI, EXTRA>;
     const size_t ring = static_cast<size_t>(kWarps) * ST * kStagePitch + 128;
     const size_t smem = ring + (PRO == kProNorm ? fused_smem_bytes(a.K, a.G) : 0);
     {  // per device, so on every launch (a host-side table write)
@@ -970,11 +1020,12 @@ template <int MT, int GM>
 int launch_pro(const LinearArgs& a, const Plan& pl, int* status, cudaStream_t s) {
     if constexpr (MT == 1) {
         if (pl.pro == kProNorm) {
-            if (a.K <= 2560) return launch_variant<1, GM, kProNorm, 2, 10>(a, pl, status, s);
-            return launch_variant<1, GM, kProNorm, 2, 16>(a, pl, status, s);
+            if (a.K <= 2560) return launch_variant<1, GM, kProNorm, 2, 10, false>(a, pl, status, s);
+            return launch_variant<1, GM, kProNorm, 2, 16, false>(a, pl, status, s);
         }
     }
-    return launch_variant<MT, GM, kProCodes, 3, 1>(a, pl, status, s);
+    if (a.dump || a.tail_kind != kTailNone) return launch_variant<MT, GM, kProCodes, 3, 1, true>(a, pl, status, s);
+    return launch_variant<MT, GM, kProCodes, 3, 1, false>(a, pl, status, s);
 }
 
 template <int MT>

@@ -669,6 +669,44 @@ def test_gemm_tcgen05_tile_widths(ctx, oracle, pkg, monkeypatch, M, N, K, bt, fo
     assert np.array_equal(dY.cpu().numpy().view(np.uint16), oracle.linear_q(W, ws, Xq, Xs, g).view(np.uint16))
 
 
+@pytest.mark.parametrize("g", [64, 128, 256, 512])
+@pytest.mark.parametrize("M", [8, 9, 16, 17, 32])
+def test_packed_linear_many_weights_back_to_back(ctx, oracle, pkg, M, g):
+    """The decode kernel with its stages refilled under load: several weights streamed one launch after another (early
+    launch, cold weights, up to two CTAs per SM), each launch's whole output against the row-major kernel's. A stage that
+    is refilled before its last read, or a partial tile parked where another warp still reads, shows as whole tiles that are
+    off by a group's share. Two kernels may add the groups in another order: at most 4 * 2^-24 of the sum of absolute
+    terms, here bounded by 2^-9 of the row's largest output plus one fp16 rounding each."""
+    N, K, n = 2576, 6144 if g == 512 else 9728, 6
+    gen = torch.Generator(device="cuda").manual_seed(M + g)
+    ws, outs, want = [], [], []
+    for _ in range(n):
+        W = torch.randint(-127, 128, (N, K), dtype=torch.int8, device="cuda", generator=gen)
+        S = torch.empty((N, K // g), device="cuda").uniform_(1e-3, 5e-3, generator=gen).half()
+        P = torch.empty((ctx.packed_weight_bytes(N, K, g),), dtype=torch.uint8, device="cuda")
+        ctx.pack_weight(W, S, N, K, g, P)
+        ws.append((W, S, P))
+        outs.append(torch.empty((M, N), dtype=torch.float16, device="cuda"))
+        want.append(torch.empty((M, N), dtype=torch.float16, device="cuda"))
+    Xq = torch.randint(-127, 128, (M, K), dtype=torch.int8, device="cuda", generator=gen)
+    Xs = torch.empty((M, K // g), device="cuda").uniform_(1e-3, 1e-2, generator=gen)
+    try:
+        for (W, S, P), Y in zip(ws, want):
+            ctx.linear_q(W, S, g, Xq, Xs, Y, M, N, K, kernel=pkg.KERNEL_GEMM_SINGLE)
+            ctx.register_packed_weight(W, P, N, K, g)
+        for _ in range(4):
+            for (W, S, P), Y in zip(ws, outs):
+                ctx.linear_q(W, S, g, Xq, Xs, Y, M, N, K)
+            torch.cuda.synchronize()
+            ctx.check_device_status()
+            for Y, Z in zip(outs, want):
+                diff = (Y.float() - Z.float()).abs()
+                assert bool((diff <= Z.float().abs().amax(1, keepdim=True) * 2.0 ** -9).all()), float(diff.max())
+    finally:
+        for W, S, P in ws:
+            ctx.register_packed_weight(W, None)
+
+
 @pytest.mark.parametrize("split_k", [1, 2, 3, 4, 5, 8])
 def test_gemv_split_k_is_deterministic_and_correct(ctx, oracle, pkg, split_k):
     M, N, K, g = 16, 320, 2560, 256
