@@ -11,13 +11,9 @@
 // Both follow the reference's fp16 rounding points; (1) also follows its summation order, so q, k and
 // the cache contents are bit-identical to the reference chain. (2) sums in a different order than
 // the reference's one-warp-per-head loop and is compared at a tolerance.
-#include <cooperative_groups.h>
-
 #include "sm100_ptx.cuh"
 #include "w8a8_internal.h"
 #include "w8a8_trace.cuh"
-
-namespace cg = cooperative_groups;
 
 namespace w8a8 {
 namespace {
@@ -168,21 +164,40 @@ __device__ __forceinline__ uint32_t kv_chunk(int r, int c16) {
 }
 
 
+// Cosine and sine of the 64 rotation angles, two per lane (pairs lane and lane + 32). They depend on the position alone, so they
+// are made before the dependency wait, and in a rolled loop: sixteen inlined evaluations per head (one per element) were some
+// 700 instructions that a launch runs once, cold.
+struct RopeAngles {
+    float c[2], s[2];
+    __device__ __forceinline__ void make(const float* freqs, int pos, int lane) {
+        const float f[2] = {freqs[lane], freqs[lane + 32]};
+#pragma unroll 1
+        for (int i = 0; i < 2; ++i) {
+            const float angle = (i ? f[1] : f[0]) * static_cast<float>(pos);
+            const float ca = cosf(angle), sa = sinf(angle);
+            if (i) { c[1] = ca; s[1] = sa; } else { c[0] = ca; s[0] = sa; }
+        }
+    }
+};
+
 // One warp, one head of the new token: per-head RMSNorm in the reference's order (rms_norm.cu:23-49 with a
 // 128-thread block) and interleaved-pair RoPE (rope.cu:36-45) — the arithmetic of qknorm_rope_kvwrite_kernel.
-// h: elements lane, 32+lane, 64+lane, 96+lane; w, fr: norm weights and frequencies of the same elements.
+// h: elements lane, 32+lane, 64+lane, 96+lane; w: norm weights of the same elements. (A butterfly leaves in every lane the sum
+// that the reference's shuffle-down tree leaves in lane 0: the same pairs, and addition commutes.)
 __device__ __forceinline__ void head_norm_rope(__half (&h)[4], bool with_norm, const __half (&w)[4], float eps,
-                                               const float (&fr)[4], int pos, int lane) {
+                                               const RopeAngles& rot, int lane) {
     if (with_norm) {
         float part[4];
 #pragma unroll
         for (int v = 0; v < 4; ++v) {
             float val = __half2float(h[v]);
-            float local_sum = 0.0f;
-            local_sum += val * val;
-            for (int offset = 16; offset > 0; offset /= 2) local_sum += __shfl_down_sync(0xffffffffu, local_sum, offset);
-            part[v] = __shfl_sync(0xffffffffu, local_sum, 0);
+            part[v] = 0.0f;
+            part[v] += val * val;
         }
+#pragma unroll
+        for (int offset = 16; offset > 0; offset /= 2)
+#pragma unroll
+            for (int v = 0; v < 4; ++v) part[v] += __shfl_xor_sync(0xffffffffu, part[v], offset);
         float total_sum = (part[0] + part[2]) + (part[1] + part[3]);
         const float rms = rsqrtf(total_sum / kHeadDim + eps);
 #pragma unroll
@@ -192,9 +207,9 @@ __device__ __forceinline__ void head_norm_rope(__half (&h)[4], bool with_norm, c
         }
     }
 #pragma unroll
-    for (int v = 0; v < 4; ++v) {
-        float angle = fr[v] * static_cast<float>(pos);
-        float cos_a = cosf(angle), sin_a = sinf(angle);
+    for (int v = 0; v < 4; ++v) {  // element 32 v + lane belongs to pair 16 v + lane / 2
+        const int from = ((v & 1) << 4) + (lane >> 1);
+        const float cos_a = __shfl_sync(0xffffffffu, rot.c[v >> 1], from), sin_a = __shfl_sync(0xffffffffu, rot.s[v >> 1], from);
         const float mine = __half2float(h[v]);
         const float other = __shfl_xor_sync(0xffffffffu, mine, 1);
         float q0 = (lane & 1) ? other : mine, q1 = (lane & 1) ? mine : other;
@@ -255,8 +270,28 @@ __device__ unsigned long long g_attn_phase[8];
 #define ATTN_PHASE(i) do {} while (0)
 #endif
 
+constexpr int kMaxSlices = 8;
+struct __align__(16) SliceState {
+    float acc[kQPerKv][kHeadDim];
+    float m[kQPerKv], l[kQPerKv];
+};
+// Four-byte and eight-byte stores into the shared memory of the cluster's CTA 0 (at the same offset as `local` here).
+__device__ __forceinline__ uint32_t in_cta0(const void* local) {
+    uint32_t r;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, 0;" : "=r"(r) : "r"(ptx::smem_u32(local)));
+    return r;
+}
+__device__ __forceinline__ void st_cluster(uint32_t addr, float v) {
+    asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(addr), "f"(v) : "memory");
+}
+__device__ __forceinline__ void st_cluster2(uint32_t addr, float a, float b) {
+    asm volatile("st.shared::cluster.v2.f32 [%0], {%1, %2};" ::"r"(addr), "f"(a), "f"(b) : "memory");
+}
+__device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
+__device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
+
 template <bool ROPE>
-__global__ void __maxnreg__(120) paged_attention_decode_kernel(const __grid_constant__ CUtensorMap map_k,
+__global__ void __maxnreg__(128) paged_attention_decode_kernel(const __grid_constant__ CUtensorMap map_k,
                                                                const __grid_constant__ CUtensorMap map_v,
                                                                const AttnParams p) {
     extern __shared__ unsigned char attn_smem[];
@@ -265,9 +300,8 @@ __global__ void __maxnreg__(120) paged_attention_decode_kernel(const __grid_cons
     __shared__ __align__(16) __half kv_new_s[2][kHeadDim];
     __shared__ float red_m[kAttnWarps][kQPerKv], red_l[kAttnWarps][kQPerKv];
     __shared__ float red_acc[kAttnWarps][kQPerKv][kHeadDim];
-    __shared__ float cta_m[kQPerKv], cta_l[kQPerKv];
-    __shared__ __align__(16) float cta_acc[kQPerKv][kHeadDim];
-    __shared__ __align__(16) __half out_s[kQPerKv * kHeadDim];
+    __shared__ SliceState slice_s[kMaxSlices];  // in CTA 0 of the cluster: the partial state of every context slice
+    __shared__ float amax_s[kAttnWarps];
     __shared__ int s_fail;
     W8A8_TRACE_SCOPE();
     ATTN_PHASE(0);
@@ -277,18 +311,19 @@ __global__ void __maxnreg__(120) paged_attention_decode_kernel(const __grid_cons
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int g = lane >> 2, t = lane & 3;
     const uint32_t ring = (ptx::smem_u32(attn_smem) + 1023u) & ~1023u;  // the swizzle pattern repeats every 1024 bytes
-    if (threadIdx.x == 0) {
-        ptx::prefetch_tensormap(&map_k);
-        ptx::prefetch_tensormap(&map_v);
-        for (int i = 0; i < kRing; ++i) {
-            ptx::mbar_init(&full_bar[i], 1);
-            ptx::mbar_init(&empty_bar[i], 1);
+    if (threadIdx.x < kRing) {
+        if (threadIdx.x == 0) {
+            ptx::prefetch_tensormap(&map_k);
+            ptx::prefetch_tensormap(&map_v);
+            s_fail = 0;
         }
-        s_fail = 0;
+        ptx::mbar_init(&full_bar[threadIdx.x], 1);
+        ptx::mbar_init(&empty_bar[threadIdx.x], 1);
         ptx::fence_barrier_init();
         ptx::fence_proxy_async();
     }
     __syncthreads();  // the only whole-CTA barrier: from here on the producer warp runs by itself
+    if (S > 1) cluster_arrive();  // (waited for before anything is written to another CTA: that CTA has started then)
 
     // Read before the dependency wait: these are not results of the launch before this one. The producer asks for the
     // first 32 block numbers without waiting for the sequence length (the read is bounded by the table's width), so
@@ -347,11 +382,10 @@ __global__ void __maxnreg__(120) paged_attention_decode_kernel(const __grid_cons
         // ------------------------------ consumers ------------------------------
         int pos = 0;
         bool owner = false;
-        float fr[4];
+        RopeAngles rot;
         if constexpr (ROPE) {  // parameters first: they do not depend on the launch before this one
             pos = p.positions[b];
-#pragma unroll
-            for (int v = 0; v < 4; ++v) fr[v] = p.freqs[(v * 32 + lane) >> 1];
+            rot.make(p.freqs, pos, lane);
             owner = ((pos / kBlockTokens) % S) == s;  // this CTA attends over the block the new token joins
         }
         ptx::pdl_wait();
@@ -372,7 +406,7 @@ __global__ void __maxnreg__(120) paged_attention_decode_kernel(const __grid_cons
                     hq[v] = src[v * 32 + lane];
                     wq[v] = (norm_w && !is_v) ? norm_w[v * 32 + lane] : __float2half(1.0f);
                 }
-                if (!is_v) head_norm_rope(hq, norm_w != nullptr, wq, p.eps, fr, pos, lane);
+                if (!is_v) head_norm_rope(hq, norm_w != nullptr, wq, p.eps, rot, lane);
                 if (role_q) {
 #pragma unroll
                     for (int v = 0; v < 4; ++v) q_s[h][v * 32 + lane] = hq[v];
@@ -499,71 +533,80 @@ __global__ void __maxnreg__(120) paged_attention_decode_kernel(const __grid_cons
             }
         }
         consumer_barrier();
-        // ---- merge the warps: thread -> (head, 4 dims) ----
-        if (threadIdx.x < kQPerKv * 32) {
-            const int hh = threadIdx.x >> 5, d0 = (threadIdx.x & 31) * 4;
-            float m = -1e30f;
-            for (int w = 0; w < kAttnWarps; ++w) m = fmaxf(m, red_m[w][hh]);
-            float l = 0.0f, a[4] = {0.0f, 0.0f, 0.0f, 0.0f};
-            for (int w = 0; w < kAttnWarps; ++w) {
-                const float scw = __expf(red_m[w][hh] - m);
-                l += red_l[w][hh] * scw;
+    }
+    // ---- merge the warps (thread -> head, 2 dims) and hand the slice's state to CTA 0 of the cluster. Everything is pushed: CTA 0
+    // then reads its own shared memory, and one cluster barrier is enough. (Pulled by CTA 0, every value was a round trip
+    // through the cluster, eight deep at eight slices, and the others had to be kept alive with a second barrier.) ----
+    ATTN_PHASE(5);
+    __syncwarp();
+    if (S > 1) cluster_wait();  // (every thread, the producer warp included: CTA 0 has started)
+    const int hh = (warp & 7) >> 1, d0 = (warp & 1) * 64 + 2 * lane;
+    if (warp < kAttnWarps) {
+        float m = -1e30f;
 #pragma unroll
-                for (int i = 0; i < 4; ++i) a[i] += red_acc[w][hh][d0 + i] * scw;
-            }
+        for (int w = 0; w < kAttnWarps; ++w) m = fmaxf(m, red_m[w][hh]);
+        float l = 0.0f, a[2] = {0.0f, 0.0f};
 #pragma unroll
-            for (int i = 0; i < 4; ++i) cta_acc[hh][d0 + i] = a[i];
-            if ((threadIdx.x & 31) == 0) { cta_m[hh] = m; cta_l[hh] = l; }
+        for (int w = 0; w < kAttnWarps; ++w) {
+            const float scw = __expf(red_m[w][hh] - m);
+            const float2 v2 = *reinterpret_cast<const float2*>(&red_acc[w][hh][d0]);
+            l += red_l[w][hh] * scw;
+            a[0] += v2.x * scw;
+            a[1] += v2.y * scw;
+        }
+        SliceState& mine = slice_s[s];
+        if (S > 1) {
+            st_cluster2(in_cta0(&mine.acc[hh][d0]), a[0], a[1]);
+            if (d0 == 0) { st_cluster(in_cta0(&mine.m[hh]), m); st_cluster(in_cta0(&mine.l[hh]), l); }
+        } else {
+            *reinterpret_cast<float2*>(&mine.acc[hh][d0]) = make_float2(a[0], a[1]);
+            if (d0 == 0) { mine.m[hh] = m; mine.l[hh] = l; }
         }
     }
-    // ---- every thread of the cluster (the producer warps included) ----
-    ATTN_PHASE(5);  // warps merged
-    cg::cluster_group cluster = cg::this_cluster();
-    if (S > 1) cluster.sync(); else __syncthreads();
-    ATTN_PHASE(6);  // every CTA of the cluster has its partial state ready
-    // ---- CTA 0 of the cluster merges the S context slices and writes the 4 heads ----
-    if (s == 0 && threadIdx.x < kQPerKv * 32) {
-        const int hh = threadIdx.x >> 5, d0 = (threadIdx.x & 31) * 4;
+    __syncwarp();
+    if (S > 1) { cluster_arrive(); cluster_wait(); } else __syncthreads();
+    ATTN_PHASE(6);  // every CTA of the cluster has its partial state in CTA 0
+    // ---- CTA 0 of the cluster merges the S context slices, writes the 4 heads and quantises them for the o-projection ----
+    if (s == 0 && warp < kAttnWarps) {
         float m = -1e30f;
-        for (int r = 0; r < S; ++r) m = fmaxf(m, (S > 1 ? cluster.map_shared_rank(cta_m, r) : cta_m)[hh]);
-        float l = 0.0f, a[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+        for (int r = 0; r < S; ++r) m = fmaxf(m, slice_s[r].m[hh]);
+        float l = 0.0f, a[2] = {0.0f, 0.0f};
         for (int r = 0; r < S; ++r) {
-            const float* pm = S > 1 ? cluster.map_shared_rank(cta_m, r) : cta_m;
-            const float* pl = S > 1 ? cluster.map_shared_rank(cta_l, r) : cta_l;
-            const float* pa = S > 1 ? cluster.map_shared_rank(&cta_acc[0][0], r) : &cta_acc[0][0];
-            const float scr = __expf(pm[hh] - m);
-            l += pl[hh] * scr;
-            const float4 v4 = *reinterpret_cast<const float4*>(pa + hh * kHeadDim + d0);
-            a[0] += v4.x * scr; a[1] += v4.y * scr; a[2] += v4.z * scr; a[3] += v4.w * scr;
+            const float scr = __expf(slice_s[r].m[hh] - m);
+            const float2 v2 = *reinterpret_cast<const float2*>(&slice_s[r].acc[hh][d0]);
+            l += slice_s[r].l[hh] * scr;
+            a[0] += v2.x * scr;
+            a[1] += v2.y * scr;
         }
         const float inv = seq_len > 0 ? 1.0f / l : 0.0f;  // empty sequence -> zeros (paged_attention.cu:44-50)
-        __align__(8) __half o4[4];
-#pragma unroll
-        for (int i = 0; i < 4; ++i) o4[i] = __float2half(seq_len > 0 ? a[i] * inv : 0.0f);
-#pragma unroll
-        for (int i = 0; i < 4; ++i) out_s[hh * kHeadDim + d0 + i] = o4[i];
-        const size_t oo = (static_cast<size_t>(b) * p.n_q + kvh * heads_here + hh) * kHeadDim + d0;
-        if (p.out) *reinterpret_cast<uint2*>(p.out + oo) = *reinterpret_cast<const uint2*>(o4);
-    }
-    if (S > 1) cluster.sync(); else __syncthreads();
-    // ---- optional: quantise these 512 channels for the o-projection (int8_gemm.cu:147-211) ----
-    if (s == 0 && p.Xq && warp < kAttnWarps) {
-        const int gsz = p.g, K = p.n_q * kHeadDim, G = K / gsz;
-        const int ch0 = kvh * heads_here * kHeadDim;          // first channel of this CTA
-        const int groups_here = (kQPerKv * kHeadDim) / gsz;   // 2 at g=256, 8 at g=64
-        for (int j = warp; j < groups_here; j += kAttnWarps) {
-            float amax = 0.0f;
-            for (int e = lane; e < gsz; e += 32) amax = fmaxf(amax, fabsf(__half2float(out_s[j * gsz + e])));
-            for (int off = 16; off > 0; off >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, off));
-            float scale = amax / 127.0f;
-            if (scale < 1e-8f) scale = 1e-8f;
-            if (lane == 0) p.Xs[static_cast<size_t>(b) * G + ch0 / gsz + j] = scale;
-            const float inv_scale = 1.0f / scale;
-            for (int e = lane; e < gsz; e += 32) {
-                int qv = __float2int_rn(__half2float(out_s[j * gsz + e]) * inv_scale);
-                qv = max(-127, min(127, qv));
-                p.Xq[static_cast<size_t>(b) * K + ch0 + j * gsz + e] = static_cast<int8_t>(qv);
+        const __half2 o2 = __floats2half2_rn(seq_len > 0 ? a[0] * inv : 0.0f, seq_len > 0 ? a[1] * inv : 0.0f);
+        const int K = p.n_q * kHeadDim, ch = kvh * heads_here * kHeadDim + hh * kHeadDim + d0;  // this thread's first channel
+        const size_t oo = static_cast<size_t>(b) * K + ch;
+        if (p.out) *reinterpret_cast<__half2*>(p.out + oo) = o2;
+        if (p.Xq) {  // int8_gemm.cu:147-211; a group is g / 2 threads (g divides 512: a power of two)
+            const float2 f = __half22float2(o2);
+            float amax = fmaxf(fabsf(f.x), fabsf(f.y));
+            const int span = p.g / 2 < 32 ? p.g / 2 : 32;
+            for (int off = span / 2; off > 0; off >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, off));
+            if (p.g > 64) {  // two, four or eight warps to a group
+                if (lane == 0) amax_s[warp] = amax;
+                consumer_barrier();
+                const int wpg = p.g / 64, w0 = warp & ~(wpg - 1);
+                for (int w = 0; w < wpg; ++w) amax = fmaxf(amax, amax_s[w0 + w]);
             }
+            float am[2] = {amax, amax};
+            if (p.g == 1) { am[0] = fabsf(f.x); am[1] = fabsf(f.y); }
+            int q[2];
+#pragma unroll
+            for (int e = 0; e < 2; ++e) {
+                float scale = am[e] / 127.0f;
+                if (scale < 1e-8f) scale = 1e-8f;
+                if ((ch + e) % p.g == 0) p.Xs[static_cast<size_t>(b) * (K / p.g) + (ch + e) / p.g] = scale;
+                const float inv_scale = 1.0f / scale;
+                q[e] = max(-127, min(127, __float2int_rn((e ? f.y : f.x) * inv_scale)));
+            }
+            p.Xq[oo] = static_cast<int8_t>(q[0]);
+            p.Xq[oo + 1] = static_cast<int8_t>(q[1]);
         }
     }
     if (s_fail) {  // a bounded wait ran out: give copies that may still be in flight time to land before the CTA goes
@@ -643,8 +686,10 @@ int launch_attention(const AttnParams& base, int B, int splits, cudaStream_t str
             sms = 148;
         const int want = sms / (B * n_kv);
         splits = want >= 8 ? 8 : want >= 4 ? 4 : want >= 2 ? 2 : 1;
+        // no more slices than give each consumer warp a block of the longest sequence the table can hold
+        while (splits > 1 && (splits / 2) * kAttnWarps >= base.max_blocks) splits /= 2;
     }
-    if (splits > 8) splits = 8;
+    if (splits > kMaxSlices) splits = kMaxSlices;
     AttnParams p = base;
     p.S = splits;
     // The caches as rows of 256 bytes (one token of one head); a box is 16 rows x 128 bytes. The row count only bounds
