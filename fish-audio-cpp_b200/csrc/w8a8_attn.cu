@@ -145,7 +145,7 @@ struct AttnParams {
 #define W8A8_ATTN_WARPS 8
 #endif
 #ifndef W8A8_ATTN_RING
-#define W8A8_ATTN_RING 16
+#define W8A8_ATTN_RING 24
 #endif
 constexpr int kAttnWarps = W8A8_ATTN_WARPS;      // consumer warps
 constexpr int kAttnThreads = (kAttnWarps + 1) * 32;  // + one producer warp
@@ -153,8 +153,11 @@ constexpr int kQPerKv = 4;                       // query heads per kv head hand
 constexpr int kBoxBytes = kBlockTokens * 128;    // a TMA box: 16 token rows x 128 bytes (64 dims), 128-byte swizzle
 constexpr int kBlkBytes = 2 * kBoxBytes;         // one 16-token block of K (or of V): dims 0..63, then dims 64..127
 constexpr int kStageBytes = 2 * kBlkBytes;       // K block, then V block
-constexpr int kRing = W8A8_ATTN_RING;            // stages of the CTA's ring, 8 KB each: two per consumer warp, so that a
-                                                 // warp's next block is on its way while it works on the current one
+// Stages of the CTA's ring, 8 KB each: three blocks per consumer warp on their way before the query arrives, as many as fit.
+// A multiple of the consumer warps: a stage then belongs to one warp, and that warp alone waits for its phases (a warp that
+// meets a stage for the first time in its second phase would take "phase -1 is complete" for its block).
+constexpr int kRing = W8A8_ATTN_RING;
+static_assert(kRing % kAttnWarps == 0, "a stage belongs to one consumer warp");
 
 // Byte offset, inside a K or V block in shared memory, of the 16-byte chunk that holds dims [8 c16, 8 c16 + 8) of
 // token row r: the box of its 64-dim half, the row's 128 bytes, the chunk XOR-ed with the row (what the tensor
@@ -300,7 +303,7 @@ __global__ void __maxnreg__(128) paged_attention_decode_kernel(const __grid_cons
     __shared__ __align__(16) __half kv_new_s[2][kHeadDim];
     __shared__ float red_m[kAttnWarps][kQPerKv], red_l[kAttnWarps][kQPerKv];
     __shared__ float red_acc[kAttnWarps][kQPerKv][kHeadDim];
-    __shared__ SliceState slice_s[kMaxSlices];  // in CTA 0 of the cluster: the partial state of every context slice
+    __shared__ SliceState slice_s[kMaxSlices - 1];  // in CTA 0 of the cluster: the partial states of context slices 1, 2, ...
     __shared__ float amax_s[kAttnWarps];
     __shared__ int s_fail;
     W8A8_TRACE_SCOPE();
@@ -388,11 +391,20 @@ __global__ void __maxnreg__(128) paged_attention_decode_kernel(const __grid_cons
             rot.make(p.freqs, pos, lane);
             owner = ((pos / kBlockTokens) % S) == s;  // this CTA attends over the block the new token joins
         }
-        ptx::pdl_wait();
-        W8A8_TRACE_WAITED();
-        ATTN_PHASE(1);
         const int new_bi = pos / kBlockTokens;
+        if constexpr (!ROPE) ptx::pdl_wait();
         if constexpr (ROPE) {
+            // The first pass is a rehearsal on zeros, before the dependency wait: cold code costs about six clocks an instruction
+            // (step at batch 8: 1554 -> 1536 us). Rehearsing the block loop and the merges as well takes longer than the wait
+            // it hides in (1517 -> 1756 us).
+#pragma unroll 1
+            for (int pass = 0; pass < 2; ++pass) {
+            const bool real = pass == 1;
+            if (real) {
+                ptx::pdl_wait();
+                W8A8_TRACE_WAITED();
+                ATTN_PHASE(1);
+            }
             // six head rows of the new token: the group's four query heads, then its k and its v; a warp per row
             const int total_heads = p.n_q + 2 * p.n_kv;
             for (int h = warp; h < kQPerKv + 2; h += kAttnWarps) {
@@ -403,7 +415,8 @@ __global__ void __maxnreg__(128) paged_attention_decode_kernel(const __grid_cons
                 __half hq[4], wq[4];
 #pragma unroll
                 for (int v = 0; v < 4; ++v) {
-                    hq[v] = src[v * 32 + lane];
+                    hq[v] = __float2half(0.0f);
+                    if (real) hq[v] = src[v * 32 + lane];
                     wq[v] = (norm_w && !is_v) ? norm_w[v * 32 + lane] : __float2half(1.0f);
                 }
                 if (!is_v) head_norm_rope(hq, norm_w != nullptr, wq, p.eps, rot, lane);
@@ -413,7 +426,7 @@ __global__ void __maxnreg__(128) paged_attention_decode_kernel(const __grid_cons
                 } else {
 #pragma unroll
                     for (int v = 0; v < 4; ++v) kv_new_s[is_v ? 1 : 0][v * 32 + lane] = hq[v];
-                    if (owner) {
+                    if (owner && real) {
                         const int phys = p.block_table[static_cast<size_t>(b) * p.max_blocks + new_bi];
                         if (phys >= 0) {
                             __half* dst = (is_k ? p.k_cache_w : p.v_cache_w) +
@@ -424,6 +437,7 @@ __global__ void __maxnreg__(128) paged_attention_decode_kernel(const __grid_cons
                         }
                     }
                 }
+            }
             }
             consumer_barrier();  // q and the new k / v rows are in shared memory
         }
@@ -541,11 +555,10 @@ __global__ void __maxnreg__(128) paged_attention_decode_kernel(const __grid_cons
     __syncwarp();
     if (S > 1) cluster_wait();  // (every thread, the producer warp included: CTA 0 has started)
     const int hh = (warp & 7) >> 1, d0 = (warp & 1) * 64 + 2 * lane;
+    float m = -1e30f, l = 0.0f, a[2] = {0.0f, 0.0f};  // of this CTA's slice, then (CTA 0) of all
     if (warp < kAttnWarps) {
-        float m = -1e30f;
 #pragma unroll
         for (int w = 0; w < kAttnWarps; ++w) m = fmaxf(m, red_m[w][hh]);
-        float l = 0.0f, a[2] = {0.0f, 0.0f};
 #pragma unroll
         for (int w = 0; w < kAttnWarps; ++w) {
             const float scw = __expf(red_m[w][hh] - m);
@@ -554,29 +567,34 @@ __global__ void __maxnreg__(128) paged_attention_decode_kernel(const __grid_cons
             a[0] += v2.x * scw;
             a[1] += v2.y * scw;
         }
-        SliceState& mine = slice_s[s];
-        if (S > 1) {
+        if (s > 0) {
+            SliceState& mine = slice_s[s - 1];
             st_cluster2(in_cta0(&mine.acc[hh][d0]), a[0], a[1]);
             if (d0 == 0) { st_cluster(in_cta0(&mine.m[hh]), m); st_cluster(in_cta0(&mine.l[hh]), l); }
-        } else {
-            *reinterpret_cast<float2*>(&mine.acc[hh][d0]) = make_float2(a[0], a[1]);
-            if (d0 == 0) { mine.m[hh] = m; mine.l[hh] = l; }
         }
     }
-    __syncwarp();
-    if (S > 1) { cluster_arrive(); cluster_wait(); } else __syncthreads();
+    if (S > 1) {
+        __syncwarp();
+        cluster_arrive();
+        cluster_wait();
+    }
     ATTN_PHASE(6);  // every CTA of the cluster has its partial state in CTA 0
     // ---- CTA 0 of the cluster merges the S context slices, writes the 4 heads and quantises them for the o-projection ----
     if (s == 0 && warp < kAttnWarps) {
-        float m = -1e30f;
-        for (int r = 0; r < S; ++r) m = fmaxf(m, slice_s[r].m[hh]);
-        float l = 0.0f, a[2] = {0.0f, 0.0f};
-        for (int r = 0; r < S; ++r) {
-            const float scr = __expf(slice_s[r].m[hh] - m);
-            const float2 v2 = *reinterpret_cast<const float2*>(&slice_s[r].acc[hh][d0]);
-            l += slice_s[r].l[hh] * scr;
-            a[0] += v2.x * scr;
-            a[1] += v2.y * scr;
+        if (S > 1) {
+            const float m_own = m;
+            for (int r = 0; r < S - 1; ++r) m = fmaxf(m, slice_s[r].m[hh]);
+            const float own = __expf(m_own - m);
+            l *= own;
+            a[0] *= own;
+            a[1] *= own;
+            for (int r = 0; r < S - 1; ++r) {
+                const float scr = __expf(slice_s[r].m[hh] - m);
+                const float2 v2 = *reinterpret_cast<const float2*>(&slice_s[r].acc[hh][d0]);
+                l += slice_s[r].l[hh] * scr;
+                a[0] += v2.x * scr;
+                a[1] += v2.y * scr;
+            }
         }
         const float inv = seq_len > 0 ? 1.0f / l : 0.0f;  // empty sequence -> zeros (paged_attention.cu:44-50)
         const __half2 o2 = __floats2half2_rn(seq_len > 0 ? a[0] * inv : 0.0f, seq_len > 0 ? a[1] * inv : 0.0f);
