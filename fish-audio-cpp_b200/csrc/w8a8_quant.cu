@@ -330,112 +330,109 @@ __global__ void __launch_bounds__(1024) rowquant_fast_kernel(const RowQuantParam
     }
 }
 
-// residual add + RMSNorm + group quantiser for the decode step, in little code: 256 threads per row, the row
-// staged in shared memory, g in {64, 128, 256}, K a multiple of 256 up to 4096. The sum of squares follows the
-// reference's T-thread launch (rms_norm.cu:23-49, :69-70): real warp w plays virtual warps w*VW .. w*VW+VW-1
-// (VW = T / 256), so the normed values are the reference's; normalising and quantising then go 8 elements (one
-// 128-bit piece) per thread, the g/8 threads of a group finding its absmax with shuffles. Plain loops on purpose:
-// a launch runs this code once, and what it costs is the instruction fetch as much as the arithmetic.
+// residual add + RMSNorm + group quantiser of one token row by 128 threads, for the decode step; K a multiple of 256 up to
+// 4096, g in {64, 128, 256}. At 8 rows a launch is a latency chain: what counts is its length. Thread t owns the 16-byte
+// pieces t + 128 i, i.e. elements 8 t + j + 1024 i (j < 8): ALL the elements of the reference's virtual threads 8 t + j of its
+// 1024-thread launch (rms_norm.cu:23-27), in its order of addition. (For K <= 512 the reference launches fewer threads; the
+// virtual threads past K then add zeros, which changes no sum.) Its shuffle-down tree over a virtual warp (virtual lanes
+// 8 (l % 4) + j) crosses real lanes twice and stays inside a thread three times; the 32 sums go through shared memory, one
+// barrier, and every warp runs the second tree (rms_norm.cu:36-42) itself. (Before: the row staged in shared memory by 256
+// threads, rounds of serial sums and five-step trees, five barriers.)
+// The first pass is a rehearsal on the norm weights, with nothing stored, while the kernel before this one still runs: code
+// that runs for the first time after another kernel costs about six clocks an instruction, warm code a fifth of that,
+// and a launch of this kernel runs its code once. (Decode step, batch 8: 1726 -> 1700 us together with the quantiser's.
+// The same in the linear's CTAs made the step slower.)
 template <int GM>
-__global__ void __launch_bounds__(256) rowquant_compact_kernel(const RowQuantParams p, int T) {
-    constexpr int LANES = GM / 8, kThreads = 256;
-    __shared__ float s_red[32];
-    __shared__ __align__(16) __half row_s[4096];
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const int K = p.K, VW = T / kThreads, G = p.G, row = blockIdx.x;
+__global__ void __launch_bounds__(128) rowquant_compact_kernel(const __grid_constant__ RowQuantParams p) {
+    constexpr int LANES = GM / 8, kPieces = 4;
+    __shared__ float s_red[2][32];
+    const int tid = threadIdx.x, lane = tid & 31, K = p.K, pieces = K / 8, row = blockIdx.x;
     const size_t base = static_cast<size_t>(row) * K;
-    const int pieces = K / 8;
     W8A8_TRACE_SCOPE();
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-    uint4 xv[2], dv[2], wv[2];
+    uint4 wv[kPieces];
 #pragma unroll
-    for (int i = 0; i < 2; ++i) {
-        const int c8 = tid + i * kThreads;
+    for (int i = 0; i < kPieces; ++i) {
+        const int c8 = tid + i * 128;
         wv[i] = __ldg(reinterpret_cast<const uint4*>(p.norm_weight) + (c8 < pieces ? c8 : 0));
     }
-    // The first pass is a rehearsal on the norm weights, with nothing stored, while the kernel before this one still runs: code
-    // that runs for the first time after another kernel costs about six clocks an instruction, warm code a fifth of that,
-    // and a launch of this kernel runs its code once. (Decode step, batch 8: 1726 -> 1700 us together with the quantiser's.
-    // The same in the linear's CTAs made the step slower: they evict the code of the kernel that is still running.)
+    const __half* res = p.residual ? p.residual : p.x_in;
 #pragma unroll 1
     for (int pass = 0; pass < 2; ++pass) {
-    const bool real = pass == 1;
-    if (real) {
-        asm volatile("griddepcontrol.wait;" ::: "memory");
-        W8A8_TRACE_WAITED();
-    }
-#pragma unroll
-    for (int i = 0; i < 2; ++i) {  // every load first (at most two pieces per thread)
-        const int c8 = tid + i * kThreads;
-        const int cc = c8 < pieces ? c8 : 0;
-        xv[i] = dv[i] = wv[i];
+        const bool real = pass == 1;
         if (real) {
-            xv[i] = *reinterpret_cast<const uint4*>(p.x_in + base + cc * 8);
-            dv[i] = *reinterpret_cast<const uint4*>((p.residual ? p.residual : p.x_in) + base + cc * 8);
+            asm volatile("griddepcontrol.wait;" ::: "memory");
+            W8A8_TRACE_WAITED();
         }
-    }
+        uint4 xv[kPieces], dv[kPieces];
 #pragma unroll
-    for (int i = 0; i < 2; ++i) {
-        const int c8 = tid + i * kThreads;
-        if (c8 < pieces) {
-            if (p.residual) {
-                __half* hx = reinterpret_cast<__half*>(&xv[i]);
-                const __half* hd = reinterpret_cast<const __half*>(&dv[i]);
-#pragma unroll
-                for (int e = 0; e < 8; ++e) hx[e] = __float2half(__half2float(hx[e]) + __half2float(hd[e]));
-                if (real && p.x_out) *reinterpret_cast<uint4*>(p.x_out + base + c8 * 8) = xv[i];
+        for (int i = 0; i < kPieces; ++i) {  // every load first
+            const int c8 = tid + i * 128;
+            xv[i] = dv[i] = wv[i];
+            if (real && c8 < pieces) {
+                xv[i] = *reinterpret_cast<const uint4*>(p.x_in + base + c8 * 8);
+                dv[i] = *reinterpret_cast<const uint4*>(res + base + c8 * 8);
             }
-            reinterpret_cast<uint4*>(row_s)[c8] = xv[i];
         }
-    }
-    __syncthreads();
-#pragma unroll 1
-    for (int k = 0; k < VW; ++k) {
-        float local_sum = 0.0f;
-#pragma unroll 1
-        for (int e = (warp * VW + k) * 32 + lane; e < K; e += T) {
-            float val = __half2float(row_s[e]);
-            local_sum += val * val;
+        float ls[8];
+#pragma unroll
+        for (int j = 0; j < 8; ++j) ls[j] = 0.0f;
+#pragma unroll
+        for (int i = 0; i < kPieces; ++i) {
+            const int c8 = tid + i * 128;
+            if (c8 < pieces) {
+                __half* hx = reinterpret_cast<__half*>(&xv[i]);
+                if (p.residual) {
+                    const __half* hd = reinterpret_cast<const __half*>(&dv[i]);
+#pragma unroll
+                    for (int e = 0; e < 8; ++e) hx[e] = __float2half(__half2float(hx[e]) + __half2float(hd[e]));
+                    if (real && p.x_out) *reinterpret_cast<uint4*>(p.x_out + base + c8 * 8) = xv[i];
+                }
+#pragma unroll
+                for (int j = 0; j < 8; ++j) {
+                    const float val = __half2float(hx[j]);
+                    ls[j] += val * val;
+                }
+            }
         }
-        for (int offset = 16; offset > 0; offset /= 2) local_sum += __shfl_down_sync(0xffffffffu, local_sum, offset);
-        if (lane == 0) s_red[warp * VW + k] = local_sum;
-    }
-    __syncthreads();
-    float total_sum = 0.0f;
-    if (warp == 0) {
-        if (lane < T / 32) total_sum = s_red[lane];
-        for (int offset = 16; offset > 0; offset /= 2) total_sum += __shfl_down_sync(0xffffffffu, total_sum, offset);
-    }
-    __syncthreads();
-    if (tid == 0) s_red[0] = rsqrtf(total_sum / K + p.eps);
-    __syncthreads();
-    const float rms = s_red[0];
 #pragma unroll
-    for (int i = 0; i < 2; ++i) {
-        const int c8 = tid + i * kThreads;
-        const bool live = c8 < pieces;  // whole warps are live or not (pieces is a multiple of 32)
-        __half* hx = reinterpret_cast<__half*>(&xv[i]);
-        const __half* hw = reinterpret_cast<const __half*>(&wv[i]);
-        float v[8], amax = 0.0f;
+        for (int j = 0; j < 8; ++j) ls[j] += __shfl_down_sync(0xffffffffu, ls[j], 2);  // virtual offset 16
 #pragma unroll
-        for (int e = 0; e < 8; ++e) {
-            float val = __half2float(hx[e]) * rms;
-            hx[e] = __float2half(val * __half2float(hw[e]));
-            v[e] = __half2float(hx[e]);
-            amax = fmaxf(amax, fabsf(v[e]));
+        for (int j = 0; j < 8; ++j) ls[j] += __shfl_down_sync(0xffffffffu, ls[j], 1);  // virtual offset 8
+#pragma unroll
+        for (int j = 0; j < 4; ++j) ls[j] += ls[j + 4];
+        ls[0] += ls[2];
+        ls[1] += ls[3];
+        if ((lane & 3) == 0) s_red[pass][tid >> 2] = ls[0] + ls[1];
+        __syncthreads();
+        float total_sum = s_red[pass][lane];
+#pragma unroll
+        for (int offset = 16; offset > 0; offset /= 2) total_sum += __shfl_xor_sync(0xffffffffu, total_sum, offset);
+        const float rms = rsqrtf(total_sum / K + p.eps);
+#pragma unroll
+        for (int i = 0; i < kPieces; ++i) {
+            const int c8 = tid + i * 128;
+            if (c8 >= pieces) break;  // (whole warps: pieces is a multiple of 32)
+            __half* hx = reinterpret_cast<__half*>(&xv[i]);
+            const __half* hw = reinterpret_cast<const __half*>(&wv[i]);
+            float v[8], amax = 0.0f;
+#pragma unroll
+            for (int e = 0; e < 8; ++e) {
+                const float val = __half2float(hx[e]) * rms;
+                hx[e] = __float2half(val * __half2float(hw[e]));
+                v[e] = __half2float(hx[e]);
+                amax = fmaxf(amax, fabsf(v[e]));
+            }
+            if (real && p.normed_out) *reinterpret_cast<uint4*>(p.normed_out + base + c8 * 8) = xv[i];
+            if (!p.Xq) continue;
+#pragma unroll
+            for (int o = LANES / 2; o > 0; o >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, o));
+            float scale = amax / 127.0f;
+            if (scale < 1e-8f) scale = 1e-8f;
+            if (real && (lane & (LANES - 1)) == 0) p.Xs[static_cast<size_t>(row) * p.G + (c8 * 8) / GM] = scale;
+            const uint2 cd = codes8(v, 1.0f / scale, false);
+            if (real) *reinterpret_cast<uint2*>(p.Xq + base + c8 * 8) = cd;
         }
-        if (live && real && p.normed_out) *reinterpret_cast<uint4*>(p.normed_out + base + c8 * 8) = xv[i];
-        if (!p.Xq) continue;
-#pragma unroll
-        for (int o = LANES / 2; o > 0; o >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, o));
-        if (!live) continue;
-        float scale = amax / 127.0f;
-        if (scale < 1e-8f) scale = 1e-8f;
-        if (real && (lane & (LANES - 1)) == 0) p.Xs[static_cast<size_t>(row) * G + (c8 * 8) / GM] = scale;
-        const uint2 cd = codes8(v, 1.0f / scale, false);
-        if (real) *reinterpret_cast<uint2*>(p.Xq + base + c8 * 8) = cd;
-    }
-    __syncthreads();
     }
     W8A8_TRACE_END(2u);
 }
@@ -708,7 +705,7 @@ int launch_rowquant(const __half* x_in, __half* x_out, const __half* residual,
                                                                                 : launch_rownorm_warp<256>(p, M, stream);
         return launch_row_kernel("rowquant_compact", gm == 64    ? rowquant_compact_kernel<64>
                                                      : gm == 128 ? rowquant_compact_kernel<128>
-                                                                 : rowquant_compact_kernel<256>, M, 256, 0, stream, p, threads);
+                                                                 : rowquant_compact_kernel<256>, M, 128, 0, stream, p);
     }
     if (norm_weight && threads >= 32 && K <= kFastElems * threads && p.g % 32 == 0 && p.G <= 160)
         return launch_row_kernel("rowquant_fast", rowquant_fast_kernel, M, threads, 0, stream, p);
