@@ -431,6 +431,14 @@ int w8a8_linear(w8a8_ctx* ctx, const void* W, const void* w_scale, int group_siz
     const int act_mode = opts ? opts->act_mode : W8A8_ACT_PER_TOKEN_GROUP;
     const int kernel = opts ? opts->kernel : W8A8_KERNEL_AUTO;
 
+    if (M <= 8 && act_mode == W8A8_ACT_PER_TOKEN_GROUP && !smooth_inv && !act_scale &&
+        (kernel == W8A8_KERNEL_AUTO || kernel == W8A8_KERNEL_GEMV_PACKED)) {
+        LinearArgs f = a;
+        f.X = static_cast<const __half*>(X);
+        fill_scratch(ctx, f);
+        if (f.packed && quant_form_wins(f) && gemv_packed_supports(f)) return launch_linear_gemv_packed(f, ctx->device_status, s);
+    }
+
     // Codes and scales into the context's scratch (row kernel), then the integer kernel; the two are
     // chained with programmatic dependent launch, so the second starts streaming weights early.
     const size_t need = quant_scratch_bytes(M, K, group_size);

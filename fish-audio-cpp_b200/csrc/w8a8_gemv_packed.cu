@@ -44,7 +44,8 @@ constexpr int kBlockW = 16 * 256;        // weight bytes of a block
 constexpr int kStagePitch = kBlockW + 128;  // room for the largest scale tail, keeps stages 128-byte aligned
 // How the activations arrive (template parameter PRO):
 enum { kProCodes = 0,   // int8 codes + fp32 scales made by an earlier launch (Xq, Xs)
-       kProNorm = 1 };  // fp16 rows: every CTA does [x + residual] -> RMSNorm -> quantiser itself, in its prologue
+       kProNorm = 1,    // fp16 rows: every CTA does [x + residual] -> RMSNorm -> quantiser itself, in its prologue
+       kProQuant = 2 }; // fp16 rows: a warp quantises the activations of each block it consumes, in registers
 
 // Forms of the kernel, by 8-token B tiles and group size class (reasons: see the consumer loop).
 constexpr bool in_place(int mt, int gm) { return mt == 4 || (mt == 2 && gm != 64); }
@@ -323,6 +324,10 @@ __device__ __forceinline__ void tail_group_quant(const LinearArgs& a, int ct0, i
 // One warp per token row (M <= 8), the row in registers from the load to the codes; only the codes and scales
 // go to shared memory. This replaces a separate launch of a kernel that runs on M CTAs and leaves the rest of
 // the GPU idle, and the trip of its results through L2.
+// PRO == kProQuant (M <= 8, g = 64, 128 or 256): the linear without the quantiser's launch before it. A lane's B fragments of a
+// block are 64 activations of one token, the four lanes of a quad hold the block's 256 of that token: a group's absmax is a
+// few packed maxima and two shuffles, and the codes go from registers into the MMA. Every warp that meets a K block quantises
+// it again, some 300 instructions per block, so the form is chosen where a CTA has few row tiles (see quant_form_wins).
 // ST: stages of a warp's ring (3; 2 for kProNorm so that two CTAs fit an SM beside the code rows).
 // KI: kProNorm only, the 16-byte pieces of a row a lane holds (K <= 256 * KI): 10 for the stack's K = 2560, else 16.
 // EXTRA: the call wants the group sums dumped or has a tail. An instance of its own: the check per promote alone cost 0.1-1.1 us
@@ -330,10 +335,10 @@ __device__ __forceinline__ void tail_group_quant(const LinearArgs& a, int ct0, i
 template <int MT, int GM, int PRO, int ST, int KI, bool EXTRA>
 __global__ void __launch_bounds__(kThreads, two_per_sm(MT, GM) ? 2 : 1)
 gemv_packed_kernel(const GemvPackedParams p) {
-    constexpr bool FUSED = PRO == kProNorm;
+    constexpr bool FUSED = PRO == kProNorm, QUANT = PRO == kProQuant;
     constexpr int kStages = ST;
     constexpr int kRingBytes = kStages * kStagePitch;
-    static_assert(PRO == kProCodes || MT == 1, "the fused prologue handles one row per warp");
+    static_assert(PRO == kProCodes || MT == 1, "the fused prologue handles one row per warp, the fused quantiser one token per quad");
     extern __shared__ unsigned char smem_raw[];
     W8A8_TRACE_SCOPE();
     unsigned long long tl[8] = {0, 0, 0, 0, 0, 0, 0, 0};
@@ -586,7 +591,7 @@ gemv_packed_kernel(const GemvPackedParams p) {
         xq_s = ptx::smem_u32(codes_s) + min(gq, a.M - 1) * pitch + c * 16;
         xsp_s[0] = scales_s + min(2 * c, a.M - 1) * a.G;
         xsp_s[1] = scales_s + min(2 * c + 1, a.M - 1) * a.G;
-    } else {
+    } else if constexpr (!QUANT) {
 #pragma unroll
         for (int nt = 0; nt < MT; ++nt) {
             xq[nt] = a.Xq + static_cast<size_t>(min(nt * 8 + gq, a.M - 1)) * a.K + c * 16;
@@ -702,7 +707,7 @@ gemv_packed_kernel(const GemvPackedParams p) {
     int si = 0;
     int ub = static_cast<int>(u0 % p.upt), rt = static_cast<int>(u0 / p.upt);
     bool ok = true;
-    constexpr bool kInPlace = in_place(MT, GM) && !FUSED;
+    constexpr bool kInPlace = (in_place(MT, GM) && !FUSED) || QUANT;
     constexpr int NX = kInPlace ? 1 : 2;
     uint4 x[NX][4][MT];
     float xs[NX][GPU][MT][2];
@@ -724,7 +729,62 @@ gemv_packed_kernel(const GemvPackedParams p) {
                 else xs[buf][q][nt][e] = __ldg(xsp[nt][e] + unit_b * GPU + q);
             }
     };
-    if (T > 0) {
+    // kProQuant: this lane's 64 activations of a block (chunk ch: 16 from ch * 64 + c * 16 on), requested a block ahead
+    uint4 raw[QUANT ? 8 : 1];
+    auto load_raw = [&](int kbase) {
+        const __half* src = a.X + static_cast<size_t>(min(gq, a.M - 1)) * a.K + kbase + c * 16;
+#pragma unroll
+        for (int i = 0; i < 8; ++i) raw[i] = __ldg(reinterpret_cast<const uint4*>(src + (i >> 1) * 64) + (i & 1));
+    };
+    auto quantise = [&]() {  // raw -> codes in x[0], scales of tokens 2c and 2c + 1 in xs[0] (int8_gemm.cu:147-211)
+        float am[GPU];
+#pragma unroll
+        for (int q = 0; q < GPU; ++q) {
+            __half2 m2 = __float2half2_rn(0.0f);
+#pragma unroll
+            for (int i = q * (8 / GPU); i < (q + 1) * (8 / GPU); ++i) {
+                const __half2* h = reinterpret_cast<const __half2*>(&raw[i]);
+#pragma unroll
+                for (int e = 0; e < 4; ++e) m2 = __hmax2(m2, __habs2(h[e]));
+            }
+            float m = fmaxf(__low2float(m2), __high2float(m2));
+            m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, 1));
+            am[q] = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, 2));
+        }
+        // lane c of a quad makes the scale of group c (of c % GPU), the others get it by shuffles
+        float mine = am[0];
+#pragma unroll
+        for (int q = 1; q < GPU; ++q)
+            if ((c & (GPU - 1)) == q) mine = am[q];
+        float scale = mine / 127.0f;
+        if (scale < 1e-8f) scale = 1e-8f;
+        const float inv_mine = 1.0f / scale;
+#pragma unroll
+        for (int q = 0; q < GPU; ++q) {
+            const float inv = GPU == 1 ? inv_mine : __shfl_sync(0xffffffffu, inv_mine, (lane & ~3) + q);
+#pragma unroll
+            for (int e = 0; e < 2; ++e) xs[0][q][0][e] = __shfl_sync(0xffffffffu, scale, (2 * c + e) * 4 + q);
+#pragma unroll
+            for (int ch = q * (4 / GPU); ch < (q + 1) * (4 / GPU); ++ch) {
+                uint32_t w[4];
+#pragma unroll
+                for (int k = 0; k < 4; ++k) {
+                    const __half2* h = reinterpret_cast<const __half2*>(&raw[2 * ch + (k >> 1)]) + 2 * (k & 1);
+                    const float2 f0 = __half22float2(h[0]), f1 = __half22float2(h[1]);
+                    // (no code of a group's own scale leaves [-127, 127])
+                    const int q0 = __float2int_rn(f0.x * inv), q1 = __float2int_rn(f0.y * inv);
+                    const int q2 = __float2int_rn(f1.x * inv), q3 = __float2int_rn(f1.y * inv);
+                    uint32_t hi;
+                    asm("cvt.pack.sat.s8.s32.b32 %0, %1, %2, %3;" : "=r"(hi) : "r"(q3), "r"(q2), "r"(0));
+                    asm("cvt.pack.sat.s8.s32.b32 %0, %1, %2, %3;" : "=r"(w[k]) : "r"(q1), "r"(q0), "r"(hi));
+                }
+                x[0][ch][0] = make_uint4(w[0], w[1], w[2], w[3]);
+            }
+        }
+    };
+    if constexpr (QUANT) {
+        if (T > 0) load_raw(ub * 256);
+    } else if (T > 0) {
 #pragma unroll
         for (int ch = 0; ch < 4; ++ch) load_x(ub * p.bpu * 256, ch, 0);
 #pragma unroll
@@ -736,6 +796,10 @@ gemv_packed_kernel(const GemvPackedParams p) {
         int nsi = si + 1, nub = ub;
         if (nsi == p.bpu) { nsi = 0; if (++nub == p.upt) nub = 0; }
         const int nkb = (nub * p.bpu + nsi) * 256;
+        if constexpr (QUANT) {
+            quantise();
+            if (t + 1 < T) load_raw(nkb);
+        }
         if (!kInPlace && t + 1 < T) {
 #pragma unroll
             for (int ch = 0; ch < 4; ++ch) load_x(nkb, ch, NX - 1);
@@ -766,14 +830,14 @@ gemv_packed_kernel(const GemvPackedParams p) {
                 mma_s8(P[nt], wa.x, wb.x, wa.y, wb.y, x[0][ch][nt].x, x[0][ch][nt].y);
                 mma_s8(Q[nt], wa.z, wb.z, wa.w, wb.w, x[0][ch][nt].z, x[0][ch][nt].w);
             }
-            if (kInPlace) load_x(nkb, ch, 0);  // (after the range's last block: a block of the same rows, read for nothing)
+            if (kInPlace && !QUANT) load_x(nkb, ch, 0);  // (after the range's last block: a block of the same rows, read for nothing)
             if (GM == 64) {
                 promote(rt, ub * 4 + ch, sa[ch % GPU], sb[ch % GPU], xs[0][ch % GPU]);
-                if (kInPlace) load_xs(nub, ch % GPU, 0);
+                if (kInPlace && !QUANT) load_xs(nub, ch % GPU, 0);
             }
             if (GM == 128 && (ch & 1)) {
                 promote(rt, ub * 2 + (ch >> 1), sa[(ch >> 1) % GPU], sb[(ch >> 1) % GPU], xs[0][(ch >> 1) % GPU]);
-                if (kInPlace) load_xs(nub, (ch >> 1) % GPU, 0);
+                if (kInPlace && !QUANT) load_xs(nub, (ch >> 1) % GPU, 0);
             }
         }
         // The block's bytes are in registers: the slot may be refilled.
@@ -792,7 +856,7 @@ gemv_packed_kernel(const GemvPackedParams p) {
             si = 0;
             if (GM == 256) {
                 promote(rt, ub, sa[0], sb[0], xs[0][0]);
-                if (kInPlace) load_xs(nub, 0, 0);
+                if (kInPlace && !QUANT) load_xs(nub, 0, 0);
             }
             // one call site for the tile end: the row tile is complete, or the range ends inside it
             ++ub;
@@ -922,7 +986,7 @@ size_t fused_smem_bytes(int K, int G) {  // norm weight + padded code rows + sca
 }
 
 bool make_plan(const LinearArgs& a, Plan& pl) {
-    const bool fused = a.norm_weight != nullptr;
+    const bool fused = a.norm_weight != nullptr, quant = !fused && a.X && !a.Xq;
     if (a.M < 1 || a.M > 32 || !a.packed) return false;
     if (!packable(a.N, a.K, a.g)) return false;
     if (fused) {
@@ -934,6 +998,9 @@ bool make_plan(const LinearArgs& a, Plan& pl) {
              reinterpret_cast<uintptr_t>(a.codes_out)) & 15u)
             return false;
         if (a.norm_residual && a.norm_x_out == a.X) return false;  // other CTAs still read X
+    } else if (quant) {
+        if (a.M > 8 || !(a.g == 64 || a.g == 128 || a.g == 256) || a.dump || a.smooth_inv || a.act_scale) return false;
+        if (a.tail_kind != kTailNone || a.tp.world > 0 || (reinterpret_cast<uintptr_t>(a.X) & 15u)) return false;
     } else {
         if (!a.Xq || !a.Xs) return false;
         if (reinterpret_cast<uintptr_t>(a.Xq) & 15u) return false;
@@ -962,7 +1029,7 @@ bool make_plan(const LinearArgs& a, Plan& pl) {
             if ((reinterpret_cast<uintptr_t>(a.Y) | reinterpret_cast<uintptr_t>(a.tail_Xq)) & 15u) return false;
         }
     }
-    pl.pro = fused ? kProNorm : kProCodes;
+    pl.pro = fused ? kProNorm : quant ? kProQuant : kProCodes;
     pl.stages = fused ? 2 : 3;
     pl.MT = a.M <= 8 ? 1 : (a.M <= 16 ? 2 : 4);
     pl.GM = a.g == 64 ? 64 : a.g == 128 ? 128 : 256;
@@ -1023,6 +1090,7 @@ int launch_pro(const LinearArgs& a, const Plan& pl, int* status, cudaStream_t s)
             if (a.K <= 2560) return launch_variant<1, GM, kProNorm, 2, 10, false>(a, pl, status, s);
             return launch_variant<1, GM, kProNorm, 2, 16, false>(a, pl, status, s);
         }
+        if (pl.pro == kProQuant) return launch_variant<1, GM, kProQuant, 3, 1, false>(a, pl, status, s);
     }
     if (a.dump || a.tail_kind != kTailNone) return launch_variant<MT, GM, kProCodes, 3, 1, true>(a, pl, status, s);
     return launch_variant<MT, GM, kProCodes, 3, 1, false>(a, pl, status, s);
@@ -1091,6 +1159,14 @@ int launch_pack_weight(const int8_t* W, const __half* S, int N, int K, int g, vo
     pack_weight_kernel<<<static_cast<unsigned>((total16 + 255) / 256), 256, 0, s>>>(
         W, S, N, K, g, num_groups(K, g), block_bytes, static_cast<unsigned char*>(out), total16);
     return check_launch("pack_weight_kernel");
+}
+
+// At most two blocks per warp: there the fused quantiser costs what the launch it replaces costs in a replayed graph (4097 x
+// 2560 at M = 8: 4.66 against 4.72 us) and saves that launch on the host (eager: 7.2 -> 5 us a call). With longer runs every
+// block is quantised by every row tile's warps again: 2560 x 9728 at M = 8 8.0 -> 9.5 us.
+bool quant_form_wins(const LinearArgs& a) {
+    const int tiles = (a.N + 15) / 16, ctas = gemv_packed_ctas(tiles, num_sms(), true);
+    return static_cast<long long>(tiles) * (a.K / 256) <= 2ll * kWarps * ctas;
 }
 
 bool gemv_packed_supports(const LinearArgs& a) {

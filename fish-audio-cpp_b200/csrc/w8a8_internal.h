@@ -114,6 +114,7 @@ size_t packed_weight_bytes(int N, int K, int g);
 int launch_pack_weight(const int8_t* W, const __half* S, int N, int K, int g, void* out, cudaStream_t s);
 int gemv_packed_ctas(int tiles, int sms, bool two_per_sm);  // CTAs that share a linear's row tiles
 bool gemv_packed_supports(const LinearArgs& a);  // also answers for the prologue and tail forms (fields of a set)
+bool quant_form_wins(const LinearArgs& a);       // whether fp16 rows (X set, Xq null) should be quantised inside the linear
 int launch_linear_gemv_packed(const LinearArgs& a, int* device_status, cudaStream_t s);
 // w8a8_attn.cu : decode-step neighbours (qk-norm + RoPE + KV write; paged attention).
 int launch_qknorm_rope_kvwrite(const __half* qkv, const __half* q_norm_w, const __half* k_norm_w, float eps,

@@ -707,6 +707,37 @@ def test_packed_linear_many_weights_back_to_back(ctx, oracle, pkg, M, g):
             ctx.register_packed_weight(W, None)
 
 
+@pytest.mark.parametrize("g", [64, 128, 256])
+@pytest.mark.parametrize("M,N,K", [(1, 16, 256), (3, 4097, 2560), (8, 40, 4096), (8, 4736, 4096), (5, 2360, 512), (7, 264, 768)])
+def test_packed_linear_quantises_in_registers(ctx, oracle, pkg, M, N, K, g):
+    """The decode linear that quantises fp16 rows itself (at most two blocks per warp): one unit in all, runs of one and two
+    blocks, token counts that leave quads without a token, a group of zeros. Codes and sums are the two-launch form's (whose
+    sums the dump checks), added in the same order: bit for bit the same outputs, and the oracle's within the bars."""
+    X, W, ws = synth.linear_case(M + N + K + g, M, N, K, g)
+    X[0, :g] = 0
+    dW, dS, dX = dev(W), dev(ws), dev(X)
+    P = torch.empty((ctx.packed_weight_bytes(N, K, g),), dtype=torch.uint8, device="cuda")
+    ctx.pack_weight(dW, dS, N, K, g, P)
+    ctx.register_packed_weight(dW, P, N, K, g)
+    try:
+        buf, dY = guarded((M, N), torch.float16, 21.0)
+        ctx.linear(dW, dS, g, dX, dY, M, N, K)
+        dq = torch.empty((M, K), dtype=torch.int8, device="cuda")
+        ds = torch.empty((M, K // g), dtype=torch.float32, device="cuda")
+        dZ = torch.empty((M, N), dtype=torch.float16, device="cuda")
+        ctx.quantize(dX, M, K, g, dq, ds)
+        ctx.linear_q(dW, dS, g, dq, ds, dZ, M, N, K)
+        torch.cuda.synchronize()
+        ctx.check_device_status()
+        assert guards_intact(buf, 21.0)
+        assert torch.equal(dY.view(torch.int16), dZ.view(torch.int16))
+        Xq, Xs = oracle.quantize(X, g)
+        assert_close_fp16(oracle, dY.cpu().numpy(), oracle.linear_q(W, ws, Xq, Xs, g), "quantised in registers",
+                          abs_terms=abs_term_sum(oracle.group_sums(W, Xq, g), ws, Xs))
+    finally:
+        ctx.register_packed_weight(dW, None)
+
+
 @pytest.mark.parametrize("split_k", [1, 2, 3, 4, 5, 8])
 def test_gemv_split_k_is_deterministic_and_correct(ctx, oracle, pkg, split_k):
     M, N, K, g = 16, 320, 2560, 256
