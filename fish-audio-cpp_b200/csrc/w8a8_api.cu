@@ -13,8 +13,6 @@ struct w8a8_ctx {
     unsigned char* workspace = nullptr;
     size_t workspace_bytes = 0;
     int* device_status = nullptr;  // set by kernels whose bounded waits run out
-    void* splitk_partials = nullptr;  // per-warp fp32 partial tiles of the stream-K GEMV
-    int* splitk_counters = nullptr;   // one arrival counter per 16-row tile, zero between launches
     // raw weight pointer -> its packed image; filled by the loader (w8a8_register_packed_weight), the
     // same pointer-keyed lookup as DualAREngine::weight_quant_meta_ (src/engine/dual_ar_engine.h:105)
     struct PackedEntry {
@@ -26,9 +24,6 @@ struct w8a8_ctx {
     int* tail_counters = nullptr;     // arrival counters of the decode kernel's tails, zero between launches
     w8a8::TpState* tp = nullptr;  // tensor-parallel exchange, when w8a8_tp_create was called
 };
-
-static constexpr size_t kSplitkPartialBytes = size_t(16) << 20;
-static constexpr size_t kSplitkCounters = size_t(1) << 18;
 
 namespace w8a8 {
 
@@ -112,23 +107,19 @@ int dispatch_linear_q(const LinearArgs& a, int kernel, int* device_status, cudaS
         case W8A8_KERNEL_GEMM: return launch_linear_gemm(a, device_status, s);
         case W8A8_KERNEL_GEMM_SINGLE: return launch_linear_gemm(a, device_status, s, 0);
         case W8A8_KERNEL_GEMM_PAIR: return launch_linear_gemm(a, device_status, s, 1);
-        case W8A8_KERNEL_GEMV_TMA: return launch_linear_gemv_tma(a, device_status, s);
+        case W8A8_KERNEL_GEMV_TMA: return launch_linear_gemv_rows(a, device_status, s);
         case W8A8_KERNEL_GEMV_PACKED: return launch_linear_gemv_packed(a, device_status, s);
         default: break;
     }
     if (a.M <= 32 && gemv_packed_supports(a)) return launch_linear_gemv_packed(a, device_status, s);
-    if (a.M <= 32 && gemv_tma_supports(a)) return launch_linear_gemv_tma(a, device_status, s);
+    if (a.M <= 32 && gemv_rows_supports(a)) return launch_linear_gemv_rows(a, device_status, s);
     if (a.M <= 32 && gemv_supports(a)) return launch_linear_gemv(a, s);
     if (gemm_supports(a)) return launch_linear_gemm(a, device_status, s);
     return launch_linear_generic(a, s);
 }
 
-// Points the arguments at the context's split-K scratch and at the packed image of the weight, if registered.
+// Points the arguments at the context's tail counters and at the packed image of the weight, if registered.
 static void fill_scratch(w8a8_ctx* ctx, LinearArgs& a) {
-    a.splitk_partials = ctx->splitk_partials;
-    a.splitk_partial_bytes = kSplitkPartialBytes;
-    a.splitk_counters = ctx->splitk_counters;
-    a.splitk_counter_count = kSplitkCounters;
     a.tail_counters = ctx->tail_counters;
     if (a.M <= 32 && !ctx->packed.empty()) {
         std::lock_guard<std::mutex> lock(ctx->packed_mu);
@@ -194,17 +185,12 @@ int w8a8_create(w8a8_ctx** out, int device, size_t workspace_bytes) {
     e = cudaMalloc(&c->workspace, c->workspace_bytes);
     if (e == cudaSuccess) e = cudaMalloc(&c->device_status, sizeof(int));
     if (e == cudaSuccess) e = cudaMemset(c->device_status, 0, sizeof(int));
-    if (e == cudaSuccess) e = cudaMalloc(&c->splitk_partials, kSplitkPartialBytes);
-    if (e == cudaSuccess) e = cudaMalloc(&c->splitk_counters, kSplitkCounters * sizeof(int));
-    if (e == cudaSuccess) e = cudaMemset(c->splitk_counters, 0, kSplitkCounters * sizeof(int));
     if (e == cudaSuccess) e = cudaMalloc(&c->tail_counters, kTailCounterInts * sizeof(int));
     if (e == cudaSuccess) e = cudaMemset(c->tail_counters, 0, kTailCounterInts * sizeof(int));
     cudaSetDevice(prev);
     if (e != cudaSuccess) {
         cudaFree(c->workspace);
         cudaFree(c->device_status);
-        cudaFree(c->splitk_partials);
-        cudaFree(c->splitk_counters);
         cudaFree(c->tail_counters);
         delete c;
         return fail(W8A8_ERR_CUDA, "context allocation: %s", cudaGetErrorString(e));
@@ -217,8 +203,6 @@ int w8a8_destroy(w8a8_ctx* ctx) {
     if (!ctx) return W8A8_OK;
     cudaFree(ctx->workspace);
     cudaFree(ctx->device_status);
-    cudaFree(ctx->splitk_partials);
-    cudaFree(ctx->splitk_counters);
     cudaFree(ctx->tail_counters);
     tp_destroy(ctx->tp);
     delete ctx;
@@ -436,7 +420,10 @@ int w8a8_linear(w8a8_ctx* ctx, const void* W, const void* w_scale, int group_siz
         LinearArgs f = a;
         f.X = static_cast<const __half*>(X);
         fill_scratch(ctx, f);
-        if (f.packed && quant_form_wins(f) && gemv_packed_supports(f)) return launch_linear_gemv_packed(f, ctx->device_status, s);
+        if (quant_form_wins(f)) {
+            if (gemv_packed_supports(f)) return launch_linear_gemv_packed(f, ctx->device_status, s);
+            if (kernel == W8A8_KERNEL_AUTO && gemv_rows_supports(f)) return launch_linear_gemv_rows(f, ctx->device_status, s);
+        }
     }
 
     // Codes and scales into the context's scratch (row kernel), then the integer kernel; the two are
@@ -517,8 +504,7 @@ size_t w8a8_decode_stack_workspace_bytes(const w8a8_decode_stack* stack) {
 
 int w8a8_decode_stack_step(w8a8_ctx* ctx, const w8a8_decode_stack* stack, void* stream) {
     if (!ctx || !stack) return fail(W8A8_ERR_INVALID_ARG, "null context or stack descriptor");
-    return launch_decode_stack(*stack, ctx->workspace, ctx->workspace_bytes, static_cast<float*>(ctx->splitk_partials),
-                               kSplitkPartialBytes, ctx->splitk_counters, kSplitkCounters, ctx->device_status,
+    return launch_decode_stack(*stack, ctx->workspace, ctx->workspace_bytes, ctx->device_status,
                                static_cast<cudaStream_t>(stream));
 }
 

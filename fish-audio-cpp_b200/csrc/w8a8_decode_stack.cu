@@ -1027,8 +1027,7 @@ int decode_stack_timeline(const w8a8_decode_stack& d, const unsigned char* works
     return n;
 }
 
-int launch_decode_stack(const w8a8_decode_stack& d, unsigned char* workspace, size_t workspace_bytes, float* partials,
-                        size_t partial_bytes, int* counters, size_t counter_count, int* status, cudaStream_t stream) {
+int launch_decode_stack(const w8a8_decode_stack& d, unsigned char* workspace, size_t workspace_bytes, int* status, cudaStream_t stream) {
     if (const char* why = check(d)) return fail(W8A8_ERR_UNSUPPORTED, "decode stack: %s", why);
     const int sms = num_sms();
     StackParams p = {};
@@ -1062,7 +1061,6 @@ int launch_decode_stack(const w8a8_decode_stack& d, unsigned char* workspace, si
     p.barrier = reinterpret_cast<unsigned*>(workspace + sc.barrier);
     p.timeline = reinterpret_cast<unsigned long long*>(workspace + sc.timeline);
     p.status = status;
-    (void)partials; (void)partial_bytes; (void)counters; (void)counter_count;  // the step adds cut tiles in shared memory
     const int Ns[4] = {(d.n_q_heads + 2 * d.n_kv_heads) * kHeadDim, d.dim, 2 * d.inter, d.dim};
     const int Ks[4] = {d.dim, d.n_q_heads * kHeadDim, d.dim, d.inter};
     const unsigned warps = static_cast<unsigned>(sms) * kWarps;

@@ -55,11 +55,6 @@ struct LinearArgs {
     int epilogue;
     int split_k;
     const void* packed;     // the weight re-packed by launch_pack_weight (null: not packed)
-    // scratch for kernels that cut K across CTAs (owned by the context; null: such kernels are not used)
-    void* splitk_partials;
-    size_t splitk_partial_bytes;
-    int* splitk_counters;        // zero between launches
-    size_t splitk_counter_count;
     // Fused prologue (packed GEMV, M <= 8): norm_weight != null means that Xq / Xs are absent and every CTA
     // forms them itself in shared memory from X: [x = half(x + norm_residual)] -> RMSNorm -> quantiser.
     const __half* norm_weight;    // [K]
@@ -106,9 +101,9 @@ int launch_linear_generic(const LinearArgs& a, cudaStream_t s);
 // w8a8_gemv.cu : M <= 32.
 bool gemv_supports(const LinearArgs& a);
 int launch_linear_gemv(const LinearArgs& a, cudaStream_t s);
-// w8a8_gemv_tma.cu : M <= 32, TMA-fed persistent stream-K form.
-bool gemv_tma_supports(const LinearArgs& a);
-int launch_linear_gemv_tma(const LinearArgs& a, int* device_status, cudaStream_t s);
+// w8a8_gemv_rows.cu : M <= 32 over the row-major matrix, TMA-fed (also answers for fp16 rows: X set, Xq null).
+bool gemv_rows_supports(const LinearArgs& a);
+int launch_linear_gemv_rows(const LinearArgs& a, int* device_status, cudaStream_t s);
 // w8a8_gemv_packed.cu : M <= 32 over pre-packed weights (linear byte stream, 1-D bulk copies).
 size_t packed_weight_bytes(int N, int K, int g);
 int launch_pack_weight(const int8_t* W, const __half* S, int N, int K, int g, void* out, cudaStream_t s);
@@ -132,8 +127,7 @@ int launch_qkv_attention_decode(const __half* qkv, const __half* q_norm_w, const
                                 int splits, int* status, cudaStream_t stream);
 // w8a8_decode_stack.cu : a whole decode step as one persistent cooperative kernel.
 size_t decode_stack_workspace_bytes(const w8a8_decode_stack& d);
-int launch_decode_stack(const w8a8_decode_stack& d, unsigned char* workspace, size_t workspace_bytes, float* partials,
-                        size_t partial_bytes, int* counters, size_t counter_count, int* status, cudaStream_t stream);
+int launch_decode_stack(const w8a8_decode_stack& d, unsigned char* workspace, size_t workspace_bytes, int* status, cudaStream_t stream);
 int decode_stack_timeline(const w8a8_decode_stack& d, const unsigned char* workspace, unsigned long long* out, int capacity,
                           cudaStream_t stream);
 // w8a8_tp.cu : one-shot all-reduce over peer memory fused with residual add + RMSNorm + quantiser.

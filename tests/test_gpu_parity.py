@@ -708,17 +708,20 @@ def test_packed_linear_many_weights_back_to_back(ctx, oracle, pkg, M, g):
 
 
 @pytest.mark.parametrize("g", [64, 128, 256])
+@pytest.mark.parametrize("packed", [True, False])
 @pytest.mark.parametrize("M,N,K", [(1, 16, 256), (3, 4097, 2560), (8, 40, 4096), (8, 4736, 4096), (5, 2360, 512), (7, 264, 768)])
-def test_packed_linear_quantises_in_registers(ctx, oracle, pkg, M, N, K, g):
-    """The decode linear that quantises fp16 rows itself (at most two blocks per warp): one unit in all, runs of one and two
-    blocks, token counts that leave quads without a token, a group of zeros. Codes and sums are the two-launch form's (whose
-    sums the dump checks), added in the same order: bit for bit the same outputs, and the oracle's within the bars."""
+def test_decode_linear_quantises_in_registers(ctx, oracle, pkg, M, N, K, g, packed):
+    """The decode linear that quantises fp16 rows itself (short runs of blocks per warp), over packed and over row-major weights:
+    one unit in all, runs of one to three blocks, token counts that leave quads without a token, rows past N in the last
+    tile, a group of zeros. Codes and sums are the two-launch form's (whose sums the dump checks), added in the same order:
+    bit for bit the same outputs, and the oracle's within the bars."""
     X, W, ws = synth.linear_case(M + N + K + g, M, N, K, g)
     X[0, :g] = 0
     dW, dS, dX = dev(W), dev(ws), dev(X)
-    P = torch.empty((ctx.packed_weight_bytes(N, K, g),), dtype=torch.uint8, device="cuda")
-    ctx.pack_weight(dW, dS, N, K, g, P)
-    ctx.register_packed_weight(dW, P, N, K, g)
+    if packed:
+        P = torch.empty((ctx.packed_weight_bytes(N, K, g),), dtype=torch.uint8, device="cuda")
+        ctx.pack_weight(dW, dS, N, K, g, P)
+        ctx.register_packed_weight(dW, P, N, K, g)
     try:
         buf, dY = guarded((M, N), torch.float16, 21.0)
         ctx.linear(dW, dS, g, dX, dY, M, N, K)
@@ -735,7 +738,8 @@ def test_packed_linear_quantises_in_registers(ctx, oracle, pkg, M, N, K, g):
         assert_close_fp16(oracle, dY.cpu().numpy(), oracle.linear_q(W, ws, Xq, Xs, g), "quantised in registers",
                           abs_terms=abs_term_sum(oracle.group_sums(W, Xq, g), ws, Xs))
     finally:
-        ctx.register_packed_weight(dW, None)
+        if packed:
+            ctx.register_packed_weight(dW, None)
 
 
 @pytest.mark.parametrize("split_k", [1, 2, 3, 4, 5, 8])
