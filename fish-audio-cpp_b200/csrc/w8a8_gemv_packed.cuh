@@ -411,20 +411,25 @@ __device__ __forceinline__ void gemv_body(const GemvPackedParams& p, const CUten
     const unsigned char* src = ROWS ? nullptr : p.packed + static_cast<size_t>(u0) * p.bpu * p.block_bytes;
     int pkb = 0, prt = 0;  // ROWS: the next box's 128-byte K block and row tile
     if constexpr (ROWS) { prt = static_cast<int>(u0 / p.upt); pkb = static_cast<int>(u0 % p.upt) * p.bpu * 2; }
+    // Weights are read once per launch and a stack's do not fit in L2: as evict-first lines they do not push out the activations,
+    // scales and cache rows that the next launches read, nor wait behind their write-back (decode step, batch 8: 1517 -> 1488 us;
+    // ten fast-AR steps 1710 -> 1666). Marking a quarter of them evict-last, to find it again at the next step: 1502 and 1687.
+    unsigned long long once;
+    asm volatile("createpolicy.fractional.L2::evict_first.b64 %0, 1.0;" : "=l"(once));
     auto issue = [&]() {  // lane 0 only
         const int slot = pt % kStages;
         if constexpr (ROWS) {
             ptx::mbar_arrive_expect_tx(&bar[slot], kBlockW);
             asm volatile(
-                "cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5}], [%2];"
-                ::"r"(ring + slot * kPitch), "l"(map), "r"(ptx::smem_u32(&bar[slot])), "r"(0), "r"(pkb), "r"(prt * 16)
+                "cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes.L2::cache_hint [%0], [%1, {%3, %4, %5}], [%2], %6;"
+                ::"r"(ring + slot * kPitch), "l"(map), "r"(ptx::smem_u32(&bar[slot])), "r"(0), "r"(pkb), "r"(prt * 16), "l"(once)
                 : "memory");
             pkb += 2;
             if (pkb == p.upt * p.bpu * 2) { pkb = 0; ++prt; }
         } else {
             ptx::mbar_arrive_expect_tx(&bar[slot], p.block_bytes);
-            asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
-                         ::"r"(ring + slot * kPitch), "l"(src), "r"(p.block_bytes), "r"(ptx::smem_u32(&bar[slot]))
+            asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes.L2::cache_hint [%0], [%1], %2, [%3], %4;"
+                         ::"r"(ring + slot * kPitch), "l"(src), "r"(p.block_bytes), "r"(ptx::smem_u32(&bar[slot])), "l"(once)
                          : "memory");
             src += p.block_bytes;
         }
