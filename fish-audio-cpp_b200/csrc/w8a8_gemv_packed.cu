@@ -164,7 +164,7 @@ int launch_pro(const LinearArgs& a, const Plan& pl, int* status, cudaStream_t s)
         }
         if (pl.pro == kProQuant) return launch_variant<1, GM, kProQuant, 3, 1, false>(a, pl, status, s);
     }
-    if (a.dump || a.tail_kind != kTailNone) return launch_variant<MT, GM, kProCodes, 3, 1, true>(a, pl, status, s);
+    if (a.dump || a.tail_kind != kTailNone || a.tp.world > 0) return launch_variant<MT, GM, kProCodes, 3, 1, true>(a, pl, status, s);
     return launch_variant<MT, GM, kProCodes, 3, 1, false>(a, pl, status, s);
 }
 

@@ -332,13 +332,14 @@ __device__ __forceinline__ void tail_group_quant(const LinearArgs& a, int ct0, i
 // it again, some 300 instructions per block, so the form is chosen where a CTA has few row tiles (see quant_form_wins).
 // ST: stages of a warp's ring (3; 2 for kProNorm so that two CTAs fit an SM beside the code rows).
 // KI: kProNorm only, the 16-byte pieces of a row a lane holds (K <= 256 * KI): 10 for the stack's K = 2560, else 16.
-// EXTRA: the call wants the group sums dumped or has a tail. An instance of its own: the check per promote alone cost 0.1-1.1 us
-// per launch.
+// EXTRA: the call wants the group sums dumped, has a tail or sends to a tensor-parallel exchange. An instance of its own: the check
+// per promote alone cost 0.1-1.1 us per launch, and the exchange's stores were half of a decode launch's code, which runs cold.
 // ROWS: the weights are the row-major matrix itself. A block is then a TMA box of 16 rows x two 128-byte K blocks (128-byte
 // swizzle), its scales come from the matrix's own scale array a unit ahead, and everything else is the same.
 template <int MT, int GM, int PRO, int ST, int KI, bool EXTRA, bool ROWS>
 __device__ __forceinline__ void gemv_body(const GemvPackedParams& p, const CUtensorMap* map) {
     constexpr bool FUSED = PRO == kProNorm, QUANT = PRO == kProQuant;
+    constexpr bool TP = EXTRA || FUSED;  // instances that can send to a tensor-parallel exchange
     constexpr int kStages = ST;
     constexpr int kPitch = ROWS ? kBlockW : kStagePitch;
     constexpr int kRingBytes = kStages * kPitch;
@@ -483,7 +484,7 @@ __device__ __forceinline__ void gemv_body(const GemvPackedParams& p, const CUten
     W8A8_STAMP(1);
     // tensor-parallel send: this exchange's epoch = the last finished one + 1 (advanced by the receive kernel)
     int tp_ep = 0;
-    if (a.tp.world > 0)
+    if (TP && a.tp.world > 0)
         tp_ep = *reinterpret_cast<const volatile int*>(a.tp.peers[a.tp.rank] + a.tp.ctl_off) + 1;
 
     const int8_t* xq[MT];
@@ -685,7 +686,7 @@ __device__ __forceinline__ void gemv_body(const GemvPackedParams& p, const CUten
                         const int row = rA + 8 * hrow;
                         if (row >= a.N) continue;
                         const size_t o = static_cast<size_t>(tok) * a.N + row;
-                        if (a.tp.world > 0) {
+                        if (TP && a.tp.world > 0) {
                             // the fp32 partial as a self-validating word {value, epoch} into slot [rank] of every rank
                             const size_t word = (static_cast<size_t>((tp_ep & 1) * a.tp.world + a.tp.rank) * a.tp.max_tokens + tok) *
                                                     a.N + row;
@@ -984,7 +985,7 @@ __device__ __forceinline__ void gemv_body(const GemvPackedParams& p, const CUten
         for (int row = rA; row <= rA + 8 && row < a.N; row += 8) {
             const size_t o = static_cast<size_t>(tok) * a.N + row;
             const float val = row == rA ? v[0] : v[1];
-            if (a.tp.world > 0) {
+            if (TP && a.tp.world > 0) {
                 const size_t word = (static_cast<size_t>((tp_ep & 1) * a.tp.world + a.tp.rank) * a.tp.max_tokens + tok) * a.N + row;
                 const uint2 wd = make_uint2(__float_as_uint(val), static_cast<unsigned>(tp_ep));
                 for (int r = 0; r < a.tp.world; ++r) reinterpret_cast<uint2*>(a.tp.peers[r])[word] = wd;
