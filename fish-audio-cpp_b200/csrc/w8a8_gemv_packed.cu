@@ -122,17 +122,17 @@ void gemv::fill_params(const LinearArgs& a, const Plan& pl, int* status, GemvPac
 
 namespace {
 
-template <int MT, int GM, int PRO, int ST, int KI, bool EXTRA>
+template <int MT, int GM, int PRO, int ST, int KI, int EPI, bool EXTRA>
 __global__ void __launch_bounds__(kThreads, two_per_sm(MT, GM) ? 2 : 1)
 gemv_packed_kernel(const __grid_constant__ GemvPackedParams p) {
-    gemv_body<MT, GM, PRO, ST, KI, EXTRA, false>(p, nullptr);
+    gemv_body<MT, GM, PRO, ST, KI, EPI, EXTRA, false>(p, nullptr);
 }
 
-template <int MT, int GM, int PRO, int ST, int KI, bool EXTRA>
+template <int MT, int GM, int PRO, int ST, int KI, int EPI, bool EXTRA>
 int launch_variant(const LinearArgs& a, const Plan& pl, int* status, cudaStream_t stream) {
     GemvPackedParams p;
     fill_params(a, pl, status, p);
-    auto kern = gemv_packed_kernel<MT, GM, PRO, ST, KI, EXTRA>;
+    auto kern = gemv_packed_kernel<MT, GM, PRO, ST, KI, EPI, EXTRA>;
     const size_t ring = static_cast<size_t>(kWarps) * ST * kStagePitch + 128;
     const size_t smem = ring + (PRO == kProNorm ? fused_smem_bytes(a.K, a.G) : 0);
     {  // per device, so on every launch (a host-side table write)
@@ -159,13 +159,17 @@ template <int MT, int GM>
 int launch_pro(const LinearArgs& a, const Plan& pl, int* status, cudaStream_t s) {
     if constexpr (MT == 1) {
         if (pl.pro == kProNorm) {
-            if (a.K <= 2560) return launch_variant<1, GM, kProNorm, 2, 10, false>(a, pl, status, s);
-            return launch_variant<1, GM, kProNorm, 2, 16, false>(a, pl, status, s);
+            if (a.K <= 2560) return launch_variant<1, GM, kProNorm, 2, 10, -1, false>(a, pl, status, s);
+            return launch_variant<1, GM, kProNorm, 2, 16, -1, false>(a, pl, status, s);
         }
-        if (pl.pro == kProQuant) return launch_variant<1, GM, kProQuant, 3, 1, false>(a, pl, status, s);
+        if (pl.pro == kProQuant) return launch_variant<1, GM, kProQuant, 3, 1, -1, false>(a, pl, status, s);
     }
-    if (a.dump || a.tail_kind != kTailNone || a.tp.world > 0) return launch_variant<MT, GM, kProCodes, 3, 1, true>(a, pl, status, s);
-    return launch_variant<MT, GM, kProCodes, 3, 1, false>(a, pl, status, s);
+    if (a.dump || a.tail_kind != kTailNone || a.tp.world > 0) return launch_variant<MT, GM, kProCodes, 3, 1, -1, true>(a, pl, status, s);
+    switch (a.epilogue) {
+        case W8A8_EPI_NONE: return launch_variant<MT, GM, kProCodes, 3, 1, W8A8_EPI_NONE, false>(a, pl, status, s);
+        case W8A8_EPI_SWIGLU: return launch_variant<MT, GM, kProCodes, 3, 1, W8A8_EPI_SWIGLU, false>(a, pl, status, s);
+        default: return launch_variant<MT, GM, kProCodes, 3, 1, W8A8_EPI_RESIDUAL, false>(a, pl, status, s);
+    }
 }
 
 template <int MT>

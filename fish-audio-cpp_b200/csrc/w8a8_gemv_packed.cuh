@@ -334,11 +334,13 @@ __device__ __forceinline__ void tail_group_quant(const LinearArgs& a, int ct0, i
 // KI: kProNorm only, the 16-byte pieces of a row a lane holds (K <= 256 * KI): 10 for the stack's K = 2560, else 16.
 // EXTRA: the call wants the group sums dumped, has a tail or sends to a tensor-parallel exchange. An instance of its own: the check
 // per promote alone cost 0.1-1.1 us per launch, and the exchange's stores were half of a decode launch's code, which runs cold.
+// EPI: the epilogue, or -1: the call's (one of three code paths is fetched past).
 // ROWS: the weights are the row-major matrix itself. A block is then a TMA box of 16 rows x two 128-byte K blocks (128-byte
 // swizzle), its scales come from the matrix's own scale array a unit ahead, and everything else is the same.
-template <int MT, int GM, int PRO, int ST, int KI, bool EXTRA, bool ROWS>
+template <int MT, int GM, int PRO, int ST, int KI, int EPI, bool EXTRA, bool ROWS>
 __device__ __forceinline__ void gemv_body(const GemvPackedParams& p, const CUtensorMap* map) {
     constexpr bool FUSED = PRO == kProNorm, QUANT = PRO == kProQuant;
+    const int epilogue = EPI >= 0 ? EPI : p.a.epilogue;
     constexpr bool TP = EXTRA || FUSED;  // instances that can send to a tensor-parallel exchange
     constexpr int kStages = ST;
     constexpr int kPitch = ROWS ? kBlockW : kStagePitch;
@@ -673,7 +675,7 @@ __device__ __forceinline__ void gemv_body(const GemvPackedParams& p, const CUten
             for (int e = 0; e < 2; ++e) {
                 const int tok = nt * 8 + 2 * c + e;
                 if (tok >= a.M) continue;
-                if (a.epilogue == W8A8_EPI_SWIGLU) {
+                if (epilogue == W8A8_EPI_SWIGLU) {
                     if (rA + 8 < a.N) {
                         const float g16 = __half2float(__float2half(v[nt][e]));
                         const __half s16 = __float2half(g16 / (1.0f + expf(-g16)));
@@ -695,7 +697,7 @@ __device__ __forceinline__ void gemv_body(const GemvPackedParams& p, const CUten
                         }
                         if (!a.Y || W8A8_ABLATED(4)) continue;
                         __half y = __float2half(v[nt][2 * hrow + e]);
-                        if (a.epilogue == W8A8_EPI_RESIDUAL)
+                        if (epilogue == W8A8_EPI_RESIDUAL)
                             y = __float2half(__half2float(y) + __half2float(a.residual[o]));
                         a.Y[o] = y;
                     }
@@ -965,6 +967,7 @@ __device__ __forceinline__ void gemv_body(const GemvPackedParams& p, const CUten
         const int f = i % (MT * 64), nt = f >> 6, e = (f >> 5) & 1, fl = f & 31, last = cut_s[w][2];
         const float* src = (cut_s[w][1] ? slot1(w) : red_s[w]) + (nt * 4 + e) * 32 + fl;
         float v[2] = {0.0f + src[0], 0.0f + src[64]};
+#pragma unroll 1
         for (int ww = w + 1; ww <= last; ++ww) {
             const float* more = red_s[ww] + (nt * 4 + e) * 32 + fl;
             v[0] += more[0];
@@ -972,7 +975,7 @@ __device__ __forceinline__ void gemv_body(const GemvPackedParams& p, const CUten
         }
         const int tok = nt * 8 + 2 * (fl & 3) + e, rA = rt_cut * 16 + row_of(fl >> 2);
         if (tok >= a.M) continue;
-        if (a.epilogue == W8A8_EPI_SWIGLU) {
+        if (epilogue == W8A8_EPI_SWIGLU) {
             if (rA + 8 < a.N) {
                 const float g16 = __half2float(__float2half(v[0]));
                 const __half s16 = __float2half(g16 / (1.0f + expf(-g16)));
@@ -992,7 +995,7 @@ __device__ __forceinline__ void gemv_body(const GemvPackedParams& p, const CUten
             }
             if (!a.Y || W8A8_ABLATED(4)) continue;
             __half y = __float2half(val);
-            if (a.epilogue == W8A8_EPI_RESIDUAL) y = __float2half(__half2float(y) + __half2float(a.residual[o]));
+            if (epilogue == W8A8_EPI_RESIDUAL) y = __float2half(__half2float(y) + __half2float(a.residual[o]));
             a.Y[o] = y;
         }
     }

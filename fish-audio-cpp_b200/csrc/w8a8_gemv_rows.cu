@@ -12,7 +12,7 @@ using namespace gemv;
 template <int MT, int GM, int PRO, bool EXTRA>
 __global__ void __launch_bounds__(kThreads, two_per_sm(MT, GM) ? 2 : 1)
 gemv_rows_kernel(const __grid_constant__ CUtensorMap map, const __grid_constant__ GemvPackedParams p) {
-    gemv_body<MT, GM, PRO, 3, 1, EXTRA, true>(p, &map);
+    gemv_body<MT, GM, PRO, 3, 1, -1, EXTRA, true>(p, &map);
 }
 
 template <int MT, int GM, int PRO, bool EXTRA>
