@@ -483,6 +483,7 @@ __global__ void __maxnreg__(128) paged_attention_decode_kernel(const __grid_cons
             }
             // V rows past the sequence's end: their weights are exactly zero, but whatever lies there (it may not be
             // a number) must not meet the multiply. (K rows past the end only feed scores that are replaced below.)
+#pragma unroll 1
             for (int r = tokens; r < kBlockTokens; ++r)
                 asm volatile("st.shared.v2.u32 [%0], {%1,%1};" ::"r"(vs + (lane >> 4) * kBoxBytes + r * 128 + (lane & 15) * 8), "r"(0u)
                              : "memory");
@@ -610,16 +611,18 @@ __global__ void __maxnreg__(128) paged_attention_decode_kernel(const __grid_cons
                 if (lane == 0) amax_s[warp] = amax;
                 consumer_barrier();
                 const int wpg = p.g / 64, w0 = warp & ~(wpg - 1);
+#pragma unroll 1
                 for (int w = 0; w < wpg; ++w) amax = fmaxf(amax, amax_s[w0 + w]);
             }
             float am[2] = {amax, amax};
             if (p.g == 1) { am[0] = fabsf(f.x); am[1] = fabsf(f.y); }
+            const int lg = 31 - __clz(p.g);
             int q[2];
 #pragma unroll
             for (int e = 0; e < 2; ++e) {
                 float scale = am[e] / 127.0f;
                 if (scale < 1e-8f) scale = 1e-8f;
-                if ((ch + e) % p.g == 0) p.Xs[static_cast<size_t>(b) * (K / p.g) + (ch + e) / p.g] = scale;
+                if (((ch + e) & (p.g - 1)) == 0) p.Xs[static_cast<size_t>(b) * (K >> lg) + ((ch + e) >> lg)] = scale;
                 const float inv_scale = 1.0f / scale;
                 q[e] = max(-127, min(127, __float2int_rn((e ? f.y : f.x) * inv_scale)));
             }
@@ -628,6 +631,7 @@ __global__ void __maxnreg__(128) paged_attention_decode_kernel(const __grid_cons
         }
     }
     if (s_fail) {  // a bounded wait ran out: give copies that may still be in flight time to land before the CTA goes
+#pragma unroll 1  // (unrolled copies of the runtime loops were a quarter of the kernel's code, which runs cold)
         for (int i = 0; i < 1000; ++i) __nanosleep(1000);
     }
     ATTN_PHASE(7);
