@@ -164,7 +164,7 @@ int launch_pro(const LinearArgs& a, const Plan& pl, int* status, cudaStream_t s)
         }
         if (pl.pro == kProQuant) return launch_variant<1, GM, kProQuant, 3, 1, -1, false>(a, pl, status, s);
     }
-    if (a.dump || a.tail_kind != kTailNone || a.tp.world > 0) return launch_variant<MT, GM, kProCodes, 3, 1, -1, true>(a, pl, status, s);
+    if (!plain_instance(a)) return launch_variant<MT, GM, kProCodes, 3, 1, -1, true>(a, pl, status, s);
     switch (a.epilogue) {
         case W8A8_EPI_NONE: return launch_variant<MT, GM, kProCodes, 3, 1, W8A8_EPI_NONE, false>(a, pl, status, s);
         case W8A8_EPI_SWIGLU: return launch_variant<MT, GM, kProCodes, 3, 1, W8A8_EPI_SWIGLU, false>(a, pl, status, s);

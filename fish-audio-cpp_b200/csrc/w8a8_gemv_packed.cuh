@@ -786,6 +786,26 @@ __device__ __forceinline__ void gemv_body(const GemvPackedParams& p, const CUten
                 else xs[buf][q][nt][e] = __ldg(xsp[nt][e] + unit_b * GPU + q);
             }
     };
+    // The scales of a unit at once: a word of two or four where the instance may (the host checks the address).
+    constexpr bool kWideXs = GPU > 1 && PRO == kProCodes && !EXTRA && !kInPlace;
+    auto load_xs_unit = [&](int unit_b, int buf) {
+        if constexpr (kWideXs) {
+#pragma unroll
+            for (int nt = 0; nt < MT; ++nt)
+#pragma unroll
+                for (int e = 0; e < 2; ++e) {
+                    const float* s = xsp[nt][e] + unit_b * GPU;
+                    __align__(16) float v[4];
+                    if constexpr (GPU == 4) *reinterpret_cast<float4*>(v) = __ldg(reinterpret_cast<const float4*>(s));
+                    else *reinterpret_cast<float2*>(v) = __ldg(reinterpret_cast<const float2*>(s));
+#pragma unroll
+                    for (int q = 0; q < GPU; ++q) xs[buf][q][nt][e] = v[q];
+                }
+        } else {
+#pragma unroll
+            for (int q = 0; q < GPU; ++q) load_xs(unit_b, q, buf);
+        }
+    };
     // kProQuant: this lane's 64 activations of a block (chunk ch: 16 from ch * 64 + c * 16 on), requested a block ahead
     uint4 raw[QUANT ? 8 : 1];
     auto load_raw = [&](int kbase) {
@@ -844,8 +864,7 @@ __device__ __forceinline__ void gemv_body(const GemvPackedParams& p, const CUten
     } else if (T > 0) {
 #pragma unroll
         for (int ch = 0; ch < 4; ++ch) load_x(ub * p.bpu * 256, ch, 0);
-#pragma unroll
-        for (int q = 0; q < GPU; ++q) load_xs(ub, q, 0);
+        load_xs_unit(ub, 0);
     }
     for (int t = 0; t < T; ++t) {
         const int slot = t % kStages;
@@ -860,10 +879,7 @@ __device__ __forceinline__ void gemv_body(const GemvPackedParams& p, const CUten
         if (!kInPlace && t + 1 < T) {
 #pragma unroll
             for (int ch = 0; ch < 4; ++ch) load_x(nkb, ch, NX - 1);
-            if (nsi == 0) {
-#pragma unroll
-                for (int q = 0; q < GPU; ++q) load_xs(nub, q, NX - 1);
-            }
+            if (nsi == 0) load_xs_unit(nub, NX - 1);
         }
         if (!ptx::mbar_wait_bounded(&bar[slot], (t / kStages) & 1)) {
             if (lane == 0) atomicExch(p.status, 600 + slot);
@@ -1028,6 +1044,10 @@ struct Plan {
     long long U;
 };
 bool make_plan(const LinearArgs& a, Plan& pl, bool rows);
+// The plain instances read the activation scales of a unit as one word; a call whose scales are not aligned for that runs EXTRA.
+inline bool plain_instance(const LinearArgs& a) {
+    return !a.dump && a.tail_kind == kTailNone && a.tp.world == 0 && (reinterpret_cast<uintptr_t>(a.Xs) & (a.g == 64 ? 15u : a.g == 128 ? 7u : 3u)) == 0;
+}
 void fill_params(const LinearArgs& a, const Plan& pl, int* status, GemvPackedParams& p);
 
 }  // namespace gemv

@@ -46,7 +46,7 @@ int launch_variant(const LinearArgs& a, const Plan& pl, int* status, cudaStream_
 template <int GM>
 int launch_gm(const LinearArgs& a, const Plan& pl, int* status, cudaStream_t s) {
     if (pl.pro == kProQuant) return launch_variant<1, GM, kProQuant, false>(a, pl, status, s);
-    if (a.dump)
+    if (!plain_instance(a))
         return pl.MT == 1 ? launch_variant<1, GM, kProCodes, true>(a, pl, status, s)
                : pl.MT == 2 ? launch_variant<2, GM, kProCodes, true>(a, pl, status, s) : launch_variant<4, GM, kProCodes, true>(a, pl, status, s);
     return pl.MT == 1 ? launch_variant<1, GM, kProCodes, false>(a, pl, status, s)
