@@ -42,20 +42,34 @@ int launch_linear_gemm(const LinearArgs& a, int* device_status, cudaStream_t str
     const Form* table = forms(a.dump ? 0 : a.g, &count);
     const Form* best = nullptr;
     double best_ns = 0;
+    int best_splits = 1;
     // The tile form that ends first: whole waves of tiles over the SMs (or pairs), each tile at its measured cost. A width
     // that leaves the last wave nearly empty loses to one that fills it; narrow tiles win where there are few tokens.
-    // (W8A8_GEMM_BT: take this token width, where the form asked for has it.)
+    // A tile's K is split over two or four CTAs where all of them fit the chip at once (a cluster of four leaves some SMs of a
+    // GPC over: 128 of 148 taken as usable); meeting and adding up measured 3-4 us for two and about 6 for four. A
+    // split adds the groups in another order than the other kernels do, so it has to save 15 % at least (K = 2560 never does).
+    // (W8A8_GEMM_BT, W8A8_GEMM_SPLIT: take this token width, this split, where the form asked for has it.)
     const char* env = std::getenv("W8A8_GEMM_BT");
     const int only_bt = env ? std::atoi(env) : 0;
-    for (int pass = only_bt ? 0 : 1; pass < 2 && !best; ++pass)
+    const char* env_split = std::getenv("W8A8_GEMM_SPLIT");
+    const int only_split = env_split ? std::atoi(env_split) : 0;
+    const int unit = a.g > BK ? a.g / BK : 1, kb_total = a.K / BK;  // a split takes whole K-groups
+    auto split_kb = [&](int splits) { return (kb_total / unit + splits - 1) / splits * unit; };
+    for (int pass = only_bt || only_split ? 0 : 1; pass < 2 && !best; ++pass)
         for (int i = 0; i < count; ++i) {
             const Form& f = table[i];
-            if (form >= 0 && f.pair != (form != 0)) continue;
-            if (pass == 0 && f.bt != only_bt) continue;
+            if (form >= 0 && (f.pair != (form != 0) || f.split)) continue;
+            if (pass == 0 && only_bt && f.bt != only_bt) continue;
             const int rows = f.pair ? 2 * BR : BR, walkers = f.pair ? sms / 2 : sms;
             const long tiles = static_cast<long>((a.M + f.bt - 1) / f.bt) * ((a.N + rows - 1) / rows);
-            const double ns = ((tiles + walkers - 1) / walkers) * (a.K / BK * double(f.stage_ns) + a.G * double(f.group_ns));
-            if (!best || ns < best_ns) { best = &f; best_ns = ns; }
+            for (int splits = f.split ? 2 : 1; splits <= (f.split ? 4 : 1); splits *= 2) {
+                if (pass == 0 && only_split && splits != only_split) continue;
+                if (f.split && (tiles * splits > (splits == 2 ? sms / 2 * 2 : sms * 7 / 8 - 1) || (splits - 1) * split_kb(splits) >= kb_total)) continue;
+                const double kb = f.split ? split_kb(splits) : kb_total;
+                double ns = ((tiles * splits + walkers - 1) / walkers) * (kb * f.stage_ns + kb * BK / a.g * f.group_ns);
+                if (f.split) ns = (ns + (splits == 2 ? 3500 : 6000)) / 0.85;
+                if (!best || ns < best_ns) { best = &f; best_ns = ns; best_splits = splits; }
+            }
         }
     if (!best) return fail(W8A8_ERR_UNSUPPORTED, "no tile form of the tcgen05 GEMM");
 
@@ -72,6 +86,8 @@ int launch_linear_gemm(const LinearArgs& a, int* device_status, cudaStream_t str
     p.status = device_status;
     p.tiles_m = (a.M + bt - 1) / bt;
     p.tiles_total = p.tiles_m * ((a.N + rows - 1) / rows);
+    p.splits = best_splits;
+    p.split_kb = split_kb(best_splits);
     p.tma_store = ycols % 8 == 0 && (reinterpret_cast<uintptr_t>(a.Y) & 15u) == 0;
     map_y = map_x;  // (a valid map in either case; only the TMA store reads it)
     if (p.tma_store) {
@@ -101,15 +117,15 @@ int launch_linear_gemm(const LinearArgs& a, int* device_status, cudaStream_t str
     // share weight tiles in L2
     const int walkers_max = best->pair ? sms / 2 : sms;
     const int walkers = p.tiles_total < walkers_max ? p.tiles_total : walkers_max;
-    cfg.gridDim = dim3(best->pair ? 2 * walkers : walkers, 1, 1);
+    cfg.gridDim = dim3(best->pair ? 2 * walkers : best->split ? best_splits * p.tiles_total : walkers, 1, 1);
     cfg.blockDim = dim3(best->threads, 1, 1);
     cfg.dynamicSmemBytes = best->smem;
     cfg.stream = stream;
     cudaLaunchAttribute attr[2];
     int na = 0;
-    if (best->pair) {
+    if (best->pair || best->split) {
         attr[na].id = cudaLaunchAttributeClusterDimension;
-        attr[na].val.clusterDim.x = 2;
+        attr[na].val.clusterDim.x = best->pair ? 2 : best_splits;
         attr[na].val.clusterDim.y = 1;
         attr[na].val.clusterDim.z = 1;
         ++na;

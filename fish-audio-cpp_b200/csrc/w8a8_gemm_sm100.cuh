@@ -61,6 +61,7 @@ struct GemmParams {
     LinearArgs a;
     int* status;
     int tiles_m, tiles_total;
+    int splits, split_kb;  // SPLIT: CTAs that share a tile's K, and the stages each of them takes (the last one what is left)
     int tma_store;  // output rows are multiples of 16 bytes and aligned: the tile leaves by TMA
 };
 
@@ -236,7 +237,12 @@ __device__ __forceinline__ uint64_t smem_desc(uint32_t saddr) {
 
 // GM: the group size when it is 64, 128 or 256; 0 = any multiple of 32 (plain loops), and whenever the group sums are asked
 // for as well.
-template <int BT, bool PAIR, int GM>
+//
+// SPLIT: few tiles and a long K. The CTAs of a cluster take one tile, each a run of its K-groups; at the end the first CTA reads
+// the others' fp32 sums from their shared memory and adds them in ascending-K order. Narrow tiles are a serial chain of some
+// 430-650 clocks per K-group, whatever the number of CTAs (tokens x rows x K, g = 64: 150 x 2560 x 9728 34.8 -> 27.0 us, 64 x
+// 2560 x 9728 34.8 -> 17.9, 150 x 2560 x 4096 19.3 -> 16.4).
+template <int BT, bool PAIR, int GM, bool SPLIT>
 __global__ void __launch_bounds__(Config<BT, PAIR>::kThreads, 1)
 gemm_i8_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_x,
                const __grid_constant__ CUtensorMap map_y, const GemmParams p) {
@@ -252,10 +258,14 @@ gemm_i8_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
     const int warp = __shfl_sync(0xffffffffu, static_cast<int>(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
     const uint32_t tiles = (ptx::smem_u32(smem_raw) + 1023u) & ~1023u;
     const uint32_t out_stage = tiles + S * C::kStageBytes, sc_ring = out_stage + C::kOutBytes;
-    const int G = a.G, num_kb = a.K / BK;
+    static_assert(!SPLIT || (!PAIR && GM != 0), "a split tile is one CTA's, of whole K-groups");
+    const int srank = SPLIT ? static_cast<int>(cluster_rank()) : 0;
+    const int kb0 = SPLIT ? srank * p.split_kb : 0;
+    const int num_kb = SPLIT ? min(p.split_kb, a.K / BK - kb0) : a.K / BK;
+    const int G = a.G, g_first = SPLIT ? kb0 * BK / GM : 0, g_end = SPLIT ? g_first + num_kb * BK / GM : G;  // this CTA's K-groups
     const uint32_t crank = PAIR ? cluster_rank() : 0u;
-    const int walker = PAIR ? static_cast<int>(blockIdx.x >> 1) : static_cast<int>(blockIdx.x);
-    const int walkers = PAIR ? static_cast<int>(gridDim.x >> 1) : static_cast<int>(gridDim.x);
+    const int walker = SPLIT ? static_cast<int>(blockIdx.x) / p.splits : PAIR ? static_cast<int>(blockIdx.x >> 1) : static_cast<int>(blockIdx.x);
+    const int walkers = SPLIT ? p.tiles_total : PAIR ? static_cast<int>(gridDim.x >> 1) : static_cast<int>(gridDim.x);
     auto tile_m0 = [&](int tile) { return (tile % p.tiles_m) * BT; };
     auto tile_n0 = [&](int tile) { return (tile / p.tiles_m) * (PAIR ? 2 * BR : BR) + static_cast<int>(crank) * BR; };
     int my_tiles = 0;
@@ -288,7 +298,7 @@ gemm_i8_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
             const bool leader = elect_one();
             // a pair's loads complete on the LEADER's barrier, which alone expects the bytes of both CTAs
             const uint32_t full0 = PAIR ? map_to_rank(ptx::smem_u32(&full_bar[0]), 0) : ptx::smem_u32(&full_bar[0]);
-            int tile = walker, kx = 0, left = my_tiles * num_kb;
+            int tile = walker, kx = kb0 * BK, left = my_tiles * num_kb;
             int m0 = tile_m0(tile) + (PAIR ? static_cast<int>(crank) * C::kRowsB : 0), n0 = tile_n0(tile);
             uint32_t parity = 1;
             bool ok = true;
@@ -409,8 +419,8 @@ gemm_i8_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
                 const int m0 = tile_m0(tile), n0 = tile_n0(tile);
                 const __half* ws0 = a.w_scale + static_cast<size_t>(min(n0 + t64, a.N - 1)) * G;
                 const __half* ws1 = a.w_scale + static_cast<size_t>(min(n0 + 64 + t64, a.N - 1)) * G;
-                for (int j0 = 0; j0 < G; j0 += kScGroups) {
-                    const int nj = min(kScGroups, G - j0);
+                for (int j0 = g_first; j0 < g_end; j0 += kScGroups) {
+                    const int nj = min(kScGroups, g_end - j0);
                     __half w[2][kScGroups];  // on their way while the slot is waited for
 #pragma unroll
                     for (int q = 0; q < kScGroups; ++q) {
@@ -442,6 +452,7 @@ gemm_i8_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
             asm volatile("cp.async.wait_all;" ::: "memory");
         }
         __syncwarp();
+        if constexpr (SPLIT) cluster_sync_all();  // (the epilogue's meeting below)
     } else {
         if constexpr (C::kMoveRegs) asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(kHighRegs) : "memory");
         // ---------------- epilogue: each warp 32 weight rows x a part of the tokens ----------------
@@ -474,7 +485,7 @@ gemm_i8_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
                 tmem_ld(taddr + (16u << 16), r[1]);
             };
 #pragma unroll 1
-            for (int j0 = 0; j0 < G && ok; j0 += kScGroups) {
+            for (int j0 = g_first; j0 < g_end && ok; j0 += kScGroups) {
                 if (!wait(&sc_full[slot], sc_parity)) {
                     if (lane == 0) atomicExch(p.status, 700 + slot);
                     ok = false;
@@ -482,7 +493,7 @@ gemm_i8_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
                 }
                 uint32_t xs_addr = sc_ring + slot * C::kScSlot + (part * HC + 2 * (lane & 3)) * 4;
                 uint32_t ws_addr = sc_ring + slot * C::kScSlot + (kScGroups * BT + quad * 32 + (lane >> 2)) * 4;
-                const int j1 = min(j0 + kScGroups, G);
+                const int j1 = min(j0 + kScGroups, g_end);
 #pragma unroll 1
                 for (int j = j0; j < j1; ++j) {
                     uint64_t w2[2][2];
@@ -546,6 +557,34 @@ gemm_i8_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
                 __syncwarp();
                 if (lane == 0) ptx::mbar_arrive(&sc_empty[slot]);
                 if (++slot == kScRing) { slot = 0; sc_parity ^= 1u; }
+            }
+            if constexpr (SPLIT) {
+                // Every stage of this CTA's ring has been loaded and multiplied: its memory holds the sums now. One tile per CTA.
+                static_assert(4 * OCT * kEpiThreads * 8 <= S * C::kStageBytes, "the sums fit the ring");
+                const uint32_t mine = tiles + et * 8;
+                if (srank > 0) {
+#pragma unroll
+                    for (int i = 0; i < 4 * OCT; ++i)
+                        asm volatile("st.shared.b64 [%0], %1;" ::"r"(mine + i * kEpiThreads * 8), "l"(acc[i / (2 * OCT)][i / OCT % 2][i % OCT]) : "memory");
+                }
+                __syncwarp();
+                cluster_sync_all();
+                if (srank > 0) {
+                    if (epi_barrier_any<kEpiThreads>(!ok)) failed_s = 1;
+                    break;
+                }
+                for (int c = 1; c < p.splits; ++c) {
+                    const uint32_t theirs = map_to_rank(mine, c);
+                    uint64_t v[4 * OCT];
+#pragma unroll
+                    for (int i = 0; i < 4 * OCT; ++i)
+                        asm volatile("ld.shared::cluster.b64 %0, [%1];" : "=l"(v[i]) : "r"(theirs + i * kEpiThreads * 8) : "memory");
+#pragma unroll
+                    for (int i = 0; i < 4 * OCT; ++i) {
+                        uint64_t& mine_i = acc[i / (2 * OCT)][i / OCT % 2][i % OCT];
+                        mine_i = pack2(lo2(mine_i) + lo2(v[i]), hi2(mine_i) + hi2(v[i]));
+                    }
+                }
             }
             // ---- the tile as fp16 in shared memory: panels of [BT tokens][64 columns], 128-byte rows, swizzled ----
             if (et == 0) asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");  // the tile before has left it
@@ -626,7 +665,7 @@ gemm_i8_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
     __syncthreads();
     if (failed_s)  // a bounded wait ran out: give copies and MMAs that may still be in flight time to land
         for (int i = 0; i < 1000; ++i) __nanosleep(1000);
-    if constexpr (PAIR) cluster_sync_all();  // nothing of the peer still signals this CTA's barriers or uses its tensor memory
+    if constexpr (PAIR || SPLIT) cluster_sync_all();  // (SPLIT: the others' sums have been read); nothing of the peer still signals this CTA's barriers or uses its tensor memory
     if (warp == 1) {
         tc_fence_after();
         tmem_dealloc<PAIR>(tmem_base, C::kTmemCols);
@@ -638,20 +677,22 @@ using Kernel = void (*)(const CUtensorMap, const CUtensorMap, const CUtensorMap,
 // K and per K-group, fitted to 8192 x 19456 x 2560 at g = 256 and g = 64 (the two overlap; their sum is what was measured).
 struct Form {
     int bt;
-    bool pair;
+    bool pair, split;
     Kernel kernel;
     int threads, smem;
     bool move_regs;
     float stage_ns, group_ns;
 };
-template <int BT, bool PAIR, int GM>
+template <int BT, bool PAIR, int GM, bool SPLIT = false>
 constexpr Form form(float stage_ns, float group_ns) {
-    return Form{BT, PAIR, gemm_i8_kernel<BT, PAIR, GM>, Config<BT, PAIR>::kThreads, Config<BT, PAIR>::kSmem, Config<BT, PAIR>::kMoveRegs, stage_ns, group_ns};
+    return Form{BT, PAIR, SPLIT, gemm_i8_kernel<BT, PAIR, GM, SPLIT>, Config<BT, PAIR>::kThreads, Config<BT, PAIR>::kSmem, Config<BT, PAIR>::kMoveRegs, stage_ns, group_ns};
 }
 template <int GM>
 const Form* all_forms(int* count) {
-    static const Form table[] = {form<32, false, GM>(148, 157), form<64, false, GM>(136, 196), form<96, false, GM>(106, 280),
-                                 form<128, false, GM>(135, 330), form<192, true, GM>(215, 440), form<256, true, GM>(247, 557)};
+    static const Form table[] = {form<32, false, GM>(148, 157), form<64, false, GM>(136, 196), form<96, false, GM>(106, 300),
+                                 form<128, false, GM>(135, 330), form<192, true, GM>(215, 440), form<256, true, GM>(247, 557),
+                                 form<32, false, GM, true>(148, 157), form<64, false, GM, true>(136, 196), form<96, false, GM, true>(106, 300),
+                                 form<128, false, GM, true>(135, 330)};
     *count = static_cast<int>(sizeof(table) / sizeof(table[0]));
     return table;
 }

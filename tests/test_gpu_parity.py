@@ -669,6 +669,56 @@ def test_gemm_tcgen05_tile_widths(ctx, oracle, pkg, monkeypatch, M, N, K, bt, fo
     assert np.array_equal(dY.cpu().numpy().view(np.uint16), oracle.linear_q(W, ws, Xq, Xs, g).view(np.uint16))
 
 
+@pytest.mark.parametrize("g", [64, 128, 256])
+@pytest.mark.parametrize("splits", [2, 4])
+@pytest.mark.parametrize("bt", [32, 64, 96, 128])
+@pytest.mark.parametrize("M,N,K", [(33, 136, 1024), (97, 40, 1280), (150, 272, 2816)])
+def test_gemm_tcgen05_split_k(ctx, oracle, pkg, monkeypatch, M, N, K, bt, splits, g):
+    """A tile's K over two or four CTAs: runs of one K-group and of many, a last run that is shorter, ragged tokens and rows. The
+    sums are the whole-K kernel's, added in another order (the bar with the sum of absolute terms covers that)."""
+    monkeypatch.setenv("W8A8_GEMM_BT", str(bt))
+    monkeypatch.setenv("W8A8_GEMM_SPLIT", str(splits))
+    X, W, ws = synth.linear_case(M + N + K + bt, M, N, K, g)
+    Xq, Xs = oracle.quantize(X, g)
+    buf, dY = guarded((M, N), torch.float16, 99.0)
+    ctx.linear_q(dev(W), dev(ws), g, dev(Xq), dev(Xs), dY, M, N, K)
+    torch.cuda.synchronize()
+    ctx.check_device_status()
+    assert guards_intact(buf, 99.0)
+    assert_close_fp16(oracle, dY.cpu().numpy(), oracle.linear_q(W, ws, Xq, Xs, g), "split K",
+                      abs_terms=abs_term_sum(oracle.group_sums(W, Xq, g), ws, Xs))
+
+
+@pytest.mark.parametrize("packed", [True, False])
+@pytest.mark.parametrize("M,g", [(3, 64), (16, 64), (8, 128)])
+def test_decode_linear_scales_at_any_address(ctx, oracle, pkg, M, g, packed):
+    """Activation scales that are not aligned for the word-wide reads of the plain instances: the same outputs bit for bit."""
+    N, K = 264, 1280
+    X, W, ws = synth.linear_case(M + g, M, N, K, g)
+    Xq, Xs = oracle.quantize(X, g)
+    dW, dS, dq, aligned = dev(W), dev(ws), dev(Xq), dev(Xs)
+    odd = torch.empty((aligned.numel() + 1,), dtype=torch.float32, device="cuda")[1:].view(aligned.shape)
+    odd.copy_(aligned)
+    if packed:
+        P = torch.empty((ctx.packed_weight_bytes(N, K, g),), dtype=torch.uint8, device="cuda")
+        ctx.pack_weight(dW, dS, N, K, g, P)
+        ctx.register_packed_weight(dW, P, N, K, g)
+    try:
+        outs = []
+        for xs in (aligned, odd):
+            dY = torch.empty((M, N), dtype=torch.float16, device="cuda")
+            ctx.linear_q(dW, dS, g, dq, xs, dY, M, N, K)
+            outs.append(dY.view(torch.int16))
+        torch.cuda.synchronize()
+        ctx.check_device_status()
+        assert torch.equal(outs[0], outs[1])
+        assert_close_fp16(oracle, outs[1].view(torch.float16).cpu().numpy(), oracle.linear_q(W, ws, Xq, Xs, g), "odd scales",
+                          abs_terms=abs_term_sum(oracle.group_sums(W, Xq, g), ws, Xs))
+    finally:
+        if packed:
+            ctx.register_packed_weight(dW, None)
+
+
 @pytest.mark.parametrize("g", [64, 128, 256, 512])
 @pytest.mark.parametrize("M", [8, 9, 16, 17, 32])
 def test_packed_linear_many_weights_back_to_back(ctx, oracle, pkg, M, g):
