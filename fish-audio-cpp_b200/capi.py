@@ -2,6 +2,7 @@
 from __future__ import annotations
 
 import ctypes as C
+import threading
 from pathlib import Path
 
 ACT_PER_TOKEN_GROUP, ACT_PER_TOKEN = 0, 1
@@ -168,6 +169,18 @@ def _stream(stream) -> int | None:
             _RAW_STREAM = _raw_stream_fn()
         return _RAW_STREAM() or None
     return stream or None
+
+
+_ERRORS = threading.local()
+
+
+def _error_buffer():
+    """512 bytes for an error text, one buffer per thread (making one costs a shim call 1 us)."""
+    try:
+        return _ERRORS.buf
+    except AttributeError:
+        _ERRORS.buf = C.create_string_buffer(512)
+        return _ERRORS.buf
 
 
 def static_scratch_bytes() -> int:
@@ -385,7 +398,7 @@ class Context:
                     "w8a8_register_packed_weight")
 
     def _shim(self, name, *args, stream=None):
-        buf = C.create_string_buffer(512)
+        buf = _error_buffer()
         rc = getattr(self.lib, name)(*args, _stream(stream), buf, 512)
         if rc:
             raise RuntimeError(buf.value.decode())
@@ -406,7 +419,7 @@ class Context:
     def shim_int8_dequant_gemm_fp16(self, W, scale, group_size, act_scale, smooth_inv, X, Y, M_out, N_tok, K,
                                     stream=None):
         """Drives the C++ entry point with the reference's own signature and argument order."""
-        buf = C.create_string_buffer(512)
+        buf = _error_buffer()
         rc = self.lib.fish_shim_int8_dequant_gemm_fp16(_ptr(W), _ptr(scale), group_size, _ptr(act_scale),
                                                        _ptr(smooth_inv), _ptr(X), _ptr(Y), M_out, N_tok, K,
                                                        _stream(stream), buf, 512)

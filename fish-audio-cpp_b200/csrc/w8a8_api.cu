@@ -47,6 +47,16 @@ bool pdl_enabled(int kernel_class) {
     return (mask & kernel_class) != 0;
 }
 
+int device_sms() {
+    static std::atomic<int> known[64];
+    int dev = 0, v = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess) return 148;
+    if (dev < 64 && (v = known[dev].load(std::memory_order_relaxed)) > 0) return v;
+    if (cudaDeviceGetAttribute(&v, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || v <= 0) return 148;
+    if (dev < 64) known[dev].store(v, std::memory_order_relaxed);
+    return v;
+}
+
 int check_launch(const char* what) {
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return fail(W8A8_ERR_CUDA, "%s: %s", what, cudaGetErrorString(e));

@@ -702,10 +702,7 @@ int launch_attention(const AttnParams& base, int B, int splits, cudaStream_t str
     if (Xq && (g <= 0 || (kQPerKv * kHeadDim) % g != 0))
         return fail(W8A8_ERR_UNSUPPORTED, "fused output quantisation needs a group size dividing 512 (got %d)", g);
     if (splits <= 0) {  // one CTA per SM: as many context slices as the (sequence, kv head) pairs leave room for
-        int dev = 0, sms = 0;
-        if (cudaGetDevice(&dev) != cudaSuccess ||
-            cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sms <= 0)
-            sms = 148;
+        const int sms = device_sms();
         const int want = sms / (B * n_kv);
         splits = want >= 8 ? 8 : want >= 4 ? 4 : want >= 2 ? 2 : 1;
         // no more slices than give each consumer warp a block of the longest sequence the table can hold

@@ -982,14 +982,6 @@ Scratch layout(const w8a8_decode_stack& d, int S) {
     return sc;
 }
 
-int num_sms() {
-    int dev = 0, v = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&v, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess ||
-        v <= 0)
-        v = 148;
-    return v;
-}
-
 int slices_for(const w8a8_decode_stack& d, int sms) {
     const int want = sms / (d.batch * d.n_kv_heads);
     return want >= 8 ? 8 : want >= 4 ? 4 : want >= 2 ? 2 : 1;  // the stand-alone attention launch picks the same
@@ -1012,13 +1004,13 @@ const char* check(const w8a8_decode_stack& d) {
 
 size_t decode_stack_workspace_bytes(const w8a8_decode_stack& d) {
     if (check(d)) return 0;
-    return layout(d, slices_for(d, num_sms())).total;
+    return layout(d, slices_for(d, device_sms())).total;
 }
 
 int decode_stack_timeline(const w8a8_decode_stack& d, const unsigned char* workspace, unsigned long long* out, int capacity,
                           cudaStream_t stream) {
     if (const char* why = check(d)) return fail(W8A8_ERR_UNSUPPORTED, "decode stack: %s", why);
-    const Scratch sc = layout(d, slices_for(d, num_sms()));
+    const Scratch sc = layout(d, slices_for(d, device_sms()));
     const int n = 18 * d.n_layers + 2;
     if (capacity < n) return fail(W8A8_ERR_INVALID_ARG, "timeline needs room for %d stamps", n);
     cudaError_t e = cudaMemcpyAsync(out, workspace + sc.timeline, static_cast<size_t>(n) * 8, cudaMemcpyDeviceToHost, stream);
@@ -1029,7 +1021,7 @@ int decode_stack_timeline(const w8a8_decode_stack& d, const unsigned char* works
 
 int launch_decode_stack(const w8a8_decode_stack& d, unsigned char* workspace, size_t workspace_bytes, int* status, cudaStream_t stream) {
     if (const char* why = check(d)) return fail(W8A8_ERR_UNSUPPORTED, "decode stack: %s", why);
-    const int sms = num_sms();
+    const int sms = device_sms();
     StackParams p = {};
     p.S = slices_for(d, sms);
     const Scratch sc = layout(d, p.S);

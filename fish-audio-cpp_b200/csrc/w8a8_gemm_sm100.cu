@@ -35,8 +35,7 @@ bool gemm_supports(const LinearArgs& a) {
 int launch_linear_gemm(const LinearArgs& a, int* device_status, cudaStream_t stream, int form) {
     using namespace gemm;
     if (!gemm_supports(a)) return fail(W8A8_ERR_UNSUPPORTED, "tcgen05 GEMM does not take this shape");
-    int sms = 148, dev = 0;
-    if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    const int sms = device_sms();
 
     int count = 0;
     const Form* table = forms(a.dump ? 0 : a.g, &count);

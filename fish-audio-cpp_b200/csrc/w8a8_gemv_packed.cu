@@ -3,18 +3,6 @@
 #include "w8a8_gemv_packed.cuh"
 
 namespace w8a8 {
-namespace {
-
-int num_sms() {  // of the current device (not cached: one process may drive several devices)
-    int dev = 0, v = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess ||
-        cudaDeviceGetAttribute(&v, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || v <= 0)
-        v = 148;
-    return v;
-}
-
-}  // namespace
-
 // How many CTAs share the row tiles of a linear. Up to two per SM (their shared memory fits twice when M <= 8),
 // as many as make the tiles per CTA equal: 160 row tiles on 148 SMs are 160 CTAs of one tile, not 136 of one
 // and 12 of two. An SM that hosts two CTAs has twice the copies in flight and pulls twice the bytes in the same
@@ -101,7 +89,7 @@ bool gemv::make_plan(const LinearArgs& a, Plan& pl, bool rows) {
     pl.tiles = (a.N + 15) / 16;
     pl.U = static_cast<long long>(pl.tiles) * pl.upt;
     // Up to two CTAs per SM where their registers and shared memory fit twice, never more CTAs than row tiles.
-    pl.ctas = gemv_packed_ctas(pl.tiles, num_sms(), two_per_sm(pl.MT, pl.GM));
+    pl.ctas = gemv_packed_ctas(pl.tiles, device_sms(), two_per_sm(pl.MT, pl.GM));
     if ((pl.U + 1) * static_cast<long long>(pl.ctas) * kWarps >= (1ll << 32)) return false;  // 32-bit range math
     return true;
 }
@@ -135,11 +123,7 @@ int launch_variant(const LinearArgs& a, const Plan& pl, int* status, cudaStream_
     auto kern = gemv_packed_kernel<MT, GM, PRO, ST, KI, EPI, EXTRA>;
     const size_t ring = static_cast<size_t>(kWarps) * ST * kStagePitch + 128;
     const size_t smem = ring + (PRO == kProNorm ? fused_smem_bytes(a.K, a.G) : 0);
-    {  // per device, so on every launch (a host-side table write)
-        const size_t most = ring + (PRO == kProNorm ? fused_smem_bytes(256 * KI, 4 * KI) : 0);
-        cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(most));
-        if (e != cudaSuccess) return fail(W8A8_ERR_CUDA, "cudaFuncSetAttribute: %s", cudaGetErrorString(e));
-    }
+    const size_t most = ring + (PRO == kProNorm ? fused_smem_bytes(256 * KI, 4 * KI) : 0);
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(pl.ctas, 1, 1);
     cfg.blockDim = dim3(kThreads, 1, 1);
@@ -150,7 +134,8 @@ int launch_variant(const LinearArgs& a, const Plan& pl, int* status, cudaStream_
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
     cfg.numAttrs = pdl_enabled(kPdlLinear) ? 1 : 0;
-    cudaError_t e = cudaLaunchKernelEx(&cfg, kern, p);
+    static SmemAttribute attribute;
+    cudaError_t e = launch_with_smem(attribute, static_cast<int>(most), cfg, kern, p);
     if (e != cudaSuccess) return fail(W8A8_ERR_CUDA, "gemv_packed launch: %s", cudaGetErrorString(e));
     return W8A8_OK;
 }
@@ -242,7 +227,7 @@ int launch_pack_weight(const int8_t* W, const __half* S, int N, int K, int g, vo
 // (eager: 7.4 -> 5.2 and 7.4 -> 6.9 us a call). With longer runs every block is quantised by every row tile's warps again:
 // packed 2560 x 9728 at M = 8 8.0 -> 9.5 us, row-major 19456 x 2560 12.4 -> 13.8.
 bool quant_form_wins(const LinearArgs& a) {
-    const int tiles = (a.N + 15) / 16, ctas = gemv_packed_ctas(tiles, num_sms(), true);
+    const int tiles = (a.N + 15) / 16, ctas = gemv_packed_ctas(tiles, device_sms(), true);
     return static_cast<long long>(tiles) * (a.K / 256) <= 3ll * kWarps * ctas;
 }
 

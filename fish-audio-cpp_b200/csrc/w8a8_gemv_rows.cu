@@ -26,8 +26,6 @@ int launch_variant(const LinearArgs& a, const Plan& pl, int* status, cudaStream_
     fill_params(a, pl, status, p);
     auto kern = gemv_rows_kernel<MT, GM, PRO, EXTRA>;
     const size_t smem = static_cast<size_t>(kWarps) * 3 * kBlockW + 1024;
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
-    if (e != cudaSuccess) return fail(W8A8_ERR_CUDA, "cudaFuncSetAttribute: %s", cudaGetErrorString(e));
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(pl.ctas, 1, 1);
     cfg.blockDim = dim3(kThreads, 1, 1);
@@ -38,7 +36,8 @@ int launch_variant(const LinearArgs& a, const Plan& pl, int* status, cudaStream_
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
     cfg.numAttrs = pdl_enabled(kPdlLinear) ? 1 : 0;
-    e = cudaLaunchKernelEx(&cfg, kern, map, p);
+    static SmemAttribute attribute;
+    cudaError_t e = launch_with_smem(attribute, static_cast<int>(smem), cfg, kern, map, p);
     if (e != cudaSuccess) return fail(W8A8_ERR_CUDA, "gemv_rows launch: %s", cudaGetErrorString(e));
     return W8A8_OK;
 }

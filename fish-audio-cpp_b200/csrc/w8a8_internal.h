@@ -4,6 +4,7 @@
 #include <cuda_fp16.h>
 #include <cuda_runtime.h>
 
+#include <atomic>
 #include <cstddef>
 #include <cstdint>
 
@@ -24,6 +25,39 @@ enum { kPdlLinear = 1, kPdlRow = 2, kPdlAttn = 4 };
 // first K/V blocks overlap the end of wqkv: 1696 -> 1650 us per step at batch 8, 1517 -> 1495 at batch 1).
 constexpr int kPdlDefaultMask = kPdlLinear | kPdlRow | kPdlAttn;
 bool pdl_enabled(int kernel_class);
+
+// SMs of the current device, asked for once per device.
+int device_sms();
+// Lets a kernel use `bytes` of dynamic shared memory: once per device (the call costs an eager launch 0.3 us of host time).
+// A launch that fails all the same asks again (`anew`): a device reset takes the attribute back. One object per kernel, static.
+class SmemAttribute {
+  public:
+    cudaError_t operator()(const void* kernel, int bytes, bool anew = false) {
+        int dev = 0;
+        cudaError_t e = cudaGetDevice(&dev);
+        if (e != cudaSuccess) return e;
+        const unsigned long long bit = dev < 64 ? 1ull << dev : 0ull;
+        if (!anew && (done_.load(std::memory_order_acquire) & bit)) return cudaSuccess;
+        e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+        if (e == cudaSuccess) done_.fetch_or(bit, std::memory_order_release);
+        return e;
+    }
+
+  private:
+    std::atomic<unsigned long long> done_{0};
+};
+// Launches `kern`; `attr` as above.
+template <class... P, class... A>
+cudaError_t launch_with_smem(SmemAttribute& attr, int max_smem, const cudaLaunchConfig_t& cfg, void (*kern)(P...), const A&... args) {
+    cudaError_t e = attr(reinterpret_cast<const void*>(kern), max_smem);
+    if (e != cudaSuccess) return e;
+    e = cudaLaunchKernelEx(&cfg, kern, args...);
+    if (e == cudaErrorInvalidValue && attr(reinterpret_cast<const void*>(kern), max_smem, true) == cudaSuccess) {
+        cudaGetLastError();
+        e = cudaLaunchKernelEx(&cfg, kern, args...);
+    }
+    return e;
+}
 
 inline int norm_group(int K, int group_size) {
     return (group_size <= 0 || group_size > K) ? K : group_size;
