@@ -928,8 +928,7 @@ def main():
     ap.add_argument("--no-pack", action="store_true", help="leave weights row-major (skip the loader-side pack)")
     ap.add_argument("--eager", action="store_true", help="launch kernels one by one instead of replaying a graph")
     ap.add_argument("--trace", action="store_true",
-                    help="decode_stack: add the per-kernel device timeline of one replayed step to the line; prefill: add "
-                         "the per-K-group timeline of the GEMM's MMA lane, epilogue and producer (both need a library "
+                    help="decode_stack: add the per-kernel device timeline of one replayed step to the line (needs a library "
                          "built with --define W8A8_TRACE, named by W8A8_LIBRARY)")
     ap.add_argument("--timeline", action="store_true",
                     help="with --step-form one-launch: add the device-side per-phase medians of one step to the line")
