@@ -417,6 +417,13 @@ gemm_i8_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
             bool ok = true;
             for (int tile = walker; tile < p.tiles_total && ok; tile += walkers) {
                 const int m0 = tile_m0(tile), n0 = tile_n0(tile);
+                if (a.epilogue == W8A8_EPI_RESIDUAL && srank == 0) {  // the tile's residual rows to L2, long before its end needs them
+                    for (int i = t64; i < 2 * BT; i += 64) {
+                        const int t = m0 + (i >> 1), col = n0 + (i & 1) * 64;
+                        if (t < a.M && col < a.N)
+                            asm volatile("prefetch.global.L2 [%0];" ::"l"(a.residual + static_cast<size_t>(t) * a.N + col));
+                    }
+                }
                 const __half* ws0 = a.w_scale + static_cast<size_t>(min(n0 + t64, a.N - 1)) * G;
                 const __half* ws1 = a.w_scale + static_cast<size_t>(min(n0 + 64 + t64, a.N - 1)) * G;
                 for (int j0 = g_first; j0 < g_end; j0 += kScGroups) {
@@ -626,19 +633,36 @@ gemm_i8_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
                 if (p.tma_store) {  // residual: 16-byte pieces, sixteen threads per token row
                     const int piece = et & 15, rt = et >> 4;
                     if (piece * 8 < width) {
-                        for (int t = rt; t < tokens; t += kEpiThreads / 16) {
-                            const size_t o = static_cast<size_t>(m0 + t) * ycols + y0 + piece * 8;
-                            uint4 v, rv = *reinterpret_cast<const uint4*>(a.residual + o);
-                            asm volatile("ld.shared.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w)
-                                         : "r"(out_stage + (piece >> 3) * C::kPanelBytes + t * 128 + (((piece & 7) ^ (t & 7)) << 4)));
-                            __half2* hv = reinterpret_cast<__half2*>(&v);
-                            const __half2* hr = reinterpret_cast<const __half2*>(&rv);
+                        // Up to four rows at a time: their reads are memory latencies, one after the other eight to a tile of 256
+                        // tokens. (All of them at once, or four in the forms for any group size, spill registers in the loop above.)
+                        constexpr int kRowStep = kEpiThreads / 16;
+                        constexpr int kRows = GM == 0 ? 2 : BT % (4 * kRowStep) == 0 ? 4 : BT % (3 * kRowStep) == 0 ? 3 : 2;
+                        static_assert(BT % (kRows * kRowStep) == 0, "whole rounds");
+                        const size_t o0 = static_cast<size_t>(m0) * ycols + y0 + piece * 8;
+#pragma unroll 1
+                        for (int t0 = rt; t0 < tokens; t0 += kRows * kRowStep) {
+                            uint4 rv[kRows];
 #pragma unroll
-                            for (int i = 0; i < 4; ++i) {
-                                const float2 x = __half22float2(hv[i]), y = __half22float2(hr[i]);
-                                hv[i] = __floats2half2_rn(x.x + y.x, x.y + y.y);
+                            for (int i = 0; i < kRows; ++i) {
+                                const int t = t0 + i * kRowStep < tokens ? t0 + i * kRowStep : t0;
+                                rv[i] = *reinterpret_cast<const uint4*>(a.residual + o0 + static_cast<size_t>(t) * ycols);
                             }
-                            *reinterpret_cast<uint4*>(a.Y + o) = v;
+#pragma unroll
+                            for (int i = 0; i < kRows; ++i) {
+                                const int t = t0 + i * kRowStep;
+                                if (t >= tokens) break;
+                                uint4 v;
+                                asm volatile("ld.shared.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w)
+                                             : "r"(out_stage + (piece >> 3) * C::kPanelBytes + t * 128 + (((piece & 7) ^ (t & 7)) << 4)));
+                                __half2* hv = reinterpret_cast<__half2*>(&v);
+                                const __half2* hr = reinterpret_cast<const __half2*>(&rv[i]);
+#pragma unroll
+                                for (int k = 0; k < 4; ++k) {
+                                    const float2 x = __half22float2(hv[k]), y = __half22float2(hr[k]);
+                                    hv[k] = __floats2half2_rn(x.x + y.x, x.y + y.y);
+                                }
+                                *reinterpret_cast<uint4*>(a.Y + o0 + static_cast<size_t>(t) * ycols) = v;
+                            }
                         }
                     }
                 } else {  // any row pitch: element by element
