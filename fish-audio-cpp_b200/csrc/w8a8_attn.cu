@@ -139,6 +139,7 @@ struct AttnParams {
     __half* k_cache_w;        // the caches again, writable
     __half* v_cache_w;
     int* status;              // error word for bounded waits that ran out
+    bool ahead;               // ROPE form: all it reads but qkv may be read before the dependency wait (see the kernel)
 };
 
 #ifndef W8A8_ATTN_WARPS
@@ -245,10 +246,8 @@ __device__ __forceinline__ void consumer_barrier() {  // the eight consumer warp
 // The K and V of one (sequence, kv head) are 4 KB blocks scattered over the paged cache. The producer warp brings them
 // into a ring of shared-memory stages with TMA (cp.async.bulk.tensor.2d over the cache seen as rows of 256 bytes,
 // two 16 x 128-byte boxes per block, 128-byte swizzle, completion counted on the stage's mbarrier; single 256-byte
-// row copies were tried first and are bound by the copy engine's request rate) — no registers are tied up by bytes in flight, so the kernel fits beside a CTA of
-// the linear before it, and everything the producer needs (sequence length, block table, every block but the
-// sequence's last) does not depend on that linear: with programmatic dependent launch the ring is already full when
-// the query arrives. 16-token blocks are dealt round-robin, first over the cluster's CTAs, then over the consumer
+// row copies were tried first and are bound by the copy engine's request rate), so no registers are tied up by bytes in
+// flight. 16-token blocks are dealt round-robin, first over the cluster's CTAs, then over the consumer
 // warps; a consumer waits for its block, computes on it from shared memory (ldmatrix into mma.sync.m16n8k16 with
 // fp32 accumulation: scores = Q K^T with the four query heads of the group as rows 0..3 of the tile, then
 // out += P V with P rounded to fp16 and the softmax denominator summed from the same rounded values) and hands the
@@ -259,8 +258,15 @@ __device__ __forceinline__ void consumer_barrier() {  // the eight consumer warp
 // query heads into shared memory; warps 4 and 5 do the same for the new k and v rows, which go to shared memory and,
 // in the CTA that owns the block the new token joins, to the cache. That block is read from the cache like any other
 // (possibly before the new rows are there) and the new rows are put over it in shared memory.
-// Without ROPE the new rows were written by the launch before this one, so the sequence's last block is requested
-// only after the dependency wait.
+//
+// What may be read before the dependency wait. The kernels ahead on the stream that are launched early let their dependents
+// start at their first instruction, so this kernel can be running while several of them still are, a cache write or an
+// update of the positions among them; the wait covers them all, an earlier read none. By default the kernel therefore
+// waits before it reads anything, and lets its own dependents start after that: once any kernel behind it runs, all
+// that was ahead of it is complete. Such a kernel is what `ahead` rests on (ROPE form only): the caller says that the
+// positions, lengths, block table and cached rows were complete before it, and the ring is filled and the rotation angles
+// are made while the projection ahead still runs (decode step at batch 8 / 1 and fast-AR frame with every layer waiting 1455 / 1260 /
+// 1577 us, with the first layer waiting and the others ahead 1421 / 1252 / 1560).
 #ifdef W8A8_TRACE
 // Diagnostic build only: nanosecond stamps of the phases of CTA (0, 0, 0), written by consumer thread 0, kept from
 // the last launch; read out by w8a8_trace_read_attn_phases.
@@ -308,7 +314,8 @@ __global__ void __maxnreg__(128) paged_attention_decode_kernel(const __grid_cons
     __shared__ int s_fail;
     W8A8_TRACE_SCOPE();
     ATTN_PHASE(0);
-    ptx::pdl_launch_dependents();
+    const bool ahead = ROPE && p.ahead;
+    if (ahead) ptx::pdl_launch_dependents();
 
     const int s = blockIdx.x, kvh = blockIdx.y, b = blockIdx.z, S = p.S;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -325,12 +332,15 @@ __global__ void __maxnreg__(128) paged_attention_decode_kernel(const __grid_cons
         ptx::fence_barrier_init();
         ptx::fence_proxy_async();
     }
+    if (!ahead) {
+        ptx::pdl_wait();
+        ptx::pdl_launch_dependents();
+    }
     __syncthreads();  // the only whole-CTA barrier: from here on the producer warp runs by itself
     if (S > 1) cluster_arrive();  // (waited for before anything is written to another CTA: that CTA has started then)
 
-    // Read before the dependency wait: these are not results of the launch before this one. The producer asks for the
-    // first 32 block numbers without waiting for the sequence length (the read is bounded by the table's width), so
-    // that the two reads are one round trip, not two.
+    // The producer asks for the first 32 block numbers without waiting for the sequence length (the read is bounded by the
+    // table's width), so that the two reads are one round trip, not two.
     int phys_first = 0;
     if (warp == kAttnWarps) {
         const int bi = s + lane * S;
@@ -345,7 +355,6 @@ __global__ void __maxnreg__(128) paged_attention_decode_kernel(const __grid_cons
         // ------------------------------ producer ------------------------------
         // Eight blocks per round, four lanes per block (one TMA box each): a single lane issuing every copy of the
         // CTA one after the other costs more than the copies take.
-        bool waited = false;
         int phys_mine = phys_first;
         bool failed = false;
         for (int li0 = 0; li0 < n_local && !failed; li0 += 8) {
@@ -357,12 +366,6 @@ __global__ void __maxnreg__(128) paged_attention_decode_kernel(const __grid_cons
             const int phys = __shfl_sync(0xffffffffu, phys_mine, li & 31);
             const int bi = s + li * S, st = li % kRing;
             const bool live = li < n_local;
-            // Without ROPE the newest rows come from the launch before this one: wait for it before the round that
-            // holds the sequence's last block.
-            if (!ROPE && !waited && s + (li0 + 7) * S >= n_blocks - 1) {
-                ptx::pdl_wait();
-                waited = true;
-            }
             if (live && li >= kRing && !ptx::mbar_wait_bounded(&empty_bar[st], ((li / kRing) - 1) & 1)) {
                 if (box == 0) { atomicExch(p.status, 800 + st); s_fail = 1; }
                 failed = true;
@@ -380,25 +383,24 @@ __global__ void __maxnreg__(128) paged_attention_decode_kernel(const __grid_cons
                     : "memory");
             }
         }
-        if (!waited) ptx::pdl_wait();
+        ptx::pdl_wait();
     } else {
         // ------------------------------ consumers ------------------------------
         int pos = 0;
         bool owner = false;
         RopeAngles rot;
-        if constexpr (ROPE) {  // parameters first: they do not depend on the launch before this one
+        if constexpr (ROPE) {
             pos = p.positions[b];
             rot.make(p.freqs, pos, lane);
             owner = ((pos / kBlockTokens) % S) == s;  // this CTA attends over the block the new token joins
         }
         const int new_bi = pos / kBlockTokens;
-        if constexpr (!ROPE) ptx::pdl_wait();
         if constexpr (ROPE) {
-            // The first pass is a rehearsal on zeros, before the dependency wait: cold code costs about six clocks an instruction
+            // With `ahead` the first pass is a rehearsal on zeros, before the dependency wait: cold code costs about six clocks an instruction
             // (step at batch 8: 1554 -> 1536 us). Rehearsing the block loop and the merges as well takes longer than the wait
             // it hides in (1517 -> 1756 us).
 #pragma unroll 1
-            for (int pass = 0; pass < 2; ++pass) {
+            for (int pass = ahead ? 0 : 1; pass < 2; ++pass) {
             const bool real = pass == 1;
             if (real) {
                 ptx::pdl_wait();
@@ -681,9 +683,10 @@ int launch_qkv_attention_decode(const __half* qkv, const __half* q_norm_w, const
                                 const float* freqs, const int* positions, __half* k_cache, __half* v_cache,
                                 const int* block_table, const int* seq_lens, int B, int n_q, int n_kv, int max_blocks,
                                 float sm_scale, int layer, int n_layers, __half* out, int g, int8_t* Xq, float* Xs,
-                                int splits, int* status, cudaStream_t stream) {
+                                int splits, bool ahead, int* status, cudaStream_t stream) {
     AttnParams p = {};
     p.status = status;
+    p.ahead = ahead;
     p.k_cache = k_cache; p.v_cache = v_cache; p.block_table = block_table; p.seq_lens = seq_lens;
     p.max_blocks = max_blocks; p.n_q = n_q; p.n_kv = n_kv; p.layer = layer; p.n_layers = n_layers; p.sm_scale = sm_scale;
     p.out = out; p.Xq = Xq; p.Xs = Xs; p.g = g;

@@ -21,8 +21,9 @@ int check_launch(const char* what);
 // the environment variable W8A8_PDL=<mask> can switch them one by one; W8A8_NO_PDL=1 switches all off.
 enum { kPdlLinear = 1, kPdlRow = 2, kPdlAttn = 4 };
 // Measured over the decode stack: early launch pays for the linears (weights are requested while the small kernel
-// before them runs), for the row kernels, which rehearse while they wait, and for the attention (its set-up and its
-// first K/V blocks overlap the end of wqkv: 1696 -> 1650 us per step at batch 8, 1517 -> 1495 at batch 1).
+// before them runs), for the row kernels, which rehearse while they wait, and for the attention whose caller says that its
+// inputs are complete (its set-up and its first K/V blocks overlap the end of wqkv: 1696 -> 1650 us per step at batch 8,
+// 1517 -> 1495 at batch 1).
 constexpr int kPdlDefaultMask = kPdlLinear | kPdlRow | kPdlAttn;
 bool pdl_enabled(int kernel_class);
 
@@ -158,7 +159,7 @@ int launch_qkv_attention_decode(const __half* qkv, const __half* q_norm_w, const
                                 const float* freqs, const int* positions, __half* k_cache, __half* v_cache,
                                 const int* block_table, const int* seq_lens, int B, int n_q, int n_kv, int max_blocks,
                                 float sm_scale, int layer, int n_layers, __half* out, int g, int8_t* Xq, float* Xs,
-                                int splits, int* status, cudaStream_t stream);
+                                int splits, bool ahead, int* status, cudaStream_t stream);
 // w8a8_decode_stack.cu : a whole decode step as one persistent cooperative kernel.
 size_t decode_stack_workspace_bytes(const w8a8_decode_stack& d);
 int launch_decode_stack(const w8a8_decode_stack& d, unsigned char* workspace, size_t workspace_bytes, int* status, cudaStream_t stream);

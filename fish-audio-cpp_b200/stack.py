@@ -250,7 +250,9 @@ class SlowARStack:
     # ------------------------------------------------------------------------------------------
     def decode_step(self, x_in=None):
         """One token for every sequence. x_in fp16 [B, dim] (the embedding of the new token); returns
-        the final-normed hidden state in self.out. All launches go to the current stream."""
+        the final-normed hidden state in self.out. All launches go to the current stream. The first layer's attention
+        waits for all that is ahead on the stream (positions, lengths, cache rows of earlier steps), so the other layers'
+        may read those before the kernels directly ahead of them have finished."""
         c, ctx, B, g = self.cfg, self.ctx, self.B, self.cfg.group
         D = c.head_dim
         if x_in is not None:
@@ -278,7 +280,7 @@ class SlowARStack:
                 ctx.qkv_attention_decode(self.qkv, lw["q_norm"], lw["k_norm"], c.eps, self.freqs, self.positions,
                                          self.k_cache, self.v_cache, self.block_table, self.seq_lens, None, B, self.nq_l,
                                          D, self.max_blocks, sm_scale, l, c.n_layer, self.nkv_l, quant_group_size=g,
-                                         Xq=self.aq, Xs=self.as_, context_splits=self.attn_splits)
+                                         Xq=self.aq, Xs=self.as_, context_splits=self.attn_splits, ahead=l > 0)
             else:
                 ctx.qknorm_rope_kvwrite(self.qkv, lw["q_norm"], lw["k_norm"], c.eps, self.freqs, self.positions,
                                         self.block_table, self.max_blocks, self.k_cache, self.v_cache, l, c.n_layer, B,
@@ -329,7 +331,7 @@ class SlowARStack:
             ctx.qkv_attention_decode(self.qkv, lw["q_norm"], lw["k_norm"], c.eps, self.freqs, self.positions,
                                      self.k_cache, self.v_cache, self.block_table, self.seq_lens, None, B, self.nq_l,
                                      D, self.max_blocks, sm_scale, l, c.n_layer, self.nkv_l, quant_group_size=g,
-                                     Xq=self.aq, Xs=self.as_, context_splits=self.attn_splits)
+                                     Xq=self.aq, Xs=self.as_, context_splits=self.attn_splits, ahead=l > 0)
         else:
             ctx.qknorm_rope_kvwrite(self.qkv, lw["q_norm"], lw["k_norm"], c.eps, self.freqs, self.positions,
                                     self.block_table, self.max_blocks, self.k_cache, self.v_cache, l, c.n_layer, B,

@@ -268,6 +268,19 @@ W8A8_API int w8a8_qkv_attention_decode(w8a8_ctx* ctx, const void* qkv, const voi
                               float sm_scale, int layer, int n_layers, int n_kv_heads, int quant_group_size,
                               void* Xq, void* Xs, int context_splits, void* stream);
 
+/* The same for a caller who states that everything the call reads except qkv (positions, seq_lens, block_table, the
+ * parameters, and this layer's cache rows of all tokens but the new one) was written ahead of an ordinary launch or copy,
+ * or of a w8a8_qkv_attention_decode / w8a8_paged_attention_decode call, that itself lies ahead of this call on the same
+ * stream. The kernel may then read them before the kernels directly ahead of it have finished: in a decode step the
+ * first layer calls w8a8_qkv_attention_decode and the others this one. Results are the same. Where the statement does not
+ * hold (e.g. two consecutive positions of one layer with no such launch between them) the result is undefined. */
+W8A8_API int w8a8_qkv_attention_decode_ahead(w8a8_ctx* ctx, const void* qkv, const void* q_norm_w,
+                                    const void* k_norm_w, float eps, const float* freqs, const int* positions,
+                                    void* k_cache, void* v_cache, const int* block_table, const int* seq_lens,
+                                    void* out, int batch, int n_heads, int head_dim, int max_blocks_per_seq,
+                                    float sm_scale, int layer, int n_layers, int n_kv_heads, int quant_group_size,
+                                    void* Xq, void* Xs, int context_splits, void* stream);
+
 /* ---- one decode step of the whole stack as one launch ------------------------------------------ */
 
 typedef struct w8a8_decode_layer {

@@ -136,3 +136,92 @@ def test_qkv_attention_decode_equals_the_two_calls(ctx, B, positions, splits):
     for w, gt, what in zip(want, got, ("attention output", "codes", "scales", "k cache", "v cache")):
         assert torch.equal(w.view(torch.uint8) if w.dtype != torch.int8 else w, gt.view(torch.uint8) if gt.dtype != torch.int8 else gt), what
     assert not torch.equal(got[3], dev(kc)), "the new k rows were written"
+
+
+def chained_setup(oracle, B, context, steps, max_blocks):
+    """`steps` consecutive tokens of one layer: their qkv rows, positions and lengths, all on the device before the first call."""
+    rng = np.random.default_rng(context + steps)
+    kc, vc, bt = make_cache(rng, B, context, max_blocks)
+    # values over the whole cache are as large as the new rows', so a row read before it was written shows
+    qkv = dev(rng.standard_normal((steps, B, (N_Q + 2 * N_KV) * D)).astype(np.float16))
+    pos = dev((context + np.arange(steps, dtype=np.int32)[:, None]).repeat(B, 1))
+    return dict(kc=kc, vc=vc, bt=dev(bt), qkv=qkv, pos=pos, seq=pos + 1, freqs=dev(oracle.rope_freqs(D, 1e6)),
+                w=dev(rng.uniform(0.5, 1.5, D).astype(np.float16)))
+
+
+@pytest.mark.parametrize("B,context,splits", [(1, 990, 0), (1, 1000, 4), (8, 500, 0), (1, 40, 1)])
+@pytest.mark.parametrize("writer", ["fused", "kvwrite", "mixed"])
+def test_consecutive_positions_back_to_back(ctx, oracle, B, context, splits, writer):
+    """Twenty consecutive positions of one layer with no other kernel between the calls, over a block boundary: each call reads the
+    rows that the one directly ahead writes. The same bits as with a synchronisation after every call."""
+    steps, max_blocks, layer, sm = 20, 128, 1, 1.0 / np.sqrt(D)
+    c = chained_setup(oracle, B, context, steps, max_blocks)
+
+    def run(sync):
+        dk, dv = dev(c["kc"]), dev(c["vc"])
+        out = torch.zeros((steps, B, N_Q, D), dtype=torch.float16, device="cuda")
+        q = torch.zeros((steps, B, N_Q, D), dtype=torch.float16, device="cuda")
+        torch.cuda.synchronize()
+        for i in range(steps):
+            if writer == "fused" or (writer == "mixed" and i % 2):
+                ctx.qkv_attention_decode(c["qkv"][i], c["w"], c["w"], 1e-6, c["freqs"], c["pos"][i], dk, dv, c["bt"], c["seq"][i], out[i],
+                                         B, N_Q, D, max_blocks, sm, layer, LAYERS, N_KV, context_splits=splits)
+            else:
+                ctx.qknorm_rope_kvwrite(c["qkv"][i], c["w"], c["w"], 1e-6, c["freqs"], c["pos"][i], c["bt"], max_blocks, dk, dv, layer,
+                                        LAYERS, B, N_Q, N_KV, D, q[i])
+                if writer == "mixed" or i % 3 == 2:  # (two writes ahead of one read, too)
+                    ctx.paged_attention_decode(q[i], dk, dv, c["bt"], c["seq"][i], out[i], B, N_Q, D, max_blocks, sm, layer, LAYERS,
+                                               N_KV, context_splits=splits)
+            if sync:
+                torch.cuda.synchronize()
+        torch.cuda.synchronize()
+        ctx.check_device_status()
+        return out, dk, dv
+
+    want = run(True)
+    for _ in range(3):
+        for w, g in zip(want, run(False)):
+            assert torch.equal(w.view(torch.int16), g.view(torch.int16))
+
+
+def test_prompt_written_then_read_at_once(ctx, oracle):
+    """A prompt's K and V written as one batch of positions of one sequence, the attention over them the next call."""
+    tokens, max_blocks, layer, sm = 900, 64, 2, 1.0 / np.sqrt(D)
+    rng = np.random.default_rng(5)
+    kc, vc, bt = make_cache(rng, 1, tokens, max_blocks)
+    dbt, dqkv = dev(bt), dev(rng.standard_normal((tokens, (N_Q + 2 * N_KV) * D)).astype(np.float16))
+    tables = dbt.expand(tokens, max_blocks).contiguous()
+    pos, seq = torch.arange(tokens, dtype=torch.int32, device="cuda"), torch.full((1,), tokens, dtype=torch.int32, device="cuda")
+    freqs, q = dev(oracle.rope_freqs(D, 1e6)), torch.empty((tokens, N_Q, D), dtype=torch.float16, device="cuda")
+    outs = []
+    for sync in (True, False, False):
+        dk, dv = dev(kc), dev(vc)
+        out = torch.empty((1, N_Q, D), dtype=torch.float16, device="cuda")
+        torch.cuda.synchronize()
+        ctx.qknorm_rope_kvwrite(dqkv, None, None, 1e-6, freqs, pos, tables, max_blocks, dk, dv, layer, LAYERS, tokens, N_Q, N_KV, D, q)
+        if sync:
+            torch.cuda.synchronize()
+        ctx.paged_attention_decode(q[-1], dk, dv, dbt, seq, out, 1, N_Q, D, max_blocks, sm, layer, LAYERS, N_KV)
+        torch.cuda.synchronize()
+        outs.append(out.view(torch.int16))
+    assert torch.equal(outs[0], outs[1]) and torch.equal(outs[0], outs[2])
+
+
+@pytest.mark.parametrize("B,positions,splits", [(1, [1937], 0), (8, [1024] * 8, 0), (3, [5, 300, 1000], 3)])
+def test_attention_ahead_equals_the_plain_call(ctx, oracle, B, positions, splits):
+    """The form that may read its inputs early, with all of them complete: the plain form's bits."""
+    rng = np.random.default_rng(B)
+    max_blocks, layer, sm = 128, 2, 1.0 / np.sqrt(D)
+    kc, vc, bt = make_cache(rng, B, max(positions), max_blocks)
+    qkv, w, fr = dev(rng.standard_normal((B, (N_Q + 2 * N_KV) * D)).astype(np.float16)), dev(rng.uniform(0.5, 1.5, D).astype(np.float16)), dev(oracle.rope_freqs(D, 1e6))
+    pos, seq, dbt = dev(np.array(positions, np.int32)), dev(np.array(positions, np.int32) + 1), dev(bt)
+    res = []
+    for ahead in (False, True):
+        dk, dv = dev(kc), dev(vc)
+        out, xq, xs = torch.empty((B, N_Q, D), dtype=torch.float16, device="cuda"), torch.empty((B, N_Q * D), dtype=torch.int8, device="cuda"), torch.empty((B, N_Q * D // 64), device="cuda")
+        torch.cuda.synchronize()
+        ctx.qkv_attention_decode(qkv, w, w, 1e-6, fr, pos, dk, dv, dbt, seq, out, B, N_Q, D, max_blocks, sm, layer, LAYERS, N_KV,
+                                 quant_group_size=64, Xq=xq, Xs=xs, context_splits=splits, ahead=ahead)
+        torch.cuda.synchronize()
+        res.append((out.view(torch.int16), xq, xs, dk.view(torch.int16), dv.view(torch.int16)))
+    assert all(torch.equal(a, b) for a, b in zip(*res))

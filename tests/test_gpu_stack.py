@@ -249,6 +249,36 @@ def test_one_launch_step_matches_the_chain_of_launches(ctx, group, dim, n_kv, in
     st.close()
 
 
+@pytest.mark.parametrize("layers,fuse_rope", [(1, True), (3, True), (2, False)])
+def test_steps_one_after_another_equal_synchronised_steps(ctx, monkeypatch, layers, fuse_rope):
+    """Twelve eager steps over a block boundary without a synchronisation: every step reads the cache rows and positions that the
+    steps ahead wrote, in the layers whose attention reads early too. The bits of steps that wait for each other."""
+    monkeypatch.setenv("W8A8_STACK_FUSE_ROPE", "1" if fuse_rope else "0")
+    cfg = S.SlowARConfig(n_layer=layers, dim=512, n_head=4, n_kv=1, inter=512, group=64)
+    st = S.SlowARStack(torch, ctx, cfg, 2, 500, max_new=16, seed=5)
+    x_in = torch.from_numpy(np.random.default_rng(layers).standard_normal((12, 2, cfg.dim)).astype(np.float16)).cuda()
+    k0, v0 = st.k_cache.clone(), st.v_cache.clone()
+    outs = []
+    for sync in (True, False, False):
+        st.reset_positions()
+        st.k_cache.copy_(k0); st.v_cache.copy_(v0)
+        got = []
+        for i in range(12):
+            if i % 3 == 2:  # (a step on the stream left by the step before, too)
+                st.decode_step()
+            else:
+                st.decode_step(x_in[i])
+            got.append(st.out.clone())
+            if sync:
+                torch.cuda.synchronize()
+        torch.cuda.synchronize()
+        ctx.check_device_status()
+        outs.append((torch.stack(got).view(torch.int16), st.k_cache.clone().view(torch.int16), st.v_cache.clone().view(torch.int16)))
+    for o in outs[1:]:
+        assert all(torch.equal(a, b) for a, b in zip(outs[0], o))
+    st.close()
+
+
 @pytest.mark.parametrize("tp,rank", [(2, 1), (4, 0), (4, 3), (8, 0), (8, 7)])
 @pytest.mark.parametrize("group", [256, 64])
 def test_every_tensor_parallel_shard_shape_runs(ctx, tp, rank, group):
