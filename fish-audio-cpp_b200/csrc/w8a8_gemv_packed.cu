@@ -51,6 +51,12 @@ bool gemv::make_plan(const LinearArgs& a, Plan& pl, bool rows) {
     } else if (quant) {
         if (a.M > 8 || !(a.g == 64 || a.g == 128 || a.g == 256) || a.dump || a.smooth_inv || a.act_scale) return false;
         if (a.tail_kind != kTailNone || a.tp.world > 0 || (reinterpret_cast<uintptr_t>(a.X) & 15u)) return false;
+        // CTAs that are done store rows of Y while others still quantise X: an output over the input (in place, N == K) needs
+        // the two launches, where all of X is codes before the first store.
+        const uintptr_t x0 = reinterpret_cast<uintptr_t>(a.X), y0 = reinterpret_cast<uintptr_t>(a.Y);
+        const size_t x_bytes = static_cast<size_t>(a.M) * a.K * 2;
+        const size_t y_bytes = static_cast<size_t>(a.M) * (a.epilogue == W8A8_EPI_SWIGLU ? a.N / 2 : a.N) * 2;
+        if (x0 < y0 + y_bytes && y0 < x0 + x_bytes) return false;
     } else {
         if (!a.Xq || !a.Xs) return false;
         if (reinterpret_cast<uintptr_t>(a.Xq) & 15u) return false;

@@ -792,6 +792,35 @@ def test_decode_linear_quantises_in_registers(ctx, oracle, pkg, M, N, K, g, pack
             ctx.register_packed_weight(dW, None)
 
 
+@pytest.mark.parametrize("packed", [True, False])
+@pytest.mark.parametrize("M", [1, 8])
+@pytest.mark.parametrize("shift", [0, 1280])
+def test_linear_over_its_own_input(ctx, oracle, pkg, M, shift, packed):
+    """Y over X, whole (N == K, in place) and over the last half of X's rows: all of X is read before the first output is stored."""
+    N = K = 2560
+    g = 256
+    X, W, ws = synth.linear_case(M + shift, M, N, K, g)
+    dW, dS = dev(W), dev(ws)
+    if packed:
+        P = torch.empty((ctx.packed_weight_bytes(N, K, g),), dtype=torch.uint8, device="cuda")
+        ctx.pack_weight(dW, dS, N, K, g, P)
+        ctx.register_packed_weight(dW, P, N, K, g)
+    try:
+        apart = torch.empty((M, N), dtype=torch.float16, device="cuda")
+        ctx.linear(dW, dS, g, dev(X), apart, M, N, K)
+        for _ in range(5):
+            buf = torch.zeros((M * K + shift,), dtype=torch.float16, device="cuda")
+            buf[:M * K] = dev(X).view(-1)
+            Y = buf[shift:shift + M * N].view(M, N)
+            ctx.linear(dW, dS, g, buf[:M * K].view(M, K), Y, M, N, K)
+            torch.cuda.synchronize()
+            ctx.check_device_status()
+            assert torch.equal(Y.view(torch.int16), apart.view(torch.int16))
+    finally:
+        if packed:
+            ctx.register_packed_weight(dW, None)
+
+
 @pytest.mark.parametrize("split_k", [1, 2, 3, 4, 5, 8])
 def test_gemv_split_k_is_deterministic_and_correct(ctx, oracle, pkg, split_k):
     M, N, K, g = 16, 320, 2560, 256
