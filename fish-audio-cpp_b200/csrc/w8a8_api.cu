@@ -424,6 +424,10 @@ int w8a8_linear(w8a8_ctx* ctx, const void* W, const void* w_scale, int group_siz
     LinearArgs a = make_args(W, w_scale, group_size, Y, M, N, K, opts);
     const int act_mode = opts ? opts->act_mode : W8A8_ACT_PER_TOKEN_GROUP;
     const int kernel = opts ? opts->kernel : W8A8_KERNEL_AUTO;
+    // (asked of every form, so that what fits a context does not depend on the form a shape gets)
+    const size_t need = quant_scratch_bytes(M, K, group_size);
+    if (need > ctx->workspace_bytes)
+        return fail(W8A8_ERR_WORKSPACE, "need %zu bytes of scratch, context has %zu", need, ctx->workspace_bytes);
 
     if (M <= 8 && act_mode == W8A8_ACT_PER_TOKEN_GROUP && !smooth_inv && !act_scale &&
         (kernel == W8A8_KERNEL_AUTO || kernel == W8A8_KERNEL_GEMV_PACKED)) {
@@ -438,9 +442,6 @@ int w8a8_linear(w8a8_ctx* ctx, const void* W, const void* w_scale, int group_siz
 
     // Codes and scales into the context's scratch (row kernel), then the integer kernel; the two are
     // chained with programmatic dependent launch, so the second starts streaming weights early.
-    const size_t need = quant_scratch_bytes(M, K, group_size);
-    if (need > ctx->workspace_bytes)
-        return fail(W8A8_ERR_WORKSPACE, "need %zu bytes of scratch, context has %zu", need, ctx->workspace_bytes);
     int8_t* Xq = reinterpret_cast<int8_t*>(ctx->workspace);
     float* Xs = reinterpret_cast<float*>(ctx->workspace + align256(static_cast<size_t>(M) * K));
     rc = launch_rowquant(static_cast<const __half*>(X), nullptr, nullptr, nullptr, 0.0f,

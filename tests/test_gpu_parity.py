@@ -821,6 +821,26 @@ def test_linear_over_its_own_input(ctx, oracle, pkg, M, shift, packed):
             ctx.register_packed_weight(dW, None)
 
 
+@pytest.mark.parametrize("packed", [True, False])
+@pytest.mark.parametrize("M,K,g", [(1, 2560, 256), (8, 2560, 64), (9, 2560, 64)])
+def test_linear_is_refused_where_its_scratch_does_not_fit(pkg, M, K, g, packed):
+    """One 256-byte step less than w8a8_workspace_bytes says: refused with nothing launched, whichever form the shape would get."""
+    N = 256
+    small = pkg.Context(0, pkg.load_library().w8a8_workspace_bytes(M, N, K, g) - 256)
+    W, S = torch.zeros((N, K), dtype=torch.int8, device="cuda"), torch.zeros((N, K // g), dtype=torch.float16, device="cuda")
+    X, buf = torch.zeros((M, K), dtype=torch.float16, device="cuda"), torch.full((M, N), 3.0, dtype=torch.float16, device="cuda")
+    if packed:
+        P = torch.empty((small.packed_weight_bytes(N, K, g),), dtype=torch.uint8, device="cuda")
+        small.pack_weight(W, S, N, K, g, P)
+        small.register_packed_weight(W, P, N, K, g)
+    with pytest.raises(pkg.W8A8Error) as e:
+        small.linear(W, S, g, X, buf, M, N, K)
+    assert e.value.status == 5  # W8A8_ERR_WORKSPACE
+    torch.cuda.synchronize()
+    assert bool((buf == 3.0).all())
+    small.close()
+
+
 @pytest.mark.parametrize("split_k", [1, 2, 3, 4, 5, 8])
 def test_gemv_split_k_is_deterministic_and_correct(ctx, oracle, pkg, split_k):
     M, N, K, g = 16, 320, 2560, 256
