@@ -587,8 +587,9 @@ __global__ void __launch_bounds__(128) groupquant_kernel(const __half* __restric
 #pragma unroll
         for (int i = 0; i < 8; ++i) v[i] = __half2float(h[i]);
         const unsigned c8 = (smooth_inv || act_scale) ? pc % K8 : 0u;  // piece inside its row
-        if (smooth_inv) {
-            const uint4 su = __ldg(reinterpret_cast<const uint4*>(smooth_inv) + c8);
+        // (Neither smoothing nor static scales are read by the rehearsal: they may be results of the launch ahead.)
+        if (smooth_inv && real) {
+            const uint4 su = *(reinterpret_cast<const uint4*>(smooth_inv) + c8);
             const __half* sh = reinterpret_cast<const __half*>(&su);
 #pragma unroll
             for (int i = 0; i < 8; ++i) v[i] *= __half2float(sh[i]);
@@ -598,7 +599,7 @@ __global__ void __launch_bounds__(128) groupquant_kernel(const __half* __restric
 #pragma unroll
         for (int o = LANES / 2; o > 0; o >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, o));
         if (!live) continue;
-        float scale = act_scale ? __half2float(act_scale[c8 / LANES]) : amax / 127.0f;
+        float scale = act_scale && real ? __half2float(act_scale[c8 / LANES]) : amax / 127.0f;
         if (scale < 1e-8f) scale = 1e-8f;
         if (real && (threadIdx.x & (LANES - 1)) == 0) Xs[pc / LANES] = scale;
         const uint2 cd = codes8(v, 1.0f / scale, act_scale != nullptr);

@@ -263,6 +263,29 @@ def test_quantize_flat_form(ctx, oracle, M, K, g, mode):
     assert np.array_equal(dq.cpu().numpy(), wq) and np.array_equal(ds.cpu().numpy(), wsc)
 
 
+@pytest.mark.parametrize("g", [64, 256])
+@pytest.mark.parametrize("what", ["smooth_inv", "act_scale"])
+def test_quantize_with_a_vector_made_by_the_launch_ahead(ctx, oracle, what, g):
+    """The smoothing vector, or the static scales, as the output of the library's own kernel directly ahead (which lets the
+    quantiser start early): the vector's new values are used, not those that its buffer held before."""
+    M, K = 8, 2560
+    n = K if what == "smooth_inv" else K // g
+    rng = np.random.default_rng(g)
+    X = synth.activations(rng, M, K)
+    src, ones = dev(rng.uniform(0.5, 2.0, (1, n)).astype(np.float16)), dev(np.ones(n, np.float16))
+    vec, dX = torch.full((1, n), 0.25, dtype=torch.float16, device="cuda"), dev(X)
+    for _ in range(10):
+        vec.fill_(0.25)
+        dq, ds = torch.empty((M, K), dtype=torch.int8, device="cuda"), torch.empty((M, K // g), dtype=torch.float32, device="cuda")
+        torch.cuda.synchronize()
+        ctx.quantize(dX, M, K, g, dq, ds, **{what: vec})  # (the old values into every SM's L1)
+        ctx.rms_norm(src, ones, vec, 1, n, 1e-6)
+        ctx.quantize(dX, M, K, g, dq, ds, **{what: vec})
+        torch.cuda.synchronize()
+        wq, wsc = oracle.quantize(X, g, **{what: vec.cpu().numpy().reshape(-1)})
+        assert np.array_equal(dq.cpu().numpy(), wq) and np.array_equal(ds.cpu().numpy(), wsc)
+
+
 # ---------------------------------------------------------------- linear (A3-A8)
 def run_linear(ctx, oracle, M, N, K, g, seed=0, fused_quant=True, **kw):
     X, W, ws = synth.linear_case(seed, M, N, K, g)
