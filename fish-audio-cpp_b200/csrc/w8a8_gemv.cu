@@ -25,6 +25,7 @@
 // activations is still running. Weights must not be written by that kernel.
 #include <cooperative_groups.h>
 
+#include "sm100_ptx.cuh"
 #include "w8a8_internal.h"
 
 namespace cg = cooperative_groups;
@@ -139,7 +140,7 @@ __global__ void __launch_bounds__(kThreads) gemv_kernel(const GemvParams p) {
         const float fa = __half2float(hsa), fb = __half2float(hsb);
 #pragma unroll
         for (int nt = 0; nt < MT; ++nt) {
-            const float x0 = __ldg(xsp[nt][0] + jl), x1 = __ldg(xsp[nt][1] + jl);
+            const float x0 = ptx::ld_result_f32(xsp[nt][0] + jl), x1 = ptx::ld_result_f32(xsp[nt][1] + jl);
             if (a.dump) {
                 const int t0 = nt * 8 + 2 * c, j = j0 + jl;
                 const size_t NG = static_cast<size_t>(a.N) * a.G;
@@ -172,7 +173,7 @@ __global__ void __launch_bounds__(kThreads) gemv_kernel(const GemvParams p) {
 #pragma unroll
                 for (int nt = 0; nt < MT; ++nt)
                     if (blk * 4 + i0 + i < total_chunks)
-                        xv[i][nt] = __ldg(reinterpret_cast<const uint4*>(xq[nt] + (blk * 4 + i0 + i) * 64));
+                        xv[i][nt] = ptx::ld_result_v4(xq[nt] + (blk * 4 + i0 + i) * 64);
 #pragma unroll
             for (int ii = 0; ii < XB; ++ii) {
                 const int i = i0 + ii;

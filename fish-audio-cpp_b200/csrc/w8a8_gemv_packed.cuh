@@ -773,7 +773,7 @@ __device__ __forceinline__ void gemv_body(const GemvPackedParams& p, const CUten
         for (int nt = 0; nt < MT; ++nt) {
             if constexpr (FUSED) x[buf][ch][nt] = lds128(xq_s + kbase + ch * 64);
             else if (W8A8_ABLATED(1)) x[buf][ch][nt] = make_uint4(0x01010101u, 0x01010101u, 0x01010101u, 0x01010101u);
-            else x[buf][ch][nt] = __ldg(reinterpret_cast<const uint4*>(xq[nt] + kbase + ch * 64));
+            else x[buf][ch][nt] = ptx::ld_result_v4(xq[nt] + kbase + ch * 64);
         }
     };
     auto load_xs = [&](int unit_b, int q, int buf) {
@@ -783,7 +783,7 @@ __device__ __forceinline__ void gemv_body(const GemvPackedParams& p, const CUten
             for (int e = 0; e < 2; ++e) {
                 if constexpr (FUSED) xs[buf][q][nt][e] = xsp_s[e][unit_b * GPU + q];
                 else if (W8A8_ABLATED(2)) xs[buf][q][nt][e] = 1.0f;
-                else xs[buf][q][nt][e] = __ldg(xsp[nt][e] + unit_b * GPU + q);
+                else xs[buf][q][nt][e] = ptx::ld_result_f32(xsp[nt][e] + unit_b * GPU + q);
             }
     };
     // The scales of a unit at once: a word of two or four where the instance may (the host checks the address).
@@ -796,8 +796,8 @@ __device__ __forceinline__ void gemv_body(const GemvPackedParams& p, const CUten
                 for (int e = 0; e < 2; ++e) {
                     const float* s = xsp[nt][e] + unit_b * GPU;
                     __align__(16) float v[4];
-                    if constexpr (GPU == 4) *reinterpret_cast<float4*>(v) = __ldg(reinterpret_cast<const float4*>(s));
-                    else *reinterpret_cast<float2*>(v) = __ldg(reinterpret_cast<const float2*>(s));
+                    if constexpr (GPU == 4) *reinterpret_cast<uint4*>(v) = ptx::ld_result_v4(s);
+                    else *reinterpret_cast<uint2*>(v) = ptx::ld_result_v2(s);
 #pragma unroll
                     for (int q = 0; q < GPU; ++q) xs[buf][q][nt][e] = v[q];
                 }
@@ -811,7 +811,7 @@ __device__ __forceinline__ void gemv_body(const GemvPackedParams& p, const CUten
     auto load_raw = [&](int kbase) {
         const __half* src = a.X + static_cast<size_t>(min(gq, a.M - 1)) * a.K + kbase + c * 16;
 #pragma unroll
-        for (int i = 0; i < 8; ++i) raw[i] = __ldg(reinterpret_cast<const uint4*>(src + (i >> 1) * 64) + (i & 1));
+        for (int i = 0; i < 8; ++i) raw[i] = ptx::ld_result_v4(src + (i >> 1) * 64 + (i & 1) * 8);
     };
     auto quantise = [&]() {  // raw -> codes in x[0], scales of tokens 2c and 2c + 1 in xs[0] (int8_gemm.cu:147-211)
         float am[GPU];

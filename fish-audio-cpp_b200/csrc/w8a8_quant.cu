@@ -10,6 +10,7 @@
 // bit-identical to those of the unfused reference chain.
 #include <cstdlib>
 
+#include "sm100_ptx.cuh"
 #include "w8a8_internal.h"
 #include "w8a8_trace.cuh"
 
@@ -559,11 +560,8 @@ __global__ void __launch_bounds__(128, KI > 10 ? 4 : 5) rownorm_warp_kernel(cons
 // few KB, and what counts is the length of the dependency chain (one load, log2(g/8) shuffles, one divide, one store): one
 // piece per thread (U = 1). At prefill sizes it is bandwidth: four loads in flight per thread (8192 x 9728: 86 -> 37 us, 6.5 TB/s).
 template <int LANES, int U>  // LANES: threads per group = g / 8
-__global__ void __launch_bounds__(128) groupquant_kernel(const __half* __restrict__ X,
-                                                         const __half* __restrict__ smooth_inv,
-                                                         const __half* __restrict__ act_scale,
-                                                         int8_t* __restrict__ Xq, float* __restrict__ Xs, unsigned pieces,
-                                                         unsigned K8) {
+__global__ void __launch_bounds__(128) groupquant_kernel(const __half* X, const __half* smooth_inv, const __half* act_scale,
+                                                         int8_t* Xq, float* Xs, unsigned pieces, unsigned K8) {
     W8A8_TRACE_SCOPE();
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 #pragma unroll 1
@@ -577,7 +575,7 @@ __global__ void __launch_bounds__(128) groupquant_kernel(const __half* __restric
     uint4 u[U];
 #pragma unroll
     for (int k = 0; k < U; ++k)  // (a whole group is live or not: pieces is a multiple of LANES)
-        u[k] = real && p0 + k * 128u < pieces ? *(reinterpret_cast<const uint4*>(X) + p0 + k * 128u) : make_uint4(0, 0, 0, 0);
+        u[k] = real && p0 + k * 128u < pieces ? ptx::ld_result_v4(reinterpret_cast<const uint4*>(X) + p0 + k * 128u) : make_uint4(0, 0, 0, 0);
 #pragma unroll
     for (int k = 0; k < U; ++k) {
         const unsigned pc = p0 + k * 128u;
