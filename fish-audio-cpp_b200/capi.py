@@ -89,6 +89,8 @@ def load_library() -> C.CDLL:
         "w8a8_rmsnorm_linear": (I, [P, P, P, I, P, P, P, P, F, P, I, I, I, C.POINTER(LinearOpts), P, P, P]),
         "w8a8_linear_q_tail": (I, [P, P, P, I, P, P, P, I, I, I, C.POINTER(LinearOpts), C.POINTER(Tail), P]),
         "w8a8_debug_tail_counters": (I, [P, P, I, P]),
+        "w8a8_debug_force_gemm_form": (I, [P, I, I]),
+        "w8a8_debug_gemm_form": (I, [I, I, I, I, I, I, I, I, P]),
         "w8a8_pack_gate_up": (I, [P, P, P, P, P, I, I, I, P, P, P]),
         "w8a8_decode_stack_workspace_bytes": (Z, [C.POINTER(DecodeStack)]),
         "w8a8_decode_stack_step": (I, [P, C.POINTER(DecodeStack), P]),
@@ -124,7 +126,8 @@ EXPORTS = [
     "w8a8_status_string", "w8a8_last_error", "w8a8_create", "w8a8_destroy", "w8a8_workspace_bytes",
     "w8a8_ctx_workspace_bytes", "w8a8_check_device_status", "w8a8_quantize", "w8a8_rms_norm",
     "w8a8_rmsnorm_quantize", "w8a8_silu", "w8a8_mul", "w8a8_residual_add", "w8a8_linear", "w8a8_linear_q",
-    "w8a8_rmsnorm_linear", "w8a8_linear_q_tail", "w8a8_debug_tail_counters", "w8a8_decode_stack_workspace_bytes", "w8a8_decode_stack_step",
+    "w8a8_rmsnorm_linear", "w8a8_linear_q_tail", "w8a8_debug_tail_counters", "w8a8_debug_force_gemm_form", "w8a8_debug_gemm_form",
+    "w8a8_decode_stack_workspace_bytes", "w8a8_decode_stack_step",
     "w8a8_decode_stack_timeline",
     "w8a8_pack_gate_up", "w8a8_qknorm_rope_kvwrite", "w8a8_paged_attention_decode", "w8a8_qkv_attention_decode",
     "w8a8_qkv_attention_decode_ahead", "w8a8_tp_create", "w8a8_tp_connect",
@@ -210,6 +213,13 @@ def static_scratch_check_status(stream=None):
     rc = lib.w8a8_static_scratch_check_status(_stream(stream))
     if rc != 0:
         raise W8A8Error(rc, "w8a8_static_scratch_check_status", lib.w8a8_last_error().decode())
+
+
+def debug_gemm_form(M, N, K, group_size, sms=148, kernel=KERNEL_GEMM, token_width=0, splits=0):
+    """(tokens per tile, CTAs per tile's rows, CTAs along its K) of the tcgen05 GEMM, or None where no form takes the shape."""
+    out = (C.c_int * 3)()
+    rc = load_library().w8a8_debug_gemm_form(M, N, K, group_size, sms, kernel, token_width, splits, out)
+    return None if rc else tuple(out)
 
 
 class Context:
@@ -306,6 +316,9 @@ class Context:
         buf = (C.c_int * count)()
         self._check(self.lib.w8a8_debug_tail_counters(self.handle, buf, count, _stream(stream)), "w8a8_debug_tail_counters")
         return list(buf)
+
+    def debug_force_gemm_form(self, token_width=0, splits=0):
+        self._check(self.lib.w8a8_debug_force_gemm_form(self.handle, token_width, splits), "w8a8_debug_force_gemm_form")
 
     def rmsnorm_linear(self, W, w_scale, group_size, x, norm_weight, eps, Y, M, N, K, residual=None, x_out=None,
                        epilogue=EPI_NONE, epi_residual=None, kernel=KERNEL_AUTO, act_mode=ACT_PER_TOKEN_GROUP,

@@ -21,6 +21,7 @@ struct w8a8_ctx {
     };
     std::unordered_map<const void*, PackedEntry> packed;
     std::mutex packed_mu;
+    int gemm_bt = 0, gemm_splits = 0;  // w8a8_debug_force_gemm_form
     int* tail_counters = nullptr;     // arrival counters of the decode kernel's tails, zero between launches
     w8a8::TpState* tp = nullptr;  // tensor-parallel exchange, when w8a8_tp_create was called
 };
@@ -131,6 +132,8 @@ int dispatch_linear_q(const LinearArgs& a, int kernel, int* device_status, cudaS
 // Points the arguments at the context's tail counters and at the packed image of the weight, if registered.
 static void fill_scratch(w8a8_ctx* ctx, LinearArgs& a) {
     a.tail_counters = ctx->tail_counters;
+    a.gemm_bt = ctx->gemm_bt;
+    a.gemm_splits = ctx->gemm_splits;
     if (a.M <= 32 && !ctx->packed.empty()) {
         std::lock_guard<std::mutex> lock(ctx->packed_mu);
         auto it = ctx->packed.find(a.W);
@@ -596,6 +599,21 @@ int w8a8_debug_tail_counters(w8a8_ctx* ctx, int* out, int count, void* stream) {
     if (e == cudaSuccess) e = cudaStreamSynchronize(s);
     if (e != cudaSuccess) return fail(W8A8_ERR_CUDA, "counter read: %s", cudaGetErrorString(e));
     return W8A8_OK;
+}
+
+int w8a8_debug_force_gemm_form(w8a8_ctx* ctx, int token_width, int splits) {
+    if (!ctx || token_width < 0 || splits < 0) return fail(W8A8_ERR_INVALID_ARG, "debug_force_gemm_form: bad arguments");
+    ctx->gemm_bt = token_width;
+    ctx->gemm_splits = splits;
+    return W8A8_OK;
+}
+
+int w8a8_debug_gemm_form(int M, int N, int K, int group_size, int sms, int kernel, int token_width, int splits, int* form_out3) {
+    if (!form_out3 || (kernel != W8A8_KERNEL_GEMM && kernel != W8A8_KERNEL_GEMM_SINGLE && kernel != W8A8_KERNEL_GEMM_PAIR))
+        return fail(W8A8_ERR_INVALID_ARG, "debug_gemm_form: bad arguments");
+    const int pair = kernel == W8A8_KERNEL_GEMM ? -1 : kernel == W8A8_KERNEL_GEMM_PAIR;
+    const int rc = gemm_form(M, N, K, norm_group(K, group_size), sms, pair, token_width, splits, form_out3);
+    return rc ? fail(rc, "no tile form of the tcgen05 GEMM for this shape") : W8A8_OK;
 }
 
 size_t w8a8_packed_weight_bytes(int N, int K, int group_size) { return packed_weight_bytes(N, K, group_size); }

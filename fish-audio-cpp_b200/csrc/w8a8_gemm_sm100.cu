@@ -1,6 +1,4 @@
 // Chooses and launches the tcgen05 GEMM (kernel and its reasons: w8a8_gemm_sm100.cuh).
-#include <cstdlib>
-
 #include "w8a8_gemm_sm100.cuh"
 
 namespace w8a8 {
@@ -19,6 +17,48 @@ const Form* forms(int g, int* count) {
     return g == 64 ? forms_g64(count) : g == 128 ? forms_g128(count) : g == 256 ? forms_g256(count) : forms_any(count);
 }
 
+// Stages of 128 bytes that each CTA of a split takes: whole K-groups.
+int split_kb(int K, int g, int splits) {
+    const int unit = g > BK ? g / BK : 1;
+    return (K / BK / unit + splits - 1) / splits * unit;
+}
+
+struct Choice {
+    const Form* form;
+    int splits;
+};
+
+// The tile form that ends first: whole waves of tiles over the SMs (or pairs), each tile at its measured cost. A width
+// that leaves the last wave nearly empty loses to one that fills it; narrow tiles win where there are few tokens.
+// A tile's K is split over two or four CTAs where all of them fit the chip at once (a cluster of four leaves some SMs of a
+// GPC over: 128 of 148 taken as usable); meeting and adding up measured 3-4 us for two and about 6 for four. A
+// split adds the groups in another order than the other kernels do, so it has to save 15 % at least (K = 2560 never does).
+// table_g: the group size whose forms are looked at (0: those of any group size). pair: -1 either, 0 one CTA per tile, 1 a pair.
+// only_bt, only_splits: 0, or the token width and the split (1: none) to take; no form where they do not fit the shape.
+Choice choose(int M, int N, int K, int table_g, int g, int sms, int pair, int only_bt, int only_splits) {
+    int count = 0;
+    const Form* table = forms(table_g, &count);
+    Choice best = {nullptr, 1};
+    double best_ns = 0;
+    for (int i = 0; i < count; ++i) {
+        const Form& f = table[i];
+        if (pair >= 0 && (f.pair != (pair != 0) || f.split)) continue;
+        if (only_bt && f.bt != only_bt) continue;
+        const int rows = f.pair ? 2 * BR : BR, walkers = f.pair ? sms / 2 : sms, kb_total = K / BK;
+        const long tiles = static_cast<long>((M + f.bt - 1) / f.bt) * ((N + rows - 1) / rows);
+        for (int splits = f.split ? 2 : 1; splits <= (f.split ? 4 : 1); splits *= 2) {
+            if (only_splits && splits != only_splits) continue;
+            if (f.split && (tiles * splits > (splits == 2 ? sms / 2 * 2 : sms * 7 / 8 - 1) || (splits - 1) * split_kb(K, g, splits) >= kb_total))
+                continue;
+            const double kb = f.split ? split_kb(K, g, splits) : kb_total;
+            double ns = ((tiles * splits + walkers - 1) / walkers) * (kb * f.stage_ns + kb * BK / g * f.group_ns);
+            if (f.split) ns = (ns + (splits == 2 ? 3500 : 6000)) / 0.85;
+            if (!best.form || ns < best_ns) { best = {&f, splits}; best_ns = ns; }
+        }
+    }
+    return best;
+}
+
 }  // namespace
 }  // namespace gemm
 
@@ -32,45 +72,27 @@ bool gemm_supports(const LinearArgs& a) {
     return true;
 }
 
+int gemm_form(int M, int N, int K, int g, int sms, int form, int only_bt, int only_splits, int* out3) {
+    using namespace gemm;
+    if (M < 1 || N < 1 || K < 1 || sms < 2 || K % BK != 0 || g % 32 != 0 || K % g != 0) return W8A8_ERR_UNSUPPORTED;
+    const Choice c = choose(M, N, K, g, g, sms, form, only_bt, only_splits);
+    if (!c.form) return W8A8_ERR_UNSUPPORTED;
+    out3[0] = c.form->bt;
+    out3[1] = c.form->pair ? 2 : 1;
+    out3[2] = c.splits;
+    return W8A8_OK;
+}
+
 int launch_linear_gemm(const LinearArgs& a, int* device_status, cudaStream_t stream, int form) {
     using namespace gemm;
     if (!gemm_supports(a)) return fail(W8A8_ERR_UNSUPPORTED, "tcgen05 GEMM does not take this shape");
     const int sms = device_sms();
 
-    int count = 0;
-    const Form* table = forms(a.dump ? 0 : a.g, &count);
-    const Form* best = nullptr;
-    double best_ns = 0;
-    int best_splits = 1;
-    // The tile form that ends first: whole waves of tiles over the SMs (or pairs), each tile at its measured cost. A width
-    // that leaves the last wave nearly empty loses to one that fills it; narrow tiles win where there are few tokens.
-    // A tile's K is split over two or four CTAs where all of them fit the chip at once (a cluster of four leaves some SMs of a
-    // GPC over: 128 of 148 taken as usable); meeting and adding up measured 3-4 us for two and about 6 for four. A
-    // split adds the groups in another order than the other kernels do, so it has to save 15 % at least (K = 2560 never does).
-    // (W8A8_GEMM_BT, W8A8_GEMM_SPLIT: take this token width, this split, where the form asked for has it.)
-    const char* env = std::getenv("W8A8_GEMM_BT");
-    const int only_bt = env ? std::atoi(env) : 0;
-    const char* env_split = std::getenv("W8A8_GEMM_SPLIT");
-    const int only_split = env_split ? std::atoi(env_split) : 0;
-    const int unit = a.g > BK ? a.g / BK : 1, kb_total = a.K / BK;  // a split takes whole K-groups
-    auto split_kb = [&](int splits) { return (kb_total / unit + splits - 1) / splits * unit; };
-    for (int pass = only_bt || only_split ? 0 : 1; pass < 2 && !best; ++pass)
-        for (int i = 0; i < count; ++i) {
-            const Form& f = table[i];
-            if (form >= 0 && (f.pair != (form != 0) || f.split)) continue;
-            if (pass == 0 && only_bt && f.bt != only_bt) continue;
-            const int rows = f.pair ? 2 * BR : BR, walkers = f.pair ? sms / 2 : sms;
-            const long tiles = static_cast<long>((a.M + f.bt - 1) / f.bt) * ((a.N + rows - 1) / rows);
-            for (int splits = f.split ? 2 : 1; splits <= (f.split ? 4 : 1); splits *= 2) {
-                if (pass == 0 && only_split && splits != only_split) continue;
-                if (f.split && (tiles * splits > (splits == 2 ? sms / 2 * 2 : sms * 7 / 8 - 1) || (splits - 1) * split_kb(splits) >= kb_total)) continue;
-                const double kb = f.split ? split_kb(splits) : kb_total;
-                double ns = ((tiles * splits + walkers - 1) / walkers) * (kb * f.stage_ns + kb * BK / a.g * f.group_ns);
-                if (f.split) ns = (ns + (splits == 2 ? 3500 : 6000)) / 0.85;
-                if (!best || ns < best_ns) { best = &f; best_ns = ns; best_splits = splits; }
-            }
-        }
-    if (!best) return fail(W8A8_ERR_UNSUPPORTED, "no tile form of the tcgen05 GEMM");
+    const Choice choice = choose(a.M, a.N, a.K, a.dump ? 0 : a.g, a.g, sms, form, a.gemm_bt, a.gemm_splits);
+    const Form* best = choice.form;
+    const int best_splits = choice.splits;
+    if (!best) return fail(W8A8_ERR_UNSUPPORTED, "no tile form of the tcgen05 GEMM for this shape (token width %d, splits %d asked for)",
+                           a.gemm_bt, a.gemm_splits);
 
     const int bt = best->bt, rows = best->pair ? 2 * BR : BR;
     CUtensorMap map_w, map_x, map_y;
@@ -86,7 +108,7 @@ int launch_linear_gemm(const LinearArgs& a, int* device_status, cudaStream_t str
     p.tiles_m = (a.M + bt - 1) / bt;
     p.tiles_total = p.tiles_m * ((a.N + rows - 1) / rows);
     p.splits = best_splits;
-    p.split_kb = split_kb(best_splits);
+    p.split_kb = split_kb(a.K, a.g, best_splits);
     p.tma_store = ycols % 8 == 0 && (reinterpret_cast<uintptr_t>(a.Y) & 15u) == 0;
     map_y = map_x;  // (a valid map in either case; only the TMA store reads it)
     if (p.tma_store) {

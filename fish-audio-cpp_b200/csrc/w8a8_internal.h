@@ -89,6 +89,7 @@ struct LinearArgs {
     int M, N, K, g, G;
     int epilogue;
     int split_k;
+    int gemm_bt, gemm_splits;  // 0, or the token width and the split of K that the tcgen05 GEMM has to take
     const void* packed;     // the weight re-packed by launch_pack_weight (null: not packed)
     // Fused prologue (packed GEMV, M <= 8): norm_weight != null means that Xq / Xs are absent and every CTA
     // forms them itself in shared memory from X: [x = half(x + norm_residual)] -> RMSNorm -> quantiser.
@@ -178,5 +179,6 @@ int launch_tp_allreduce_rowquant(TpState* t, __half* x, const __half* partial, c
 bool gemm_supports(const LinearArgs& a);
 // form: -1 picks between one CTA per tile (0) and a CTA pair per tile (1) by shape
 int launch_linear_gemm(const LinearArgs& a, int* device_status, cudaStream_t s, int form = -1);
+int gemm_form(int M, int N, int K, int g, int sms, int form, int only_bt, int only_splits, int* out3);  // what it would take
 
 }  // namespace w8a8

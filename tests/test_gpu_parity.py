@@ -674,14 +674,24 @@ def test_prefill_shapes_full_size(ctx, oracle, pkg, name, g, M):
     assert np.array_equal(got.view(np.uint16), want.view(np.uint16))
 
 
+@pytest.fixture
+def gemm_form(ctx):
+    """The context with the tcgen05 GEMM held to a token width and a split of K (a call that has no such form is refused)."""
+    def hold(token_width, splits):
+        ctx.debug_force_gemm_form(token_width, splits)
+        return ctx
+    yield hold
+    ctx.debug_force_gemm_form(0, 0)
+
+
 @pytest.mark.parametrize("g", [64, 128, 256])
 @pytest.mark.parametrize("bt,form", [(32, "SINGLE"), (64, "SINGLE"), (96, "SINGLE"), (128, "SINGLE"), (192, "PAIR"), (256, "PAIR")])
 @pytest.mark.parametrize("M,N,K", [(1, 136, 256), (257, 272, 1280), (383, 40, 768)])
-def test_gemm_tcgen05_tile_widths(ctx, oracle, pkg, monkeypatch, M, N, K, bt, form, g):
+def test_gemm_tcgen05_tile_widths(gemm_form, oracle, pkg, M, N, K, bt, form, g):
     """Every token width of a tile: one token, tiles that end one past or one short of a width, rows that end inside a
     warp's 32, K of 2, 6 and 10 stages (the ring of stages and the ring of scale chunks wrap at other places than the
     tiles do), an odd and an even number of groups. Bit for bit the oracle's."""
-    monkeypatch.setenv("W8A8_GEMM_BT", str(bt))
+    ctx = gemm_form(bt, 1)
     X, W, ws = synth.linear_case(M + N + K + bt, M, N, K, g)
     Xq, Xs = oracle.quantize(X, g)
     buf, dY = guarded((M, N), torch.float16, 99.0)
@@ -696,14 +706,19 @@ def test_gemm_tcgen05_tile_widths(ctx, oracle, pkg, monkeypatch, M, N, K, bt, fo
 @pytest.mark.parametrize("splits", [2, 4])
 @pytest.mark.parametrize("bt", [32, 64, 96, 128])
 @pytest.mark.parametrize("M,N,K", [(33, 136, 1024), (97, 40, 1280), (150, 272, 2816)])
-def test_gemm_tcgen05_split_k(ctx, oracle, pkg, monkeypatch, M, N, K, bt, splits, g):
+def test_gemm_tcgen05_split_k(gemm_form, oracle, pkg, M, N, K, bt, splits, g):
     """A tile's K over two or four CTAs: runs of one K-group and of many, a last run that is shorter, ragged tokens and rows. The
-    sums are the whole-K kernel's, added in another order (the bar with the sum of absolute terms covers that)."""
-    monkeypatch.setenv("W8A8_GEMM_BT", str(bt))
-    monkeypatch.setenv("W8A8_GEMM_SPLIT", str(splits))
+    sums are the whole-K kernel's, added in another order (the bar with the sum of absolute terms covers that). The form is taken
+    or the call is refused; five groups are not four runs of whole groups."""
+    ctx = gemm_form(bt, splits)
     X, W, ws = synth.linear_case(M + N + K + bt, M, N, K, g)
     Xq, Xs = oracle.quantize(X, g)
     buf, dY = guarded((M, N), torch.float16, 99.0)
+    if K // g == 5 and splits == 4:
+        with pytest.raises(pkg.W8A8Error) as e:
+            ctx.linear_q(dev(W), dev(ws), g, dev(Xq), dev(Xs), dY, M, N, K)
+        assert e.value.status == 2  # W8A8_ERR_UNSUPPORTED
+        return
     ctx.linear_q(dev(W), dev(ws), g, dev(Xq), dev(Xs), dY, M, N, K)
     torch.cuda.synchronize()
     ctx.check_device_status()

@@ -69,6 +69,27 @@ def test_null_context_is_rejected(pkg):
     assert lib.w8a8_destroy(None) == 0
 
 
+def test_gemm_form_follows_what_is_asked_for(pkg):
+    """The rule that picks the tcgen05 GEMM's form, on the host: a width or split that is asked for is taken or refused, never
+    replaced; one CTA per tile and pairs keep to their widths."""
+    assert pkg.debug_gemm_form(8192, 19456, 2560, 256)[0] in (192, 256)
+    assert pkg.debug_gemm_form(33, 2560, 9728, 64)[2] > 1, "few tiles and a long K: split"
+    for g in (64, 128, 256):
+        for bt in (32, 64, 96, 128):
+            assert pkg.debug_gemm_form(150, 2560, 2560, g, token_width=bt, splits=1) == (bt, 1, 1)
+            assert pkg.debug_gemm_form(150, 2560, 2560, g, token_width=bt, kernel=pkg.KERNEL_GEMM_PAIR) is None
+            assert pkg.debug_gemm_form(33, 136, 1024, g, token_width=bt, splits=2) == (bt, 1, 2)
+            # K = 1280 in groups of 256 is five groups: four runs of whole groups would leave the last one empty
+            want = None if g == 256 else (bt, 1, 4)
+            assert pkg.debug_gemm_form(97, 40, 1280, g, token_width=bt, splits=4) == want
+        for bt in (192, 256):
+            assert pkg.debug_gemm_form(150, 2560, 2560, g, token_width=bt) == (bt, 2, 1)
+            assert pkg.debug_gemm_form(150, 2560, 2560, g, token_width=bt, splits=2) is None
+    assert pkg.debug_gemm_form(8192, 2560, 9728, 64, splits=2) is None, "more tiles than the chip holds at once"
+    assert pkg.debug_gemm_form(150, 2560, 2560, 256, token_width=100) is None
+    assert pkg.debug_gemm_form(150, 2560, 2500, 250) is None
+
+
 def test_product_never_touches_the_oracle():
     """Nothing under the package may import, link or read oracle/ (checker only)."""
     pat = re.compile(r"(^|\s)(import|from)\s+oracle\b|oracle/|w8a8o_|libw8a8_oracle|fishref")
