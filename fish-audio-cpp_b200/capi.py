@@ -90,7 +90,7 @@ def load_library() -> C.CDLL:
         "w8a8_linear_q_tail": (I, [P, P, P, I, P, P, P, I, I, I, C.POINTER(LinearOpts), C.POINTER(Tail), P]),
         "w8a8_debug_tail_counters": (I, [P, P, I, P]),
         "w8a8_debug_force_gemm_form": (I, [P, I, I]),
-        "w8a8_debug_gemm_form": (I, [I, I, I, I, I, I, I, I, P]),
+        "w8a8_debug_gemm_form": (I, [I, I, I, I, I, I, I, I, I, P]),
         "w8a8_pack_gate_up": (I, [P, P, P, P, P, I, I, I, P, P, P]),
         "w8a8_decode_stack_workspace_bytes": (Z, [C.POINTER(DecodeStack)]),
         "w8a8_decode_stack_step": (I, [P, C.POINTER(DecodeStack), P]),
@@ -215,10 +215,10 @@ def static_scratch_check_status(stream=None):
         raise W8A8Error(rc, "w8a8_static_scratch_check_status", lib.w8a8_last_error().decode())
 
 
-def debug_gemm_form(M, N, K, group_size, sms=148, kernel=KERNEL_GEMM, token_width=0, splits=0):
+def debug_gemm_form(M, N, K, group_size, sms=148, kernel=KERNEL_GEMM, token_width=0, splits=0, moved_registers=True):
     """(tokens per tile, CTAs per tile's rows, CTAs along its K) of the tcgen05 GEMM, or None where no form takes the shape."""
     out = (C.c_int * 3)()
-    rc = load_library().w8a8_debug_gemm_form(M, N, K, group_size, sms, kernel, token_width, splits, out)
+    rc = load_library().w8a8_debug_gemm_form(M, N, K, group_size, sms, kernel, token_width, splits, int(moved_registers), out)
     return None if rc else tuple(out)
 
 

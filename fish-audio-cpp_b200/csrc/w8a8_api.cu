@@ -608,11 +608,12 @@ int w8a8_debug_force_gemm_form(w8a8_ctx* ctx, int token_width, int splits) {
     return W8A8_OK;
 }
 
-int w8a8_debug_gemm_form(int M, int N, int K, int group_size, int sms, int kernel, int token_width, int splits, int* form_out3) {
+int w8a8_debug_gemm_form(int M, int N, int K, int group_size, int sms, int kernel, int token_width, int splits, int moved_registers,
+                         int* form_out3) {
     if (!form_out3 || (kernel != W8A8_KERNEL_GEMM && kernel != W8A8_KERNEL_GEMM_SINGLE && kernel != W8A8_KERNEL_GEMM_PAIR))
         return fail(W8A8_ERR_INVALID_ARG, "debug_gemm_form: bad arguments");
     const int pair = kernel == W8A8_KERNEL_GEMM ? -1 : kernel == W8A8_KERNEL_GEMM_PAIR;
-    const int rc = gemm_form(M, N, K, norm_group(K, group_size), sms, pair, token_width, splits, form_out3);
+    const int rc = gemm_form(M, N, K, norm_group(K, group_size), sms, pair, token_width, splits, moved_registers != 0, form_out3);
     return rc ? fail(rc, "no tile form of the tcgen05 GEMM for this shape") : W8A8_OK;
 }
 

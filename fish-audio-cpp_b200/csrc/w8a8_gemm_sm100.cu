@@ -23,6 +23,23 @@ int split_kb(int K, int g, int splits) {
     return (K / BK / unit + splits - 1) / splits * unit;
 }
 
+// setmaxnreg moves registers between the warpgroups of the widest form; the sums balance only for the register count the kernel
+// was compiled to (kLaunchRegs per thread). An unbalanced sum blocks for ever in setmaxnreg.inc, a wait nothing bounds, so in a
+// build that came out differently that form is not taken.
+bool balanced(const Form& f) {
+    if (!f.move_regs) return true;
+    int r = f.state->registers.load(std::memory_order_relaxed);
+    if (r == 0) {
+        cudaFuncAttributes fa;
+        if (cudaFuncGetAttributes(&fa, f.kernel) != cudaSuccess) {
+            cudaGetLastError();
+            return false;
+        }
+        f.state->registers.store(r = fa.numRegs, std::memory_order_relaxed);
+    }
+    return r == kLaunchRegs;
+}
+
 struct Choice {
     const Form* form;
     int splits;
@@ -35,7 +52,8 @@ struct Choice {
 // split adds the groups in another order than the other kernels do, so it has to save 15 % at least (K = 2560 never does).
 // table_g: the group size whose forms are looked at (0: those of any group size). pair: -1 either, 0 one CTA per tile, 1 a pair.
 // only_bt, only_splits: 0, or the token width and the split (1: none) to take; no form where they do not fit the shape.
-Choice choose(int M, int N, int K, int table_g, int g, int sms, int pair, int only_bt, int only_splits) {
+template <class Usable>
+Choice choose(int M, int N, int K, int table_g, int g, int sms, int pair, int only_bt, int only_splits, Usable usable) {
     int count = 0;
     const Form* table = forms(table_g, &count);
     Choice best = {nullptr, 1};
@@ -53,7 +71,7 @@ Choice choose(int M, int N, int K, int table_g, int g, int sms, int pair, int on
             const double kb = f.split ? split_kb(K, g, splits) : kb_total;
             double ns = ((tiles * splits + walkers - 1) / walkers) * (kb * f.stage_ns + kb * BK / g * f.group_ns);
             if (f.split) ns = (ns + (splits == 2 ? 3500 : 6000)) / 0.85;
-            if (!best.form || ns < best_ns) { best = {&f, splits}; best_ns = ns; }
+            if ((!best.form || ns < best_ns) && usable(f)) { best = {&f, splits}; best_ns = ns; }
         }
     }
     return best;
@@ -72,10 +90,10 @@ bool gemm_supports(const LinearArgs& a) {
     return true;
 }
 
-int gemm_form(int M, int N, int K, int g, int sms, int form, int only_bt, int only_splits, int* out3) {
+int gemm_form(int M, int N, int K, int g, int sms, int form, int only_bt, int only_splits, bool moved_registers, int* out3) {
     using namespace gemm;
     if (M < 1 || N < 1 || K < 1 || sms < 2 || K % BK != 0 || g % 32 != 0 || K % g != 0) return W8A8_ERR_UNSUPPORTED;
-    const Choice c = choose(M, N, K, g, g, sms, form, only_bt, only_splits);
+    const Choice c = choose(M, N, K, g, g, sms, form, only_bt, only_splits, [&](const Form& f) { return moved_registers || !f.move_regs; });
     if (!c.form) return W8A8_ERR_UNSUPPORTED;
     out3[0] = c.form->bt;
     out3[1] = c.form->pair ? 2 : 1;
@@ -88,7 +106,7 @@ int launch_linear_gemm(const LinearArgs& a, int* device_status, cudaStream_t str
     if (!gemm_supports(a)) return fail(W8A8_ERR_UNSUPPORTED, "tcgen05 GEMM does not take this shape");
     const int sms = device_sms();
 
-    const Choice choice = choose(a.M, a.N, a.K, a.dump ? 0 : a.g, a.g, sms, form, a.gemm_bt, a.gemm_splits);
+    const Choice choice = choose(a.M, a.N, a.K, a.dump ? 0 : a.g, a.g, sms, form, a.gemm_bt, a.gemm_splits, balanced);
     const Form* best = choice.form;
     const int best_splits = choice.splits;
     if (!best) return fail(W8A8_ERR_UNSUPPORTED, "no tile form of the tcgen05 GEMM for this shape (token width %d, splits %d asked for)",
@@ -118,21 +136,6 @@ int launch_linear_gemm(const LinearArgs& a, int* device_status, cudaStream_t str
                                    static_cast<uint64_t>(ycols) * 2, 128, bt, 1);
         if (rc) return rc;
     }
-    // The attribute is per device and this library serves several devices of one process: set it on every launch (a
-    // host-side table write) rather than remember it per process.
-    cudaError_t e = cudaFuncSetAttribute(best->kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, best->smem);
-    if (e != cudaSuccess) return fail(W8A8_ERR_CUDA, "cudaFuncSetAttribute: %s", cudaGetErrorString(e));
-    if (best->move_regs) {
-        // setmaxnreg moves registers between the warpgroups; the sums balance only for the register count the kernel was
-        // compiled to (kLaunchRegs per thread). An unbalanced sum blocks for ever in setmaxnreg.inc, a wait nothing
-        // bounds, so a build that came out differently is refused here.
-        cudaFuncAttributes fa;
-        e = cudaFuncGetAttributes(&fa, best->kernel);
-        if (e != cudaSuccess) return fail(W8A8_ERR_CUDA, "cudaFuncGetAttributes: %s", cudaGetErrorString(e));
-        if (fa.numRegs != kLaunchRegs)
-            return fail(W8A8_ERR_UNSUPPORTED, "gemm_i8_kernel was compiled to %d registers per thread, its setmaxnreg balance needs %d",
-                        fa.numRegs, kLaunchRegs);
-    }
     cudaLaunchConfig_t cfg = {};
     // persistent: one CTA (or CTA pair) per SM (pair of SMs) walks its tiles, tokens fastest, so that concurrent CTAs
     // share weight tiles in L2
@@ -158,7 +161,7 @@ int launch_linear_gemm(const LinearArgs& a, int* device_status, cudaStream_t str
     }
     cfg.attrs = attr;
     cfg.numAttrs = na;
-    e = cudaLaunchKernelEx(&cfg, best->kernel, map_w, map_x, map_y, p);
+    const cudaError_t e = launch_with_smem(best->state->attribute, best->smem, cfg, best->kernel, map_w, map_x, map_y, p);
     if (e != cudaSuccess) return fail(W8A8_ERR_CUDA, "gemm launch: %s", cudaGetErrorString(e));
     return W8A8_OK;
 }

@@ -699,6 +699,10 @@ gemm_i8_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
 using Kernel = void (*)(const CUtensorMap, const CUtensorMap, const CUtensorMap, const GemmParams);
 // A tile form: its kernel and what the launch needs to know about it. stage_ns, group_ns: what a tile takes per 128 bytes of
 // K and per K-group, fitted to 8192 x 19456 x 2560 at g = 256 and g = 64 (the two overlap; their sum is what was measured).
+struct FormState {
+    SmemAttribute attribute;
+    std::atomic<int> registers{0};  // per thread, as compiled (0: not asked for yet)
+};
 struct Form {
     int bt;
     bool pair, split;
@@ -706,10 +710,14 @@ struct Form {
     int threads, smem;
     bool move_regs;
     float stage_ns, group_ns;
+    FormState* state;
 };
+template <int BT, bool PAIR, int GM, bool SPLIT>
+inline FormState form_state;
 template <int BT, bool PAIR, int GM, bool SPLIT = false>
-constexpr Form form(float stage_ns, float group_ns) {
-    return Form{BT, PAIR, SPLIT, gemm_i8_kernel<BT, PAIR, GM, SPLIT>, Config<BT, PAIR>::kThreads, Config<BT, PAIR>::kSmem, Config<BT, PAIR>::kMoveRegs, stage_ns, group_ns};
+Form form(float stage_ns, float group_ns) {
+    return Form{BT, PAIR, SPLIT, gemm_i8_kernel<BT, PAIR, GM, SPLIT>, Config<BT, PAIR>::kThreads, Config<BT, PAIR>::kSmem, Config<BT, PAIR>::kMoveRegs, stage_ns, group_ns,
+                &form_state<BT, PAIR, GM, SPLIT>};
 }
 template <int GM>
 const Form* all_forms(int* count) {

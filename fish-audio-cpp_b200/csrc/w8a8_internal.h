@@ -179,6 +179,7 @@ int launch_tp_allreduce_rowquant(TpState* t, __half* x, const __half* partial, c
 bool gemm_supports(const LinearArgs& a);
 // form: -1 picks between one CTA per tile (0) and a CTA pair per tile (1) by shape
 int launch_linear_gemm(const LinearArgs& a, int* device_status, cudaStream_t s, int form = -1);
-int gemm_form(int M, int N, int K, int g, int sms, int form, int only_bt, int only_splits, int* out3);  // what it would take
+int gemm_form(int M, int N, int K, int g, int sms, int form, int only_bt, int only_splits, bool moved_registers,
+              int* out3);  // what it would take
 
 }  // namespace w8a8

@@ -208,9 +208,10 @@ W8A8_API int w8a8_debug_tail_counters(w8a8_ctx* ctx, int* out, int count, void* 
 W8A8_API int w8a8_debug_force_gemm_form(w8a8_ctx* ctx, int token_width, int splits);
 /* Diagnostic, host only (needs no device): the form that the tcgen05 GEMM takes on a GPU of `sms` SMs: {tokens per tile, CTAs that
  * share its rows (1 or 2), CTAs that share its K (1, 2 or 4)}. kernel: W8A8_KERNEL_GEMM, _GEMM_SINGLE or _GEMM_PAIR; token_width
- * and splits as above. */
+ * and splits as above; moved_registers 0: without the form that is left out where its kernel was not compiled to the register
+ * count that its split between warps needs. */
 W8A8_API int w8a8_debug_gemm_form(int M, int N, int K, int group_size, int sms, int kernel, int token_width, int splits,
-                                  int* form_out3);
+                                  int moved_registers, int* form_out3);
 
 /* No counterpart in the reference. The same computation as w8a8_linear for callers that may not
  * allocate device memory and therefore cannot create a context (w8a8_create allocates): a plugin

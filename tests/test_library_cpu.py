@@ -88,6 +88,11 @@ def test_gemm_form_follows_what_is_asked_for(pkg):
     assert pkg.debug_gemm_form(8192, 2560, 9728, 64, splits=2) is None, "more tiles than the chip holds at once"
     assert pkg.debug_gemm_form(150, 2560, 2560, 256, token_width=100) is None
     assert pkg.debug_gemm_form(150, 2560, 2500, 250) is None
+    # the widest form, where its register balance does not hold: another one takes the shape
+    for g in (64, 128, 256):
+        assert pkg.debug_gemm_form(256, 37888, 2560, g, kernel=pkg.KERNEL_GEMM_PAIR) == (256, 2, 1)
+        assert pkg.debug_gemm_form(256, 37888, 2560, g, kernel=pkg.KERNEL_GEMM_PAIR, moved_registers=False) == (192, 2, 1)
+        assert pkg.debug_gemm_form(8192, 19456, 2560, g, moved_registers=False) is not None
 
 
 def test_product_never_touches_the_oracle():
