@@ -722,14 +722,6 @@ int launch_attention(const AttnParams& base, int B, int splits, cudaStream_t str
     rc = make_tensor_map_2d_u8(&map_v, p.v_cache, kHeadDim * 2, uint64_t(1) << 30, kHeadDim * 2, 128, kBlockTokens, 1);
     if (rc) return rc;
     const size_t smem = static_cast<size_t>(kRing) * kStageBytes + 1024;
-    {  // per device, so on every launch (a host-side table write)
-        cudaError_t e = cudaFuncSetAttribute(paged_attention_decode_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                             static_cast<int>(smem));
-        if (e == cudaSuccess)
-            e = cudaFuncSetAttribute(paged_attention_decode_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                     static_cast<int>(smem));
-        if (e != cudaSuccess) return fail(W8A8_ERR_CUDA, "cudaFuncSetAttribute: %s", cudaGetErrorString(e));
-    }
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(splits, n_kv, B);
     cfg.blockDim = dim3(kAttnThreads, 1, 1);
@@ -744,8 +736,10 @@ int launch_attention(const AttnParams& base, int B, int splits, cudaStream_t str
     attr[1].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
     cfg.numAttrs = pdl_enabled(kPdlAttn) ? 2 : 1;
-    cudaError_t e = p.qkv ? cudaLaunchKernelEx(&cfg, paged_attention_decode_kernel<true>, map_k, map_v, p)
-                          : cudaLaunchKernelEx(&cfg, paged_attention_decode_kernel<false>, map_k, map_v, p);
+    static SmemAttribute attribute[2];
+    const int most = static_cast<int>(smem);
+    const cudaError_t e = p.qkv ? launch_with_smem(attribute[1], most, cfg, paged_attention_decode_kernel<true>, map_k, map_v, p)
+                                : launch_with_smem(attribute[0], most, cfg, paged_attention_decode_kernel<false>, map_k, map_v, p);
     if (e != cudaSuccess) return fail(W8A8_ERR_CUDA, "paged_attention_decode launch: %s", cudaGetErrorString(e));
     return W8A8_OK;
 }
