@@ -48,7 +48,7 @@ int launch(__half* a, const __half* b, long n, cudaStream_t s) {
                  (OP == OP_SILU || (reinterpret_cast<uintptr_t>(b) & 15u) == 0);
     long work = vec_ok ? (n + 7) / 8 : n;
     long blocks = (work + 255) / 256;
-    if (blocks > 148L * 16) blocks = 148L * 16;  // grid-stride beyond 16 CTAs per SM
+    if (blocks > device_sms() * 16L) blocks = device_sms() * 16L;  // grid-stride beyond 16 CTAs per SM
     eltwise_kernel<OP><<<static_cast<unsigned>(blocks), 256, 0, s>>>(a, b, n, vec_ok);
     return check_launch("eltwise_kernel");
 }

@@ -37,7 +37,6 @@ constexpr int kWarps = 4;
 constexpr int kThreads = kWarps * 32;
 constexpr int kTileRows = kWarps * 16;
 constexpr int kPartPitch = kTileRows + 4;  // floats; keeps fragment stores bank-conflict-free
-constexpr int kNumSMs = 148;
 
 struct GemvParams {
     LinearArgs a;
@@ -278,11 +277,12 @@ bool make_plan(const LinearArgs& a, Plan& pl) {
     if (S <= 0) {
         // Pick the slice count that minimises (CTAs per SM, rounded up) x (bytes per CTA + a fixed
         // per-CTA cost): enough CTAs to cover the SMs, slices of equal group counts preferred.
+        const int sms = device_sms();
         double best = 1e30;
         S = 1;
         for (int cand = 1; cand <= 8 && cand <= a.G; ++cand) {
             const int slice_groups = (a.G + cand - 1) / cand;
-            const int waves = (tiles * cand + kNumSMs - 1) / kNumSMs;
+            const int waves = (tiles * cand + sms - 1) / sms;
             const double cost = static_cast<double>(waves) * (static_cast<double>(slice_groups) * a.g + 768.0);
             if (cost < best * 0.999) { best = cost; S = cand; }
         }

@@ -629,7 +629,7 @@ template <int LANES>
 int launch_groupquant(const __half* X, const __half* smooth_inv, const __half* act_scale, int8_t* Xq, float* Xs,
                       unsigned pieces, unsigned K8, cudaStream_t stream) {
     // four pieces per thread once the single-piece form would fill every SM with more than two rounds of threads
-    if (pieces > 148u * 2048u * 2u)
+    if (pieces > static_cast<unsigned>(device_sms()) * 2048u * 2u)
         return launch_row_kernel("groupquant", groupquant_kernel<LANES, 4>, (pieces + 511) / 512, 128, 0, stream, X, smooth_inv,
                                  act_scale, Xq, Xs, pieces, K8);
     return launch_row_kernel("groupquant", groupquant_kernel<LANES, 1>, (pieces + 127) / 128, 128, 0, stream, X, smooth_inv, act_scale,
@@ -699,7 +699,7 @@ int launch_rowquant(const __half* x_in, __half* x_out, const __half* residual,
         (!normed_out || aligned16(normed_out)) && (!Xq || (reinterpret_cast<uintptr_t>(Xq) & 7u) == 0)) {
         // A CTA per row has the shorter chain, a warp per row more bytes in flight: the line is where the CTAs no longer all
         // fit the chip at once (eight per SM). At 150 rows a warp per row leaves three SMs of four idle: 8 us against 5.
-        if (threads == 1024 && M > 148 * 8)
+        if (threads == 1024 && M > device_sms() * 8)
             return gm == 64 ? launch_rownorm_warp<64>(p, M, stream) : gm == 128 ? launch_rownorm_warp<128>(p, M, stream)
                                                                                 : launch_rownorm_warp<256>(p, M, stream);
         return launch_row_kernel("rowquant_compact", gm == 64    ? rowquant_compact_kernel<64>
