@@ -21,7 +21,7 @@ struct w8a8_ctx {
     };
     std::unordered_map<const void*, PackedEntry> packed;
     std::mutex packed_mu;
-    int gemm_bt = 0, gemm_splits = 0;  // w8a8_debug_force_gemm_form
+    short gemm_bt = 0, gemm_splits = 0;  // w8a8_debug_force_gemm_form
     int* tail_counters = nullptr;     // arrival counters of the decode kernel's tails, zero between launches
     w8a8::TpState* tp = nullptr;  // tensor-parallel exchange, when w8a8_tp_create was called
 };
@@ -602,9 +602,9 @@ int w8a8_debug_tail_counters(w8a8_ctx* ctx, int* out, int count, void* stream) {
 }
 
 int w8a8_debug_force_gemm_form(w8a8_ctx* ctx, int token_width, int splits) {
-    if (!ctx || token_width < 0 || splits < 0) return fail(W8A8_ERR_INVALID_ARG, "debug_force_gemm_form: bad arguments");
-    ctx->gemm_bt = token_width;
-    ctx->gemm_splits = splits;
+    if (!ctx || token_width < 0 || token_width > 256 || splits < 0 || splits > 8) return fail(W8A8_ERR_INVALID_ARG, "debug_force_gemm_form: bad arguments");
+    ctx->gemm_bt = static_cast<short>(token_width);
+    ctx->gemm_splits = static_cast<short>(splits);
     return W8A8_OK;
 }
 
