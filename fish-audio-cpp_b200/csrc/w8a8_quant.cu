@@ -33,6 +33,7 @@ struct RowQuantParams {
     int K, g, G;
     int per_token;
     int vec_ok;               // K % 8 == 0 and all fp16 pointers 16-byte aligned
+    int first_pass;           // 0: the compact kernel runs a rehearsal before its dependency wait (see rehearses)
 };
 
 __device__ __forceinline__ float warp_max(float v) {
@@ -342,7 +343,7 @@ __global__ void __launch_bounds__(1024) rowquant_fast_kernel(const RowQuantParam
 // The first pass is a rehearsal on the norm weights, with nothing stored, while the kernel before this one still runs: code
 // that runs for the first time after another kernel costs about six clocks an instruction, warm code a fifth of that,
 // and a launch of this kernel runs its code once. (Decode step, batch 8: 1726 -> 1700 us together with the quantiser's.
-// The same in the linear's CTAs made the step slower.)
+// The same in the linear's CTAs made the step slower. Which launches rehearse: see rehearses.)
 template <int GM>
 __global__ void __launch_bounds__(128) rowquant_compact_kernel(const __grid_constant__ RowQuantParams p) {
     constexpr int LANES = GM / 8, kPieces = 4;
@@ -359,7 +360,7 @@ __global__ void __launch_bounds__(128) rowquant_compact_kernel(const __grid_cons
     }
     const __half* res = p.residual ? p.residual : p.x_in;
 #pragma unroll 1
-    for (int pass = 0; pass < 2; ++pass) {
+    for (int pass = p.first_pass; pass < 2; ++pass) {
         const bool real = pass == 1;
         if (real) {
             asm volatile("griddepcontrol.wait;" ::: "memory");
@@ -561,11 +562,11 @@ __global__ void __launch_bounds__(128, KI > 10 ? 4 : 5) rownorm_warp_kernel(cons
 // piece per thread (U = 1). At prefill sizes it is bandwidth: four loads in flight per thread (8192 x 9728: 86 -> 37 us, 6.5 TB/s).
 template <int LANES, int U>  // LANES: threads per group = g / 8
 __global__ void __launch_bounds__(128) groupquant_kernel(const __half* X, const __half* smooth_inv, const __half* act_scale,
-                                                         int8_t* Xq, float* Xs, unsigned pieces, unsigned K8) {
+                                                         int8_t* Xq, float* Xs, unsigned pieces, unsigned K8, int first_pass) {
     W8A8_TRACE_SCOPE();
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 #pragma unroll 1
-    for (int pass = U == 1 ? 0 : 1; pass < 2; ++pass) {
+    for (int pass = U == 1 ? first_pass : 1; pass < 2; ++pass) {
     const bool real = pass == 1;
     if (real) {
         asm volatile("griddepcontrol.wait;" ::: "memory");
@@ -625,15 +626,20 @@ int launch_row_kernel(const char* what, void (*kernel)(Params...), unsigned bloc
     return W8A8_OK;
 }
 
+// A rehearsal pays where the kernel ahead lets this one start early and is still busy: behind the decode linears, up to 32 rows. The
+// GEMM lets nothing start before its end, so behind it, as behind other kernels, the rehearsal is time added, once per CTA
+// (quantiser at 600 x 4096 3.8 us without and 4.7 with, at 150 x 2560 2.3 and 2.7; row kernel at 600 x 2560 6.6 and 6.9).
+bool rehearses(int rows) { return rows <= 32; }
+
 template <int LANES>
 int launch_groupquant(const __half* X, const __half* smooth_inv, const __half* act_scale, int8_t* Xq, float* Xs,
-                      unsigned pieces, unsigned K8, cudaStream_t stream) {
+                      unsigned pieces, unsigned K8, int first_pass, cudaStream_t stream) {
     // four pieces per thread once the single-piece form would fill every SM with more than two rounds of threads
     if (pieces > static_cast<unsigned>(device_sms()) * 2048u * 2u)
         return launch_row_kernel("groupquant", groupquant_kernel<LANES, 4>, (pieces + 511) / 512, 128, 0, stream, X, smooth_inv,
-                                 act_scale, Xq, Xs, pieces, K8);
+                                 act_scale, Xq, Xs, pieces, K8, first_pass);
     return launch_row_kernel("groupquant", groupquant_kernel<LANES, 1>, (pieces + 127) / 128, 128, 0, stream, X, smooth_inv, act_scale,
-                             Xq, Xs, pieces, K8);
+                             Xq, Xs, pieces, K8, first_pass);
 }
 
 template <int GM>
@@ -656,9 +662,10 @@ int launch_rowquant(const __half* x_in, __half* x_out, const __half* residual,
             (gn == 64 || gn == 128 || gn == 256) && K % gn == 0 && static_cast<long long>(M) * K / 8 < (1ll << 31) && aligned16(x_in) &&
             (reinterpret_cast<uintptr_t>(Xq) & 7u) == 0 && (!smooth_inv || aligned16(smooth_inv))) {
             const unsigned pieces = static_cast<unsigned>(static_cast<long long>(M) * K / 8), K8 = static_cast<unsigned>(K / 8);
-            if (gn == 64) return launch_groupquant<8>(x_in, smooth_inv, act_scale, Xq, Xs, pieces, K8, stream);
-            if (gn == 128) return launch_groupquant<16>(x_in, smooth_inv, act_scale, Xq, Xs, pieces, K8, stream);
-            return launch_groupquant<32>(x_in, smooth_inv, act_scale, Xq, Xs, pieces, K8, stream);
+            const int first = rehearses(M) ? 0 : 1;
+            if (gn == 64) return launch_groupquant<8>(x_in, smooth_inv, act_scale, Xq, Xs, pieces, K8, first, stream);
+            if (gn == 128) return launch_groupquant<16>(x_in, smooth_inv, act_scale, Xq, Xs, pieces, K8, first, stream);
+            return launch_groupquant<32>(x_in, smooth_inv, act_scale, Xq, Xs, pieces, K8, first, stream);
         }
     }
     RowQuantParams p;
@@ -676,6 +683,7 @@ int launch_rowquant(const __half* x_in, __half* x_out, const __half* residual,
     p.g = norm_group(K, g);
     p.G = num_groups(K, g);
     p.per_token = act_mode == W8A8_ACT_PER_TOKEN;
+    p.first_pass = rehearses(M) ? 0 : 1;
     p.vec_ok = (K % 8 == 0) && aligned16(x_in) && (!residual || aligned16(residual)) &&
                (!x_out || aligned16(x_out));
     // The norm must run with the reference's block size to reproduce its summation order:
