@@ -454,7 +454,7 @@ __global__ void __launch_bounds__(128, KI > 10 ? 4 : 5) rownorm_warp_kernel(cons
     if (row >= M) return;
     const int K = p.K, iters = K / 256;
     const size_t base = static_cast<size_t>(row) * K;
-    const __half* res = p.residual ? p.residual + base : nullptr;
+    const __half* res = KI <= 10 && p.residual ? p.residual + base : nullptr;  // (wider rows with a residual: a CTA per row)
     uint4 v[KI];
 #pragma unroll
     for (int i = 0; i < KI; ++i)
@@ -713,9 +713,14 @@ int launch_rowquant(const __half* x_in, __half* x_out, const __half* residual,
     if (compact_ok && norm_weight && threads >= 256 && K % 256 == 0 && K <= 4096 && !smooth_inv && !act_scale && (!p.per_token || !Xq) &&
         (gm == 64 || gm == 128 || gm == 256) && p.vec_ok && aligned16(norm_weight) &&
         (!normed_out || aligned16(normed_out)) && (!Xq || (reinterpret_cast<uintptr_t>(Xq) & 7u) == 0)) {
-        // A CTA per row has the shorter chain, a warp per row more bytes in flight: the line is where the CTAs no longer all
-        // fit the chip at once (eight per SM). At 150 rows a warp per row leaves three SMs of four idle: 8 us against 5.
-        if (threads == 1024 && M > device_sms() * 8)
+        // A CTA per row has the shorter chain, a warp per row more bytes in flight. CTA / warp, us: 1185 x 2560 5.8 / 7.6, 1700 6.9 /
+        // 7.8, 2048 8.4 / 7.9, 8192 31.8 / 21.2; 1185 x 1024 4.3 / 4.6, 1400 4.8 / 4.7. Past 2560 columns a warp per row fits an SM
+        // sixteen times, and a second wave has to be worth it: 2368 x 4096 11.5 / 10.7, 2500 12.7 / 18.9, 4001 19.4 / 21.5, 8192 38.6 /
+        // 36.5; with a residual it never is (sixteen loads, then four rounds of the residual): 1185 x 4096 7.8 / 13.4, 8192 47 / 69.
+        const int sms = device_sms();
+        const bool warp_per_row = threads == 1024 && M > sms * (K <= 1024 ? 9 : 13) &&
+                                  (K <= 2560 || (!residual && (M <= sms * 16 || M > sms * 40)));
+        if (warp_per_row)
             return gm == 64 ? launch_rownorm_warp<64>(p, M, stream) : gm == 128 ? launch_rownorm_warp<128>(p, M, stream)
                                                                                 : launch_rownorm_warp<256>(p, M, stream);
         return launch_row_kernel("rowquant_compact", gm == 64    ? rowquant_compact_kernel<64>

@@ -220,11 +220,12 @@ def test_elementwise(ctx, oracle, n):
         assert torch.equal(ra, dr)
 
 
-@pytest.mark.parametrize("M,K,g", [(1185, 768, 256), (1186, 2560, 64), (1187, 2816, 128), (1200, 4096, 256), (1185, 4096, 64)])
+@pytest.mark.parametrize("M,K,g", [(1185, 768, 256), (1186, 2560, 64), (1187, 2816, 128), (1200, 4096, 256), (1185, 4096, 64),
+                                   (1333, 768, 256), (1925, 2560, 64), (1926, 2816, 128), (1927, 4096, 256), (1933, 1280, 64)])
 @pytest.mark.parametrize("with_residual", [False, True])
 def test_rmsnorm_quantize_many_rows(ctx, oracle, M, K, g, with_residual):
-    """More rows than eight per SM: the warp-per-row form (its shortest row, the last row count that fills a CTA of four and the ones
-    that do not, the widths at which its register rows end). The sum of squares follows the reference's order; the device's
+    """Many rows, a CTA or (the last five, without a residual where they are wider than 2560) a warp for each: the warp form's shortest
+    row, row counts that fill its CTAs of four and ones that do not, the widths at which its register rows end). The sum of squares follows the reference's order; the device's
     rsqrtf may move a normed value by one fp16 ulp against the oracle's, and codes are compared on the device's own norm."""
     rng = np.random.default_rng(M + K)
     x = synth.activations(rng, M, K)
@@ -245,6 +246,28 @@ def test_rmsnorm_quantize_many_rows(ctx, oracle, M, K, g, with_residual):
     ctx.rms_norm(dev(want_x), dev(w), alone, M, K, 1e-6)
     torch.cuda.synchronize()
     assert torch.equal(alone, dn)
+
+
+@pytest.mark.parametrize("M", [1333, 1925, 2369, 5921])
+@pytest.mark.parametrize("K,g", [(256, 64), (512, 128), (768, 256), (1024, 64), (1280, 128), (2560, 64), (2816, 256), (4096, 128)])
+@pytest.mark.parametrize("with_residual", [False, True])
+def test_rmsnorm_many_rows_equal_few_rows(ctx, M, K, g, with_residual):
+    """Row counts just past the lines between a CTA and a warp per row, widths on both sides of them, against few rows: the same bits on
+    the first, some middle and the last rows, since both forms sum in the order of the reference's launch."""
+    gen = torch.Generator(device="cuda").manual_seed(M + K)
+    x0 = torch.randn((M, K), device="cuda", generator=gen).half() * 3
+    r = torch.randn((M, K), device="cuda", generator=gen).half() if with_residual else None
+    w = torch.empty((K,), device="cuda").uniform_(0.8, 1.2, generator=gen).half()
+
+    def run(rows):
+        x, res, m = x0[rows].clone(), r[rows].clone() if with_residual else None, x0[rows].shape[0]
+        dn, dq, ds = torch.empty_like(x), torch.empty((m, K), dtype=torch.int8, device="cuda"), torch.empty((m, K // g), device="cuda")
+        ctx.rmsnorm_quantize(x, w, 1e-6, m, K, g, dq, ds, residual=res, normed_out=dn)
+        torch.cuda.synchronize()
+        return x.view(torch.int16), dn.view(torch.int16), dq, ds
+    many = run(slice(0, M))
+    for rows in (slice(0, 3), slice(700, 716), slice(M - 5, M)):
+        assert all(torch.equal(a[rows], b) for a, b in zip(many, run(rows)))
 
 
 @pytest.mark.parametrize("M,K,g", [(613, 9728, 64), (1901, 2560, 256), (947, 5120, 128)])
