@@ -387,7 +387,9 @@ gemm_i8_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
                             if (kLoopGroups < C::kAcc && s == S - 1 && (as_any = kLoopGroups - as_any) == 0) acc_parity ^= 1u;
                         } else {
                             if (!wait(&full_bar[s], parity)) { code = 300 + s; break; }
-#pragma unroll 1
+                            // (Rolled up, the four MMAs of a stage took the issuing warp longer than they take: one scale per channel,
+                            // 4096 x 19456 x 2560 309 -> 204 us, groups of 512 342 -> 234.)
+#pragma unroll
                             for (int sub = 0; sub < 4; ++sub) {
                                 if (q_in_group == 0) {
                                     if (!wait(&acc_empty[as_any], acc_parity)) { code = 400 + as_any; break; }
