@@ -349,7 +349,7 @@ TMA_SHAPES = [(1, 128, 256, 64), (4, 200, 512, 128), (8, 64, 2560, 256), (9, 192
 
 @pytest.mark.parametrize("M,N,K,g", TMA_SHAPES)
 def test_gemv_tma_small_shapes(ctx, oracle, pkg, M, N, K, g):
-    """The stream-K TMA kernel: tiles cut by warp-range boundaries, N not a multiple of 16, every
+    """The decode kernel over TMA boxes of the row-major matrix: tiles cut by warp-range boundaries, N not a multiple of 16, every
     group-size branch; two runs must agree bit for bit (the partial sums are added in a fixed order)."""
     (X, W, ws, Xq, Xs), Y, P = run_linear(ctx, oracle, M, N, K, g, seed=M + N, kernel=pkg.KERNEL_GEMV_TMA)
     Pw = oracle.group_sums(W, Xq, g)
@@ -671,8 +671,8 @@ def test_prefill_shapes_full_size(ctx, oracle, pkg, name, g, M):
     """configs[2], all sixteen cases (four projections x g in {256, 64} x M in {2048, 8192}): the whole GEMM
     runs on the GPU; a random 48-token x 192-row sub-problem is recomputed by the oracle (each output
     depends only on its own token row and weight row) and must agree bit for bit; a second run of the full
-    problem, through the form of the kernel that the default did NOT pick (CTA pairs at g = 256, single CTAs at
-    g = 64 by default), must agree with the first bit for bit as well."""
+    problem, through the form of the kernel that the default did NOT pick (a CTA pair per tile where it takes one CTA, and the
+    other way round), must agree with the first bit for bit as well."""
     K, N = synth.PROJECTIONS[name]
     rng = np.random.default_rng(7 + g)
     X = synth.activations(rng, M, K)
@@ -684,7 +684,9 @@ def test_prefill_shapes_full_size(ctx, oracle, pkg, name, g, M):
     dX = dev(X)
     ctx.linear(dW, dS, g, dX, dY, M, N, K)
     dY2 = torch.empty_like(dY)
-    ctx.linear(dW, dS, g, dX, dY2, M, N, K, kernel=pkg.KERNEL_GEMM_SINGLE if g >= 128 else pkg.KERNEL_GEMM_PAIR)
+    _, ctas, splits = pkg.debug_gemm_form(M, N, K, g, sms=torch.cuda.get_device_properties(0).multi_processor_count)
+    assert splits == 1
+    ctx.linear(dW, dS, g, dX, dY2, M, N, K, kernel=pkg.KERNEL_GEMM_SINGLE if ctas == 2 else pkg.KERNEL_GEMM_PAIR)
     torch.cuda.synchronize()
     ctx.check_device_status()
     assert torch.equal(dY.view(torch.int16), dY2.view(torch.int16))
