@@ -86,7 +86,6 @@ bool gemv::make_plan(const LinearArgs& a, Plan& pl, bool rows) {
         }
     }
     pl.pro = fused ? kProNorm : quant ? kProQuant : kProCodes;
-    pl.stages = fused ? 2 : 3;
     pl.MT = a.M <= 8 ? 1 : (a.M <= 16 ? 2 : 4);
     pl.GM = a.g == 64 ? 64 : a.g == 128 ? 128 : 256;
     pl.bpu = a.g > 256 ? a.g / 256 : 1;

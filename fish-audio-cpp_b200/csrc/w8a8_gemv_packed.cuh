@@ -415,8 +415,8 @@ __device__ __forceinline__ void gemv_body(const GemvPackedParams& p, const CUten
     int pkb = 0, prt = 0;  // ROWS: the next box's 128-byte K block and row tile
     if constexpr (ROWS) { prt = static_cast<int>(u0 / p.upt); pkb = static_cast<int>(u0 % p.upt) * p.bpu * 2; }
     // Weights are read once per launch and a stack's do not fit in L2: as evict-first lines they do not push out the activations,
-    // scales and cache rows that the next launches read, nor wait behind their write-back (decode step, batch 8: 1517 -> 1488 us;
-    // ten fast-AR steps 1710 -> 1666). Marking a quarter of them evict-last, to find it again at the next step: 1502 and 1687.
+    // scales and cache rows that the next launches read, nor wait behind their write-back (decode step, batch 8: 1517 -> 1490 us;
+    // ten fast-AR steps 1710 -> 1650). Marking a quarter of them evict-last, to find it again at the next step: 1502 and 1687.
     unsigned long long once;
     asm volatile("createpolicy.fractional.L2::evict_first.b64 %0, 1.0;" : "=l"(once));
     auto issue = [&]() {  // lane 0 only
@@ -1040,7 +1040,7 @@ __device__ __forceinline__ void gemv_body(const GemvPackedParams& p, const CUten
 
 // How a linear is cut over CTAs and warps.
 struct Plan {
-    int MT, GM, upt, bpu, block_bytes, tiles, ctas, pro, stages;
+    int MT, GM, upt, bpu, block_bytes, tiles, ctas, pro;
     long long U;
 };
 bool make_plan(const LinearArgs& a, Plan& pl, bool rows);
