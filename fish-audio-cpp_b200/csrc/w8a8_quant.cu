@@ -560,9 +560,11 @@ __global__ void __launch_bounds__(128, KI > 10 ? 4 : 5) rownorm_warp_kernel(cons
 // [M, G] are contiguous and K is a multiple of g), so the whole matrix is one flat run of pieces. At decode sizes it is a
 // few KB, and what counts is the length of the dependency chain (one load, log2(g/8) shuffles, one divide, one store): one
 // piece per thread (U = 1). At prefill sizes it is bandwidth: four loads in flight per thread (8192 x 9728: 86 -> 37 us, 6.5 TB/s).
+// Twelve CTAs of that form fit an SM with 40 registers a thread; compiled to 44 it ran at eleven (8192 x 9728 36.5 -> 38.4 us). Only the
+// outputs are __restrict__: loads may move past stores, and are still not taken for constant.
 template <int LANES, int U>  // LANES: threads per group = g / 8
-__global__ void __launch_bounds__(128) groupquant_kernel(const __half* X, const __half* smooth_inv, const __half* act_scale,
-                                                         int8_t* Xq, float* Xs, unsigned pieces, unsigned K8, int first_pass) {
+__global__ void __launch_bounds__(128, U == 1 ? 1 : 12) groupquant_kernel(const __half* X, const __half* smooth_inv, const __half* act_scale,
+                                                         int8_t* __restrict__ Xq, float* __restrict__ Xs, unsigned pieces, unsigned K8, int first_pass) {
     W8A8_TRACE_SCOPE();
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 #pragma unroll 1
@@ -582,7 +584,7 @@ __global__ void __launch_bounds__(128) groupquant_kernel(const __half* X, const 
         u[k] = real && p0 + k * 128u < pieces ? ptx::ld_result_v4(reinterpret_cast<const uint4*>(X) + p0 + k * 128u) : make_uint4(0, 0, 0, 0);
     auto load_vectors = [&](unsigned pc) {
         const unsigned c8 = pc % K8;  // piece inside its row
-        if (smooth_inv) su = ptx::ld_result_v4(reinterpret_cast<const uint4*>(smooth_inv) + c8);
+        if (smooth_inv) su = *(reinterpret_cast<const uint4*>(smooth_inv) + c8);
         if (act_scale) st = __half2float(act_scale[c8 / LANES]);
     };
     const bool vectors = real && (smooth_inv || act_scale);
