@@ -49,6 +49,7 @@
 
 #include "sm100_ptx.cuh"
 #include "w8a8_internal.h"
+#include "w8a8_swiglu.cuh"
 
 namespace w8a8 {
 namespace gemm {
@@ -217,14 +218,8 @@ __device__ __forceinline__ uint32_t half2_bits(uint64_t v) {
     const __half2 h = __floats2half2_rn(lo2(v), hi2(v));
     return *reinterpret_cast<const uint32_t*>(&h);
 }
-// silu(gate) * up with the roundings of the reference's GEMM, silu, GEMM, mul chain (ffn_activations.cu:12-17, :35-40)
-__device__ __forceinline__ __half swiglu1(float gate, float up) {
-    const float g16 = __half2float(__float2half(gate)), u16 = __half2float(__float2half(up));
-    const __half s16 = __float2half(g16 / (1.0f + expf(-g16)));
-    return __float2half(__half2float(s16) * u16);
-}
 __device__ __forceinline__ uint32_t swiglu2_bits(uint64_t gate, uint64_t up) {
-    const __half2 h = __halves2half2(swiglu1(lo2(gate), lo2(up)), swiglu1(hi2(gate), hi2(up)));
+    const __half2 h = swiglu2(__floats2half2_rn(lo2(gate), hi2(gate)), __floats2half2_rn(lo2(up), hi2(up)));
     return *reinterpret_cast<const uint32_t*>(&h);
 }
 

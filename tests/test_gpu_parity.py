@@ -752,6 +752,33 @@ def test_gemm_tcgen05_split_k(gemm_form, oracle, pkg, M, N, K, bt, splits, g):
                       abs_terms=abs_term_sum(oracle.group_sums(W, Xq, g), ws, Xs))
 
 
+def test_fused_swiglu_of_every_gate(ctx, pkg):
+    """The SwiGLU epilogue's quotient against the divide of the separate silu, for every fp16 gate (one token each; an infinite one
+    by overflow): bit for bit."""
+    bits = np.arange(65536, dtype=np.uint32).astype(np.uint16)
+    gates = bits.view(np.float16)
+    M, K, g = 65536, 128, 64
+    Xq = np.zeros((M, K), np.int8)
+    Xq[:, 0] = Xq[:, g] = 1
+    Xs = np.ones((M, 2), np.float32)
+    Xs[:, 0] = np.where(np.isinf(gates), np.sign(gates.astype(np.float32)) * 1e5, gates.astype(np.float32))
+    W = np.zeros((16, K), np.int8)  # gate rows read the first group, up rows the second: up = 1
+    W[:8, 0] = W[8:, g] = 1
+    # (a zero weight times a NaN scale is NaN: the up rows of those tokens are, and so is the product either way)
+    dY = torch.empty((M, 8), dtype=torch.float16, device="cuda")
+    ctx.linear_q(dev(W), dev(np.ones((16, 2), np.float16)), g, dev(Xq), dev(Xs), dY, M, 16, K, epilogue=pkg.EPI_SWIGLU)
+    want = dev(gates.copy())
+    ctx.shim_silu_forward(want, M)
+    torch.cuda.synchronize()
+    got = dY.cpu().numpy()
+    want = want.cpu().numpy()
+    nan = np.isnan(want)
+    assert np.isnan(got[nan]).all() and nan.sum() == 2 * 1023 + 1  # NaN arguments, and -infinity
+    # -0: the sum of a zero group is +0, so the gate is
+    want[0x8000] = 0
+    assert np.array_equal(got[~nan].view(np.uint16), np.repeat(want[~nan].view(np.uint16)[:, None], 8, axis=1))
+
+
 @pytest.mark.parametrize("packed", [True, False])
 @pytest.mark.parametrize("M,g", [(3, 64), (16, 64), (8, 128)])
 def test_decode_linear_scales_at_any_address(ctx, oracle, pkg, M, g, packed):
