@@ -6,7 +6,7 @@ namespace gemm {
 
 // Group sizes without a case of their own, and calls that want the group sums.
 const Form* forms_any(int* count) {
-    static const Form table[] = {form<128, false, 0>(135, 330), form<128, true, 0>(165, 360)};
+    static const Form table[] = {form<128, false, 0>(135, 330, 1300), form<128, true, 0>(165, 360, 1300)};
     *count = static_cast<int>(sizeof(table) / sizeof(table[0]));
     return table;
 }
@@ -24,10 +24,10 @@ int split_kb(int K, int g, int splits) {
 }
 
 // setmaxnreg moves registers between the warpgroups of the widest form; the sums balance only for the register count the kernel
-// was compiled to (kLaunchRegs per thread). An unbalanced sum blocks for ever in setmaxnreg.inc, a wait nothing bounds, so in a
+// was compiled to (Form::launch_regs per thread). An unbalanced sum blocks for ever in setmaxnreg.inc, a wait nothing bounds, so in a
 // build that came out differently that form is not taken.
 bool balanced(const Form& f) {
-    if (!f.move_regs) return true;
+    if (f.launch_regs == 0) return true;
     int r = f.state->registers.load(std::memory_order_relaxed);
     if (r == 0) {
         cudaFuncAttributes fa;
@@ -37,7 +37,7 @@ bool balanced(const Form& f) {
         }
         f.state->registers.store(r = fa.numRegs, std::memory_order_relaxed);
     }
-    return r == kLaunchRegs;
+    return r == f.launch_regs;
 }
 
 struct Choice {
@@ -49,7 +49,7 @@ struct Choice {
 // that leaves the last wave nearly empty loses to one that fills it; narrow tiles win where there are few tokens.
 // A tile's K is split over two or four CTAs where all of them fit the chip at once (a cluster of four leaves some SMs of a
 // GPC over: 128 of 148 taken as usable); meeting and adding up measured 3-4 us for two and about 6 for four. A
-// split adds the groups in another order than the other kernels do, so it has to save 15 % at least (K = 2560 never does).
+// split adds the groups in another order than the other kernels do, so it has to save 10 % at least.
 // table_g: the group size whose forms are looked at (0: those of any group size). pair: -1 either, 0 one CTA per tile, 1 a pair.
 // only_bt, only_splits: 0, or the token width and the split (1: none) to take; no form where they do not fit the shape.
 template <class Usable>
@@ -69,8 +69,8 @@ Choice choose(int M, int N, int K, int table_g, int g, int sms, int pair, int on
             if (f.split && (tiles * splits > (splits == 2 ? sms / 2 * 2 : sms * 7 / 8 - 1) || (splits - 1) * split_kb(K, g, splits) >= kb_total))
                 continue;
             const double kb = f.split ? split_kb(K, g, splits) : kb_total;
-            double ns = ((tiles * splits + walkers - 1) / walkers) * (kb * f.stage_ns + kb * BK / g * f.group_ns);
-            if (f.split) ns = (ns + (splits == 2 ? 3500 : 6000)) / 0.85;
+            double ns = ((tiles * splits + walkers - 1) / walkers) * (kb * f.stage_ns + kb * BK / g * f.group_ns + f.tile_ns);
+            if (f.split) ns = (ns + (splits == 2 ? 3500 : 6000)) / 0.9;
             if ((!best.form || ns < best_ns) && usable(f)) { best = {&f, splits}; best_ns = ns; }
         }
     }
@@ -93,7 +93,7 @@ bool gemm_supports(const LinearArgs& a) {
 int gemm_form(int M, int N, int K, int g, int sms, int form, int only_bt, int only_splits, bool moved_registers, int* out3) {
     using namespace gemm;
     if (M < 1 || N < 1 || K < 1 || sms < 2 || K % BK != 0 || g % 32 != 0 || K % g != 0) return W8A8_ERR_UNSUPPORTED;
-    const Choice c = choose(M, N, K, g, g, sms, form, only_bt, only_splits, [&](const Form& f) { return moved_registers || !f.move_regs; });
+    const Choice c = choose(M, N, K, g, g, sms, form, only_bt, only_splits, [&](const Form& f) { return moved_registers || f.launch_regs == 0; });
     if (!c.form) return W8A8_ERR_UNSUPPORTED;
     out3[0] = c.form->bt;
     out3[1] = c.form->pair ? 2 : 1;

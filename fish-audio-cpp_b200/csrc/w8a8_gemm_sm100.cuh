@@ -12,7 +12,7 @@
 //   warp 0       producer: TMA loads of 128 weight rows and BT token rows, 128 bytes of K each (both matrices are
 //                row-major with K contiguous, i.e. already the K-major operand; TMA applies the 128-byte swizzle)
 //   warp 1       MMA issuer: four tcgen05.mma (K = 32) per stage; every K-group accumulates into its own BT-column slice
-//                of tensor memory (two or four slices), starting with "overwrite"
+//                of tensor memory (two to eight slices), starting with "overwrite" or, at g = 64, with a bias (below)
 //   warps 2, 3   stage the scales of four K-groups at a time in a ring of their own
 //   warps 4 ...  epilogue, eight or sixteen warps, each 32 weight rows x a part of the tokens. For every K-group
 //                acc = fma(float(P) * ws, xs, acc), groups ascending -- the arithmetic and order of
@@ -31,17 +31,29 @@
 // latency, and descriptors computed in divergent code are moved to uniform registers one by one): the tensor pipe ran at
 // 0.6 of its rate. Hence: the whole warp runs the loop and one elected lane issues; the loop is unrolled over the stages
 // so that stage, accumulator slice and descriptor offsets are immediates; group sizes 64 / 128 / 256 are template cases.
-// The promote is the other side, and at g = 64 the bound: per sum one int -> fp32 conversion (64 a clock and SM), half a
-// packed multiply and half a packed FMA, about 3 clocks per warp and scheduler, 770 clocks per group of a 128 x 256 tile
-// against 256 of MMAs; with tensor-memory and shared loads 870-900 (measured alone). So the sums are read in the layout of
-// an mma.sync accumulator (16x256b): a lane then holds 4 weight rows x 2 tokens of every 16 x 8 block and needs one
-// 8-byte read of activation scales per eight sums. With a thread per row (32x32b) it was a 16-byte read per four, and a
-// 16-byte read costs 8 clocks per scheduler even when all lanes read the same address: the promote took twice as long.
-// The other exact conversions (integer add into the mantissa of 1.5 * 2^23, the bias taken out by a subtract or inside
-// the multiply) measured 15-25 % slower than the conversion instruction: they compete with the FMAs for their pipe.
+// The promote is the other side, and the bound in most forms: stamps of the clock in the epilogue warps showed 1280 (g = 64) and 1390
+// (g = 256) clocks per K-group of a 128 x 256 tile against 256 and 1024 of MMAs. What it is made of, measured alone (16 warps):
+//   * per two sums two conversions, a packed multiply and a packed FMA; by themselves 4.3 clocks per warp and scheduler, with the
+//     tensor-memory and shared-memory reads around them 6.9-7.2, as if conversions and those reads shared a way into the registers.
+//     Without conversions, two packed FMAs, 5.1-5.6. Hence the BIAS at g = 64 (promote2): each group's accumulator starts from a
+//     constant, made by one more MMA of a constant operand with itself, that makes every sum positive; as bits it then is an fp32
+//     number, and the multiply that had to follow the conversion takes the bias out again, exactly. At g = 128 it would take two more MMAs per
+//     four, and at g = 256 the tensor pipe is the next bound.
+//   * about 360 clocks per K-group whatever the tile's width: two waits, the arrive, the loop. Hence UNITS of two K-groups of 64
+//     on the tiles of up to 128 tokens. (Four, or units at g = 128 and 256, would need a slot that is not known at compile time, as a
+//     tile may end inside a unit. With it in a register the lanes of the issuing warp have to meet at every wait and before it moves
+//     on; without that two builds ended with an illegal memory access, and with it g = 128 and 256 lost 10-40 %.)
+//   * the sums are read in the layout of an mma.sync accumulator (16x256b): a lane then holds 4 weight rows x 2 tokens of every 16 x 8
+//     block and reads the activation scales of eight sums with 8 bytes. (32x32b, a thread per row, is three times as fast out of tensor
+//     memory but needs a 16-byte read per four sums: 1.3-2 times as long in all, most while the MMAs read shared memory.)
+// The integer conversions (add into the mantissa of 1.5 * 2^23) measured 15-25 % slower than the conversion instruction.
+// The SwiGLU of a tile's end took 5900 of the 19 800 clocks of a tile at g = 256 (w8a8_swiglu.cuh).
 //
-// Measured, M x N x K = 8192 x 19456 x 2560: g = 256 591 us -> 346 us (1381 -> 2360 TOPS), g = 64 1511 us -> 898 us
-// (540 -> 909 TOPS), against the form before (tokens as A, one lane issuing, a thread per token row).
+// Measured back to back, us, before the bias, the units, the 16-byte scale reads, the SwiGLU and the costs fitted anew, and with
+// them (M x N x K):
+//   8192 x 19456 x 2560, g = 64   962 -> 788 (848 -> 1036 TOPS); g = 256 365 -> 343 (2236 -> 2380 TOPS)
+//   2048 x  2560 x 9728, g = 64   155 -> 124;  613 x 2560 x 9728  53.5 -> 43.3;  150 x 19456 x 2560  53 -> 36.7
+//   at g = 128 and 256 rows without SwiGLU within 4 % either way (pairs of 192 tokens 2-5 % slower: 4001 x 6144 x 2560 54.9 -> 57.2)
 //
 // Every mbarrier wait is bounded; a wait that runs out records an error word, and the CTA still frees its tensor memory
 // before it returns.
@@ -55,7 +67,7 @@ namespace w8a8 {
 namespace gemm {
 
 constexpr int BR = 128, BK = 128;            // weight rows per CTA; bytes of K per stage
-constexpr int kScGroups = 4, kScRing = 4;    // K-groups per chunk of scales, chunks in the ring
+constexpr int kScGroups = 4, kScRing = 3;    // K-groups per chunk of scales, chunks in the ring
 constexpr uint32_t kSpin = 1u << 21;
 
 struct GemmParams {
@@ -66,28 +78,41 @@ struct GemmParams {
     int tma_store;  // output rows are multiples of 16 bytes and aligned: the tile leaves by TMA
 };
 
-// Registers per thread of the 640-thread form that moves some between its warpgroups: at launch, in warpgroup 0, in the others.
-constexpr int kLaunchRegs = 96, kLowRegs = 56, kHighRegs = 104;
-static_assert(128 * (kLaunchRegs - kLowRegs) >= 512 * (kHighRegs - kLaunchRegs), "setmaxnreg sums must balance");
+// g = 64: the sums come out of the MMAs with kBias added, by a first MMA of a constant operand with itself.
+constexpr int kBiasByte = 184, kBias = kBiasByte * kBiasByte * 32, kConstBytes = BR * 32;
+static_assert(kBias > 128 * 128 * 64 && kBias + 128 * 128 * 64 < (1 << 23) && kBias % (1 << 11) == 0 && (kBias >> 11) < (1 << 13),
+              "sums above zero and below 2^23; 11 bits of a weight scale times the bias are exact in fp32");
 
-template <int BT, bool PAIR>
+template <int BT, bool PAIR, int GM>
 struct Config {
+    static constexpr bool kBiased = GM == 64 && BT >= 96;  // (narrower tiles are a chain, and the MMA would lengthen it: 1.05)
     static constexpr int kRowsB = PAIR ? BT / 2 : BT;                 // token rows this CTA loads
     static constexpr int kStageBytes = (BR + kRowsB) * BK;
     static constexpr int kPanelBytes = BT * 128;                      // BT tokens x 64 fp16 columns, 128-byte swizzle
     static constexpr int kOutBytes = 2 * kPanelBytes;
     static constexpr int kScSlot = kScGroups * (BT + BR) * 4;         // activation scales [4][BT], weight scales [4][128]
     static constexpr int kScBytes = kScRing * kScSlot;
-    static constexpr int kRoom = 226 * 1024 - 1024 - kOutBytes - kScBytes;
+    static constexpr int kConst = kBiased ? kConstBytes : 0;
+    static constexpr int kRoom = 226 * 1024 - 1024 - kOutBytes - kScBytes - kConst;
     static constexpr int kStages = kRoom / kStageBytes >= 8 ? 8 : 4;  // a multiple of four (see the issuer)
-    static constexpr int kSmem = kStages * kStageBytes + kOutBytes + kScBytes + 1024;
-    // Epilogue warps: four per part of the tokens (one per 32 weight rows). Four warps per scheduler on the wide tiles: with
-    // two, half of the issue slots stay empty (g = 64, 8192 x 19456 x 2560: 1012 us with eight warps, 900 with sixteen).
-    static constexpr int kParts = BT >= 128 ? 4 : 2;
+    static constexpr int kSmem = kStages * kStageBytes + kOutBytes + kScBytes + kConst + 1024;
+    // Epilogue warps: four per part of the tokens (one per 32 weight rows). Sixteen on the wide tiles; with the bias eight are as good
+    // at 256 tokens (steps of 32 tokens; 16: 1.03) and better at 128 (613 x 2560 x 9728 54.3 us for 55.7), not at 192
+    // (2048 x 19456 x 2560 247 us for 232).
+    static constexpr int kParts = BT >= 128 && !(kBiased && BT != 192) ? 4 : 2;
+    static constexpr int kStep = kBiased && BT == 256 ? 32 : 16;      // tokens per step of the promote
     static constexpr int kEpiWarps = 4 * kParts, kThreads = 128 + kEpiWarps * 32;
-    // The widest tile needs more registers in sixteen epilogue warps than 640 threads can have each: warpgroup 0 gives some up.
+    // The widest tile needs more registers in its epilogue warps than all threads can have: warpgroup 0 gives some up.
     static constexpr bool kMoveRegs = BT > 192;
-    static constexpr int kAcc = BT <= 128 ? 4 : 2;                    // accumulator slices
+    // Registers per thread of the form that moves some: at launch, in warpgroup 0, in the others.
+    static constexpr int kLaunchRegs = kParts == 2 ? 168 : 96, kLowRegs = kParts == 2 ? 40 : 56, kHighRegs = kParts == 2 ? 232 : 104;
+    static_assert(128 * (kLaunchRegs - kLowRegs) >= kEpiWarps * 32 * (kHighRegs - kLaunchRegs), "setmaxnreg sums must balance");
+    // K-groups per unit: what issuer and epilogue hand one another (see above). Two groups of 64: K is a multiple of 128, so every
+    // tile and every run of a split is whole units. Two units in tensor memory, four where they are small.
+    static constexpr int kUnit = GM == 64 && BT <= 128 ? 2 : 1;
+    static constexpr int kSlots = BT <= 64 || (kUnit == 1 && BT <= 128) ? 4 : 2;
+    static constexpr int kAcc = kUnit * kSlots;                       // accumulator slices
+    static constexpr int kBatch = GM != 0 && (BT == 64 || (BT == 32 && kUnit > 1)) ? 2 : 1;  // steps whose sums are requested together
     static constexpr int kTmemCols = kAcc * BT <= 128 ? 128 : kAcc * BT <= 256 ? 256 : 512;
     static_assert(kStages * kStageBytes <= kRoom, "stages do not fit");
     static_assert(BT % 32 == 0 && BT <= 256, "token width");
@@ -199,15 +224,25 @@ __device__ __forceinline__ void promote2(uint64_t& acc, uint32_t p0, uint32_t p1
         "mul.rn.f32x2 t, t, %3;\n\tfma.rn.f32x2 %0, t, %4, %0;\n\t}"
         : "+l"(acc) : "r"(p0), "r"(p1), "l"(ws), "l"(xs));
 }
-__device__ __forceinline__ uint64_t lds64(uint32_t addr) {
-    uint64_t v;
-    asm volatile("ld.shared.u64 %0, [%1];" : "=l"(v) : "r"(addr));
-    return v;
+// The same where the sums carry kBias: as bits, P + kBias is the fp32 number (P + kBias) * 2^-149, so one FMA converts, takes the
+// bias out and multiplies, with one rounding, that of float(P) * ws: ws comes times 2^111, bias is -kBias * 2^-149 times that, and
+// acc is 2^-38 times the sum.
+__device__ __forceinline__ void promote2(uint64_t& acc, uint32_t p0, uint32_t p1, uint64_t ws, uint64_t bias, uint64_t xs) {
+    asm("{\n\t.reg .b64 t;\n\tmov.b64 t, {%1, %2};\n\tfma.rn.f32x2 t, t, %3, %4;\n\tfma.rn.f32x2 %0, t, %5, %0;\n\t}"
+        : "+l"(acc) : "r"(p0), "r"(p1), "l"(ws), "l"(bias), "l"(xs));
 }
-__device__ __forceinline__ float lds32(uint32_t addr) {
-    float v;
-    asm volatile("ld.shared.f32 %0, [%1];" : "=f"(v) : "r"(addr));
-    return v;
+__device__ __forceinline__ void mul2(uint64_t& v, uint64_t f) { asm("mul.rn.f32x2 %0, %0, %1;" : "+l"(v) : "l"(f)); }
+// Where the scales of token t and of weight row n lie in their [groups][BT] and [groups][128] of shared memory: what a lane reads for
+// sixteen tokens (two neighbouring ones of either eight), or for its four weight rows, is one 16-byte piece. Such a read, its
+// address shared by the lanes of a row or column, takes shared memory as long as one of 8 bytes (two clocks, twice that while the
+// MMAs read their operands), of which there would be two, or four of 4 bytes.
+__device__ __forceinline__ int xs_slot(int t) { return (t & ~15) | ((t & 6) << 1) | ((t >> 2) & 2) | (t & 1); }
+__device__ __forceinline__ int ws_slot(int n) { return (n & ~31) | ((n & 7) << 2) | ((n >> 3) & 3); }
+__device__ __forceinline__ void lds_2x64(uint32_t addr, uint64_t& a, uint64_t& b) {
+    asm volatile("ld.shared.v2.u64 {%0, %1}, [%2];" : "=l"(a), "=l"(b) : "r"(addr));
+}
+__device__ __forceinline__ void lds_4x32(uint32_t addr, float (&v)[4]) {
+    asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v[0]), "=f"(v[1]), "=f"(v[2]), "=f"(v[3]) : "r"(addr));
 }
 // Four 8 x 8 fp16 matrices held as accumulator fragments, stored TRANSPOSED: lane l gives the address of the 16-byte row
 // l % 8 of matrix l / 8.
@@ -230,6 +265,45 @@ __device__ __forceinline__ uint64_t smem_desc(uint32_t saddr) {
            (2ull << 61) /* SWIZZLE_128B */;
 }
 
+// With the bias (promote2), an infinite weight scale gives infinity less infinity. The output columns of such weight rows, in the
+// tile that lies in shared memory, are formed anew, from the operands: signed infinities and NaN as float(P) * ws has them. Slow, and
+// only run once a CTA has met an infinite scale.
+template <class C>
+__device__ __forceinline__ void infinite_rows(const LinearArgs& a, uint32_t out_stage, int m0, int n0, int tokens, bool swiglu, int et) {
+    auto infinite = [&](int n) {
+        bool any = false;
+        for (int j = 0; j < a.G; ++j) any |= isinf(__half2float(a.w_scale[static_cast<size_t>(n) * a.G + j]));
+        return any;
+    };
+    auto sum = [&](int n, int m) {
+        const int* w = reinterpret_cast<const int*>(a.W + static_cast<size_t>(n) * a.K);
+        const int* x = reinterpret_cast<const int*>(a.Xq + static_cast<size_t>(m) * a.K);
+        float acc = 0.0f;
+#pragma unroll 1
+        for (int j = 0; j < a.G; ++j) {
+            int p = 0;
+#pragma unroll 1
+            for (int k = 0; k < a.g / 4; ++k) p = __dp4a(w[j * (a.g / 4) + k], x[j * (a.g / 4) + k], p);
+            acc = fmaf(static_cast<float>(p) * __half2float(a.w_scale[static_cast<size_t>(n) * a.G + j]), a.Xs[static_cast<size_t>(m) * a.G + j], acc);
+        }
+        return acc;
+    };
+#pragma unroll 1
+    for (int row = 0; row < BR && n0 + row < a.N; ++row) {
+        if (swiglu && (row & 8)) continue;  // (taken with its gate row)
+        const int n = n0 + row;
+        if (!infinite(n) && !(swiglu && infinite(n + 8))) continue;
+        const int col = swiglu ? (row >> 4) * 8 + (row & 7) : row;
+#pragma unroll 1
+        for (int t = et; t < tokens; t += C::kEpiWarps * 32) {
+            __half y = __float2half(sum(n, m0 + t));
+            if (swiglu) y = __low2half(swiglu2(__half2half2(y), __half2half2(__float2half(sum(n + 8, m0 + t)))));
+            asm volatile("st.shared.u16 [%0], %1;" ::"r"(out_stage + (col >> 6) * C::kPanelBytes + t * 128 +
+                                                         ((((col & 63) >> 3) ^ (t & 7)) << 4) + (col & 7) * 2), "h"(__half_as_ushort(y)) : "memory");
+        }
+    }
+}
+
 // GM: the group size when it is 64, 128 or 256; 0 = any multiple of 32 (plain loops), and whenever the group sums are asked
 // for as well.
 //
@@ -238,21 +312,23 @@ __device__ __forceinline__ uint64_t smem_desc(uint32_t saddr) {
 // 430-650 clocks per K-group, whatever the number of CTAs (tokens x rows x K, g = 64: 150 x 2560 x 9728 34.8 -> 27.0 us, 64 x
 // 2560 x 9728 34.8 -> 17.9, 150 x 2560 x 4096 19.3 -> 16.4).
 template <int BT, bool PAIR, int GM, bool SPLIT>
-__global__ void __launch_bounds__(Config<BT, PAIR>::kThreads, 1)
+__global__ void __launch_bounds__(Config<BT, PAIR, GM>::kThreads, 1)
 gemm_i8_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_x,
                const __grid_constant__ CUtensorMap map_y, const GemmParams p) {
-    using C = Config<BT, PAIR>;
+    using C = Config<BT, PAIR, GM>;
     constexpr int S = C::kStages, kEpiWarps = C::kEpiWarps, kEpiThreads = kEpiWarps * 32;
     extern __shared__ unsigned char smem_raw[];
-    __shared__ __align__(8) uint64_t full_bar[S], empty_bar[S], acc_full[C::kAcc], acc_empty[C::kAcc], sc_full[kScRing], sc_empty[kScRing];
+    __shared__ __align__(8) uint64_t full_bar[S], empty_bar[S], acc_full[C::kSlots], acc_empty[C::kSlots], sc_full[kScRing], sc_empty[kScRing];
     __shared__ uint32_t tmem_base_s;
     __shared__ int failed_s;
+    // kBiased: a weight scale that this CTA has met is infinite; the same, as all epilogue threads are to see it at a tile's end
+    __shared__ int infinite_s, infinite_tile_s;
 
     const LinearArgs& a = p.a;
     // (through a shuffle, so that the compiler knows it is the same in all lanes and keeps what follows from it in uniform registers)
     const int warp = __shfl_sync(0xffffffffu, static_cast<int>(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
     const uint32_t tiles = (ptx::smem_u32(smem_raw) + 1023u) & ~1023u;
-    const uint32_t out_stage = tiles + S * C::kStageBytes, sc_ring = out_stage + C::kOutBytes;
+    const uint32_t out_stage = tiles + S * C::kStageBytes, sc_ring = out_stage + C::kOutBytes, const_tile = sc_ring + C::kScBytes;
     static_assert(!SPLIT || (!PAIR && GM != 0), "a split tile is one CTA's, of whole K-groups");
     const int srank = SPLIT ? static_cast<int>(cluster_rank()) : 0;
     const int kb0 = SPLIT ? srank * p.split_kb : 0;
@@ -268,13 +344,19 @@ gemm_i8_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
 
     if (threadIdx.x == 0) {
         for (int s = 0; s < S; ++s) { ptx::mbar_init(&full_bar[s], 1); ptx::mbar_init(&empty_bar[s], 1); }
-        for (int s = 0; s < C::kAcc; ++s) {
+        for (int s = 0; s < C::kSlots; ++s) {
             ptx::mbar_init(&acc_full[s], 1);
             ptx::mbar_init(&acc_empty[s], PAIR ? 2 * kEpiWarps : kEpiWarps);
         }
         for (int s = 0; s < kScRing; ++s) { ptx::mbar_init(&sc_full[s], 128); ptx::mbar_init(&sc_empty[s], kEpiWarps); }
         failed_s = 0;
+        infinite_s = 0;
         ptx::fence_barrier_init();
+        ptx::fence_proxy_async();
+    }
+    if constexpr (C::kBiased) {  // (the operand of the first MMA of every K-group: the same byte everywhere, so its layout is any)
+        for (int i = threadIdx.x; i < kConstBytes / 4; i += C::kThreads)
+            asm volatile("st.shared.u32 [%0], %1;" ::"r"(const_tile + i * 4), "r"(kBiasByte * 0x01010101u) : "memory");
         ptx::fence_proxy_async();
     }
     if (warp == 1) tmem_alloc<PAIR>(&tmem_base_s, C::kTmemCols);
@@ -287,7 +369,7 @@ gemm_i8_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
     ptx::pdl_wait();
 
     if (warp < 4) {
-        if constexpr (C::kMoveRegs) asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kLowRegs) : "memory");
+        if constexpr (C::kMoveRegs) asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(C::kLowRegs) : "memory");
         if (warp == 0) {
             // ---------------- producer ----------------
             const bool leader = elect_one();
@@ -344,6 +426,10 @@ gemm_i8_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
                                            (static_cast<uint32_t>(BT >> 3) << 17) | (static_cast<uint32_t>((PAIR ? 2 * BR : BR) >> 4) << 24);
                 const bool leader = elect_one();
                 const uint64_t desc0 = smem_desc(tiles);
+                // uint8 x uint8; rows of 32 bytes in groups of eight, 32-byte swizzle
+                constexpr uint32_t bias_idesc = idesc & ~((7u << 7) | (7u << 10));
+                const uint64_t bias_desc = static_cast<uint64_t>((const_tile & 0x3ffffu) >> 4) | (1ull << 16) |
+                                           (static_cast<uint64_t>(256 >> 4) << 32) | (1ull << 46) | (6ull << 61);
                 int left = my_tiles * num_kb;
                 uint32_t parity = 0, acc_parity = 1;
                 int code = 0;  // what ran out, if anything
@@ -358,28 +444,34 @@ gemm_i8_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
                         // (a step of 32 bytes along K inside the 128-byte swizzled row: +2 in the descriptor's address field)
                         if constexpr (GM != 0) {
                             // the groups of this stage: half a group, one, or two
-                            constexpr int kPerStage = GM == 64 ? 2 : 1, kMmas = 4 / kPerStage, kLoopGroups = S * 128 / GM;
+                            constexpr int kPerStage = GM == 64 ? 2 : 1, kMmas = 4 / kPerStage;
                             const bool first = GM != 256 || s % 2 == 0, last = GM != 256 || s % 2 == 1;
                             if (!wait(&full_bar[s], parity)) { code = 300 + s; break; }
 #pragma unroll
                             for (int h = 0; h < kPerStage; ++h) {
-                                const int lg = GM == 256 ? s / 2 : s * kPerStage + h;                  // group inside this turn of the ring
-                                const int as = kLoopGroups >= C::kAcc ? lg % C::kAcc : lg + as_any;     // its accumulator slice
-                                if (first) {
+                                // A turn of the ring is whole rounds of the slots, or half of one.
+                                constexpr int kTurn = S * 128 / GM / C::kUnit;  // units
+                                static_assert(S * 128 / GM % C::kUnit == 0 && (kTurn % C::kSlots == 0 || 2 * kTurn == C::kSlots), "rounds of the slots");
+                                const int lg = GM == 256 ? s / 2 : s * kPerStage + h, lu = lg / C::kUnit;  // group and unit inside this turn
+                                const int as = kTurn >= C::kSlots ? lu % C::kSlots : lu + as_any;
+                                const bool opens = first && lg % C::kUnit == 0, closes = last && lg % C::kUnit == C::kUnit - 1;
+                                if (opens) {
                                     if (!wait(&acc_empty[as], acc_parity)) { code = 400 + as; break; }
                                     tc_fence_after();
                                 }
                                 if (leader) {
+                                    const uint32_t to = tmem_base + (as * C::kUnit + lg % C::kUnit) * BT;
+                                    if (C::kBiased && first) mma_i8<PAIR>(to, bias_desc, bias_desc, bias_idesc, 0u);
 #pragma unroll
                                     for (int sub = h * kMmas; sub < (h + 1) * kMmas; ++sub)
-                                        mma_i8<PAIR>(tmem_base + as * BT, da + 2 * sub, db + 2 * sub, idesc, (first && sub == h * kMmas) ? 0u : 1u);
-                                    if (last) tc_commit<PAIR>(&acc_full[as]);  // the K-group's sums are complete
+                                        mma_i8<PAIR>(to, da + 2 * sub, db + 2 * sub, idesc, (!C::kBiased && first && sub == h * kMmas) ? 0u : 1u);
+                                    if (closes) tc_commit<PAIR>(&acc_full[as]);  // the unit's sums are complete
                                 }
-                                if (kLoopGroups >= C::kAcc && last && lg % C::kAcc == C::kAcc - 1) acc_parity ^= 1u;
+                                if (kTurn >= C::kSlots && closes && lu % C::kSlots == C::kSlots - 1) acc_parity ^= 1u;
+                                if (kTurn < C::kSlots && closes && lu == kTurn - 1 && (as_any = kTurn - as_any) == 0) acc_parity ^= 1u;
                             }
                             if (code) break;
                             if (leader) tc_commit<PAIR>(&empty_bar[s]);  // the stage may be refilled once these MMAs retire
-                            if (kLoopGroups < C::kAcc && s == S - 1 && (as_any = kLoopGroups - as_any) == 0) acc_parity ^= 1u;
                         } else {
                             if (!wait(&full_bar[s], parity)) { code = 300 + s; break; }
                             // (Rolled up, the four MMAs of a stage took the issuing warp longer than they take: one scale per channel,
@@ -394,7 +486,7 @@ gemm_i8_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
                                 if (++q_in_group == mpg) {
                                     if (leader) tc_commit<PAIR>(&acc_full[as_any]);
                                     q_in_group = 0;
-                                    if (++as_any == C::kAcc) { as_any = 0; acc_parity ^= 1u; }
+                                    if (++as_any == C::kSlots) { as_any = 0; acc_parity ^= 1u; }
                                 }
                             }
                             if (code) break;
@@ -409,9 +501,25 @@ gemm_i8_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
         } else {
             // ---------------- scales, four groups per chunk: activation scales [4][BT], weight scales [4][128], fp32 ----------------
             const int t64 = threadIdx.x - 64;
+            constexpr float kScale = C::kBiased ? 0x1p111f : 1.0f;  // (see promote2)
             int slot = 0;
             uint32_t parity = 1;
             bool ok = true;
+            // The weight scales are read a chunk ahead: a read takes as long as the narrow tiles take for a chunk.
+            __half w[2][kScGroups];
+            auto load_w = [&](int tile, int j0) {
+                if (j0 >= g_end) { tile += walkers; j0 = g_first; }
+                if (tile >= p.tiles_total) return;
+                const int n0 = tile_n0(tile);
+                const __half* ws0 = a.w_scale + static_cast<size_t>(min(n0 + t64, a.N - 1)) * G;
+                const __half* ws1 = a.w_scale + static_cast<size_t>(min(n0 + 64 + t64, a.N - 1)) * G;
+#pragma unroll
+                for (int q = 0; q < kScGroups; ++q) {
+                    w[0][q] = ws0[min(j0 + q, G - 1)];
+                    w[1][q] = ws1[min(j0 + q, G - 1)];
+                }
+            };
+            load_w(walker, g_first);
             for (int tile = walker; tile < p.tiles_total && ok; tile += walkers) {
                 const int m0 = tile_m0(tile), n0 = tile_n0(tile);
                 if (a.epilogue == W8A8_EPI_RESIDUAL && srank == 0) {  // the tile's residual rows to L2, long before its end needs them
@@ -421,16 +529,8 @@ gemm_i8_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
                             asm volatile("prefetch.global.L2 [%0];" ::"l"(a.residual + static_cast<size_t>(t) * a.N + col));
                     }
                 }
-                const __half* ws0 = a.w_scale + static_cast<size_t>(min(n0 + t64, a.N - 1)) * G;
-                const __half* ws1 = a.w_scale + static_cast<size_t>(min(n0 + 64 + t64, a.N - 1)) * G;
                 for (int j0 = g_first; j0 < g_end; j0 += kScGroups) {
                     const int nj = min(kScGroups, g_end - j0);
-                    __half w[2][kScGroups];  // on their way while the slot is waited for
-#pragma unroll
-                    for (int q = 0; q < kScGroups; ++q) {
-                        w[0][q] = ws0[min(j0 + q, G - 1)];
-                        w[1][q] = ws1[min(j0 + q, G - 1)];
-                    }
                     if (!wait(&sc_empty[slot], parity)) {
                         atomicExch(p.status, 600 + slot);
                         ok = false;
@@ -441,15 +541,18 @@ gemm_i8_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
                         const float* src = a.Xs + static_cast<size_t>(min(m0 + t, a.M - 1)) * G + j0;
 #pragma unroll
                         for (int q = 0; q < kScGroups; ++q)
-                            if (q < nj) asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(dst + (q * BT + t) * 4), "l"(src + q) : "memory");
+                            if (q < nj) asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(dst + (q * BT + xs_slot(t)) * 4), "l"(src + q) : "memory");
                     }
                     asm volatile("cp.async.mbarrier.arrive.noinc.shared.b64 [%0];" ::"r"(ptx::smem_u32(&sc_full[slot])) : "memory");
 #pragma unroll
                     for (int q = 0; q < kScGroups; ++q) {
-                        asm volatile("st.shared.f32 [%0], %1;" ::"r"(dst + (kScGroups * BT + q * BR + t64) * 4), "f"(__half2float(w[0][q])) : "memory");
-                        asm volatile("st.shared.f32 [%0], %1;" ::"r"(dst + (kScGroups * BT + q * BR + 64 + t64) * 4), "f"(__half2float(w[1][q])) : "memory");
+                        const float w0 = __half2float(w[0][q]), w1 = __half2float(w[1][q]);
+                        if (C::kBiased && (isinf(w0) || isinf(w1))) infinite_s = 1;
+                        asm volatile("st.shared.f32 [%0], %1;" ::"r"(dst + (kScGroups * BT + q * BR + ws_slot(t64)) * 4), "f"(w0 * kScale) : "memory");
+                        asm volatile("st.shared.f32 [%0], %1;" ::"r"(dst + (kScGroups * BT + q * BR + 64 + ws_slot(t64)) * 4), "f"(w1 * kScale) : "memory");
                     }
                     ptx::mbar_arrive(&sc_full[slot]);
+                    load_w(tile, j0 + kScGroups);
                     if (++slot == kScRing) { slot = 0; parity ^= 1u; }
                 }
             }
@@ -458,15 +561,18 @@ gemm_i8_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
         __syncwarp();
         if constexpr (SPLIT) cluster_sync_all();  // (the epilogue's meeting below)
     } else {
-        if constexpr (C::kMoveRegs) asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(kHighRegs) : "memory");
+        if constexpr (C::kMoveRegs) asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(C::kHighRegs) : "memory");
         // ---------------- epilogue: each warp 32 weight rows x a part of the tokens ----------------
         // A lane holds four weight rows (16 h + 8 e + lane / 4) and, of every eight tokens, two neighbouring ones.
         constexpr int HC = BT / C::kParts;              // tokens per warp
-        constexpr int CH = 16;                          // tokens per step
+        constexpr int CH = C::kStep;                    // tokens per step
         constexpr int NCH = HC / CH, OCT = HC / 8;
         const int quad = warp & 3;                      // the tensor-memory lane quadrant this warp may read
         const int part = (warp - 4) >> 2;               // which part of the tokens
         const int et = (warp - 4) * 32 + lane;
+        constexpr int U = C::kUnit;
+        constexpr int STEPS = U * NCH, BATCH = C::kBatch;
+        static_assert(STEPS % BATCH == 0 && kScGroups % U == 0, "whole batches, whole units in a chunk of scales");
         int as = 0, slot = 0;
         uint32_t acc_parity = 0, sc_parity = 0;
         bool ok = true;
@@ -481,13 +587,8 @@ gemm_i8_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
                 for (int e = 0; e < 2; ++e)
 #pragma unroll
                     for (int o = 0; o < OCT; ++o) acc[h][e][o] = 0ull;
-            // (A second buffer of sums, filled while the first is promoted, and a look-ahead into the next group were measured: no
-            // gain with four warps per scheduler, and a loss where the tensor pipe is the slower side.)
-            uint32_t r[2][CH / 2];
-            auto load_sums = [&](uint32_t taddr) {
-                tmem_ld(taddr, r[0]);
-                tmem_ld(taddr + (16u << 16), r[1]);
-            };
+            // (A second buffer of sums, filled while the first is promoted, within a group or from one to the next: no gain.)
+            uint32_t r[BATCH][2][CH / 2];
 #pragma unroll 1
             for (int j0 = g_first; j0 < g_end && ok; j0 += kScGroups) {
                 if (!wait(&sc_full[slot], sc_parity)) {
@@ -495,72 +596,111 @@ gemm_i8_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
                     ok = false;
                     break;
                 }
-                uint32_t xs_addr = sc_ring + slot * C::kScSlot + (part * HC + 2 * (lane & 3)) * 4;
-                uint32_t ws_addr = sc_ring + slot * C::kScSlot + (kScGroups * BT + quad * 32 + (lane >> 2)) * 4;
+                uint32_t xs_addr = sc_ring + slot * C::kScSlot + (part * HC + 4 * (lane & 3)) * 4;
+                uint32_t ws_addr = sc_ring + slot * C::kScSlot + (kScGroups * BT + quad * 32 + 4 * (lane >> 2)) * 4;
                 const int j1 = min(j0 + kScGroups, g_end);
 #pragma unroll 1
-                for (int j = j0; j < j1; ++j) {
-                    uint64_t w2[2][2];
-#pragma unroll
-                    for (int h = 0; h < 2; ++h)
-#pragma unroll
-                        for (int e = 0; e < 2; ++e) {
-                            const float w = lds32(ws_addr + (16 * h + 8 * e) * 4);
-                            w2[h][e] = pack2(w, w);
-                        }
-                    const uint32_t taddr = taddr0 + as * BT;
+                for (int j = j0; j < j1; j += U) {
+                    const uint32_t taddr = taddr0 + as * (U * BT);
+                    float w4[BATCH][4];
+                    if constexpr (U == 1) lds_4x32(ws_addr, w4[0]);
                     if (!wait(&acc_full[as], acc_parity)) {
                         if (lane == 0) atomicExch(p.status, 500 + as);
                         ok = false;
                         break;
                     }
                     tc_fence_after();
-                    load_sums(taddr);
+                    auto load_sums = [&](int q0) {  // the sums of the steps from q0
 #pragma unroll
-                    for (int ci = 0; ci < NCH; ++ci) {
-                        uint64_t x2[CH / 8];
+                        for (int b = 0; b < BATCH; ++b)
 #pragma unroll
-                        for (int o = 0; o < CH / 8; ++o) x2[o] = lds64(xs_addr + (ci * CH + 8 * o) * 4);
+                            for (int c = 0; c < CH; c += 16) {
+                                const uint32_t from = taddr + (q0 + b) / NCH * BT + (q0 + b) % NCH * CH + c;
+                                tmem_ld(from, *reinterpret_cast<uint32_t(*)[8]>(&r[b][0][c / 2]));
+                                tmem_ld(from + (16u << 16), *reinterpret_cast<uint32_t(*)[8]>(&r[b][1][c / 2]));
+                            }
+                    };
+                    load_sums(0);
+                    uint64_t w2[2][2], b2[2][2];
+#pragma unroll
+                    for (int q0 = 0; q0 < STEPS; q0 += BATCH) {
+                        uint64_t x2[BATCH][CH / 8];
+#pragma unroll
+                        for (int b = 0; b < BATCH; ++b)
+#pragma unroll
+                            for (int o = 0; o < CH / 8; o += 2)
+                                lds_2x64(xs_addr + ((q0 + b) / NCH * BT + (q0 + b) % NCH * CH + 8 * o) * 4, x2[b][o], x2[b][o + 1]);
+                        if constexpr (U > 1) {
+#pragma unroll
+                            for (int b = 0; b < BATCH; ++b)
+                                if ((q0 + b) % NCH == 0) lds_4x32(ws_addr + (q0 + b) / NCH * BR * 4, w4[b]);
+                        }
                         tmem_ld_wait();
-                        if (ci + 1 == NCH) {
-                            // The group's last sums are in registers: the slice may be overwritten while they are promoted.
+                        if (q0 + BATCH == STEPS) {
+                            // The unit's last sums are in registers: its slices may be overwritten while they are promoted.
                             tc_fence_before();
                             __syncwarp();
                             if (lane == 0) {
                                 if (PAIR && crank != 0) mbar_arrive_cluster(acc_empty0 + as * 8);
                                 else ptx::mbar_arrive(&acc_empty[as]);
                             }
-                            if (++as == C::kAcc) { as = 0; acc_parity ^= 1u; }
                         }
 #pragma unroll
-                        for (int o = 0; o < CH / 8; ++o)
+                        for (int b = 0; b < BATCH; ++b) {
+                            const int ci = (q0 + b) % NCH;
+                            if (ci == 0) {
 #pragma unroll
-                            for (int h = 0; h < 2; ++h)
-#pragma unroll
-                                for (int e = 0; e < 2; ++e)
-                                    promote2(acc[h][e][ci * (CH / 8) + o], r[h][4 * o + 2 * e], r[h][4 * o + 2 * e + 1], w2[h][e], x2[o]);
-                        if constexpr (GM == 0) {
-                            if (a.dump) {
-#pragma unroll
-                                for (int o = 0; o < CH / 8; ++o)
-#pragma unroll
-                                    for (int i = 0; i < 8; ++i) {
-                                        const int n = n0 + quad * 32 + 16 * (i >> 2) + 8 * ((i >> 1) & 1) + (lane >> 2);
-                                        const int m = m0 + part * HC + ci * CH + 8 * o + 2 * (lane & 3) + (i & 1);
-                                        if (m < a.M && n < a.N)
-                                            a.dump[(static_cast<size_t>(m) * a.N + n) * G + j] = static_cast<int>(r[i >> 2][4 * o + (i & 3)]);
+                                for (int i = 0; i < 4; ++i) {
+                                    const float w = w4[b][i];
+                                    w2[i / 2][i % 2] = pack2(w, w);
+                                    if constexpr (C::kBiased) {
+                                        const float bias = w * -__int_as_float(kBias);
+                                        b2[i / 2][i % 2] = pack2(bias, bias);
                                     }
+                                }
+                            }
+#pragma unroll
+                            for (int o = 0; o < CH / 8; ++o)
+#pragma unroll
+                                for (int h = 0; h < 2; ++h)
+#pragma unroll
+                                    for (int e = 0; e < 2; ++e) {
+                                        uint64_t& to = acc[h][e][ci * (CH / 8) + o];
+                                        const uint32_t p0 = r[b][h][4 * o + 2 * e], p1 = r[b][h][4 * o + 2 * e + 1];
+                                        if constexpr (C::kBiased) promote2(to, p0, p1, w2[h][e], b2[h][e], x2[b][o]);
+                                        else promote2(to, p0, p1, w2[h][e], x2[b][o]);
+                                    }
+                            if constexpr (GM == 0) {
+                                if (a.dump) {
+#pragma unroll
+                                    for (int o = 0; o < CH / 8; ++o)
+#pragma unroll
+                                        for (int i = 0; i < 8; ++i) {
+                                            const int n = n0 + quad * 32 + 16 * (i >> 2) + 8 * ((i >> 1) & 1) + (lane >> 2);
+                                            const int m = m0 + part * HC + ci * CH + 8 * o + 2 * (lane & 3) + (i & 1);
+                                            if (m < a.M && n < a.N)
+                                                a.dump[(static_cast<size_t>(m) * a.N + n) * G + j] = static_cast<int>(r[b][i >> 2][4 * o + (i & 3)]);
+                                        }
+                                }
                             }
                         }
-                        if (ci + 1 < NCH) load_sums(taddr + (ci + 1) * CH);
+                        if (q0 + BATCH < STEPS) load_sums(q0 + BATCH);
                     }
-                    xs_addr += BT * 4;
-                    ws_addr += BR * 4;
+                    if (++as == C::kSlots) { as = 0; acc_parity ^= 1u; }
+                    xs_addr += U * BT * 4;
+                    ws_addr += U * BR * 4;
                 }
                 // the chunk's scales are used up
                 __syncwarp();
                 if (lane == 0) ptx::mbar_arrive(&sc_empty[slot]);
                 if (++slot == kScRing) { slot = 0; sc_parity ^= 1u; }
+            }
+            int infinite = 0;
+            if constexpr (C::kBiased) {
+                infinite = infinite_s;
+                const uint64_t up = pack2(0x1p38f, 0x1p38f);
+#pragma unroll
+                for (int i = 0; i < 4 * OCT; ++i) mul2(acc[i / (2 * OCT)][i / OCT % 2][i % OCT], up);
             }
             if constexpr (SPLIT) {
                 // Every stage of this CTA's ring has been loaded and multiplied: its memory holds the sums now. One tile per CTA.
@@ -579,6 +719,11 @@ gemm_i8_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
                 }
                 for (int c = 1; c < p.splits; ++c) {
                     const uint32_t theirs = map_to_rank(mine, c);
+                    if constexpr (C::kBiased) {
+                        int v;
+                        asm volatile("ld.shared::cluster.s32 %0, [%1];" : "=r"(v) : "r"(map_to_rank(ptx::smem_u32(&infinite_s), c)) : "memory");
+                        infinite |= v;
+                    }
                     uint64_t v[4 * OCT];
 #pragma unroll
                     for (int i = 0; i < 4 * OCT; ++i)
@@ -591,7 +736,10 @@ gemm_i8_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
                 }
             }
             // ---- the tile as fp16 in shared memory: panels of [BT tokens][64 columns], 128-byte rows, swizzled ----
-            if (et == 0) asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");  // the tile before has left it
+            if (et == 0) {
+                asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");  // the tile before has left it
+                if constexpr (C::kBiased) infinite_tile_s = infinite;
+            }
             if (epi_barrier_any<kEpiThreads>(!ok)) {
                 failed_s = 1;
                 break;
@@ -612,6 +760,12 @@ gemm_i8_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
                 for (int o = 0; o < OCT; ++o)
                     stmatrix_x4_trans(dst + o * 8 * 128, half2_bits(acc[0][0][o]), half2_bits(acc[0][1][o]), half2_bits(acc[1][0][o]),
                                       half2_bits(acc[1][1][o]));
+            }
+            if constexpr (C::kBiased) {
+                if (infinite_tile_s) {
+                    epi_barrier<kEpiThreads>();
+                    infinite_rows<C>(a, out_stage, m0, n0, min(BT, a.M - m0), swiglu, et);
+                }
             }
             const int ycols = swiglu ? a.N / 2 : a.N, y0 = swiglu ? n0 / 2 : n0;   // first output column of this CTA
             const int width = min(swiglu ? BR / 2 : BR, ycols - y0);                // columns it owns (<= 0: none)
@@ -698,32 +852,39 @@ struct FormState {
     SmemAttribute attribute;
     std::atomic<int> registers{0};  // per thread, as compiled (0: not asked for yet)
 };
-// A tile form: its kernel and what the launch needs to know about it. stage_ns, group_ns: what a tile takes per 128 bytes of
-// K and per K-group, fitted to one shape, 8192 x 19456 x 2560 at g = 256 and g = 64 (the two overlap; their sum is what was
-// measured). There is no term for a chain's start or a tile's end (conversion, residual, store): at 2048 and 8192 tokens the
-// predicted times of w2 lie 10-25 % below measured ones, so forms that differ by a few per cent are not told apart.
+// A tile form: its kernel and what the launch needs to know about it. stage_ns, group_ns, tile_ns: what a tile takes per 128 bytes of
+// K, per K-group and for itself (the start of its chain, conversion, store), fitted to the four projections at 100 to 4001 tokens, for
+// each group size; with 2.5 us for the launch they give the measured times within 15 %. At 8192 tokens, where the codes of w2 do not
+// stay in L2, pairs of 256 tokens lose more than pairs of 192 (8192 x 2560 x 9728, g = 256: 245 us and 205), so 192 is set 3-4 %
+// lower than fitted, and 256 at groups of 128 and 256 2-4 % higher.
 struct Form {
     int bt;
     bool pair, split;
     Kernel kernel;
     int threads, smem;
-    bool move_regs;
-    float stage_ns, group_ns;
+    int launch_regs;  // per thread, if the form moves some between its warpgroups; else 0
+    float stage_ns, group_ns, tile_ns;
     FormState* state;
 };
 template <int BT, bool PAIR, int GM, bool SPLIT>
 inline FormState form_state;
 template <int BT, bool PAIR, int GM, bool SPLIT = false>
-Form form(float stage_ns, float group_ns) {
-    return Form{BT, PAIR, SPLIT, gemm_i8_kernel<BT, PAIR, GM, SPLIT>, Config<BT, PAIR>::kThreads, Config<BT, PAIR>::kSmem, Config<BT, PAIR>::kMoveRegs, stage_ns, group_ns,
-                &form_state<BT, PAIR, GM, SPLIT>};
+Form form(float stage_ns, float group_ns, float tile_ns) {
+    using C = Config<BT, PAIR, GM>;
+    return Form{BT, PAIR, SPLIT, gemm_i8_kernel<BT, PAIR, GM, SPLIT>, C::kThreads, C::kSmem, C::kMoveRegs ? C::kLaunchRegs : 0,
+                stage_ns, group_ns, tile_ns, &form_state<BT, PAIR, GM, SPLIT>};
 }
 template <int GM>
 const Form* all_forms(int* count) {
-    static const Form table[] = {form<32, false, GM>(148, 157), form<64, false, GM>(136, 196), form<96, false, GM>(106, 300),
-                                 form<128, false, GM>(135, 330), form<192, true, GM>(215, 440), form<256, true, GM>(247, 557),
-                                 form<32, false, GM, true>(148, 157), form<64, false, GM, true>(136, 196), form<96, false, GM, true>(106, 300),
-                                 form<128, false, GM, true>(135, 330)};
+    // per stage at groups of 64, 128 and 256, and per tile, for token widths 32, 64, 96, 128, 192, 256
+    constexpr float kStage[3][6] = {{332, 467, 562, 635, 940, 1176}, {210, 307, 354, 399, 596, 745}, {153, 192, 225, 235, 340, 412}};
+    constexpr float kTile[3][6] = {{311, 573, 641, 1057, 1669, 2164}, {535, 699, 799, 1411, 1952, 2547}, {166, 615, 553, 1270, 2060, 2689}};
+    constexpr int q = GM == 64 ? 0 : GM == 128 ? 1 : 2;
+    static const Form table[] = {form<32, false, GM>(kStage[q][0], 0, kTile[q][0]),       form<64, false, GM>(kStage[q][1], 0, kTile[q][1]),
+                                 form<96, false, GM>(kStage[q][2], 0, kTile[q][2]),       form<128, false, GM>(kStage[q][3], 0, kTile[q][3]),
+                                 form<192, true, GM>(kStage[q][4], 0, kTile[q][4]),       form<256, true, GM>(kStage[q][5], 0, kTile[q][5]),
+                                 form<32, false, GM, true>(kStage[q][0], 0, kTile[q][0]), form<64, false, GM, true>(kStage[q][1], 0, kTile[q][1]),
+                                 form<96, false, GM, true>(kStage[q][2], 0, kTile[q][2]), form<128, false, GM, true>(kStage[q][3], 0, kTile[q][3])};
     *count = static_cast<int>(sizeof(table) / sizeof(table[0]));
     return table;
 }

@@ -752,6 +752,43 @@ def test_gemm_tcgen05_split_k(gemm_form, oracle, pkg, M, N, K, bt, splits, g):
                       abs_terms=abs_term_sum(oracle.group_sums(W, Xq, g), ws, Xs))
 
 
+@pytest.mark.parametrize("epilogue", ["NONE", "RESIDUAL", "SWIGLU"])
+@pytest.mark.parametrize("bt,splits", [(64, 1), (96, 1), (96, 2), (128, 1), (128, 4), (192, 1), (256, 1)])
+def test_gemm_tcgen05_infinite_weight_scales(gemm_form, oracle, pkg, bt, splits, epilogue):
+    """Group size 64, where the wide forms' sums carry a bias: rows with an infinite weight scale still give what float(P) * scale
+    gives, signed infinities, and NaN where a group sum is zero; every other row is the oracle's."""
+    M, inter, K, g = 101, 72, 512, 64
+    ctx = gemm_form(bt, splits)
+    N = 2 * inter if epilogue == "SWIGLU" else 136
+    X, W, ws = synth.linear_case(bt + splits, M, N, K, g)
+    Xq, Xs = oracle.quantize(X, g)
+    bad = [3, 9, 64, 130]
+    ws[bad[0], 0], ws[bad[1], 7], ws[bad[2], 3], ws[bad[3], 5] = np.inf, -np.inf, np.inf, np.inf
+    W[bad[3], 5 * g : 6 * g] = 0  # zero times infinity
+    W[:, :g] = np.where(W[:, :g] == -127, -128, W[:, :g])  # (a code the exporter does not make, and the int8 range has)
+    R = np.random.default_rng(1).standard_normal((M, N)).astype(np.float16)
+    dY = torch.empty((M, inter if epilogue == "SWIGLU" else N), dtype=torch.float16, device="cuda")
+    ctx.linear_q(dev(W), dev(ws), g, dev(Xq), dev(Xs), dY, M, N, K, epilogue=getattr(pkg, "EPI_" + epilogue),
+                 residual=dev(R) if epilogue == "RESIDUAL" else None)
+    torch.cuda.synchronize()
+    ctx.check_device_status()
+    with np.errstate(all="ignore"):
+        want = oracle.linear_q(W, ws, Xq, Xs, g)
+        if epilogue == "RESIDUAL":
+            want = oracle.residual_add(want, R)
+        elif epilogue == "SWIGLU":  # (rows in blocks of eight gate rows and their eight up rows)
+            gate, up = want.reshape(M, -1, 2, 8).transpose(2, 0, 1, 3).reshape(2, M, inter)
+            want = oracle.mul(oracle.silu(gate), up)
+    got = dY.cpu().numpy()
+    fin = np.isfinite(want)
+    assert 2 * M <= (~fin).sum() <= 4 * M and np.isnan(want).any()
+    assert np.array_equal(np.isnan(got), np.isnan(want)) and np.array_equal(got[np.isinf(want)], want[np.isinf(want)])
+    if splits == 1 and epilogue != "SWIGLU":
+        assert np.array_equal(got[fin].view(np.uint16), want[fin].view(np.uint16))
+    else:  # (another order of the sum, or the device's expf: a last bit)
+        assert np.abs(got[fin].astype(np.float32) - want[fin].astype(np.float32)).max() <= 2e-3 * np.abs(want[fin].astype(np.float32)).max()
+
+
 def test_fused_swiglu_of_every_gate(ctx, pkg):
     """The SwiGLU epilogue's quotient against the divide of the separate silu, for every fp16 gate (one token each; an infinite one
     by overflow): bit for bit."""
