@@ -11,8 +11,8 @@ namespace w8a8 {
 // (test_fused_swiglu_of_every_gate). Large denominators are cut off where the result has long been zero in fp16, so that nothing
 // becomes infinite on the way; an infinite x gives what the divide gives.
 // Why: with the divide, a 256 x 256 tile's SwiGLU took the epilogue warps of the tcgen05 GEMM 5900 clocks of 19 800 (g = 256).
-// (The decode linears keep the divide: a launch there has one tile's worth per CTA, and ten fast-AR steps took 1559 us with the
-// divide, 1565 without.)
+// (The decode linears keep the divide: a launch there has one tile's worth per CTA, and ten fast-AR steps took 1553 us with the
+// divide, 1559 without.)
 __device__ __forceinline__ float silu_of_half(float x) {
     const float d = 1.0f + fminf(expf(-x), 0x1p100f);
     float r, n;
