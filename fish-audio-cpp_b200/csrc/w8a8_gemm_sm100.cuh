@@ -110,7 +110,9 @@ struct Config {
     // K-groups per unit: what issuer and epilogue hand one another (see above). Two groups of 64: K is a multiple of 128, so every
     // tile and every run of a split is whole units. Two units in tensor memory, four where they are small.
     static constexpr int kUnit = GM == 64 && BT <= 128 ? 2 : 1;
-    static constexpr int kSlots = BT <= 64 || (kUnit == 1 && BT <= 128) ? 4 : 2;
+    // No more of them than a turn of the ring fills, so that the issuer knows each at compile time.
+    static constexpr int kTurn = GM == 0 ? 4 : kStages * BK / GM / kUnit;  // units per turn of the ring
+    static constexpr int kSlotsRoom = BT <= 64 || (kUnit == 1 && BT <= 128) ? 4 : 2, kSlots = kSlotsRoom < kTurn ? kSlotsRoom : kTurn;
     static constexpr int kAcc = kUnit * kSlots;                       // accumulator slices
     static constexpr int kBatch = GM != 0 && (BT == 64 || (BT == 32 && kUnit > 1)) ? 2 : 1;  // steps whose sums are requested together
     static constexpr int kTmemCols = kAcc * BT <= 128 ? 128 : kAcc * BT <= 256 ? 256 : 512;
@@ -449,11 +451,11 @@ gemm_i8_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
                             if (!wait(&full_bar[s], parity)) { code = 300 + s; break; }
 #pragma unroll
                             for (int h = 0; h < kPerStage; ++h) {
-                                // A turn of the ring is whole rounds of the slots, or half of one.
-                                constexpr int kTurn = S * 128 / GM / C::kUnit;  // units
-                                static_assert(S * 128 / GM % C::kUnit == 0 && (kTurn % C::kSlots == 0 || 2 * kTurn == C::kSlots), "rounds of the slots");
+                                // A turn of the ring is whole rounds of the slots. The lanes of this warp may be apart here, some past a
+                                // wait that others are still in: what the leader issues must not be a register that moves with the loop.
+                                static_assert(S * 128 / GM % C::kUnit == 0 && C::kTurn % C::kSlots == 0, "rounds of the slots");
                                 const int lg = GM == 256 ? s / 2 : s * kPerStage + h, lu = lg / C::kUnit;  // group and unit inside this turn
-                                const int as = kTurn >= C::kSlots ? lu % C::kSlots : lu + as_any;
+                                const int as = lu % C::kSlots;
                                 const bool opens = first && lg % C::kUnit == 0, closes = last && lg % C::kUnit == C::kUnit - 1;
                                 if (opens) {
                                     if (!wait(&acc_empty[as], acc_parity)) { code = 400 + as; break; }
@@ -467,8 +469,7 @@ gemm_i8_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
                                         mma_i8<PAIR>(to, da + 2 * sub, db + 2 * sub, idesc, (!C::kBiased && first && sub == h * kMmas) ? 0u : 1u);
                                     if (closes) tc_commit<PAIR>(&acc_full[as]);  // the unit's sums are complete
                                 }
-                                if (kTurn >= C::kSlots && closes && lu % C::kSlots == C::kSlots - 1) acc_parity ^= 1u;
-                                if (kTurn < C::kSlots && closes && lu == kTurn - 1 && (as_any = kTurn - as_any) == 0) acc_parity ^= 1u;
+                                if (closes && as == C::kSlots - 1) acc_parity ^= 1u;
                             }
                             if (code) break;
                             if (leader) tc_commit<PAIR>(&empty_bar[s]);  // the stage may be refilled once these MMAs retire

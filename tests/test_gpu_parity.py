@@ -789,6 +789,32 @@ def test_gemm_tcgen05_infinite_weight_scales(gemm_form, oracle, pkg, bt, splits,
         assert np.abs(got[fin].astype(np.float32) - want[fin].astype(np.float32)).max() <= 2e-3 * np.abs(want[fin].astype(np.float32)).max()
 
 
+WIDTHS = [(32, "SINGLE"), (64, "SINGLE"), (96, "SINGLE"), (128, "SINGLE"), (192, "PAIR"), (256, "PAIR")]
+
+
+@pytest.mark.parametrize("K", [384, 768])
+@pytest.mark.parametrize("bt,form,g", [(bt, form, g) for bt, form in WIDTHS for g in (64, 128, 256)])
+def test_gemm_tcgen05_many_tiles_per_cta(gemm_form, oracle, pkg, bt, form, g, K):
+    """Two to three tiles per CTA, so that the rings of stages, accumulator slots and scale chunks run on from one tile into the
+    next: whole turns of the ring and parts of one, an odd number of groups, one chunk of scales per tile. Bit for bit the
+    oracle's, on a sample of the tokens."""
+    K -= K % g
+    ctx = gemm_form(bt, 1)
+    M, N = bt * 100 + 1, 264
+    rng = np.random.default_rng(bt + g + K)
+    W, ws = synth.weights(rng, N, K), synth.weight_scales(rng, N, K // g)
+    Xq = rng.integers(-127, 128, size=(M, K), dtype=np.int8)
+    Xs = rng.uniform(1e-3, 4e-2, size=(M, K // g)).astype(np.float32)
+    buf, dY = guarded((M, N), torch.float16, 99.0)
+    ctx.linear_q(dev(W), dev(ws), g, dev(Xq), dev(Xs), dY, M, N, K, kernel=getattr(pkg, "KERNEL_GEMM_" + form))
+    torch.cuda.synchronize()
+    ctx.check_device_status()
+    assert guards_intact(buf, 99.0)
+    pick = np.unique(np.concatenate([np.arange(0, M, 41), [M - 2, M - 1, bt - 1, bt]]))
+    want = oracle.linear_q(W, ws, Xq[pick], Xs[pick], g)
+    assert np.array_equal(dY.cpu().numpy()[pick].view(np.uint16), want.view(np.uint16))
+
+
 def test_fused_swiglu_of_every_gate(ctx, pkg):
     """The SwiGLU epilogue's quotient against the divide of the separate silu, for every fp16 gate (one token each; an infinite one
     by overflow): bit for bit."""
