@@ -474,18 +474,22 @@ gemm_i8_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
                             if (code) break;
                             if (leader) tc_commit<PAIR>(&empty_bar[s]);  // the stage may be refilled once these MMAs retire
                         } else {
-                            if (!wait(&full_bar[s], parity)) { code = 300 + s; break; }
+                            // Slot and place in the group run in registers here, so the lanes of the warp stay together: they agree on every
+                            // wait, and none moves on before the leader has issued.
+                            if (!__all_sync(0xffffffffu, wait(&full_bar[s], parity))) { code = 300 + s; break; }
                             // (Rolled up, the four MMAs of a stage took the issuing warp longer than they take: one scale per channel,
                             // 4096 x 19456 x 2560 309 -> 204 us, groups of 512 342 -> 234.)
 #pragma unroll
                             for (int sub = 0; sub < 4; ++sub) {
                                 if (q_in_group == 0) {
-                                    if (!wait(&acc_empty[as_any], acc_parity)) { code = 400 + as_any; break; }
+                                    if (!__all_sync(0xffffffffu, wait(&acc_empty[as_any], acc_parity))) { code = 400 + as_any; break; }
                                     tc_fence_after();
                                 }
                                 if (leader) mma_i8<PAIR>(tmem_base + as_any * BT, da + 2 * sub, db + 2 * sub, idesc, q_in_group != 0 ? 1u : 0u);
+                                __syncwarp();
                                 if (++q_in_group == mpg) {
                                     if (leader) tc_commit<PAIR>(&acc_full[as_any]);
+                                    __syncwarp();
                                     q_in_group = 0;
                                     if (++as_any == C::kSlots) { as_any = 0; acc_parity ^= 1u; }
                                 }

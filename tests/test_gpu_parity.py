@@ -793,11 +793,12 @@ WIDTHS = [(32, "SINGLE"), (64, "SINGLE"), (96, "SINGLE"), (128, "SINGLE"), (192,
 
 
 @pytest.mark.parametrize("K", [384, 768])
-@pytest.mark.parametrize("bt,form,g", [(bt, form, g) for bt, form in WIDTHS for g in (64, 128, 256)])
+@pytest.mark.parametrize("bt,form,g", [(bt, form, g) for bt, form in WIDTHS for g in (64, 128, 256)] +
+                         [(128, form, g) for form in ("SINGLE", "PAIR") for g in (32, 384)])
 def test_gemm_tcgen05_many_tiles_per_cta(gemm_form, oracle, pkg, bt, form, g, K):
     """Two to three tiles per CTA, so that the rings of stages, accumulator slots and scale chunks run on from one tile into the
-    next: whole turns of the ring and parts of one, an odd number of groups, one chunk of scales per tile. Bit for bit the
-    oracle's, on a sample of the tokens."""
+    next: whole turns of the ring and parts of one, an odd number of groups, one chunk of scales per tile. Groups of 32 and 384 go to
+    the forms for any group size. Bit for bit the oracle's, on a sample of the tokens."""
     K -= K % g
     ctx = gemm_form(bt, 1)
     M, N = bt * 100 + 1, 264
