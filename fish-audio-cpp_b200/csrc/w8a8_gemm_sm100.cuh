@@ -114,6 +114,11 @@ struct Config {
     static constexpr int kTurn = GM == 0 ? 4 : kStages * BK / GM / kUnit;  // units per turn of the ring
     static constexpr int kSlotsRoom = BT <= 64 || (kUnit == 1 && BT <= 128) ? 4 : 2, kSlots = kSlotsRoom < kTurn ? kSlotsRoom : kTurn;
     static constexpr int kAcc = kUnit * kSlots;                       // accumulator slices
+    // The weight scales a chunk ahead (see the scales' warps). us with and without, M x N x K: 64 tokens wide, g = 64, 64 x 2560 x 9728
+    // 36.3 and 37.1; 256 wide, g = 64, 8192 x 6144 x 2560 256.9 and 258.6; any group size, 4096 x 19456 x 2560 with one group 267 and
+    // 273. Elsewhere it costs what it holds registers for: g = 64, 192 wide, 2048 x 19456 x 2560 240.9 and 235.5; 32 wide,
+    // 40 x 2560 x 9728 26.3 and 25.4; g = 256, 192 wide, 4001 x 6144 x 2560 59.1 and 58.2; g = 128, 128 wide, 2048 x 2560 x 9728 95.2 and 93.8.
+    static constexpr bool kScalesAhead = GM == 0 || (GM == 64 && (BT == 64 || BT == 256));
     static constexpr int kBatch = GM != 0 && (BT == 64 || (BT == 32 && kUnit > 1)) ? 2 : 1;  // steps whose sums are requested together
     static constexpr int kTmemCols = kAcc * BT <= 128 ? 128 : kAcc * BT <= 256 ? 256 : 512;
     static_assert(kStages * kStageBytes <= kRoom, "stages do not fit");
@@ -510,21 +515,23 @@ gemm_i8_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
             int slot = 0;
             uint32_t parity = 1;
             bool ok = true;
-            // The weight scales are read a chunk ahead: a read takes as long as the narrow tiles take for a chunk.
+            // kScalesAhead: the weight scales are read a chunk ahead, as a read takes as long as a narrow tile takes for a chunk.
             __half w[2][kScGroups];
-            auto load_w = [&](int tile, int j0) {
-                if (j0 >= g_end) { tile += walkers; j0 = g_first; }
-                if (tile >= p.tiles_total) return;
-                const int n0 = tile_n0(tile);
-                const __half* ws0 = a.w_scale + static_cast<size_t>(min(n0 + t64, a.N - 1)) * G;
-                const __half* ws1 = a.w_scale + static_cast<size_t>(min(n0 + 64 + t64, a.N - 1)) * G;
+            auto w_row = [&](int n) { return a.w_scale + static_cast<size_t>(min(n + t64, a.N - 1)) * G; };
+            auto load_w = [&](const __half* ws0, const __half* ws1, int j0) {
 #pragma unroll
                 for (int q = 0; q < kScGroups; ++q) {
                     w[0][q] = ws0[min(j0 + q, G - 1)];
                     w[1][q] = ws1[min(j0 + q, G - 1)];
                 }
             };
-            load_w(walker, g_first);
+            auto load_w_ahead = [&](int tile, int j0) {
+                if (j0 >= g_end) { tile += walkers; j0 = g_first; }
+                if (tile >= p.tiles_total) return;
+                const int n0 = tile_n0(tile);
+                load_w(w_row(n0), w_row(n0 + 64), j0);
+            };
+            if constexpr (C::kScalesAhead) load_w_ahead(walker, g_first);
             for (int tile = walker; tile < p.tiles_total && ok; tile += walkers) {
                 const int m0 = tile_m0(tile), n0 = tile_n0(tile);
                 if (a.epilogue == W8A8_EPI_RESIDUAL && srank == 0) {  // the tile's residual rows to L2, long before its end needs them
@@ -534,8 +541,12 @@ gemm_i8_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
                             asm volatile("prefetch.global.L2 [%0];" ::"l"(a.residual + static_cast<size_t>(t) * a.N + col));
                     }
                 }
+                // (Once a tile: formed anew for every chunk they cost the tiles of 192 tokens 1 %, a call of one wave up to 2 %.)
+                const __half* ws0 = w_row(n0);
+                const __half* ws1 = w_row(n0 + 64);
                 for (int j0 = g_first; j0 < g_end; j0 += kScGroups) {
                     const int nj = min(kScGroups, g_end - j0);
+                    if constexpr (!C::kScalesAhead) load_w(ws0, ws1, j0);  // on their way while the slot is waited for
                     if (!wait(&sc_empty[slot], parity)) {
                         atomicExch(p.status, 600 + slot);
                         ok = false;
@@ -557,7 +568,7 @@ gemm_i8_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
                         asm volatile("st.shared.f32 [%0], %1;" ::"r"(dst + (kScGroups * BT + q * BR + 64 + ws_slot(t64)) * 4), "f"(w1 * kScale) : "memory");
                     }
                     ptx::mbar_arrive(&sc_full[slot]);
-                    load_w(tile, j0 + kScGroups);
+                    if constexpr (C::kScalesAhead) load_w_ahead(tile, j0 + kScGroups);
                     if (++slot == kScRing) { slot = 0; parity ^= 1u; }
                 }
             }
