@@ -119,6 +119,11 @@ struct Config {
     // 273. Elsewhere it costs what it holds registers for: g = 64, 192 wide, 2048 x 19456 x 2560 240.9 and 235.5; 32 wide,
     // 40 x 2560 x 9728 26.3 and 25.4; g = 256, 192 wide, 4001 x 6144 x 2560 59.1 and 58.2; g = 128, 128 wide, 2048 x 2560 x 9728 95.2 and 93.8.
     static constexpr bool kScalesAhead = GM == 0 || (GM == 64 && (BT == 64 || BT == 256));
+    // How the epilogue reads scales from shared memory: 16 bytes at a time (xs_slot, ws_slot), but in pieces of 8 and 4 by the pairs
+    // of 192 tokens at groups of 128 and 256 (4001 x 6144 x 2560, g = 256 58.2 -> 57.3 us, 4001 x 19456 x 2560 205.3 -> 200.2; g = 128
+    // 94.1 -> 91.8, 297 -> 289). The others lose with those: g = 128, 96 wide, 613 x 6144 x 2560 24.5 -> 25.4; g = 64, 128 wide,
+    // 2048 x 2560 x 9728 142.1 -> 144.5.
+    static constexpr bool kWideScales = GM == 64 || GM == 0 || BT != 192;
     static constexpr int kBatch = GM != 0 && (BT == 64 || (BT == 32 && kUnit > 1)) ? 2 : 1;  // steps whose sums are requested together
     static constexpr int kTmemCols = kAcc * BT <= 128 ? 128 : kAcc * BT <= 256 ? 256 : 512;
     static_assert(kStages * kStageBytes <= kRoom, "stages do not fit");
@@ -243,13 +248,22 @@ __device__ __forceinline__ void mul2(uint64_t& v, uint64_t f) { asm("mul.rn.f32x
 // sixteen tokens (two neighbouring ones of either eight), or for its four weight rows, is one 16-byte piece. Such a read, its
 // address shared by the lanes of a row or column, takes shared memory as long as one of 8 bytes (two clocks, twice that while the
 // MMAs read their operands), of which there would be two, or four of 4 bytes.
-__device__ __forceinline__ int xs_slot(int t) { return (t & ~15) | ((t & 6) << 1) | ((t >> 2) & 2) | (t & 1); }
-__device__ __forceinline__ int ws_slot(int n) { return (n & ~31) | ((n & 7) << 2) | ((n >> 3) & 3); }
+// WIDE false (Config::kWideScales): in order, and read in two and in four pieces.
+template <bool WIDE>
+__device__ __forceinline__ int xs_slot(int t) { return WIDE ? (t & ~15) | ((t & 6) << 1) | ((t >> 2) & 2) | (t & 1) : t; }
+template <bool WIDE>
+__device__ __forceinline__ int ws_slot(int n) { return WIDE ? (n & ~31) | ((n & 7) << 2) | ((n >> 3) & 3) : n; }
+template <bool WIDE>
 __device__ __forceinline__ void lds_2x64(uint32_t addr, uint64_t& a, uint64_t& b) {
-    asm volatile("ld.shared.v2.u64 {%0, %1}, [%2];" : "=l"(a), "=l"(b) : "r"(addr));
+    if constexpr (WIDE) asm volatile("ld.shared.v2.u64 {%0, %1}, [%2];" : "=l"(a), "=l"(b) : "r"(addr));
+    else asm volatile("ld.shared.u64 %0, [%2];\n\tld.shared.u64 %1, [%2 + 32];" : "=&l"(a), "=l"(b) : "r"(addr));
 }
+template <bool WIDE>
 __device__ __forceinline__ void lds_4x32(uint32_t addr, float (&v)[4]) {
-    asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v[0]), "=f"(v[1]), "=f"(v[2]), "=f"(v[3]) : "r"(addr));
+    if constexpr (WIDE) asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v[0]), "=f"(v[1]), "=f"(v[2]), "=f"(v[3]) : "r"(addr));
+    else
+        asm volatile("ld.shared.f32 %0, [%4];\n\tld.shared.f32 %1, [%4 + 32];\n\tld.shared.f32 %2, [%4 + 64];\n\tld.shared.f32 %3, [%4 + 96];"
+                     : "=&f"(v[0]), "=&f"(v[1]), "=&f"(v[2]), "=f"(v[3]) : "r"(addr));
 }
 // Four 8 x 8 fp16 matrices held as accumulator fragments, stored TRANSPOSED: lane l gives the address of the 16-byte row
 // l % 8 of matrix l / 8.
@@ -557,15 +571,15 @@ gemm_i8_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
                         const float* src = a.Xs + static_cast<size_t>(min(m0 + t, a.M - 1)) * G + j0;
 #pragma unroll
                         for (int q = 0; q < kScGroups; ++q)
-                            if (q < nj) asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(dst + (q * BT + xs_slot(t)) * 4), "l"(src + q) : "memory");
+                            if (q < nj) asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(dst + (q * BT + xs_slot<C::kWideScales>(t)) * 4), "l"(src + q) : "memory");
                     }
                     asm volatile("cp.async.mbarrier.arrive.noinc.shared.b64 [%0];" ::"r"(ptx::smem_u32(&sc_full[slot])) : "memory");
 #pragma unroll
                     for (int q = 0; q < kScGroups; ++q) {
                         const float w0 = __half2float(w[0][q]), w1 = __half2float(w[1][q]);
                         if (C::kBiased && (isinf(w0) || isinf(w1))) infinite_s = 1;
-                        asm volatile("st.shared.f32 [%0], %1;" ::"r"(dst + (kScGroups * BT + q * BR + ws_slot(t64)) * 4), "f"(w0 * kScale) : "memory");
-                        asm volatile("st.shared.f32 [%0], %1;" ::"r"(dst + (kScGroups * BT + q * BR + 64 + ws_slot(t64)) * 4), "f"(w1 * kScale) : "memory");
+                        asm volatile("st.shared.f32 [%0], %1;" ::"r"(dst + (kScGroups * BT + q * BR + ws_slot<C::kWideScales>(t64)) * 4), "f"(w0 * kScale) : "memory");
+                        asm volatile("st.shared.f32 [%0], %1;" ::"r"(dst + (kScGroups * BT + q * BR + 64 + ws_slot<C::kWideScales>(t64)) * 4), "f"(w1 * kScale) : "memory");
                     }
                     ptx::mbar_arrive(&sc_full[slot]);
                     if constexpr (C::kScalesAhead) load_w_ahead(tile, j0 + kScGroups);
@@ -612,14 +626,14 @@ gemm_i8_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
                     ok = false;
                     break;
                 }
-                uint32_t xs_addr = sc_ring + slot * C::kScSlot + (part * HC + 4 * (lane & 3)) * 4;
-                uint32_t ws_addr = sc_ring + slot * C::kScSlot + (kScGroups * BT + quad * 32 + 4 * (lane >> 2)) * 4;
+                uint32_t xs_addr = sc_ring + slot * C::kScSlot + (part * HC + (C::kWideScales ? 4 : 2) * (lane & 3)) * 4;
+                uint32_t ws_addr = sc_ring + slot * C::kScSlot + (kScGroups * BT + quad * 32 + (C::kWideScales ? 4 : 1) * (lane >> 2)) * 4;
                 const int j1 = min(j0 + kScGroups, g_end);
 #pragma unroll 1
                 for (int j = j0; j < j1; j += U) {
                     const uint32_t taddr = taddr0 + as * (U * BT);
                     float w4[BATCH][4];
-                    if constexpr (U == 1) lds_4x32(ws_addr, w4[0]);
+                    if constexpr (U == 1) lds_4x32<C::kWideScales>(ws_addr, w4[0]);
                     if (!wait(&acc_full[as], acc_parity)) {
                         if (lane == 0) atomicExch(p.status, 500 + as);
                         ok = false;
@@ -645,11 +659,11 @@ gemm_i8_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
                         for (int b = 0; b < BATCH; ++b)
 #pragma unroll
                             for (int o = 0; o < CH / 8; o += 2)
-                                lds_2x64(xs_addr + ((q0 + b) / NCH * BT + (q0 + b) % NCH * CH + 8 * o) * 4, x2[b][o], x2[b][o + 1]);
+                                lds_2x64<C::kWideScales>(xs_addr + ((q0 + b) / NCH * BT + (q0 + b) % NCH * CH + 8 * o) * 4, x2[b][o], x2[b][o + 1]);
                         if constexpr (U > 1) {
 #pragma unroll
                             for (int b = 0; b < BATCH; ++b)
-                                if ((q0 + b) % NCH == 0) lds_4x32(ws_addr + (q0 + b) / NCH * BR * 4, w4[b]);
+                                if ((q0 + b) % NCH == 0) lds_4x32<C::kWideScales>(ws_addr + (q0 + b) / NCH * BR * 4, w4[b]);
                         }
                         tmem_ld_wait();
                         if (q0 + BATCH == STEPS) {
