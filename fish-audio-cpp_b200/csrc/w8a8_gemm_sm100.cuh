@@ -633,7 +633,23 @@ gemm_i8_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
                 for (int j = j0; j < j1; j += U) {
                     const uint32_t taddr = taddr0 + as * (U * BT);
                     float w4[BATCH][4];
+                    uint64_t w2[2][2], b2[2][2];
+                    auto take_scales = [&](const float (&w)[4]) {
+#pragma unroll
+                        for (int i = 0; i < 4; ++i) {
+                            w2[i / 2][i % 2] = pack2(w[i], w[i]);
+                            if constexpr (C::kBiased) {
+                                const float bias = w[i] * -__int_as_float(kBias);
+                                b2[i / 2][i % 2] = pack2(bias, bias);
+                            }
+                        }
+                    };
+                    // One group per unit: made ready before the wait; behind it they cost every group (g = 128, M x N x K 2048 x 2560 x
+                    // 9728, 128 wide 92.8 -> 88.6 us, 4001 x 2560 x 9728, 192 wide 152.5 -> 149.6). Not so in the forms for any group size
+                    // (2048 x 6144 x 2560, g = 32 208 -> 204 us behind it).
+                    constexpr bool kBefore = U == 1 && GM != 0;
                     if constexpr (U == 1) lds_4x32<C::kWideScales>(ws_addr, w4[0]);
+                    if constexpr (kBefore) take_scales(w4[0]);
                     if (!wait(&acc_full[as], acc_parity)) {
                         if (lane == 0) atomicExch(p.status, 500 + as);
                         ok = false;
@@ -651,7 +667,6 @@ gemm_i8_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
                             }
                     };
                     load_sums(0);
-                    uint64_t w2[2][2], b2[2][2];
 #pragma unroll
                     for (int q0 = 0; q0 < STEPS; q0 += BATCH) {
                         uint64_t x2[BATCH][CH / 8];
@@ -678,17 +693,7 @@ gemm_i8_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
 #pragma unroll
                         for (int b = 0; b < BATCH; ++b) {
                             const int ci = (q0 + b) % NCH;
-                            if (ci == 0) {
-#pragma unroll
-                                for (int i = 0; i < 4; ++i) {
-                                    const float w = w4[b][i];
-                                    w2[i / 2][i % 2] = pack2(w, w);
-                                    if constexpr (C::kBiased) {
-                                        const float bias = w * -__int_as_float(kBias);
-                                        b2[i / 2][i % 2] = pack2(bias, bias);
-                                    }
-                                }
-                            }
+                            if (!kBefore && ci == 0) take_scales(w4[b]);
 #pragma unroll
                             for (int o = 0; o < CH / 8; ++o)
 #pragma unroll
