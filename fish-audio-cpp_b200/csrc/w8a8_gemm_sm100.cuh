@@ -67,7 +67,7 @@ namespace w8a8 {
 namespace gemm {
 
 constexpr int BR = 128, BK = 128;            // weight rows per CTA; bytes of K per stage
-constexpr int kScGroups = 4, kScRing = 3;    // K-groups per chunk of scales, chunks in the ring
+constexpr int kScGroups = 4;                 // K-groups per chunk of scales
 constexpr uint32_t kSpin = 1u << 21;
 
 struct GemmParams {
@@ -90,6 +90,11 @@ struct Config {
     static constexpr int kStageBytes = (BR + kRowsB) * BK;
     static constexpr int kPanelBytes = BT * 128;                      // BT tokens x 64 fp16 columns, 128-byte swizzle
     static constexpr int kOutBytes = 2 * kPanelBytes;
+    // Tiles of 64 tokens at groups of 128 and 256: a fourth chunk of scales in the ring, the sums of one step at a time, scales read in
+    // pieces of 8 and 4 bytes. With three chunks, two steps and 16 bytes: M x N x K 263 x 2560 x 4096, g = 256 9.0 -> 9.3 us, 150 x 2560 x
+    // 9728 16.0 -> 16.5; g = 128, 331 x 2560 x 4096 13.3 -> 13.7, 64 x 2560 x 9728 in two 17.0 -> 17.8.
+    static constexpr bool kNarrowChain = BT == 64 && GM >= 128;
+    static constexpr int kScRing = kNarrowChain ? 4 : 3;              // chunks of scales in the ring
     static constexpr int kScSlot = kScGroups * (BT + BR) * 4;         // activation scales [4][BT], weight scales [4][128]
     static constexpr int kScBytes = kScRing * kScSlot;
     static constexpr int kConst = kBiased ? kConstBytes : 0;
@@ -123,8 +128,8 @@ struct Config {
     // of 192 tokens at groups of 128 and 256 (4001 x 6144 x 2560, g = 256 58.2 -> 57.3 us, 4001 x 19456 x 2560 205.3 -> 200.2; g = 128
     // 94.1 -> 91.8, 297 -> 289). The others lose with those: g = 128, 96 wide, 613 x 6144 x 2560 24.5 -> 25.4; g = 64, 128 wide,
     // 2048 x 2560 x 9728 142.1 -> 144.5.
-    static constexpr bool kWideScales = GM == 64 || GM == 0 || BT != 192;
-    static constexpr int kBatch = GM != 0 && (BT == 64 || (BT == 32 && kUnit > 1)) ? 2 : 1;  // steps whose sums are requested together
+    static constexpr bool kWideScales = GM == 64 || GM == 0 || (BT != 192 && !kNarrowChain);
+    static constexpr int kBatch = GM == 64 && BT <= 64 ? 2 : 1;  // steps whose sums are requested together
     static constexpr int kTmemCols = kAcc * BT <= 128 ? 128 : kAcc * BT <= 256 ? 256 : 512;
     static_assert(kStages * kStageBytes <= kRoom, "stages do not fit");
     static_assert(BT % 32 == 0 && BT <= 256, "token width");
@@ -339,7 +344,7 @@ gemm_i8_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
     using C = Config<BT, PAIR, GM>;
     constexpr int S = C::kStages, kEpiWarps = C::kEpiWarps, kEpiThreads = kEpiWarps * 32;
     extern __shared__ unsigned char smem_raw[];
-    __shared__ __align__(8) uint64_t full_bar[S], empty_bar[S], acc_full[C::kSlots], acc_empty[C::kSlots], sc_full[kScRing], sc_empty[kScRing];
+    __shared__ __align__(8) uint64_t full_bar[S], empty_bar[S], acc_full[C::kSlots], acc_empty[C::kSlots], sc_full[C::kScRing], sc_empty[C::kScRing];
     __shared__ uint32_t tmem_base_s;
     __shared__ int failed_s;
     // kBiased: a weight scale that this CTA has met is infinite; the same, as all epilogue threads are to see it at a tile's end
@@ -369,7 +374,7 @@ gemm_i8_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
             ptx::mbar_init(&acc_full[s], 1);
             ptx::mbar_init(&acc_empty[s], PAIR ? 2 * kEpiWarps : kEpiWarps);
         }
-        for (int s = 0; s < kScRing; ++s) { ptx::mbar_init(&sc_full[s], 128); ptx::mbar_init(&sc_empty[s], kEpiWarps); }
+        for (int s = 0; s < C::kScRing; ++s) { ptx::mbar_init(&sc_full[s], 128); ptx::mbar_init(&sc_empty[s], kEpiWarps); }
         failed_s = 0;
         infinite_s = 0;
         ptx::fence_barrier_init();
@@ -583,7 +588,7 @@ gemm_i8_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
                     }
                     ptx::mbar_arrive(&sc_full[slot]);
                     if constexpr (C::kScalesAhead) load_w_ahead(tile, j0 + kScGroups);
-                    if (++slot == kScRing) { slot = 0; parity ^= 1u; }
+                    if (++slot == C::kScRing) { slot = 0; parity ^= 1u; }
                 }
             }
             asm volatile("cp.async.wait_all;" ::: "memory");
@@ -728,7 +733,7 @@ gemm_i8_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
                 // the chunk's scales are used up
                 __syncwarp();
                 if (lane == 0) ptx::mbar_arrive(&sc_empty[slot]);
-                if (++slot == kScRing) { slot = 0; sc_parity ^= 1u; }
+                if (++slot == C::kScRing) { slot = 0; sc_parity ^= 1u; }
             }
             int infinite = 0;
             if constexpr (C::kBiased) {
