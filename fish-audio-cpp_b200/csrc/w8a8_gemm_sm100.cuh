@@ -293,32 +293,38 @@ __device__ __forceinline__ uint64_t smem_desc(uint32_t saddr) {
 
 // With the bias (promote2), an infinite weight scale gives infinity less infinity. The output columns of such weight rows, in the
 // tile that lies in shared memory, are formed anew, from the operands: signed infinities and NaN as float(P) * ws has them. Slow, and
-// only run once a CTA has met an infinite scale.
+// only run for a tile that has met an infinite scale (one such row: 4001 x 6144 x 2560 997 us with a search of every row by every
+// thread in every tile that followed, 190 now, 161 without such a row). First which rows those are, a thread per row, into rows[4]:
+__device__ __forceinline__ void find_infinite_rows(const LinearArgs& a, uint32_t* rows, int n0, int et) {
+    bool any = false;
+    if (et < BR && n0 + et < a.N)
+        for (int j = 0; j < a.G; ++j) any |= isinf(__half2float(a.w_scale[static_cast<size_t>(n0 + et) * a.G + j]));
+    const uint32_t word = __ballot_sync(0xffffffffu, any);
+    if (et < BR && (et & 31) == 0) rows[et >> 5] = word;
+}
 template <class C>
-__device__ __forceinline__ void infinite_rows(const LinearArgs& a, uint32_t out_stage, int m0, int n0, int tokens, bool swiglu, int et) {
-    auto infinite = [&](int n) {
-        bool any = false;
-        for (int j = 0; j < a.G; ++j) any |= isinf(__half2float(a.w_scale[static_cast<size_t>(n) * a.G + j]));
-        return any;
-    };
+__device__ __forceinline__ void infinite_rows(const LinearArgs& a, const uint32_t* rows, uint32_t out_stage, int m0, int n0, int tokens, bool swiglu, int et) {
     auto sum = [&](int n, int m) {
-        const int* w = reinterpret_cast<const int*>(a.W + static_cast<size_t>(n) * a.K);
-        const int* x = reinterpret_cast<const int*>(a.Xq + static_cast<size_t>(m) * a.K);
+        const int4* w = reinterpret_cast<const int4*>(a.W + static_cast<size_t>(n) * a.K);
+        const int4* x = reinterpret_cast<const int4*>(a.Xq + static_cast<size_t>(m) * a.K);
         float acc = 0.0f;
 #pragma unroll 1
         for (int j = 0; j < a.G; ++j) {
             int p = 0;
 #pragma unroll 1
-            for (int k = 0; k < a.g / 4; ++k) p = __dp4a(w[j * (a.g / 4) + k], x[j * (a.g / 4) + k], p);
+            for (int k = j * (a.g / 16); k < (j + 1) * (a.g / 16); ++k) {
+                const int4 wv = w[k], xv = x[k];
+                p = __dp4a(wv.x, xv.x, __dp4a(wv.y, xv.y, __dp4a(wv.z, xv.z, __dp4a(wv.w, xv.w, p))));
+            }
             acc = fmaf(static_cast<float>(p) * __half2float(a.w_scale[static_cast<size_t>(n) * a.G + j]), a.Xs[static_cast<size_t>(m) * a.G + j], acc);
         }
         return acc;
     };
 #pragma unroll 1
-    for (int row = 0; row < BR && n0 + row < a.N; ++row) {
+    for (int row = 0; row < BR; ++row) {
         if (swiglu && (row & 8)) continue;  // (taken with its gate row)
+        if (!(rows[row >> 5] >> (row & 31) & (swiglu ? 0x101u : 1u))) continue;
         const int n = n0 + row;
-        if (!infinite(n) && !(swiglu && infinite(n + 8))) continue;
         const int col = swiglu ? (row >> 4) * 8 + (row & 7) : row;
 #pragma unroll 1
         for (int t = et; t < tokens; t += C::kEpiWarps * 32) {
@@ -347,8 +353,11 @@ gemm_i8_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
     __shared__ __align__(8) uint64_t full_bar[S], empty_bar[S], acc_full[C::kSlots], acc_empty[C::kSlots], sc_full[C::kScRing], sc_empty[C::kScRing];
     __shared__ uint32_t tmem_base_s;
     __shared__ int failed_s;
-    // kBiased: a weight scale that this CTA has met is infinite; the same, as all epilogue threads are to see it at a tile's end
-    __shared__ int infinite_s, infinite_tile_s;
+    // kBiased: infinite_s[i % kMarks] is i + 1 if a weight scale of this CTA's i-th tile is infinite (the scales' warps are up to kScRing
+    // chunks, so as many tiles, ahead of the epilogue); the same, as all epilogue threads are to see it at a tile's end
+    constexpr int kMarks = C::kScRing + 1;
+    __shared__ int infinite_s[kMarks], infinite_tile_s;
+    __shared__ uint32_t infinite_rows_s[BR / 32];
 
     const LinearArgs& a = p.a;
     // (through a shuffle, so that the compiler knows it is the same in all lanes and keeps what follows from it in uniform registers)
@@ -376,7 +385,7 @@ gemm_i8_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
         }
         for (int s = 0; s < C::kScRing; ++s) { ptx::mbar_init(&sc_full[s], 128); ptx::mbar_init(&sc_empty[s], kEpiWarps); }
         failed_s = 0;
-        infinite_s = 0;
+        for (int i = 0; i < kMarks; ++i) infinite_s[i] = 0;
         ptx::fence_barrier_init();
         ptx::fence_proxy_async();
     }
@@ -551,7 +560,8 @@ gemm_i8_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
                 load_w(w_row(n0), w_row(n0 + 64), j0);
             };
             if constexpr (C::kScalesAhead) load_w_ahead(walker, g_first);
-            for (int tile = walker; tile < p.tiles_total && ok; tile += walkers) {
+            int ith = 0;
+            for (int tile = walker; tile < p.tiles_total && ok; tile += walkers, ++ith) {
                 const int m0 = tile_m0(tile), n0 = tile_n0(tile);
                 if (a.epilogue == W8A8_EPI_RESIDUAL && srank == 0) {  // the tile's residual rows to L2, long before its end needs them
                     for (int i = t64; i < 2 * BT; i += 64) {
@@ -582,7 +592,7 @@ gemm_i8_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
 #pragma unroll
                     for (int q = 0; q < kScGroups; ++q) {
                         const float w0 = __half2float(w[0][q]), w1 = __half2float(w[1][q]);
-                        if (C::kBiased && (isinf(w0) || isinf(w1))) infinite_s = 1;
+                        if (C::kBiased && (isinf(w0) || isinf(w1))) infinite_s[ith % kMarks] = ith + 1;
                         asm volatile("st.shared.f32 [%0], %1;" ::"r"(dst + (kScGroups * BT + q * BR + ws_slot<C::kWideScales>(t64)) * 4), "f"(w0 * kScale) : "memory");
                         asm volatile("st.shared.f32 [%0], %1;" ::"r"(dst + (kScGroups * BT + q * BR + 64 + ws_slot<C::kWideScales>(t64)) * 4), "f"(w1 * kScale) : "memory");
                     }
@@ -737,7 +747,8 @@ gemm_i8_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
             }
             int infinite = 0;
             if constexpr (C::kBiased) {
-                infinite = infinite_s;
+                const int ith = (tile - walker) / walkers;
+                infinite = infinite_s[ith % kMarks] == ith + 1;
                 const uint64_t up = pack2(0x1p38f, 0x1p38f);
 #pragma unroll
                 for (int i = 0; i < 4 * OCT; ++i) mul2(acc[i / (2 * OCT)][i / OCT % 2][i % OCT], up);
@@ -761,8 +772,8 @@ gemm_i8_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
                     const uint32_t theirs = map_to_rank(mine, c);
                     if constexpr (C::kBiased) {
                         int v;
-                        asm volatile("ld.shared::cluster.s32 %0, [%1];" : "=r"(v) : "r"(map_to_rank(ptx::smem_u32(&infinite_s), c)) : "memory");
-                        infinite |= v;
+                        asm volatile("ld.shared::cluster.s32 %0, [%1];" : "=r"(v) : "r"(map_to_rank(ptx::smem_u32(&infinite_s[0]), c)) : "memory");
+                        infinite |= v;  // (a CTA's only tile: 0 or 1)
                     }
                     uint64_t v[4 * OCT];
 #pragma unroll
@@ -803,8 +814,9 @@ gemm_i8_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
             }
             if constexpr (C::kBiased) {
                 if (infinite_tile_s) {
+                    find_infinite_rows(a, infinite_rows_s, n0, et);
                     epi_barrier<kEpiThreads>();
-                    infinite_rows<C>(a, out_stage, m0, n0, min(BT, a.M - m0), swiglu, et);
+                    infinite_rows<C>(a, infinite_rows_s, out_stage, m0, n0, min(BT, a.M - m0), swiglu, et);
                 }
             }
             const int ycols = swiglu ? a.N / 2 : a.N, y0 = swiglu ? n0 / 2 : n0;   // first output column of this CTA

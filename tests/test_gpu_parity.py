@@ -816,6 +816,35 @@ def test_gemm_tcgen05_many_tiles_per_cta(gemm_form, oracle, pkg, bt, form, g, K)
     assert np.array_equal(dY.cpu().numpy()[pick].view(np.uint16), want.view(np.uint16))
 
 
+@pytest.mark.parametrize("bt,form", [(96, "SINGLE"), (128, "SINGLE"), (192, "PAIR"), (256, "PAIR")])
+def test_gemm_tcgen05_infinite_weight_scales_over_many_tiles(gemm_form, oracle, pkg, bt, form):
+    """Tiles with an infinite weight scale and tiles without one in turn on one CTA, one chunk of scales per tile, so that the
+    scales are staged up to three tiles ahead of the tile that is being written."""
+    N, K, g = 520, 256, 64
+    M = bt * 61 + 5  # 62 token tiles: with 148 CTAs (74 pairs) a CTA takes tiles of two or three row tiles
+    ctx = gemm_form(bt, 1)
+    rng = np.random.default_rng(bt)
+    W, ws = synth.weights(rng, N, K), synth.weight_scales(rng, N, K // g)
+    bad = [3, 300, 511, 519]
+    ws[bad[0], 0], ws[bad[1], 3], ws[bad[2], 1], ws[bad[3], 2] = np.inf, -np.inf, np.inf, np.inf
+    W[bad[2], g : 2 * g] = 0  # zero times infinity
+    Xq = rng.integers(-127, 128, size=(M, K), dtype=np.int8)
+    Xs = rng.uniform(1e-3, 4e-2, size=(M, K // g)).astype(np.float32)
+    buf, dY = guarded((M, N), torch.float16, 99.0)
+    ctx.linear_q(dev(W), dev(ws), g, dev(Xq), dev(Xs), dY, M, N, K, kernel=getattr(pkg, "KERNEL_GEMM_" + form))
+    torch.cuda.synchronize()
+    ctx.check_device_status()
+    assert guards_intact(buf, 99.0)
+    pick = np.unique(np.concatenate([np.arange(0, M, 19), [M - 1]]))
+    with np.errstate(all="ignore"):
+        want = oracle.linear_q(W, ws, Xq[pick], Xs[pick], g)
+    got = dY.cpu().numpy()[pick]
+    assert np.isnan(want[:, bad[2]]).all() and np.isinf(want[:, bad[0]]).any()
+    nan = np.isnan(want)
+    assert np.array_equal(np.isnan(got), nan)
+    assert np.array_equal(got[~nan].view(np.uint16), want[~nan].view(np.uint16))
+
+
 def test_fused_swiglu_of_every_gate(ctx, pkg):
     """The SwiGLU epilogue's quotient against the divide of the separate silu, for every fp16 gate (one token each; an infinite one
     by overflow): bit for bit."""
