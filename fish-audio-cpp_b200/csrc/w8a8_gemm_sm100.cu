@@ -4,9 +4,10 @@
 namespace w8a8 {
 namespace gemm {
 
-// Group sizes without a case of their own, and calls that want the group sums.
+// Group sizes without a case of their own, and calls that want the group sums. (Costs fitted at groups of 32, 320, 512 and K, 40 to 4001
+// tokens, within 15 %. Nowhere there was the pair the faster one: 5-15 % slower.)
 const Form* forms_any(int* count) {
-    static const Form table[] = {form<128, false, 0>(135, 330, 1300), form<128, true, 0>(165, 360, 1300)};
+    static const Form table[] = {form<128, false, 0>(332, 332, 1250), form<128, true, 0>(345, 355, 1840)};
     *count = static_cast<int>(sizeof(table) / sizeof(table[0]));
     return table;
 }
@@ -48,8 +49,10 @@ struct Choice {
 // The tile form that ends first: whole waves of tiles over the SMs (or pairs), each tile at its measured cost. A width
 // that leaves the last wave nearly empty loses to one that fills it; narrow tiles win where there are few tokens.
 // A tile's K is split over two or four CTAs where all of them fit the chip at once (a cluster of four leaves some SMs of a
-// GPC over: 128 of 148 taken as usable); meeting and adding up measured 3-4 us for two and about 6 for four. A
-// split adds the groups in another order than the other kernels do, so it has to save 10 % at least.
+// GPC over: 128 of 148 taken as usable); meeting and adding up came out of the fit as 2.5 us for two and 5 for four. A split adds the
+// groups in another order than the other kernels do, so it has to save 10 % at least, and two are taken as 3 us: K = 2560 never splits.
+// Rows that are no multiple of eight leave element by element: 55 ns per token of a thread's part (measured at 4097 rows), which
+// the 256-token pairs at g = 64, with half the threads, lose by (4001 x 4097 x 2560 148 us, 192 wide 134).
 // table_g: the group size whose forms are looked at (0: those of any group size). pair: -1 either, 0 one CTA per tile, 1 a pair.
 // only_bt, only_splits: 0, or the token width and the split (1: none) to take; no form where they do not fit the shape.
 template <class Usable>
@@ -63,14 +66,15 @@ Choice choose(int M, int N, int K, int table_g, int g, int sms, int pair, int on
         if (pair >= 0 && (f.pair != (pair != 0) || f.split)) continue;
         if (only_bt && f.bt != only_bt) continue;
         const int rows = f.pair ? 2 * BR : BR, walkers = f.pair ? sms / 2 : sms, kb_total = K / BK;
+        const double tile_ns = f.tile_ns + (N % 8 == 0 ? 0.0 : 55.0 * f.bt / f.parts);
         const long tiles = static_cast<long>((M + f.bt - 1) / f.bt) * ((N + rows - 1) / rows);
         for (int splits = f.split ? 2 : 1; splits <= (f.split ? 4 : 1); splits *= 2) {
             if (only_splits && splits != only_splits) continue;
             if (f.split && (tiles * splits > (splits == 2 ? sms / 2 * 2 : sms * 7 / 8 - 1) || (splits - 1) * split_kb(K, g, splits) >= kb_total))
                 continue;
             const double kb = f.split ? split_kb(K, g, splits) : kb_total;
-            double ns = ((tiles * splits + walkers - 1) / walkers) * (kb * f.stage_ns + kb * BK / g * f.group_ns + f.tile_ns);
-            if (f.split) ns = (ns + (splits == 2 ? 3500 : 6000)) / 0.9;
+            double ns = ((tiles * splits + walkers - 1) / walkers) * (kb * f.stage_ns + kb * BK / g * f.group_ns + tile_ns);
+            if (f.split) ns = (ns + (splits == 2 ? 3000 : 5000)) / 0.9;
             if ((!best.form || ns < best_ns) && usable(f)) { best = {&f, splits}; best_ns = ns; }
         }
     }

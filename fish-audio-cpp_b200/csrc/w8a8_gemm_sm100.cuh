@@ -905,10 +905,12 @@ struct FormState {
     std::atomic<int> registers{0};  // per thread, as compiled (0: not asked for yet)
 };
 // A tile form: its kernel and what the launch needs to know about it. stage_ns, group_ns, tile_ns: what a tile takes per 128 bytes of
-// K, per K-group and for itself (the start of its chain, conversion, store), fitted to the four projections at 100 to 4001 tokens, for
-// each group size; with 2.5 us for the launch they give the measured times within 15 %. At 8192 tokens, where the codes of w2 do not
-// stay in L2, pairs of 256 tokens lose more than pairs of 192 (8192 x 2560 x 9728, g = 256: 245 us and 205), so 192 is set 3-4 %
-// lower than fitted, and 256 at groups of 128 and 256 2-4 % higher.
+// K, per K-group and for itself (the start of its chain, conversion, store). Fitted to 4100 times, no cost below zero: seven shapes (the
+// four projections, 9728 x 2560, 4096 x 9728, 1000 x 1024) x 29 token counts from 33 to 8192 x every form that takes them, for each
+// group size. With 2.7-3.2 us for the launch nine in ten of the times within a third of the best form's lie within 15 % of the model's.
+// What it does not hold: a chip that is not full (at groups of 256 a stage of a lone tile of 96 tokens takes 210 ns, not 290), and what
+// several sweeps over a long prompt's codes miss L2 for. Judged by its choice, the rule lost 0.4, 0.5 and 0.4 % against the best form on
+// average (groups of 64, 128, 256), and 0.2, 1.2 and 1.2 % over eight other shapes x eleven token counts, most of it splits of K not taken.
 struct Form {
     int bt;
     bool pair, split;
@@ -916,6 +918,7 @@ struct Form {
     int threads, smem;
     int launch_regs;  // per thread, if the form moves some between its warpgroups; else 0
     float stage_ns, group_ns, tile_ns;
+    int parts;  // Config::kParts
     FormState* state;
 };
 template <int BT, bool PAIR, int GM, bool SPLIT>
@@ -924,13 +927,13 @@ template <int BT, bool PAIR, int GM, bool SPLIT = false>
 Form form(float stage_ns, float group_ns, float tile_ns) {
     using C = Config<BT, PAIR, GM>;
     return Form{BT, PAIR, SPLIT, gemm_i8_kernel<BT, PAIR, GM, SPLIT>, C::kThreads, C::kSmem, C::kMoveRegs ? C::kLaunchRegs : 0,
-                stage_ns, group_ns, tile_ns, &form_state<BT, PAIR, GM, SPLIT>};
+                stage_ns, group_ns, tile_ns, C::kParts, &form_state<BT, PAIR, GM, SPLIT>};
 }
 template <int GM>
 const Form* all_forms(int* count) {
     // per stage at groups of 64, 128 and 256, and per tile, for token widths 32, 64, 96, 128, 192, 256
-    constexpr float kStage[3][6] = {{332, 467, 562, 635, 940, 1176}, {210, 307, 354, 399, 596, 745}, {153, 192, 225, 235, 340, 412}};
-    constexpr float kTile[3][6] = {{311, 573, 641, 1057, 1669, 2164}, {535, 699, 799, 1411, 1952, 2547}, {166, 615, 553, 1270, 2060, 2689}};
+    constexpr float kStage[3][6] = {{314, 470, 514, 601, 912, 1157}, {210, 300, 351, 390, 609, 744}, {152, 177, 289, 308, 363, 451}};
+    constexpr float kTile[3][6] = {{0, 0, 600, 740, 1530, 1420}, {400, 440, 610, 930, 1230, 1660}, {300, 590, 20, 300, 1650, 1880}};
     constexpr int q = GM == 64 ? 0 : GM == 128 ? 1 : 2;
     static const Form table[] = {form<32, false, GM>(kStage[q][0], 0, kTile[q][0]),       form<64, false, GM>(kStage[q][1], 0, kTile[q][1]),
                                  form<96, false, GM>(kStage[q][2], 0, kTile[q][2]),       form<128, false, GM>(kStage[q][3], 0, kTile[q][3]),

@@ -95,6 +95,23 @@ def test_gemm_form_follows_what_is_asked_for(pkg):
         assert pkg.debug_gemm_form(8192, 19456, 2560, g, moved_registers=False) is not None
 
 
+@pytest.mark.parametrize("M,N,K,g,want", [
+    (2048, 2560, 9728, 256, (192, 2, 1)),  # 62 us; tiles of 96 tokens 74
+    (150, 2560, 9728, 256, (64, 1, 2)),    # 12.9 us; tiles of 32, not split, 14.3
+    (4001, 4097, 2560, 64, (192, 2, 1)),   # rows that leave element by element: 134 us; 256 wide 148
+])
+def test_gemm_form_that_was_measured_fastest(pkg, M, N, K, g, want):
+    assert pkg.debug_gemm_form(M, N, K, g) == want
+
+
+def test_gemm_never_splits_the_hidden_width(pkg):
+    """K = 2560: the sums of wqkv and w1|w3 are added in the order of the other kernels, whatever the number of tokens and rows."""
+    for g in (64, 128, 256):
+        for M in (33, 64, 97, 160, 300, 613, 2048, 8192):
+            for N in (16, 96, 256, 1000, 2560, 4097, 6144, 19456):
+                assert pkg.debug_gemm_form(M, N, 2560, g)[2] == 1
+
+
 def test_product_never_touches_the_oracle():
     """Nothing under the package may import, link or read oracle/ (checker only)."""
     pat = re.compile(r"(^|\s)(import|from)\s+oracle\b|oracle/|w8a8o_|libw8a8_oracle|fishref")
