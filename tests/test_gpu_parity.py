@@ -628,9 +628,9 @@ GEMM_FORMS = ["KERNEL_GEMM_SINGLE", "KERNEL_GEMM_PAIR"]  # one CTA per tile; a C
 @pytest.mark.parametrize("M,N,K,g", GEMM_SHAPES + [(640, 520, 768, 256), (385, 2560, 512, 128)])
 def test_gemm_tcgen05_small_shapes(ctx, oracle, pkg, M, N, K, g, form):
     """The tcgen05 + TMA kernel in both forms: ragged token and row tails (an odd number of 128-token tiles leaves the
-    second CTA of the last pair without rows; N = 520 and 136 end inside a 64-column store panel; N = 72 and 264 are
-    not multiples of 8 ... 16 bytes and take the direct-store epilogue), every group size a multiple of 32 including
-    groups that straddle a 128-byte stage. Groups are added in ascending order exactly like the oracle, so the fp16
+    second CTA of the last pair without rows; N = 520, 136, 72 and 264 end inside a 64-column store panel), every group size a
+    multiple of 32 including groups that straddle a 128-byte stage. With the group sums asked for, so these are the forms for any
+    group size. Groups are added in ascending order exactly like the oracle, so the fp16
     output must agree bit for bit."""
     (X, W, ws, Xq, Xs), Y, P = run_linear(ctx, oracle, M, N, K, g, seed=M + N + K, kernel=getattr(pkg, form))
     ctx.check_device_status()
@@ -816,6 +816,61 @@ def test_gemm_tcgen05_many_tiles_per_cta(gemm_form, oracle, pkg, bt, form, g, K)
     assert np.array_equal(dY.cpu().numpy()[pick].view(np.uint16), want.view(np.uint16))
 
 
+@pytest.mark.parametrize("wval,qval", [(-128, -128), (-128, 127), (127, 127), (127, -128)])
+@pytest.mark.parametrize("g", [64, 128, 256])
+@pytest.mark.parametrize("bt,splits", [(32, 1), (64, 1), (96, 1), (128, 1), (192, 1), (256, 1), (96, 2), (128, 2)])
+def test_gemm_tcgen05_largest_sums_without_dump(gemm_form, oracle, pkg, bt, splits, g, wval, qval):
+    """The forms that a call without group sums takes, at the largest sums of a group, 128 * 128 * g of either sign (at g = 64 the
+    wide forms add a bias that has to keep such a sum positive and inside 23 bits), -128 among the activation codes too. Bit for
+    bit the oracle's; a split adds two fp32 sums of one fp16 result, so its last bit may differ."""
+    M, N, K = 130, 264, 512
+    ctx = gemm_form(bt, splits)
+    rng = np.random.default_rng(7)
+    W = np.full((N, K), wval, dtype=np.int8)
+    W[1::3, ::5] = 127 if wval == -128 else -128  # (rows 0, 3, ...: every product at its largest)
+    ws = synth.weight_scales(rng, N, K // g)
+    Xq = np.full((M, K), qval, dtype=np.int8)
+    Xq[1::2, 7::11] = 127 if qval == -128 else -128
+    Xs = rng.uniform(1e-5, 1e-3, size=(M, K // g)).astype(np.float32)
+    P = oracle.group_sums(W, Xq, g)
+    assert np.abs(P).max() == abs(wval * qval) * g
+    buf, dY = guarded((M, N), torch.float16, 99.0)
+    ctx.linear_q(dev(W), dev(ws), g, dev(Xq), dev(Xs), dY, M, N, K)
+    torch.cuda.synchronize()
+    ctx.check_device_status()
+    assert guards_intact(buf, 99.0)
+    got, want = dY.cpu().numpy(), oracle.linear_q(W, ws, Xq, Xs, g)
+    assert np.isfinite(want).all()
+    if splits == 1:
+        assert np.array_equal(got.view(np.uint16), want.view(np.uint16))
+    else:
+        assert_close_fp16(oracle, got, want, "split K, largest sums", abs_terms=abs_term_sum(P, ws, Xs))
+
+
+@pytest.mark.parametrize("epilogue", ["NONE", "RESIDUAL"])
+@pytest.mark.parametrize("g", [64, 256])
+@pytest.mark.parametrize("bt,form", WIDTHS)
+@pytest.mark.parametrize("N", [133, 4097])
+def test_gemm_tcgen05_rows_that_are_no_multiple_of_eight(gemm_form, oracle, pkg, N, bt, form, g, epilogue):
+    """Output rows of any pitch leave element by element, by as many threads per token as the form has parts. A vocabulary of 4097
+    sampled rows is such a weight. Bit for bit the oracle's."""
+    M, K = (bt + 37, 512) if N == 133 else (33, 256)
+    ctx = gemm_form(bt, 1)
+    X, W, ws = synth.linear_case(N + bt, M, N, K, g)
+    Xq, Xs = oracle.quantize(X, g)
+    R = np.random.default_rng(2).standard_normal((M, N)).astype(np.float16)
+    buf, dY = guarded((M, N), torch.float16, 99.0)
+    ctx.linear_q(dev(W), dev(ws), g, dev(Xq), dev(Xs), dY, M, N, K, kernel=getattr(pkg, "KERNEL_GEMM_" + form),
+                 epilogue=getattr(pkg, "EPI_" + epilogue), residual=dev(R) if epilogue == "RESIDUAL" else None)
+    torch.cuda.synchronize()
+    ctx.check_device_status()
+    assert guards_intact(buf, 99.0)
+    want = oracle.linear_q(W, ws, Xq, Xs, g)
+    if epilogue == "RESIDUAL":
+        want = oracle.residual_add(want, R)
+    assert np.array_equal(dY.cpu().numpy().view(np.uint16), want.view(np.uint16))
+
+
 @pytest.mark.parametrize("bt,form", [(96, "SINGLE"), (128, "SINGLE"), (192, "PAIR"), (256, "PAIR")])
 def test_gemm_tcgen05_infinite_weight_scales_over_many_tiles(gemm_form, oracle, pkg, bt, form):
     """Tiles with an infinite weight scale and tiles without one in turn on one CTA, one chunk of scales per tile, so that the
@@ -870,6 +925,29 @@ def test_fused_swiglu_of_every_gate(ctx, pkg):
     # -0: the sum of a zero group is +0, so the gate is
     want[0x8000] = 0
     assert np.array_equal(got[~nan].view(np.uint16), np.repeat(want[~nan].view(np.uint16)[:, None], 8, axis=1))
+
+
+def test_fused_swiglu_of_gates_that_round_to_zero(ctx, oracle, pkg):
+    """Sums of either sign too small for fp16: gates of +0 and -0, and ups of both, against the separate silu and mul."""
+    small = np.array([1e-9, -1e-9, 1.0, -1.0, 6e-8, -6e-8], np.float32)
+    gate, up = (v.reshape(-1) for v in np.meshgrid(small, small, indexing="ij"))
+    M, K, g = gate.size, 128, 64
+    Xq = np.zeros((M, K), np.int8)
+    Xq[:, 0] = Xq[:, g] = 1
+    Xs = np.stack([gate, up], axis=1).astype(np.float32)
+    W = np.zeros((16, K), np.int8)
+    W[:8, 0] = W[8:, g] = 1
+    dY = torch.empty((M, 8), dtype=torch.float16, device="cuda")
+    for kernel in ("KERNEL_GEMM_SINGLE", "KERNEL_GEMM_PAIR"):
+        ctx.linear_q(dev(W), dev(np.ones((16, 2), np.float16)), g, dev(Xq), dev(Xs), dY, M, 16, K, epilogue=pkg.EPI_SWIGLU,
+                     kernel=getattr(pkg, kernel))
+        silu = dev(gate.astype(np.float16))
+        ctx.shim_silu_forward(silu, M)
+        ctx.shim_mul_forward(silu, dev(up.astype(np.float16)), M)
+        torch.cuda.synchronize()
+        want = silu.cpu().numpy()
+        assert (gate.astype(np.float16).view(np.uint16) == 0x8000).any() and (want.view(np.uint16) == 0x8000).any()
+        assert np.array_equal(dY.cpu().numpy().view(np.uint16), np.repeat(want.view(np.uint16)[:, None], 8, axis=1))
 
 
 @pytest.mark.parametrize("packed", [True, False])
@@ -1212,8 +1290,8 @@ def test_linear_against_reference_kernel(ctx, oracle, M, N, K, g):
 @pytest.mark.parametrize("g", [256, 64])
 @pytest.mark.parametrize("wval,qval", [(-128, 127), (127, 127), (-128, -127), (127, -127)])
 def test_gemm_tcgen05_extreme_codes(ctx, oracle, pkg, g, wval, qval, form):
-    """Every product at its largest magnitude: a group of 256 sums to 128 * 127 * 256 = 4 161 536, just under the
-    2^22 up to which the kernel's integer-add int32 -> fp32 conversion is exact. Sums and fp16 bits must match."""
+    """Every product at its largest magnitude, in the forms for any group size (the group sums are asked for): a group of 256 sums
+    to 128 * 127 * 256 = 4 161 536, which fp32 holds exactly. Sums and fp16 bits must match."""
     M, N, K = 130, 264, 512
     G = oracle.num_groups(K, g)
     rng = np.random.default_rng(7)
