@@ -12,7 +12,7 @@
 //   warp 0       producer: TMA loads of 128 weight rows and BT token rows, 128 bytes of K each (both matrices are
 //                row-major with K contiguous, i.e. already the K-major operand; TMA applies the 128-byte swizzle)
 //   warp 1       MMA issuer: four tcgen05.mma (K = 32) per stage; every K-group accumulates into its own BT-column slice
-//                of tensor memory (two to eight slices), starting with "overwrite" or, at g = 64, with a bias (below)
+//                of tensor memory (two to four, in units eight), starting with "overwrite" or, at g = 64, with a bias (below)
 //   warps 2, 3   stage the scales of four K-groups at a time in a ring of their own
 //   warps 4 ...  epilogue, eight or sixteen warps, each 32 weight rows x a part of the tokens. For every K-group
 //                acc = fma(float(P) * ws, xs, acc), groups ascending -- the arithmetic and order of
@@ -31,29 +31,32 @@
 // latency, and descriptors computed in divergent code are moved to uniform registers one by one): the tensor pipe ran at
 // 0.6 of its rate. Hence: the whole warp runs the loop and one elected lane issues; the loop is unrolled over the stages
 // so that stage, accumulator slice and descriptor offsets are immediates; group sizes 64 / 128 / 256 are template cases.
-// The promote is the other side, and the bound in most forms: stamps of the clock in the epilogue warps showed 1280 (g = 64) and 1390
-// (g = 256) clocks per K-group of a 128 x 256 tile against 256 and 1024 of MMAs. What it is made of, measured alone (16 warps):
-//   * per two sums two conversions, a packed multiply and a packed FMA; by themselves 4.3 clocks per warp and scheduler, with the
-//     tensor-memory and shared-memory reads around them 6.9-7.2, as if conversions and those reads shared a way into the registers.
-//     Without conversions, two packed FMAs, 5.1-5.6. Hence the BIAS at g = 64 (promote2): each group's accumulator starts from a
-//     constant, made by one more MMA of a constant operand with itself, that makes every sum positive; as bits it then is an fp32
-//     number, and the multiply that had to follow the conversion takes the bias out again, exactly. At g = 128 it would take two more MMAs per
-//     four, and at g = 256 the tensor pipe is the next bound.
-//   * about 360 clocks per K-group whatever the tile's width: two waits, the arrive, the loop. Hence UNITS of two K-groups of 64
-//     on the tiles of up to 128 tokens. (Four, or units at g = 128 and 256, would need a slot that is not known at compile time, as a
-//     tile may end inside a unit. With it in a register the lanes of the issuing warp have to meet at every wait and before it moves
-//     on; without that two builds ended with an illegal memory access, and with it g = 128 and 256 lost 10-40 %.)
+// The promote is the other side, and the bound in most forms: stamps of the clock in an epilogue warp (which cost some 10 % themselves;
+// profiles/gemm_i8_kernel_epilogue_clock_stamps.md) show 1216, 1424 and 1451 clocks per K-group of a 128 x 256 tile at groups of 64, 128
+// and 256, of which 224-358 are waits for the MMAs, against 384 (with the bias), 512 and 1024 of MMAs. In trial programs of sixteen such
+// warps alone, clocks per warp and scheduler for two sums (the programs are not kept):
+//   * two conversions, a packed multiply and a packed FMA 4.3 by themselves, 6.9-7.2 with the tensor-memory and shared-memory reads around
+//     them, as if conversions and those reads shared a way into the registers; two packed FMAs without conversions 5.1-5.6 with the
+//     reads. Hence the BIAS at g = 64 (promote2): each group's accumulator starts from a constant, made by one more MMA of a
+//     constant operand with itself, that makes every sum positive; as bits it then is an fp32 number, and the multiply that had to
+//     follow the conversion takes the bias out again, exactly. At g = 128 it would take two more MMAs per four, and at g = 256 the tensor pipe
+//     is the next bound.
+//   * the integer conversions (add into the mantissa of 1.5 * 2^23) 15-25 % slower than the conversion instruction.
 //   * the sums are read in the layout of an mma.sync accumulator (16x256b): a lane then holds 4 weight rows x 2 tokens of every 16 x 8
-//     block and reads the activation scales of eight sums with 8 bytes. (32x32b, a thread per row, is three times as fast out of tensor
-//     memory but needs a 16-byte read per four sums: 1.3-2 times as long in all, most while the MMAs read shared memory.)
-// The integer conversions (add into the mantissa of 1.5 * 2^23) measured 15-25 % slower than the conversion instruction.
-// The SwiGLU of a tile's end took 5900 of the 19 800 clocks of a tile at g = 256 (w8a8_swiglu.cuh).
+//     block and reads the activation scales of sixteen sums, four tokens, with 16 bytes. (32x32b, a thread per row, is three times as
+//     fast out of tensor memory but needs a 16-byte read per four sums: 1.3-2 times as long in all, most while the MMAs read shared
+//     memory.)
+// Some 270 clocks of a K-group do not depend on the tile's width (370, 501, 561 and 725 clocks for 32, 64, 96 and 128 tokens at g = 256):
+// two waits, the arrive, the loop. Hence UNITS of two K-groups of 64 on the tiles of up to 128 tokens (252 and 410 clocks per group for
+// 32 and 64 tokens, 530 for 128). Four, or units at g = 128 and 256, would need a slot that is not known at compile time, as a tile may
+// end inside a unit: with the slot in a register of the issuing warp, two trial builds ended with an illegal memory access. Its cause was not
+// shown. With the lanes of that warp agreeing on every wait and meeting before the slot moved on, the builds ran, and lost 10-40 %.
 //
-// Measured back to back, us, before the bias, the units, the 16-byte scale reads, the SwiGLU and the costs fitted anew, and with
-// them (M x N x K):
-//   8192 x 19456 x 2560, g = 64   962 -> 788 (848 -> 1036 TOPS); g = 256 365 -> 343 (2236 -> 2380 TOPS)
-//   2048 x  2560 x 9728, g = 64   155 -> 124;  613 x 2560 x 9728  53.5 -> 43.3;  150 x 19456 x 2560  53 -> 36.7
-//   at g = 128 and 256 rows without SwiGLU within 4 % either way (pairs of 192 tokens 2-5 % slower: 4001 x 6144 x 2560 54.9 -> 57.2)
+// Measured back to back in turn, us, without the bias, the units, the 16-byte scale reads and the cheaper SwiGLU, and with them
+// (M x N x K; the long ones under the power cap):
+//   8192 x 19456 x 2560, g = 64   967 -> 787 (844 -> 1037 TOPS); g = 128 617 -> 568; g = 256 447 -> 393 (1827 -> 2076 TOPS)
+//   2048 x  2560 x 9728, g = 64   154 -> 120;  613 x 2560 x 9728  52.8 -> 42.1;  150 x 19456 x 2560  52.6 -> 36.0
+//   4001 x  6144 x 2560, g = 128  95.2 -> 95.2; g = 256 66.9 -> 66.9 (no SwiGLU, pairs of 192 tokens)
 //
 // Every mbarrier wait is bounded; a wait that runs out records an error word, and the CTA still frees its tensor memory
 // before it returns.
@@ -340,9 +343,9 @@ __device__ __forceinline__ void infinite_rows(const LinearArgs& a, const uint32_
 // for as well.
 //
 // SPLIT: few tiles and a long K. The CTAs of a cluster take one tile, each a run of its K-groups; at the end the first CTA reads
-// the others' fp32 sums from their shared memory and adds them in ascending-K order. Narrow tiles are a serial chain of some
-// 430-650 clocks per K-group, whatever the number of CTAs (tokens x rows x K, g = 64: 150 x 2560 x 9728 34.8 -> 27.0 us, 64 x
-// 2560 x 9728 34.8 -> 17.9, 150 x 2560 x 4096 19.3 -> 16.4).
+// the others' fp32 sums from their shared memory and adds them in ascending-K order. Narrow tiles are a serial chain of K-groups,
+// whatever the number of CTAs (tokens x rows x K, the best form without a split and with one: g = 64, 33 x 2560 x 9728 25.0 and 16.4 us,
+// 150 x 2560 x 9728 25.2 and 23.5, 33 x 2560 x 4096 14.3 and 11.2; g = 256, 64 x 2560 x 9728 14.5 and 11.2).
 template <int BT, bool PAIR, int GM, bool SPLIT>
 __global__ void __launch_bounds__(Config<BT, PAIR, GM>::kThreads, 1)
 gemm_i8_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_x,

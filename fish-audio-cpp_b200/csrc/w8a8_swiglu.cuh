@@ -7,10 +7,12 @@
 namespace w8a8 {
 
 // x / (1 + exp(-x)) for an x that is an fp16 number. The quotient is an approximate reciprocal's, corrected once by its residual
-// (Markstein, IBM J. Res. Dev. 34, 1990); rounded to fp16 it is the divide's for every one of the 65536 arguments
-// (test_fused_swiglu_of_every_gate). Large denominators are cut off where the result has long been zero in fp16, so that nothing
-// becomes infinite on the way; an infinite x gives what the divide gives.
-// Why: with the divide, a 256 x 256 tile's SwiGLU took the epilogue warps of the tcgen05 GEMM 5900 clocks of 19 800 (g = 256).
+// (Markstein, IBM J. Res. Dev. 34, 1990); rounded to fp16 it is the divide's for every one of the 65536 arguments (tested:
+// test_fused_swiglu_of_every_gate, and for -0 test_fused_swiglu_of_gates_that_round_to_zero). Large denominators are cut off where the
+// result has long been zero in fp16, so that nothing becomes infinite on the way; an infinite x gives what the divide gives.
+// Why: with the divide it was the longest part of a tile's end. A 256 x 256 tile at g = 256 now ends in 3130 clocks, 1090 without the
+// SwiGLU, after ten K-groups of 1451 (stamps of the clock). w1|w3 at g = 256, with all that changed since the divide, 150 tokens 30.0 ->
+// 19.4 us and 8192 tokens 447 -> 393; rows without SwiGLU 7.2 -> 7.3 (6144, 150 tokens) and 126 -> 125 (8192).
 // (The decode linears keep the divide: a launch there has one tile's worth per CTA, and ten fast-AR steps took 1553 us with the
 // divide, 1559 without.)
 __device__ __forceinline__ float silu_of_half(float x) {
