@@ -13,7 +13,7 @@
 //                row-major with K contiguous, i.e. already the K-major operand; TMA applies the 128-byte swizzle)
 //   warp 1       MMA issuer: four tcgen05.mma (K = 32) per stage; every K-group accumulates into its own BT-column slice
 //                of tensor memory (two to four, in units eight), starting with "overwrite" or, at g = 64, with a bias (below)
-//   warps 2, 3   stage the scales of four K-groups at a time in a ring of their own
+//   warps 2, 3   stage the scales of eight K-groups at a time in a ring of their own
 //   warps 4 ...  epilogue, eight or sixteen warps, each 32 weight rows x a part of the tokens. For every K-group
 //                acc = fma(float(P) * ws, xs, acc), groups ascending -- the arithmetic and order of
 //                accumulate_group_kernel (int8_gemm.cu:213-234) -- in fp32 registers, then the fp16 store
@@ -70,7 +70,6 @@ namespace w8a8 {
 namespace gemm {
 
 constexpr int BR = 128, BK = 128;            // weight rows per CTA; bytes of K per stage
-constexpr int kScGroups = 4;                 // K-groups per chunk of scales
 constexpr uint32_t kSpin = 1u << 21;
 
 struct GemmParams {
@@ -93,12 +92,13 @@ struct Config {
     static constexpr int kStageBytes = (BR + kRowsB) * BK;
     static constexpr int kPanelBytes = BT * 128;                      // BT tokens x 64 fp16 columns, 128-byte swizzle
     static constexpr int kOutBytes = 2 * kPanelBytes;
-    // Tiles of 64 tokens at groups of 128 and 256: a fourth chunk of scales in the ring, the sums of one step at a time, scales read in
-    // pieces of 8 and 4 bytes. With three chunks, two steps and 16 bytes: M x N x K 263 x 2560 x 4096, g = 256 9.0 -> 9.3 us, 150 x 2560 x
-    // 9728 16.0 -> 16.5; g = 128, 331 x 2560 x 4096 13.3 -> 13.7, 64 x 2560 x 9728 in two 17.0 -> 17.8.
-    static constexpr bool kNarrowChain = BT == 64 && GM >= 128;
-    static constexpr int kScRing = kNarrowChain ? 4 : 3;              // chunks of scales in the ring
-    static constexpr int kScSlot = kScGroups * (BT + BR) * 4;         // activation scales [4][BT], weight scales [4][128]
+    // K-groups per chunk of scales, chunks in the ring. An epilogue warp spends some 240 clocks where one chunk ends and the next begins: its
+    // arrive, a wait, new addresses, and between them nothing to mix the promote with. With twelve groups in three chunks of four, us
+    // back to back: 4096 x 19456 x 2560 g = 64, 256 wide 395 and now 387, 192 wide 429 and 421, g = 128, 256 wide 281 and 275; 2048 x 6144 x
+    // 2560 g = 64, 96 wide 86.8 and 82.9; 150 x 19456 x 2560 g = 64, 32 wide 40.2 and 37.8. (Sixteen in two chunks of eight have room in every form; chunks
+    // of sixteen in the narrower ones lose stages of operands for them: 613 x 2560 x 9728 g = 256, 64 wide 29.2 and 42.7.)
+    static constexpr int kScGroups = 8, kScRing = 2;
+    static constexpr int kScSlot = kScGroups * (BT + BR) * 4;         // activation scales [8][BT], weight scales [8][128]
     static constexpr int kScBytes = kScRing * kScSlot;
     static constexpr int kConst = kBiased ? kConstBytes : 0;
     static constexpr int kRoom = 226 * 1024 - 1024 - kOutBytes - kScBytes - kConst;
@@ -122,16 +122,10 @@ struct Config {
     static constexpr int kTurn = GM == 0 ? 4 : kStages * BK / GM / kUnit;  // units per turn of the ring
     static constexpr int kSlotsRoom = BT <= 64 || (kUnit == 1 && BT <= 128) ? 4 : 2, kSlots = kSlotsRoom < kTurn ? kSlotsRoom : kTurn;
     static constexpr int kAcc = kUnit * kSlots;                       // accumulator slices
-    // The weight scales a chunk ahead (see the scales' warps). us with and without, M x N x K: 64 tokens wide, g = 64, 64 x 2560 x 9728
-    // 36.3 and 37.1; 256 wide, g = 64, 8192 x 6144 x 2560 256.9 and 258.6; any group size, 4096 x 19456 x 2560 with one group 267 and
-    // 273. Elsewhere it costs what it holds registers for: g = 64, 192 wide, 2048 x 19456 x 2560 240.9 and 235.5; 32 wide,
-    // 40 x 2560 x 9728 26.3 and 25.4; g = 256, 192 wide, 4001 x 6144 x 2560 59.1 and 58.2; g = 128, 128 wide, 2048 x 2560 x 9728 95.2 and 93.8.
-    static constexpr bool kScalesAhead = GM == 0 || (GM == 64 && (BT == 64 || BT == 256));
-    // How the epilogue reads scales from shared memory: 16 bytes at a time (xs_slot, ws_slot), but in pieces of 8 and 4 by the pairs
-    // of 192 tokens at groups of 128 and 256 (4001 x 6144 x 2560, g = 256 58.2 -> 57.3 us, 4001 x 19456 x 2560 205.3 -> 200.2; g = 128
-    // 94.1 -> 91.8, 297 -> 289). The others lose with those: g = 128, 96 wide, 613 x 6144 x 2560 24.5 -> 25.4; g = 64, 128 wide,
-    // 2048 x 2560 x 9728 142.1 -> 144.5.
-    static constexpr bool kWideScales = GM == 64 || GM == 0 || (BT != 192 && !kNarrowChain);
+    // The weight scales a chunk ahead (see the scales' warps): 256 wide, g = 64, 4096 x 19456 x 2560 380 us and 390 without; any group
+    // size, 4096 x 19456 x 2560 with one group 267 and 273. Elsewhere it costs what it holds registers for: g = 64, 64 wide, 150 x 6144 x
+    // 2560 12.2 and 11.4.
+    static constexpr bool kScalesAhead = GM == 0 || (GM == 64 && BT == 256);
     static constexpr int kBatch = GM == 64 && BT <= 64 ? 2 : 1;  // steps whose sums are requested together
     static constexpr int kTmemCols = kAcc * BT <= 128 ? 128 : kAcc * BT <= 256 ? 256 : 512;
     static_assert(kStages * kStageBytes <= kRoom, "stages do not fit");
@@ -256,22 +250,13 @@ __device__ __forceinline__ void mul2(uint64_t& v, uint64_t f) { asm("mul.rn.f32x
 // sixteen tokens (two neighbouring ones of either eight), or for its four weight rows, is one 16-byte piece. Such a read, its
 // address shared by the lanes of a row or column, takes shared memory as long as one of 8 bytes (two clocks, twice that while the
 // MMAs read their operands), of which there would be two, or four of 4 bytes.
-// WIDE false (Config::kWideScales): in order, and read in two and in four pieces.
-template <bool WIDE>
-__device__ __forceinline__ int xs_slot(int t) { return WIDE ? (t & ~15) | ((t & 6) << 1) | ((t >> 2) & 2) | (t & 1) : t; }
-template <bool WIDE>
-__device__ __forceinline__ int ws_slot(int n) { return WIDE ? (n & ~31) | ((n & 7) << 2) | ((n >> 3) & 3) : n; }
-template <bool WIDE>
+__device__ __forceinline__ int xs_slot(int t) { return (t & ~15) | ((t & 6) << 1) | ((t >> 2) & 2) | (t & 1); }
+__device__ __forceinline__ int ws_slot(int n) { return (n & ~31) | ((n & 7) << 2) | ((n >> 3) & 3); }
 __device__ __forceinline__ void lds_2x64(uint32_t addr, uint64_t& a, uint64_t& b) {
-    if constexpr (WIDE) asm volatile("ld.shared.v2.u64 {%0, %1}, [%2];" : "=l"(a), "=l"(b) : "r"(addr));
-    else asm volatile("ld.shared.u64 %0, [%2];\n\tld.shared.u64 %1, [%2 + 32];" : "=&l"(a), "=l"(b) : "r"(addr));
+    asm volatile("ld.shared.v2.u64 {%0, %1}, [%2];" : "=l"(a), "=l"(b) : "r"(addr));
 }
-template <bool WIDE>
 __device__ __forceinline__ void lds_4x32(uint32_t addr, float (&v)[4]) {
-    if constexpr (WIDE) asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v[0]), "=f"(v[1]), "=f"(v[2]), "=f"(v[3]) : "r"(addr));
-    else
-        asm volatile("ld.shared.f32 %0, [%4];\n\tld.shared.f32 %1, [%4 + 32];\n\tld.shared.f32 %2, [%4 + 64];\n\tld.shared.f32 %3, [%4 + 96];"
-                     : "=&f"(v[0]), "=&f"(v[1]), "=&f"(v[2]), "=f"(v[3]) : "r"(addr));
+    asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v[0]), "=f"(v[1]), "=f"(v[2]), "=f"(v[3]) : "r"(addr));
 }
 // Four 8 x 8 fp16 matrices held as accumulator fragments, stored TRANSPOSED: lane l gives the address of the 16-byte row
 // l % 8 of matrix l / 8.
@@ -351,7 +336,7 @@ __global__ void __launch_bounds__(Config<BT, PAIR, GM>::kThreads, 1)
 gemm_i8_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_x,
                const __grid_constant__ CUtensorMap map_y, const GemmParams p) {
     using C = Config<BT, PAIR, GM>;
-    constexpr int S = C::kStages, kEpiWarps = C::kEpiWarps, kEpiThreads = kEpiWarps * 32;
+    constexpr int S = C::kStages, kEpiWarps = C::kEpiWarps, kEpiThreads = kEpiWarps * 32, kScGroups = C::kScGroups;
     extern __shared__ unsigned char smem_raw[];
     __shared__ __align__(8) uint64_t full_bar[S], empty_bar[S], acc_full[C::kSlots], acc_empty[C::kSlots], sc_full[C::kScRing], sc_empty[C::kScRing];
     __shared__ uint32_t tmem_base_s;
@@ -540,7 +525,7 @@ gemm_i8_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
                 if (code && leader) atomicExch(p.status, code);
             }
         } else {
-            // ---------------- scales, four groups per chunk: activation scales [4][BT], weight scales [4][128], fp32 ----------------
+            // ---------------- scales, a chunk at a time: activation scales [8][BT], weight scales [8][128], fp32 ----------------
             const int t64 = threadIdx.x - 64;
             constexpr float kScale = C::kBiased ? 0x1p111f : 1.0f;  // (see promote2)
             int slot = 0;
@@ -589,15 +574,15 @@ gemm_i8_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
                         const float* src = a.Xs + static_cast<size_t>(min(m0 + t, a.M - 1)) * G + j0;
 #pragma unroll
                         for (int q = 0; q < kScGroups; ++q)
-                            if (q < nj) asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(dst + (q * BT + xs_slot<C::kWideScales>(t)) * 4), "l"(src + q) : "memory");
+                            if (q < nj) asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(dst + (q * BT + xs_slot(t)) * 4), "l"(src + q) : "memory");
                     }
                     asm volatile("cp.async.mbarrier.arrive.noinc.shared.b64 [%0];" ::"r"(ptx::smem_u32(&sc_full[slot])) : "memory");
 #pragma unroll
                     for (int q = 0; q < kScGroups; ++q) {
                         const float w0 = __half2float(w[0][q]), w1 = __half2float(w[1][q]);
                         if (C::kBiased && (isinf(w0) || isinf(w1))) infinite_s[ith % kMarks] = ith + 1;
-                        asm volatile("st.shared.f32 [%0], %1;" ::"r"(dst + (kScGroups * BT + q * BR + ws_slot<C::kWideScales>(t64)) * 4), "f"(w0 * kScale) : "memory");
-                        asm volatile("st.shared.f32 [%0], %1;" ::"r"(dst + (kScGroups * BT + q * BR + 64 + ws_slot<C::kWideScales>(t64)) * 4), "f"(w1 * kScale) : "memory");
+                        asm volatile("st.shared.f32 [%0], %1;" ::"r"(dst + (kScGroups * BT + q * BR + ws_slot(t64)) * 4), "f"(w0 * kScale) : "memory");
+                        asm volatile("st.shared.f32 [%0], %1;" ::"r"(dst + (kScGroups * BT + q * BR + 64 + ws_slot(t64)) * 4), "f"(w1 * kScale) : "memory");
                     }
                     ptx::mbar_arrive(&sc_full[slot]);
                     if constexpr (C::kScalesAhead) load_w_ahead(tile, j0 + kScGroups);
@@ -644,8 +629,8 @@ gemm_i8_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
                     ok = false;
                     break;
                 }
-                uint32_t xs_addr = sc_ring + slot * C::kScSlot + (part * HC + (C::kWideScales ? 4 : 2) * (lane & 3)) * 4;
-                uint32_t ws_addr = sc_ring + slot * C::kScSlot + (kScGroups * BT + quad * 32 + (C::kWideScales ? 4 : 1) * (lane >> 2)) * 4;
+                uint32_t xs_addr = sc_ring + slot * C::kScSlot + (part * HC + 4 * (lane & 3)) * 4;
+                uint32_t ws_addr = sc_ring + slot * C::kScSlot + (kScGroups * BT + quad * 32 + 4 * (lane >> 2)) * 4;
                 const int j1 = min(j0 + kScGroups, g_end);
 #pragma unroll 1
                 for (int j = j0; j < j1; j += U) {
@@ -666,7 +651,7 @@ gemm_i8_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
                     // 9728, 128 wide 92.8 -> 88.6 us, 4001 x 2560 x 9728, 192 wide 152.5 -> 149.6). Not so in the forms for any group size
                     // (2048 x 6144 x 2560, g = 32 208 -> 204 us behind it).
                     constexpr bool kBefore = U == 1 && GM != 0;
-                    if constexpr (U == 1) lds_4x32<C::kWideScales>(ws_addr, w4[0]);
+                    if constexpr (U == 1) lds_4x32(ws_addr, w4[0]);
                     if constexpr (kBefore) take_scales(w4[0]);
                     if (!wait(&acc_full[as], acc_parity)) {
                         if (lane == 0) atomicExch(p.status, 500 + as);
@@ -692,11 +677,11 @@ gemm_i8_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
                         for (int b = 0; b < BATCH; ++b)
 #pragma unroll
                             for (int o = 0; o < CH / 8; o += 2)
-                                lds_2x64<C::kWideScales>(xs_addr + ((q0 + b) / NCH * BT + (q0 + b) % NCH * CH + 8 * o) * 4, x2[b][o], x2[b][o + 1]);
+                                lds_2x64(xs_addr + ((q0 + b) / NCH * BT + (q0 + b) % NCH * CH + 8 * o) * 4, x2[b][o], x2[b][o + 1]);
                         if constexpr (U > 1) {
 #pragma unroll
                             for (int b = 0; b < BATCH; ++b)
-                                if ((q0 + b) % NCH == 0) lds_4x32<C::kWideScales>(ws_addr + (q0 + b) / NCH * BR * 4, w4[b]);
+                                if ((q0 + b) % NCH == 0) lds_4x32(ws_addr + (q0 + b) / NCH * BR * 4, w4[b]);
                         }
                         tmem_ld_wait();
                         if (q0 + BATCH == STEPS) {
