@@ -122,6 +122,9 @@ struct Config {
     static constexpr int kTurn = GM == 0 ? 4 : kStages * BK / GM / kUnit;  // units per turn of the ring
     static constexpr int kSlotsRoom = BT <= 64 || (kUnit == 1 && BT <= 128) ? 4 : 2, kSlots = kSlotsRoom < kTurn ? kSlotsRoom : kTurn;
     static constexpr int kAcc = kUnit * kSlots;                       // accumulator slices
+    // Where the arrive by a branch is the faster one: 256 wide, g = 64, 4096 x 19456 x 2560 384 us and 392 with arrive_lane0; 128 wide,
+    // g = 256, 2048 x 6144 x 2560 38.1 and 38.8.
+    static constexpr bool kBranchArrive = (GM == 64 && BT == 256) || (GM == 256 && BT == 128);
     // The weight scales a chunk ahead (see the scales' warps): 256 wide, g = 64, 4096 x 19456 x 2560 380 us and 390 without; any group
     // size, 4096 x 19456 x 2560 with one group 267 and 273. Elsewhere it costs what it holds registers for: g = 64, 64 wide, 150 x 6144 x
     // 2560 12.2 and 11.4.
@@ -202,6 +205,14 @@ __device__ __forceinline__ uint32_t map_to_rank(uint32_t local, uint32_t rank) {
 }
 __device__ __forceinline__ void mbar_arrive_cluster(uint32_t cluster_addr) {
     asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(cluster_addr) : "memory");
+}
+// Lane 0 arrives, by a predicate: a branch would end the block of instructions in which the compiler mixes the promote with the reads.
+// (For the hand-over of sums: reading them and waiting for them is the warp's as one, so no lane is behind.) us with a branch and without,
+// 4096 x 19456 x 2560: 192 wide, g = 64 418 and 390, g = 128 307 and 286, g = 256 213 and 207; 256 wide, g = 128 244 and 238.
+template <bool CLUSTER>
+__device__ __forceinline__ void arrive_lane0(uint32_t addr, int lane) {
+    if constexpr (CLUSTER) asm volatile("{\n\t.reg .pred p;\n\tsetp.eq.u32 p, %1, 0;\n\t@p mbarrier.arrive.shared::cluster.b64 _, [%0];\n\t}" ::"r"(addr), "r"(lane) : "memory");
+    else asm volatile("{\n\t.reg .pred p;\n\tsetp.eq.u32 p, %1, 0;\n\t@p mbarrier.arrive.shared::cta.b64 _, [%0];\n\t}" ::"r"(addr), "r"(lane) : "memory");
 }
 __device__ __forceinline__ void cluster_sync_all() {
     asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
@@ -687,10 +698,14 @@ gemm_i8_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
                         if (q0 + BATCH == STEPS) {
                             // The unit's last sums are in registers: its slices may be overwritten while they are promoted.
                             tc_fence_before();
-                            __syncwarp();
-                            if (lane == 0) {
-                                if (PAIR && crank != 0) mbar_arrive_cluster(acc_empty0 + as * 8);
-                                else ptx::mbar_arrive(&acc_empty[as]);
+                            if constexpr (C::kBranchArrive) {
+                                __syncwarp();
+                                if (lane == 0) {
+                                    if (PAIR && crank != 0) mbar_arrive_cluster(acc_empty0 + as * 8);
+                                    else ptx::mbar_arrive(&acc_empty[as]);
+                                }
+                            } else {
+                                arrive_lane0<PAIR>(acc_empty0 + as * 8, lane);
                             }
                         }
 #pragma unroll
