@@ -14,7 +14,7 @@
 //   warp 1       MMA issuer: four tcgen05.mma (K = 32) per stage; every K-group accumulates into its own BT-column slice
 //                of tensor memory (two to four, in units eight), starting with "overwrite" or, at g = 64, with a bias (below)
 //   warps 2, 3   stage the scales of eight K-groups at a time in a ring of their own
-//   warps 4 ...  epilogue, eight or sixteen warps, each 32 weight rows x a part of the tokens. For every K-group
+//   warps 4 ...  epilogue, eight to sixteen warps, each 32 weight rows x a part of the tokens. For every K-group
 //                acc = fma(float(P) * ws, xs, acc), groups ascending -- the arithmetic and order of
 //                accumulate_group_kernel (int8_gemm.cu:213-234) -- in fp32 registers, then the fp16 store
 // One persistent CTA (or CTA pair) per SM (pair of SMs) walks over the tiles; all rings keep running across tiles, so
@@ -104,11 +104,13 @@ struct Config {
     static constexpr int kRoom = 226 * 1024 - 1024 - kOutBytes - kScBytes - kConst;
     static constexpr int kStages = kRoom / kStageBytes >= 8 ? 8 : 4;  // a multiple of four (see the issuer)
     static constexpr int kSmem = kStages * kStageBytes + kOutBytes + kScBytes + kConst + 1024;
-    // Epilogue warps: four per part of the tokens (one per 32 weight rows). Sixteen on the wide tiles; with the bias eight are as good
-    // at 256 tokens (steps of 32 tokens; 16: 1.03) and better at 128 (613 x 2560 x 9728 54.3 us for 55.7), not at 192
-    // (2048 x 19456 x 2560 247 us for 232).
-    static constexpr int kParts = BT >= 128 && !(kBiased && BT != 192) ? 4 : 2;
-    static constexpr int kStep = kBiased && BT == 256 ? 32 : 16;      // tokens per step of the promote
+    // Epilogue warps: four per part of the tokens (one per 32 weight rows). More warps hide more of one another's waits, fewer have the
+    // registers to mix more of the promote with the reads; measured form by form. g = 64, 96 wide, 2048 x 6144 x 2560: three parts 70.5 us,
+    // two 79.4; 192 wide, 4096 x 19456 x 2560: four 390, three 404, two 393. g = 128, 128 wide, 2048 x 6144 x 2560: two, in steps of 32 tokens, 44.3, four 46.4;
+    // 192 wide, 4001 x 2560 x 9728: four 124.6, three 130, two 136. g = 256, 256 wide, 4096 x 19456 x 2560: two 160, four 165; 128 wide, 2048 x
+    // 6144 x 2560: two, in steps of 32, 35.4, four 36.7.
+    static constexpr int kParts = GM == 64 ? (BT == 192 ? 4 : BT == 96 ? 3 : 2) : GM == 128 ? (BT >= 192 ? 4 : 2) : GM == 256 ? (BT == 192 ? 4 : 2) : 4;
+    static constexpr int kStep = (GM == 64 && BT == 256) || (GM >= 128 && BT == 128) ? 32 : 16;  // tokens per step of the promote
     static constexpr int kEpiWarps = 4 * kParts, kThreads = 128 + kEpiWarps * 32;
     // The widest tile needs more registers in its epilogue warps than all threads can have: warpgroup 0 gives some up.
     static constexpr bool kMoveRegs = BT > 192;
