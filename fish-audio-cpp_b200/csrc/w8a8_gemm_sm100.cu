@@ -24,6 +24,9 @@ int split_kb(int K, int g, int splits) {
     return (K / BK / unit + splits - 1) / splits * unit;
 }
 
+// The stages that a run of kb takes in the form: whole units.
+int padded_kb(const Form& f, int kb) { return (kb + f.unit_kb - 1) / f.unit_kb * f.unit_kb; }
+
 // setmaxnreg moves registers between the warpgroups of the widest form; the sums balance only for the register count the kernel
 // was compiled to (Form::launch_regs per thread). An unbalanced sum blocks for ever in setmaxnreg.inc, a wait nothing bounds, so in a
 // build that came out differently that form is not taken.
@@ -49,8 +52,9 @@ struct Choice {
 // The tile form that ends first: whole waves of tiles over the SMs (or pairs), each tile at its measured cost. A width
 // that leaves the last wave nearly empty loses to one that fills it; narrow tiles win where there are few tokens.
 // A tile's K is split over two or four CTAs where all of them fit the chip at once (a cluster of four leaves some SMs of a
-// GPC over: 128 of 148 taken as usable); meeting and adding up came out of the fit as 2.5 us for two and 5 for four. A split adds the
-// groups in another order than the other kernels do, so it has to save 10 % at least, and two are taken as 3 us: K = 2560 never splits.
+// GPC over: 128 of 148 taken as usable); meeting and adding up came out of the fit as 2.6-2.9 us for two and 5-5.6 for four. A split adds
+// the groups in another order than the other kernels do, so it has to save 10 % at least, with which 2.3 and 4.5 us choose best, and K = 2560
+// never splits.
 // Rows that are no multiple of eight leave element by element: 55 ns per token of a thread's part (measured at 4097 rows), which
 // the 256-token pairs at g = 64, with half the threads, lose by (4001 x 4097 x 2560 148 us, 192 wide 134).
 // table_g: the group size whose forms are looked at (0: those of any group size). pair: -1 either, 0 one CTA per tile, 1 a pair.
@@ -72,9 +76,9 @@ Choice choose(int M, int N, int K, int table_g, int g, int sms, int pair, int on
             if (only_splits && splits != only_splits) continue;
             if (f.split && (tiles * splits > (splits == 2 ? sms / 2 * 2 : sms * 7 / 8 - 1) || (splits - 1) * split_kb(K, g, splits) >= kb_total))
                 continue;
-            const double kb = f.split ? split_kb(K, g, splits) : kb_total;
+            const double kb = padded_kb(f, f.split ? split_kb(K, g, splits) : kb_total);
             double ns = ((tiles * splits + walkers - 1) / walkers) * (kb * f.stage_ns + kb * BK / g * f.group_ns + tile_ns);
-            if (f.split) ns = (ns + (splits == 2 ? 3000 : 5000)) / 0.9;
+            if (f.split) ns = (ns + (splits == 2 ? 2300 : 4500)) / 0.9;
             if ((!best.form || ns < best_ns) && usable(f)) { best = {&f, splits}; best_ns = ns; }
         }
     }

@@ -12,7 +12,7 @@
 //   warp 0       producer: TMA loads of 128 weight rows and BT token rows, 128 bytes of K each (both matrices are
 //                row-major with K contiguous, i.e. already the K-major operand; TMA applies the 128-byte swizzle)
 //   warp 1       MMA issuer: four tcgen05.mma (K = 32) per stage; every K-group accumulates into its own BT-column slice
-//                of tensor memory (two to four, in units eight), starting with "overwrite" or, at g = 64, with a bias (below)
+//                of tensor memory (two to sixteen), starting with "overwrite" or, at g = 64, with a bias (below)
 //   warps 2, 3   stage the scales of eight K-groups at a time in a ring of their own
 //   warps 4 ...  epilogue, eight to sixteen warps, each 32 weight rows x a part of the tokens. For every K-group
 //                acc = fma(float(P) * ws, xs, acc), groups ascending -- the arithmetic and order of
@@ -46,11 +46,15 @@
 //     block and reads the activation scales of sixteen sums, four tokens, with 16 bytes. (32x32b, a thread per row, is three times as
 //     fast out of tensor memory but needs a 16-byte read per four sums: 1.3-2 times as long in all, most while the MMAs read shared
 //     memory.)
-// Some 270 clocks of a K-group do not depend on the tile's width (370, 501, 561 and 725 clocks for 32, 64, 96 and 128 tokens at g = 256):
-// two waits, the arrive, the loop. Hence UNITS of two K-groups of 64 on the tiles of up to 128 tokens (252 and 410 clocks per group for
-// 32 and 64 tokens, 530 for 128). Four, or units at g = 128 and 256, would need a slot that is not known at compile time, as a tile may
-// end inside a unit: with the slot in a register of the issuing warp, two trial builds ended with an illegal memory access. Its cause was not
-// shown. With the lanes of that warp agreeing on every wait and meeting before the slot moved on, the builds ran, and lost 10-40 %.
+// Some 270 clocks of a hand-over do not depend on the tile's width: two waits, the arrive, the loop, each of them the end of what the
+// compiler can mix. Hence UNITS: up to 128 tokens, issuer and epilogue hand one another as many K-groups as two slots of tensor
+// memory hold, up to two, four or eight, and the loop over a chunk of scales is unrolled where that measured faster. us back to back, one
+// (g = 128, 256) or two (g = 64) groups per unit in a rolled loop, and now: g = 64 150 x 19456 x 2560, 32 wide 37.8 -> 30.1, 613 x 19456 x
+// 2560, 64 wide 101.8 -> 88.6, 2048 x 6144 x 2560, 96 wide 82.9 -> 73.1; g = 128 32 wide 28.2 -> 21.7, 64 wide 68.1 -> 56.7, 96 wide 60.0 -> 52.8; g = 256
+// 32 wide 20.9 -> 20.2 (96 and 128 wide lose a sixth by units of two: there the MMAs of a unit take longer than its promote hides).
+// A tile's K, or its run of a split, is padded to whole units, so that slots and columns stay immediates of the issuer: loads past
+// K bring zeros, those past a run the next run's operands, and the scales of the groups that only fill a unit are zero, which adds
+// 0 to sums that are never -0. (700 x 2560 x 2816, g = 256, 64 wide: 11 groups as 12, 11.0 us and 11.7.)
 //
 // Measured back to back in turn, us, without the bias, the units, the 16-byte scale reads and the cheaper SwiGLU, and with them
 // (M x N x K; the long ones under the power cap):
@@ -117,12 +121,13 @@ struct Config {
     // Registers per thread of the form that moves some: at launch, in warpgroup 0, in the others.
     static constexpr int kLaunchRegs = kParts == 2 ? 168 : 96, kLowRegs = kParts == 2 ? 40 : 56, kHighRegs = kParts == 2 ? 232 : 104;
     static_assert(128 * (kLaunchRegs - kLowRegs) >= kEpiWarps * 32 * (kHighRegs - kLaunchRegs), "setmaxnreg sums must balance");
-    // K-groups per unit: what issuer and epilogue hand one another (see above). Two groups of 64: K is a multiple of 128, so every
-    // tile and every run of a split is whole units. Two units in tensor memory, four where they are small.
-    static constexpr int kUnit = GM == 64 && BT <= 128 ? 2 : 1;
+    // K-groups per unit (see above), the stages that a unit takes, units per turn of the epilogue's loop.
+    static constexpr int kUnit = GM == 64 ? (BT == 32 ? 8 : BT == 64 ? 4 : BT <= 128 ? 2 : 1) : GM == 128 ? (BT <= 64 ? 4 : BT <= 128 ? 2 : 1) : GM == 256 && BT <= 64 ? 2 : 1;
+    static constexpr int kUnitKb = kUnit * GM > BK ? kUnit * GM / BK : 1;
+    static constexpr int kUnroll = GM == 64 ? (BT >= 192 || BT == 32 ? 1 : BT == 64 ? 2 : 4) : GM == 128 ? (BT >= 192 || BT == 64 ? 1 : BT == 96 ? 4 : 2) : 1;
     // No more of them than a turn of the ring fills, so that the issuer knows each at compile time.
     static constexpr int kTurn = GM == 0 ? 4 : kStages * BK / GM / kUnit;  // units per turn of the ring
-    static constexpr int kSlotsRoom = BT <= 64 || (kUnit == 1 && BT <= 128) ? 4 : 2, kSlots = kSlotsRoom < kTurn ? kSlotsRoom : kTurn;
+    static constexpr int kSlotsRoom = 4 * kUnit * BT <= 512 ? 4 : 2, kSlots = kSlotsRoom < kTurn ? kSlotsRoom : kTurn;
     static constexpr int kAcc = kUnit * kSlots;                       // accumulator slices
     // Where the arrive by a branch is the faster one: 256 wide, g = 64, 4096 x 19456 x 2560 384 us and 392 with arrive_lane0; 128 wide,
     // g = 256, 2048 x 6144 x 2560 38.1 and 38.8.
@@ -133,6 +138,7 @@ struct Config {
     static constexpr bool kScalesAhead = GM == 0 || (GM == 64 && BT == 256);
     static constexpr int kBatch = GM == 64 && BT <= 64 ? 2 : 1;  // steps whose sums are requested together
     static constexpr int kTmemCols = kAcc * BT <= 128 ? 128 : kAcc * BT <= 256 ? 256 : 512;
+    static_assert(kSlots >= 2 && kTurn % kSlots == 0, "one unit's sums are formed while another's are promoted");
     static_assert(kStages * kStageBytes <= kRoom, "stages do not fit");
     static_assert(BT % 32 == 0 && BT <= 256, "token width");
 };
@@ -368,8 +374,10 @@ gemm_i8_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
     static_assert(!SPLIT || (!PAIR && GM != 0), "a split tile is one CTA's, of whole K-groups");
     const int srank = SPLIT ? static_cast<int>(cluster_rank()) : 0;
     const int kb0 = SPLIT ? srank * p.split_kb : 0;
-    const int num_kb = SPLIT ? min(p.split_kb, a.K / BK - kb0) : a.K / BK;
-    const int G = a.G, g_first = SPLIT ? kb0 * BK / GM : 0, g_end = SPLIT ? g_first + num_kb * BK / GM : G;  // this CTA's K-groups
+    const int real_kb = SPLIT ? min(p.split_kb, a.K / BK - kb0) : a.K / BK, num_kb = (real_kb + C::kUnitKb - 1) / C::kUnitKb * C::kUnitKb;
+    // this CTA's K-groups, and where they end with those that only fill the last unit
+    const int G = a.G, g_first = SPLIT ? kb0 * BK / GM : 0, g_end = SPLIT ? g_first + real_kb * BK / GM : G;
+    const int g_pad = GM == 0 ? G : g_first + num_kb * BK / (GM == 0 ? 1 : GM);
     const uint32_t crank = PAIR ? cluster_rank() : 0u;
     const int walker = SPLIT ? static_cast<int>(blockIdx.x) / p.splits : PAIR ? static_cast<int>(blockIdx.x >> 1) : static_cast<int>(blockIdx.x);
     const int walkers = SPLIT ? p.tiles_total : PAIR ? static_cast<int>(gridDim.x >> 1) : static_cast<int>(gridDim.x);
@@ -445,7 +453,7 @@ gemm_i8_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
                         }
                     }
                     kx += BK;
-                    if (kx == a.K) {
+                    if (kx == (kb0 + num_kb) * BK) {
                         kx = 0;
                         tile += walkers;
                         m0 = tile_m0(tile) + (PAIR ? static_cast<int>(crank) * C::kRowsB : 0);
@@ -555,7 +563,7 @@ gemm_i8_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
                 }
             };
             auto load_w_ahead = [&](int tile, int j0) {
-                if (j0 >= g_end) { tile += walkers; j0 = g_first; }
+                if (j0 >= g_pad) { tile += walkers; j0 = g_first; }
                 if (tile >= p.tiles_total) return;
                 const int n0 = tile_n0(tile);
                 load_w(w_row(n0), w_row(n0 + 64), j0);
@@ -574,7 +582,7 @@ gemm_i8_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
                 // (Once a tile: formed anew for every chunk they cost the tiles of 192 tokens 1 %, a call of one wave up to 2 %.)
                 const __half* ws0 = w_row(n0);
                 const __half* ws1 = w_row(n0 + 64);
-                for (int j0 = g_first; j0 < g_end; j0 += kScGroups) {
+                for (int j0 = g_first; j0 < g_pad; j0 += kScGroups) {
                     const int nj = min(kScGroups, g_end - j0);
                     if constexpr (!C::kScalesAhead) load_w(ws0, ws1, j0);  // on their way while the slot is waited for
                     if (!wait(&sc_empty[slot], parity)) {
@@ -586,13 +594,17 @@ gemm_i8_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
                     for (int t = t64; t < BT; t += 64) {
                         const float* src = a.Xs + static_cast<size_t>(min(m0 + t, a.M - 1)) * G + j0;
 #pragma unroll
-                        for (int q = 0; q < kScGroups; ++q)
-                            if (q < nj) asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(dst + (q * BT + xs_slot(t)) * 4), "l"(src + q) : "memory");
+                        for (int q = 0; q < kScGroups; ++q) {
+                            const uint32_t to = dst + (q * BT + xs_slot(t)) * 4;
+                            if (q < nj) asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(to), "l"(src + q) : "memory");
+                            else if (C::kUnit > 1 && j0 + q < g_pad) asm volatile("st.shared.f32 [%0], %1;" ::"r"(to), "f"(0.0f) : "memory");
+                        }
                     }
                     asm volatile("cp.async.mbarrier.arrive.noinc.shared.b64 [%0];" ::"r"(ptx::smem_u32(&sc_full[slot])) : "memory");
 #pragma unroll
                     for (int q = 0; q < kScGroups; ++q) {
-                        const float w0 = __half2float(w[0][q]), w1 = __half2float(w[1][q]);
+                        const bool real = C::kUnit == 1 || q < nj;
+                        const float w0 = real ? __half2float(w[0][q]) : 0.0f, w1 = real ? __half2float(w[1][q]) : 0.0f;
                         if (C::kBiased && (isinf(w0) || isinf(w1))) infinite_s[ith % kMarks] = ith + 1;
                         asm volatile("st.shared.f32 [%0], %1;" ::"r"(dst + (kScGroups * BT + q * BR + ws_slot(t64)) * 4), "f"(w0 * kScale) : "memory");
                         asm volatile("st.shared.f32 [%0], %1;" ::"r"(dst + (kScGroups * BT + q * BR + 64 + ws_slot(t64)) * 4), "f"(w1 * kScale) : "memory");
@@ -636,7 +648,7 @@ gemm_i8_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
             // (A second buffer of sums, filled while the first is promoted, within a group or from one to the next: no gain.)
             uint32_t r[BATCH][2][CH / 2];
 #pragma unroll 1
-            for (int j0 = g_first; j0 < g_end && ok; j0 += kScGroups) {
+            for (int j0 = g_first; j0 < g_pad && ok; j0 += kScGroups) {
                 if (!wait(&sc_full[slot], sc_parity)) {
                     if (lane == 0) atomicExch(p.status, 700 + slot);
                     ok = false;
@@ -644,8 +656,8 @@ gemm_i8_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
                 }
                 uint32_t xs_addr = sc_ring + slot * C::kScSlot + (part * HC + 4 * (lane & 3)) * 4;
                 uint32_t ws_addr = sc_ring + slot * C::kScSlot + (kScGroups * BT + quad * 32 + 4 * (lane >> 2)) * 4;
-                const int j1 = min(j0 + kScGroups, g_end);
-#pragma unroll 1
+                const int j1 = min(j0 + kScGroups, g_pad);
+#pragma unroll C::kUnroll
                 for (int j = j0; j < j1; j += U) {
                     const uint32_t taddr = taddr0 + as * (U * BT);
                     float w4[BATCH][4];
@@ -910,12 +922,11 @@ struct FormState {
     std::atomic<int> registers{0};  // per thread, as compiled (0: not asked for yet)
 };
 // A tile form: its kernel and what the launch needs to know about it. stage_ns, group_ns, tile_ns: what a tile takes per 128 bytes of
-// K, per K-group and for itself (the start of its chain, conversion, store). Fitted to 4100 times, no cost below zero: seven shapes (the
-// four projections, 9728 x 2560, 4096 x 9728, 1000 x 1024) x 29 token counts from 33 to 8192 x every form that takes them, for each
-// group size. With 2.7-3.2 us for the launch nine in ten of the times within a third of the best form's lie within 15 % of the model's.
-// What it does not hold: a chip that is not full (at groups of 256 a stage of a lone tile of 96 tokens takes 210 ns, not 290), and what
-// several sweeps over a long prompt's codes miss L2 for. Judged by its choice, the rule lost 0.4, 0.5 and 0.4 % against the best form on
-// average (groups of 64, 128, 256), and 0.2, 1.2 and 1.2 % over eight other shapes x eleven token counts, most of it splits of K not taken.
+// K, per K-group and for itself (the start of its chain, conversion, store). Fitted to 4100 times, no cost below zero, then moved by up
+// to 6 % each towards the choices that lose least: seven shapes (the four projections, 9728 x 2560, 4096 x 9728, 1000 x 1024) x 31 token
+// counts from 33 to 8192 x every form that takes them, for each group size. What it does not hold: a chip that is not full, and what
+// several sweeps over a long prompt's codes miss L2 for. Judged by its choice, the rule loses 0.5, 0.4 and 0.3 % against the best form on
+// average (groups of 64, 128, 256), and 0.8, 0.6 and 0.4 % over eight other shapes x eleven token counts.
 struct Form {
     int bt;
     bool pair, split;
@@ -923,7 +934,7 @@ struct Form {
     int threads, smem;
     int launch_regs;  // per thread, if the form moves some between its warpgroups; else 0
     float stage_ns, group_ns, tile_ns;
-    int parts;  // Config::kParts
+    int parts, unit_kb;  // Config::kParts, Config::kUnitKb
     FormState* state;
 };
 template <int BT, bool PAIR, int GM, bool SPLIT>
@@ -932,13 +943,13 @@ template <int BT, bool PAIR, int GM, bool SPLIT = false>
 Form form(float stage_ns, float group_ns, float tile_ns) {
     using C = Config<BT, PAIR, GM>;
     return Form{BT, PAIR, SPLIT, gemm_i8_kernel<BT, PAIR, GM, SPLIT>, C::kThreads, C::kSmem, C::kMoveRegs ? C::kLaunchRegs : 0,
-                stage_ns, group_ns, tile_ns, C::kParts, &form_state<BT, PAIR, GM, SPLIT>};
+                stage_ns, group_ns, tile_ns, C::kParts, C::kUnitKb, &form_state<BT, PAIR, GM, SPLIT>};
 }
 template <int GM>
 const Form* all_forms(int* count) {
     // per stage at groups of 64, 128 and 256, and per tile, for token widths 32, 64, 96, 128, 192, 256
-    constexpr float kStage[3][6] = {{314, 470, 514, 601, 912, 1157}, {210, 300, 351, 390, 609, 744}, {152, 177, 289, 308, 363, 451}};
-    constexpr float kTile[3][6] = {{0, 0, 600, 740, 1530, 1420}, {400, 440, 610, 930, 1230, 1660}, {300, 590, 20, 300, 1650, 1880}};
+    constexpr float kStage[3][6] = {{235, 380, 441, 563, 825, 1142}, {151, 245, 298, 339, 508, 670}, {141, 170, 286, 288, 321, 383}};
+    constexpr float kTile[3][6] = {{110, 260, 610, 920, 1930, 2590}, {440, 390, 720, 1150, 2220, 2550}, {290, 740, 90, 500, 2190, 2730}};
     constexpr int q = GM == 64 ? 0 : GM == 128 ? 1 : 2;
     static const Form table[] = {form<32, false, GM>(kStage[q][0], 0, kTile[q][0]),       form<64, false, GM>(kStage[q][1], 0, kTile[q][1]),
                                  form<96, false, GM>(kStage[q][2], 0, kTile[q][2]),       form<128, false, GM>(kStage[q][3], 0, kTile[q][3]),

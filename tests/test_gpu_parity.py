@@ -727,6 +727,27 @@ def test_gemm_tcgen05_tile_widths(gemm_form, oracle, pkg, M, N, K, bt, form, g):
     assert np.array_equal(dY.cpu().numpy().view(np.uint16), oracle.linear_q(W, ws, Xq, Xs, g).view(np.uint16))
 
 
+@pytest.mark.parametrize("K,g", [(128, 64), (384, 64), (640, 64), (1152, 64), (128, 128), (384, 128), (640, 128), (1152, 128), (256, 256), (768, 256), (2304, 256)])
+@pytest.mark.parametrize("bt", [32, 64, 96, 128])
+def test_gemm_tcgen05_k_that_ends_inside_a_unit(gemm_form, oracle, pkg, K, g, bt):
+    """The narrow forms hand over two to eight K-groups at a time: a K of one, three, five and nine stages or groups ends inside such
+    a unit in most of them, what is left is filled with groups of scale zero, and several tiles of a CTA follow one another.
+    Negative sums and outputs of zero among them. Bit for bit the oracle's."""
+    M, N = 149, 2 * 148 * 128 + 136  # more tiles than SMs in every form
+    ctx = gemm_form(bt, 1)
+    X, W, ws = synth.linear_case(K + bt, M, N, K, g)
+    Xq, Xs = oracle.quantize(X, g)
+    Xq[3] = 0
+    W[5] = -W[5]
+    _, dY = guarded((M, N), torch.float16, 99.0)
+    ctx.linear_q(dev(W), dev(ws), g, dev(Xq), dev(Xs), dY, M, N, K, kernel=pkg.KERNEL_GEMM_SINGLE)
+    torch.cuda.synchronize()
+    ctx.check_device_status()
+    rows = np.r_[0:300, N - 300:N]
+    assert np.array_equal(dY.cpu().numpy()[:, rows].view(np.uint16),
+                          oracle.linear_q(np.ascontiguousarray(W[rows]), np.ascontiguousarray(ws[rows]), Xq, Xs, g).view(np.uint16))
+
+
 @pytest.mark.parametrize("g", [64, 128, 256])
 @pytest.mark.parametrize("splits", [2, 4])
 @pytest.mark.parametrize("bt", [32, 64, 96, 128])
