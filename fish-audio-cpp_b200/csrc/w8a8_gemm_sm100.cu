@@ -32,17 +32,27 @@ int padded_kb(const Form& f, int kb) { return (kb + f.unit_kb - 1) / f.unit_kb *
 // build that came out differently that form is not taken.
 bool balanced(const Form& f) {
     if (f.launch_regs == 0) return true;
-    int r = f.state->registers.load(std::memory_order_relaxed);
-    if (r == 0) {
-        cudaFuncAttributes fa;
-        if (cudaFuncGetAttributes(&fa, f.kernel) != cudaSuccess) {
-            cudaGetLastError();
-            return false;
+    for (int i = 0; i < 2 && f.kernel[i]; ++i) {
+        int r = f.state[i].registers.load(std::memory_order_relaxed);
+        if (r == 0) {
+            cudaFuncAttributes fa;
+            if (cudaFuncGetAttributes(&fa, f.kernel[i]) != cudaSuccess) {
+                cudaGetLastError();
+                return false;
+            }
+            f.state[i].registers.store(r = fa.numRegs, std::memory_order_relaxed);
         }
-        f.state->registers.store(r = fa.numRegs, std::memory_order_relaxed);
+        if (r != f.launch_regs) return false;
     }
-    return r == f.launch_regs;
+    return true;
 }
+
+// Which side of the tiles is walked first. Tokens, so that concurrent CTAs share weight tiles in L2 and each weight is read from memory once;
+// but where the activation codes are the larger operand and do not stay in L2 beside the rest, every such sweep reads them from memory
+// again. Then rows: the weights stay, and the codes are read once. us back to back, tokens and rows first: 8192 x 2560 x 9728 (80 MB of
+// codes) g = 256 198 and 182, g = 128 294 and 256; 16384 x 2560 x 9728 407 and 337; 6500 (63 MB) 166 and 160; 5000 (49 MB) 129.6 and
+// 129.9; 2048 59.8 and 62.2.
+bool walk_rows_first(int M, int N, int K) { return M > N && static_cast<long long>(M) * K >= 60000000ll; }
 
 struct Choice {
     const Form* form;
@@ -131,8 +141,10 @@ int launch_linear_gemm(const LinearArgs& a, int* device_status, cudaStream_t str
     GemmParams p;
     p.a = a;
     p.status = device_status;
-    p.tiles_m = (a.M + bt - 1) / bt;
-    p.tiles_total = p.tiles_m * ((a.N + rows - 1) / rows);
+    const int tiles_m = (a.M + bt - 1) / bt, tiles_n = (a.N + rows - 1) / rows;
+    const bool rows_first = best->kernel[1] && walk_rows_first(a.M, a.N, a.K);
+    p.inner = rows_first ? tiles_n : tiles_m;
+    p.tiles_total = tiles_m * tiles_n;
     p.splits = best_splits;
     p.split_kb = split_kb(a.K, a.g, best_splits);
     p.tma_store = ycols % 8 == 0 && (reinterpret_cast<uintptr_t>(a.Y) & 15u) == 0;
@@ -145,8 +157,7 @@ int launch_linear_gemm(const LinearArgs& a, int* device_status, cudaStream_t str
         if (rc) return rc;
     }
     cudaLaunchConfig_t cfg = {};
-    // persistent: one CTA (or CTA pair) per SM (pair of SMs) walks its tiles, tokens fastest, so that concurrent CTAs
-    // share weight tiles in L2
+    // persistent: one CTA (or CTA pair) per SM (pair of SMs) walks its tiles
     const int walkers_max = best->pair ? sms / 2 : sms;
     const int walkers = p.tiles_total < walkers_max ? p.tiles_total : walkers_max;
     cfg.gridDim = dim3(best->pair ? 2 * walkers : best->split ? best_splits * p.tiles_total : walkers, 1, 1);
@@ -169,7 +180,7 @@ int launch_linear_gemm(const LinearArgs& a, int* device_status, cudaStream_t str
     }
     cfg.attrs = attr;
     cfg.numAttrs = na;
-    const cudaError_t e = launch_with_smem(best->state->attribute, best->smem, cfg, best->kernel, map_w, map_x, map_y, p);
+    const cudaError_t e = launch_with_smem(best->state[rows_first].attribute, best->smem, cfg, best->kernel[rows_first], map_w, map_x, map_y, p);
     if (e != cudaSuccess) return fail(W8A8_ERR_CUDA, "gemm launch: %s", cudaGetErrorString(e));
     return W8A8_OK;
 }

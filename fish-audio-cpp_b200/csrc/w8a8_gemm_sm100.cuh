@@ -79,7 +79,7 @@ constexpr uint32_t kSpin = 1u << 21;
 struct GemmParams {
     LinearArgs a;
     int* status;
-    int tiles_m, tiles_total;
+    int inner, tiles_total;  // tiles along the side that is walked first; in all
     int splits, split_kb;  // SPLIT: CTAs that share a tile's K, and the stages each of them takes (the last one what is left)
     int tma_store;  // output rows are multiples of 16 bytes and aligned: the tile leaves by TMA
 };
@@ -350,7 +350,10 @@ __device__ __forceinline__ void infinite_rows(const LinearArgs& a, const uint32_
 // the others' fp32 sums from their shared memory and adds them in ascending-K order. Narrow tiles are a serial chain of K-groups,
 // whatever the number of CTAs (tokens x rows x K, the best form without a split and with one: g = 64, 33 x 2560 x 9728 25.0 and 16.4 us,
 // 150 x 2560 x 9728 25.2 and 23.5, 33 x 2560 x 4096 14.3 and 11.2; g = 256, 64 x 2560 x 9728 14.5 and 11.2).
-template <int BT, bool PAIR, int GM, bool SPLIT>
+//
+// ROWS_FIRST: which side of the tiles is walked first (see walk_rows_first). An instance of its own: chosen in the kernel, by a parameter, it
+// cost the pairs of 192 tokens at g = 64 up to 3 % wherever it was not taken (code placement: 4001 x 6144 x 2560 121.7 and 126.6 us).
+template <int BT, bool PAIR, int GM, bool SPLIT, bool ROWS_FIRST>
 __global__ void __launch_bounds__(Config<BT, PAIR, GM>::kThreads, 1)
 gemm_i8_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_x,
                const __grid_constant__ CUtensorMap map_y, const GemmParams p) {
@@ -381,8 +384,8 @@ gemm_i8_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
     const uint32_t crank = PAIR ? cluster_rank() : 0u;
     const int walker = SPLIT ? static_cast<int>(blockIdx.x) / p.splits : PAIR ? static_cast<int>(blockIdx.x >> 1) : static_cast<int>(blockIdx.x);
     const int walkers = SPLIT ? p.tiles_total : PAIR ? static_cast<int>(gridDim.x >> 1) : static_cast<int>(gridDim.x);
-    auto tile_m0 = [&](int tile) { return (tile % p.tiles_m) * BT; };
-    auto tile_n0 = [&](int tile) { return (tile / p.tiles_m) * (PAIR ? 2 * BR : BR) + static_cast<int>(crank) * BR; };
+    auto tile_m0 = [&](int tile) { return (ROWS_FIRST ? tile / p.inner : tile % p.inner) * BT; };
+    auto tile_n0 = [&](int tile) { return (ROWS_FIRST ? tile % p.inner : tile / p.inner) * (PAIR ? 2 * BR : BR) + static_cast<int>(crank) * BR; };
     int my_tiles = 0;
     if (walker < p.tiles_total) my_tiles = (p.tiles_total - walker + walkers - 1) / walkers;
 
@@ -930,20 +933,22 @@ struct FormState {
 struct Form {
     int bt;
     bool pair, split;
-    Kernel kernel;
+    Kernel kernel[2];  // tokens walked first, rows walked first (or none)
     int threads, smem;
     int launch_regs;  // per thread, if the form moves some between its warpgroups; else 0
     float stage_ns, group_ns, tile_ns;
     int parts, unit_kb;  // Config::kParts, Config::kUnitKb
-    FormState* state;
+    FormState* state;  // [2]
 };
 template <int BT, bool PAIR, int GM, bool SPLIT>
-inline FormState form_state;
+inline FormState form_state[2];
 template <int BT, bool PAIR, int GM, bool SPLIT = false>
 Form form(float stage_ns, float group_ns, float tile_ns) {
     using C = Config<BT, PAIR, GM>;
-    return Form{BT, PAIR, SPLIT, gemm_i8_kernel<BT, PAIR, GM, SPLIT>, C::kThreads, C::kSmem, C::kMoveRegs ? C::kLaunchRegs : 0,
-                stage_ns, group_ns, tile_ns, C::kParts, C::kUnitKb, &form_state<BT, PAIR, GM, SPLIT>};
+    Kernel rows_first = nullptr;
+    if constexpr (BT >= 128 && !SPLIT && GM != 0) rows_first = gemm_i8_kernel<BT, PAIR, GM, SPLIT, true>;  // (a long prompt's forms)
+    return Form{BT, PAIR, SPLIT, {gemm_i8_kernel<BT, PAIR, GM, SPLIT, false>, rows_first}, C::kThreads, C::kSmem, C::kMoveRegs ? C::kLaunchRegs : 0,
+                stage_ns, group_ns, tile_ns, C::kParts, C::kUnitKb, form_state<BT, PAIR, GM, SPLIT>};
 }
 template <int GM>
 const Form* all_forms(int* count) {

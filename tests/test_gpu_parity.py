@@ -727,6 +727,36 @@ def test_gemm_tcgen05_tile_widths(gemm_form, oracle, pkg, M, N, K, bt, form, g):
     assert np.array_equal(dY.cpu().numpy().view(np.uint16), oracle.linear_q(W, ws, Xq, Xs, g).view(np.uint16))
 
 
+@pytest.mark.parametrize("N", [1000, 1003])
+@pytest.mark.parametrize("g", [64, 128, 256])
+@pytest.mark.parametrize("bt,form", [(128, "SINGLE"), (192, "PAIR"), (256, "PAIR")])
+def test_gemm_tcgen05_rows_walked_first(gemm_form, oracle, pkg, bt, form, g, N):
+    """A prompt whose codes are the larger operand is walked rows first; its parts, which are walked tokens first, give the same bits."""
+    M, K = 6301, 9728
+    assert M > N and M * K >= 60_000_000 > M // 2 * K
+    ctx = gemm_form(bt, 1)
+    gen = torch.Generator(device="cuda").manual_seed(bt + g)
+    W = torch.randint(-127, 128, (N, K), dtype=torch.int8, device="cuda", generator=gen)
+    ws = torch.empty((N, K // g), device="cuda").uniform_(1e-3, 5e-3, generator=gen).half()
+    Xq = torch.randint(-127, 128, (M, K), dtype=torch.int8, device="cuda", generator=gen)
+    Xs = torch.rand((M, K // g), device="cuda", generator=gen) * 1e-2 + 1e-4
+    kernel = getattr(pkg, "KERNEL_GEMM_" + form)
+    buf, whole = guarded((M, N), torch.float16, 99.0)
+    ctx.linear_q(W, ws, g, Xq, Xs, whole, M, N, K, kernel=kernel)
+    parts = torch.empty_like(whole)
+    for m0, m1 in ((0, M // 2), (M // 2, M)):
+        rows = torch.empty((m1 - m0, N), dtype=torch.float16, device="cuda")
+        ctx.linear_q(W, ws, g, Xq[m0:m1].contiguous(), Xs[m0:m1].contiguous(), rows, m1 - m0, N, K, kernel=kernel)
+        parts[m0:m1] = rows
+    torch.cuda.synchronize()
+    ctx.check_device_status()
+    assert guards_intact(buf, 99.0)
+    assert torch.equal(whole.view(torch.int16), parts.view(torch.int16))
+    some = [0, 1, 255, 256, M // 2, M - 1]
+    want = oracle.linear_q(W.cpu().numpy(), ws.cpu().numpy(), Xq[some].cpu().numpy(), Xs[some].cpu().numpy(), g)
+    assert np.array_equal(whole[some].cpu().numpy().view(np.uint16), want.view(np.uint16))
+
+
 @pytest.mark.parametrize("K,g", [(128, 64), (384, 64), (640, 64), (1152, 64), (128, 128), (384, 128), (640, 128), (1152, 128), (256, 256), (768, 256), (2304, 256)])
 @pytest.mark.parametrize("bt", [32, 64, 96, 128])
 def test_gemm_tcgen05_k_that_ends_inside_a_unit(gemm_form, oracle, pkg, K, g, bt):
