@@ -663,6 +663,24 @@ int launch_qknorm_rope_kvwrite(const __half* qkv, const __half* q_norm_w, const 
     return W8A8_OK;
 }
 
+// Context slices per (sequence, kv head) pair, for the longest sequence the table can hold. us of a decode layer at 8 kv heads.
+// At most as many as run at once, a cluster's CTAs lying in one GPC: sixteen clusters of eight do not fit (36 blocks 40.8, with three 35.8), nor
+// 24 of six (40.5, with four 36.3) nor 48 of three (42.1, with two 37.7); 40 of three and 32 of four do.
+// One, as long as its ring holds the whole context: every further CTA starts later (it finds no SM that the projection ahead has
+// left free) and has a state to merge. 17 blocks, batch 1 34.1 with eight and 32.9 with one, batch 5 36.6 with two and 34.1, batch 8 37.4 and 36.4; 25 blocks,
+// batch 4 36.0 and 34.8; 30 blocks, batch 8, 37.7 with two and 38.2 with one.
+// Then a slice per twelve blocks: 45 blocks, batch 1 34.4 with eight and 34.0 with three, batch 2 39.9 and 35.9; 128 blocks, batch 2 41.2 with
+// eight, 38.3 with four and 37.6 with six, batch 5 45.9 with two and 41.8 with three. Two where three fit, and 72 CTAs in three, are worse than
+// their neighbours: batch 4, 45 blocks 37.2 with two, 36.5 with three; batch 3 37.2, 37.1 and, with four, 36.3.
+int attention_slices(int pairs, int blocks, int sms) {
+    const int most = pairs * 8 <= sms / 2 ? 8 : pairs * 6 <= sms * 2 / 3 ? 6 : pairs * 4 <= sms * 7 / 8 ? 4 : pairs * 3 <= sms * 5 / 6 ? 3 : pairs * 2 <= sms ? 2 : 1;
+    if (blocks <= kRing + 1 || most == 1) return 1;
+    const int want = blocks / 12 < most ? blocks / 12 : most;
+    if (want == 2 && most >= 3 && pairs > 8) return pairs * 3 >= 64 && pairs * 3 < 90 ? 4 : 3;
+    if (want == 3 && pairs * 3 >= 64 && pairs * 3 < 90) return 4;
+    return want >= 8 ? 8 : want >= 6 ? 6 : want >= 4 ? 4 : want;
+}
+
 namespace {
 int launch_attention(const AttnParams& base, int B, int splits, cudaStream_t stream);
 }
@@ -704,13 +722,7 @@ int launch_attention(const AttnParams& base, int B, int splits, cudaStream_t str
         return fail(W8A8_ERR_UNSUPPORTED, "paged attention here handles 4 query heads per kv head (got %d / %d)", n_q, n_kv);
     if (Xq && (g <= 0 || (kQPerKv * kHeadDim) % g != 0))
         return fail(W8A8_ERR_UNSUPPORTED, "fused output quantisation needs a group size dividing 512 (got %d)", g);
-    if (splits <= 0) {  // one CTA per SM: as many context slices as the (sequence, kv head) pairs leave room for
-        const int sms = device_sms();
-        const int want = sms / (B * n_kv);
-        splits = want >= 8 ? 8 : want >= 4 ? 4 : want >= 2 ? 2 : 1;
-        // no more slices than give each consumer warp a block of the longest sequence the table can hold
-        while (splits > 1 && (splits / 2) * kAttnWarps >= base.max_blocks) splits /= 2;
-    }
+    if (splits <= 0) splits = attention_slices(B * n_kv, base.max_blocks, device_sms());
     if (splits > kMaxSlices) splits = kMaxSlices;
     AttnParams p = base;
     p.S = splits;

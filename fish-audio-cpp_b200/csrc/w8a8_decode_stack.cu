@@ -982,9 +982,8 @@ Scratch layout(const w8a8_decode_stack& d, int S) {
     return sc;
 }
 
-int slices_for(const w8a8_decode_stack& d, int sms) {
-    const int want = sms / (d.batch * d.n_kv_heads);
-    return want >= 8 ? 8 : want >= 4 ? 4 : want >= 2 ? 2 : 1;  // the stand-alone attention launch picks the same
+int slices_for(const w8a8_decode_stack& d, int sms) {  // as the stand-alone attention launch has them
+    return attention_slices(d.batch * d.n_kv_heads, d.max_blocks_per_seq, sms);
 }
 
 const char* check(const w8a8_decode_stack& d) {

@@ -145,6 +145,7 @@ int launch_linear_gemv_rows(const LinearArgs& a, int* device_status, cudaStream_
 // w8a8_gemv_packed.cu : M <= 32 over pre-packed weights (linear byte stream, 1-D bulk copies).
 size_t packed_weight_bytes(int N, int K, int g);
 int launch_pack_weight(const int8_t* W, const __half* S, int N, int K, int g, void* out, cudaStream_t s);
+int attention_slices(int pairs, int max_blocks, int sms);  // CTAs that share a (sequence, kv head) pair's context
 int gemv_packed_ctas(int tiles, int sms, bool two_per_sm);  // CTAs that share a linear's row tiles
 bool gemv_packed_supports(const LinearArgs& a);  // also answers for the prologue and tail forms (fields of a set)
 bool quant_form_wins(const LinearArgs& a);       // whether fp16 rows (X set, Xq null) should be quantised inside the linear

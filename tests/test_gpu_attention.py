@@ -97,6 +97,24 @@ def test_paged_attention_decode(ctx, oracle, B, lens, splits):
         assert (rout.float() - dout.float()).abs().max().item() <= 2e-3 * max(1.0, rout.float().abs().max().item())
 
 
+# One to eight slices as the launch chooses them (the table's width and the batch decide), the longest sequence filling the table.
+@pytest.mark.parametrize("B,max_blocks", [(8, 25), (1, 26), (8, 26), (1, 44), (5, 45), (3, 40), (4, 128), (2, 128), (1, 128), (10, 128)])
+def test_paged_attention_decode_with_chosen_slices(ctx, oracle, B, max_blocks):
+    rng = np.random.default_rng(B + max_blocks)
+    layer = 1
+    lens = [max_blocks * BS] + [int(rng.integers(0, max_blocks * BS)) for _ in range(B - 1)]
+    kc, vc, bt = make_cache(rng, B, max(lens), max_blocks)
+    q = rng.standard_normal((B, N_Q, D)).astype(np.float16)
+    seq = np.array(lens, np.int32)
+    dout = torch.full((B, N_Q, D), 9.0, dtype=torch.float16, device="cuda")
+    sm = 1.0 / np.sqrt(D)
+    ctx.paged_attention_decode(dev(q), dev(kc), dev(vc), dev(bt), dev(seq), dout, B, N_Q, D, max_blocks, sm, layer, LAYERS, N_KV)
+    torch.cuda.synchronize()
+    ctx.check_device_status()
+    want = oracle.paged_attention_decode(q, kc, vc, bt, seq, layer, sm)
+    assert np.abs(dout.cpu().numpy().astype(np.float64) - want).max() <= 2e-3 * max(1.0, np.abs(want).max())
+
+
 @pytest.mark.parametrize("B,positions", [(1, [0]), (3, [15, 16, 40]), (8, [1024] * 8), (4, [4, 299, 31, 999])])
 @pytest.mark.parametrize("splits", [0, 1, 2, 3])
 def test_qkv_attention_decode_equals_the_two_calls(ctx, B, positions, splits):
