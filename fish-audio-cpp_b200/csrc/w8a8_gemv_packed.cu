@@ -94,7 +94,15 @@ bool gemv::make_plan(const LinearArgs& a, Plan& pl, bool rows) {
     pl.tiles = (a.N + 15) / 16;
     pl.U = static_cast<long long>(pl.tiles) * pl.upt;
     // Up to two CTAs per SM where their registers and shared memory fit twice, never more CTAs than row tiles.
-    pl.ctas = gemv_packed_ctas(pl.tiles, device_sms(), two_per_sm(pl.MT, pl.GM));
+    // Two row tiles at once where the CTA that holds most has more than eight blocks per warp: half the reads of activations, twice the code,
+    // which runs cold, and a longer first step. us, one tile and two: M = 16, g = 64 2560 x 9728 12.6 and 10.5, 20000 x 2560 15.2 and 13.3,
+    // 155776 x 2560 82 and 65; g = 128 11.2 and 9.9, 14.5 and 12.8, 72 and 64; M = 32, g = 64 12000 x 9728 45.5 and 40.0, g = 256 155776 x 2560 98 and 76; but
+    // 6144 x 2560 at M = 32 11.1 and 12.3, and at g >= 128 and M = 9, where the other form fits an SM twice, 2560 x 9728 9.4 and 9.7.
+    // Decode step, batch 16: g = 64 1790 and 1733, g = 128 1662 and 1610.
+    const int sms = device_sms();
+    const int most = (pl.tiles + sms - 1) / sms * (a.K / 256);  // blocks of the CTA that holds most, a CTA per SM
+    pl.NR = pl.MT > 1 && most > 8 * kWarps && (pl.MT == 4 || pl.GM == 64 || a.M > 12) ? 2 : 1;
+    pl.ctas = gemv_packed_ctas(pl.tiles, sms, two_per_sm(pl.MT, pl.GM, pl.NR));
     if ((pl.U + 1) * static_cast<long long>(pl.ctas) * kWarps >= (1ll << 32)) return false;  // 32-bit range math
     return true;
 }
@@ -115,17 +123,17 @@ void gemv::fill_params(const LinearArgs& a, const Plan& pl, int* status, GemvPac
 
 namespace {
 
-template <int MT, int GM, int PRO, int ST, int KI, int EPI, bool EXTRA>
-__global__ void __launch_bounds__(kThreads, two_per_sm(MT, GM) ? 2 : 1)
+template <int MT, int GM, int NR, int PRO, int ST, int KI, int EPI, bool EXTRA>
+__global__ void __launch_bounds__(kThreads, two_per_sm(MT, GM, NR) ? 2 : 1)
 gemv_packed_kernel(const __grid_constant__ GemvPackedParams p) {
-    gemv_body<MT, GM, PRO, ST, KI, EPI, EXTRA, false>(p, nullptr);
+    gemv_body<MT, GM, NR, PRO, ST, KI, EPI, EXTRA, false>(p, nullptr);
 }
 
-template <int MT, int GM, int PRO, int ST, int KI, int EPI, bool EXTRA>
+template <int MT, int GM, int NR, int PRO, int ST, int KI, int EPI, bool EXTRA>
 int launch_variant(const LinearArgs& a, const Plan& pl, int* status, cudaStream_t stream) {
     GemvPackedParams p;
     fill_params(a, pl, status, p);
-    auto kern = gemv_packed_kernel<MT, GM, PRO, ST, KI, EPI, EXTRA>;
+    auto kern = gemv_packed_kernel<MT, GM, NR, PRO, ST, KI, EPI, EXTRA>;
     const size_t ring = static_cast<size_t>(kWarps) * ST * kStagePitch + 128;
     const size_t smem = ring + (PRO == kProNorm ? fused_smem_bytes(a.K, a.G) : 0);
     const size_t most = ring + (PRO == kProNorm ? fused_smem_bytes(256 * KI, 4 * KI) : 0);
@@ -145,29 +153,29 @@ int launch_variant(const LinearArgs& a, const Plan& pl, int* status, cudaStream_
     return W8A8_OK;
 }
 
-template <int MT, int GM>
+template <int MT, int GM, int NR>
 int launch_pro(const LinearArgs& a, const Plan& pl, int* status, cudaStream_t s) {
     if constexpr (MT == 1) {
         if (pl.pro == kProNorm) {
-            if (a.K <= 2560) return launch_variant<1, GM, kProNorm, 2, 10, -1, false>(a, pl, status, s);
-            return launch_variant<1, GM, kProNorm, 2, 16, -1, false>(a, pl, status, s);
+            if (a.K <= 2560) return launch_variant<1, GM, 1, kProNorm, 2, 10, -1, false>(a, pl, status, s);
+            return launch_variant<1, GM, 1, kProNorm, 2, 16, -1, false>(a, pl, status, s);
         }
-        if (pl.pro == kProQuant) return launch_variant<1, GM, kProQuant, 3, 1, -1, false>(a, pl, status, s);
+        if (pl.pro == kProQuant) return launch_variant<1, GM, 1, kProQuant, 3, 1, -1, false>(a, pl, status, s);
     }
-    if (!plain_instance(a)) return launch_variant<MT, GM, kProCodes, 3, 1, -1, true>(a, pl, status, s);
+    if (!plain_instance(a)) return launch_variant<MT, GM, NR, kProCodes, 3, 1, -1, true>(a, pl, status, s);
     switch (a.epilogue) {
-        case W8A8_EPI_NONE: return launch_variant<MT, GM, kProCodes, 3, 1, W8A8_EPI_NONE, false>(a, pl, status, s);
-        case W8A8_EPI_SWIGLU: return launch_variant<MT, GM, kProCodes, 3, 1, W8A8_EPI_SWIGLU, false>(a, pl, status, s);
-        default: return launch_variant<MT, GM, kProCodes, 3, 1, W8A8_EPI_RESIDUAL, false>(a, pl, status, s);
+        case W8A8_EPI_NONE: return launch_variant<MT, GM, NR, kProCodes, 3, 1, W8A8_EPI_NONE, false>(a, pl, status, s);
+        case W8A8_EPI_SWIGLU: return launch_variant<MT, GM, NR, kProCodes, 3, 1, W8A8_EPI_SWIGLU, false>(a, pl, status, s);
+        default: return launch_variant<MT, GM, NR, kProCodes, 3, 1, W8A8_EPI_RESIDUAL, false>(a, pl, status, s);
     }
 }
 
-template <int MT>
+template <int MT, int NR>
 int launch_gm(const LinearArgs& a, const Plan& pl, int* status, cudaStream_t s) {
     switch (pl.GM) {
-        case 64: return launch_pro<MT, 64>(a, pl, status, s);
-        case 128: return launch_pro<MT, 128>(a, pl, status, s);
-        default: return launch_pro<MT, 256>(a, pl, status, s);
+        case 64: return launch_pro<MT, 64, NR>(a, pl, status, s);
+        case 128: return launch_pro<MT, 128, NR>(a, pl, status, s);
+        default: return launch_pro<MT, 256, NR>(a, pl, status, s);
     }
 }
 
@@ -244,11 +252,9 @@ bool gemv_packed_supports(const LinearArgs& a) {
 int launch_linear_gemv_packed(const LinearArgs& a, int* device_status, cudaStream_t s) {
     Plan pl;
     if (!make_plan(a, pl, false)) return fail(W8A8_ERR_UNSUPPORTED, "packed gemv kernel does not take this shape");
-    switch (pl.MT) {
-        case 1: return launch_gm<1>(a, pl, device_status, s);
-        case 2: return launch_gm<2>(a, pl, device_status, s);
-        default: return launch_gm<4>(a, pl, device_status, s);
-    }
+    if (pl.MT == 1) return launch_gm<1, 1>(a, pl, device_status, s);
+    if (pl.NR == 1) return pl.MT == 2 ? launch_gm<2, 1>(a, pl, device_status, s) : launch_gm<4, 1>(a, pl, device_status, s);
+    return pl.MT == 2 ? launch_gm<2, 2>(a, pl, device_status, s) : launch_gm<4, 2>(a, pl, device_status, s);
 }
 
 }  // namespace w8a8

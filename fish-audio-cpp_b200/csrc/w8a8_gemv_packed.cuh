@@ -49,9 +49,9 @@ enum { kProCodes = 0,   // int8 codes + fp32 scales made by an earlier launch (X
        kProNorm = 1,    // fp16 rows: every CTA does [x + residual] -> RMSNorm -> quantiser itself, in its prologue
        kProQuant = 2 }; // fp16 rows: a warp quantises the activations of each block it consumes, in registers
 
-// Forms of the kernel, by 8-token B tiles and group size class (reasons: see the consumer loop).
-constexpr bool in_place(int mt, int gm) { return mt == 4 || (mt == 2 && gm != 64); }
-constexpr bool two_per_sm(int mt, int gm) { return mt == 1 || (mt == 2 && gm != 64); }
+// Forms of the kernel, by 8-token B tiles, group size class and tiles at once (reasons: see the consumer loop).
+constexpr bool in_place(int mt, int gm, int nr) { return mt == 4 || (mt == 2 && gm != 64 && nr == 1); }
+constexpr bool two_per_sm(int mt, int gm, int nr) { return mt == 1 || (mt == 2 && gm != 64 && nr == 1); }
 
 struct GemvPackedParams {
     LinearArgs a;
@@ -79,6 +79,23 @@ __device__ __forceinline__ void mma_s8(int (&d)[4], uint32_t a0, uint32_t a1, ui
         : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
 }
 
+// The same onto zero: no registers to clear before it.
+__device__ __forceinline__ void mma_s8_first(int (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
+    asm volatile("mma.sync.aligned.m16n8k32.row.col.s32.s8.s8.s32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%10,%10,%10,%10};\n"
+                 : "=r"(d[0]), "=r"(d[1]), "=r"(d[2]), "=r"(d[3]) : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1), "r"(0));
+}
+__device__ __forceinline__ uint64_t pack2(float a, float b) {
+    return static_cast<uint64_t>(__float_as_uint(a)) | (static_cast<uint64_t>(__float_as_uint(b)) << 32);
+}
+// Two sums of one weight row: acc = fma(float(P) * ws, xs, acc), two at a time.
+__device__ __forceinline__ void promote2(float& acc0, float& acc1, int p0, int p1, uint64_t ws, uint64_t xs) {
+    uint64_t acc = pack2(acc0, acc1);
+    asm("{\n\t.reg .f32 lo, hi;\n\t.reg .b64 t;\n\tcvt.rn.f32.s32 lo, %1;\n\tcvt.rn.f32.s32 hi, %2;\n\tmov.b64 t, {lo, hi};\n\t"
+        "mul.rn.f32x2 t, t, %3;\n\tfma.rn.f32x2 %0, t, %4, %0;\n\t}" : "+l"(acc) : "r"(p0), "r"(p1), "l"(ws), "l"(xs));
+    acc0 = __uint_as_float(static_cast<uint32_t>(acc));
+    acc1 = __uint_as_float(static_cast<uint32_t>(acc >> 32));
+}
+
 __device__ __forceinline__ uint4 lds128(uint32_t addr) {
     uint4 v;
     asm volatile("ld.shared.v4.u32 {%0,%1,%2,%3}, [%4];\n" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(addr));
@@ -89,6 +106,24 @@ __device__ __forceinline__ uint32_t lds16(uint32_t addr) {
     uint16_t v;
     asm volatile("ld.shared.u16 %0, [%1];\n" : "=h"(v) : "r"(addr));
     return v;
+}
+
+// A row's scales of a block, one word.
+template <int N>
+__device__ __forceinline__ void lds_scales(uint32_t addr, __half (&s)[N]) {
+    if constexpr (N == 4) {
+        uint32_t v[2];
+        asm volatile("ld.shared.v2.u32 {%0, %1}, [%2];\n" : "=r"(v[0]), "=r"(v[1]) : "r"(addr));
+#pragma unroll
+        for (int i = 0; i < 4; ++i) s[i] = __ushort_as_half(static_cast<unsigned short>(v[i >> 1] >> (16 * (i & 1))));
+    } else if constexpr (N == 2) {
+        uint32_t v;
+        asm volatile("ld.shared.u32 %0, [%1];\n" : "=r"(v) : "r"(addr));
+        s[0] = __ushort_as_half(static_cast<unsigned short>(v));
+        s[1] = __ushort_as_half(static_cast<unsigned short>(v >> 16));
+    } else {
+        s[0] = __ushort_as_half(static_cast<unsigned short>(lds16(addr)));
+    }
 }
 
 __device__ __forceinline__ uint4 ld_cg16(const __half* p) {
@@ -330,6 +365,8 @@ __device__ __forceinline__ void tail_group_quant(const LinearArgs& a, int ct0, i
 // block are 64 activations of one token, the four lanes of a quad hold the block's 256 of that token: a group's absmax is a
 // few packed maxima and two shuffles, and the codes go from registers into the MMA. Every warp that meets a K block quantises
 // it again, some 300 instructions per block, so the form is chosen where a CTA has few row tiles (see quant_form_wins).
+// NR: row tiles that a warp takes through a K block together, so that the activations it reads, by then as many bytes as the weights, serve
+// both (1 or 2; more than eight rows). A CTA's last tile may be alone. Which launches take two: see make_plan.
 // ST: stages of a warp's ring (3; 2 for kProNorm so that two CTAs fit an SM beside the code rows).
 // KI: kProNorm only, the 16-byte pieces of a row a lane holds (K <= 256 * KI): 10 for the stack's K = 2560, else 16.
 // EXTRA: the call wants the group sums dumped, has a tail or sends to a tensor-parallel exchange. An instance of its own: the check
@@ -337,7 +374,7 @@ __device__ __forceinline__ void tail_group_quant(const LinearArgs& a, int ct0, i
 // EPI: the epilogue, or -1: the call's (one of three code paths is fetched past).
 // ROWS: the weights are the row-major matrix itself. A block is then a TMA box of 16 rows x two 128-byte K blocks (128-byte
 // swizzle), its scales come from the matrix's own scale array a unit ahead, and everything else is the same.
-template <int MT, int GM, int PRO, int ST, int KI, int EPI, bool EXTRA, bool ROWS>
+template <int MT, int GM, int NR, int PRO, int ST, int KI, int EPI, bool EXTRA, bool ROWS>
 __device__ __forceinline__ void gemv_body(const GemvPackedParams& p, const CUtensorMap* map) {
     constexpr bool FUSED = PRO == kProNorm, QUANT = PRO == kProQuant;
     const int epilogue = EPI >= 0 ? EPI : p.a.epilogue;
@@ -363,7 +400,7 @@ __device__ __forceinline__ void gemv_body(const GemvPackedParams& p, const CUten
 
     // ---- this warp's contiguous range of units; the eight ranges of a CTA are neighbours, so that most row
     // tiles cut by a range boundary are cut between warps of ONE CTA and can be added up in shared memory ----
-    __shared__ float red_s[kWarps][MT * 4 * 32];  // a warp's part of the tile its run begins in (slot 0)
+    __shared__ float red_s[kWarps][NR * MT * 4 * 32];  // a warp's part of the tile its run begins in (slot 0)
     __shared__ int cut_s[kWarps][3];  // per boundary between two warps' runs: the row tile it cuts (-1: none, or counted with
                                       // the boundary before it), the slot of its first contributor, its last contributor
     // Whole 16-row tiles per CTA (tile t of `tiles` goes to CTA t * C / tiles), the CTA's units in equal contiguous
@@ -371,14 +408,21 @@ __device__ __forceinline__ void gemv_body(const GemvPackedParams& p, const CUten
     // this CTA.
     const unsigned tiles = p.U / p.upt;
     const unsigned ct0 = blockIdx.x * tiles / gridDim.x, ct1 = (blockIdx.x + 1) * tiles / gridDim.x;
-    const unsigned cu0 = ct0 * p.upt, n_cta = (ct1 - ct0) * p.upt;
+    // NR = 2: a unit is two neighbouring tiles (the CTA's last one may be alone) x a unit of K, counted from the CTA's first.
+    const unsigned cu0 = NR == 1 ? ct0 * p.upt : 0, n_cta = (ct1 - ct0 + NR - 1) / NR * p.upt;
     const unsigned nw_cta = n_cta < kWarps ? n_cta : kWarps;
     unsigned u0 = cu0, u1 = cu0;
     if (static_cast<unsigned>(warp) < nw_cta) {
         u0 = cu0 + warp * n_cta / nw_cta;
         u1 = cu0 + (warp + 1) * n_cta / nw_cta;
     }
-    const int T = static_cast<int>(u1 - u0) * p.bpu;  // blocks
+    auto first_tile = [&](unsigned u) { return static_cast<int>(NR == 1 ? u / p.upt : ct0 + u / p.upt * NR); };  // of a unit
+    const int T = static_cast<int>(u1 - u0) * p.bpu;  // steps: a K block of the unit's tiles
+    int blocks = T;                                    // blocks of the run
+    if constexpr (NR == 2) {
+        const unsigned paired = (ct1 - ct0) / 2 * p.upt;  // units of two tiles, ahead of those of a lone last one
+        if (u0 < paired) blocks += static_cast<int>(min(u1, paired) - u0) * p.bpu;
+    }
     // The row tiles cut by run boundaries, worked out while nothing is waited for: a division costs a lone warp some forty
     // clocks, and this used to sit between a tile's last block and its store.
     if (threadIdx.x < kWarps) {
@@ -411,9 +455,11 @@ __device__ __forceinline__ void gemv_body(const GemvPackedParams& p, const CUten
 
     // producer (lane 0): the range is one contiguous run of blocks in the packed image, of boxes in the row-major matrix
     int pt = 0;
+    const int k_blocks = p.upt * p.bpu;
     const unsigned char* src = ROWS ? nullptr : p.packed + static_cast<size_t>(u0) * p.bpu * p.block_bytes;
-    int pkb = 0, prt = 0;  // ROWS: the next box's 128-byte K block and row tile
-    if constexpr (ROWS) { prt = static_cast<int>(u0 / p.upt); pkb = static_cast<int>(u0 % p.upt) * p.bpu * 2; }
+    int pkb = 0, prt = 0, pr = 0;  // ROWS, NR = 2: the next block's K block, its unit's first tile, which of the tiles
+    if constexpr (ROWS || NR == 2) { prt = first_tile(u0); pkb = static_cast<int>(u0 % p.upt) * p.bpu; }
+    if constexpr (!ROWS && NR == 2) src = p.packed + (static_cast<size_t>(prt) * k_blocks + pkb) * p.block_bytes;
     // Weights are read once per launch and a stack's do not fit in L2: as evict-first lines they do not push out the activations,
     // scales and cache rows that the next launches read, nor wait behind their write-back (decode step, batch 8: 1517 -> 1490 us;
     // ten fast-AR steps 1710 -> 1650). Marking a quarter of them evict-last, to find it again at the next step: 1502 and 1687.
@@ -425,21 +471,31 @@ __device__ __forceinline__ void gemv_body(const GemvPackedParams& p, const CUten
             ptx::mbar_arrive_expect_tx(&bar[slot], kBlockW);
             asm volatile(
                 "cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes.L2::cache_hint [%0], [%1, {%3, %4, %5}], [%2], %6;"
-                ::"r"(ring + slot * kPitch), "l"(map), "r"(ptx::smem_u32(&bar[slot])), "r"(0), "r"(pkb), "r"(prt * 16), "l"(once)
+                ::"r"(ring + slot * kPitch), "l"(map), "r"(ptx::smem_u32(&bar[slot])), "r"(0), "r"(pkb * 2), "r"((prt + pr) * 16), "l"(once)
                 : "memory");
-            pkb += 2;
-            if (pkb == p.upt * p.bpu * 2) { pkb = 0; ++prt; }
         } else {
             ptx::mbar_arrive_expect_tx(&bar[slot], p.block_bytes);
             asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes.L2::cache_hint [%0], [%1], %2, [%3], %4;"
-                         ::"r"(ring + slot * kPitch), "l"(src), "r"(p.block_bytes), "r"(ptx::smem_u32(&bar[slot])), "l"(once)
+                         ::"r"(ring + slot * kPitch), "l"(NR == 1 ? src : src + static_cast<size_t>(pr * k_blocks) * p.block_bytes),
+                         "r"(p.block_bytes), "r"(ptx::smem_u32(&bar[slot])), "l"(once)
                          : "memory");
-            src += p.block_bytes;
         }
         ++pt;
+        if constexpr (NR == 2) {
+            if (pr == 0 && prt + 1 < static_cast<int>(ct1)) { pr = 1; return; }
+            pr = 0;
+        }
+        if constexpr (!ROWS) src += p.block_bytes;
+        if constexpr (ROWS || NR == 2) {
+            if (++pkb == k_blocks) {  // (the image goes on with the next tile, which of two was taken along)
+                pkb = 0;
+                prt += NR;
+                if constexpr (!ROWS) src += static_cast<size_t>(k_blocks) * p.block_bytes;
+            }
+        }
     };
     if (lane == 0) {
-        const int pre = T < kStages ? T : kStages;
+        const int pre = blocks < kStages ? blocks : kStages;
         for (int i = 0; i < pre; ++i) issue();
     }
     // The blocks behind the ring's go to L2 meanwhile, one or two per warp: a linear of few rows meets its activations late, and the
@@ -459,24 +515,25 @@ __device__ __forceinline__ void gemv_body(const GemvPackedParams& p, const CUten
         __syncthreads();  // staged by all threads, read by each warp on its own after the wait
     }
     // ROWS: the scales of a lane's two rows of a unit, one aligned word each (K is a multiple of 256, so G of the unit's groups)
-    __align__(8) __half wsn[2][GPU];
+    __align__(8) __half wsn[NR][2][GPU];
     auto load_ws = [&](int tile, int unit) {
 #pragma unroll
-        for (int h = 0; h < 2; ++h) {
-            const __half* src_s = a.w_scale + static_cast<size_t>(min(tile * 16 + gr + 8 * h, a.N - 1)) * a.G + unit * GPU;
+        for (int i = 0; i < 2 * NR; ++i) {
+            const int h = i & 1;
+            const __half* src_s = a.w_scale + static_cast<size_t>(min(tile * 16 + gr + 8 * i, a.N - 1)) * a.G + unit * GPU;
             if constexpr (GPU == 4) {
                 const uint2 v = __ldg(reinterpret_cast<const uint2*>(src_s));
-                *reinterpret_cast<uint2*>(wsn[h]) = v;
+                *reinterpret_cast<uint2*>(wsn[i >> 1][h]) = v;
             } else if constexpr (GPU == 2) {
                 const uint32_t v = __ldg(reinterpret_cast<const uint32_t*>(src_s));
-                *reinterpret_cast<uint32_t*>(wsn[h]) = v;
+                *reinterpret_cast<uint32_t*>(wsn[i >> 1][h]) = v;
             } else {
-                wsn[h][0] = __ldg(src_s);
+                wsn[i >> 1][h][0] = __ldg(src_s);
             }
         }
     };
     if constexpr (ROWS) {
-        if (T > 0) load_ws(static_cast<int>(u0 / p.upt), static_cast<int>(u0 % p.upt));
+        if (T > 0) load_ws(first_tile(u0), static_cast<int>(u0 % p.upt));
     }
     // Everything above touches only weights. Let the next launch begin its own prologue, then wait
     // for the kernel before this one: it produces the activations.
@@ -659,12 +716,18 @@ __device__ __forceinline__ void gemv_body(const GemvPackedParams& p, const CUten
 
     // Two integer accumulators per tile: consecutive MMAs alternate between them, so that one MMA does
     // not wait for the previous one's result (with one warp per scheduler that latency is exposed).
-    int P[MT][4], Q[MT][4];
-    float acc[MT][4];
+    // One group per four MMAs at one token tile leaves the chain bare; with more token tiles their MMAs fill it and one accumulator
+    // does. The first MMA of a group starts from zero and two sums are promoted per instruction, except in the one-tile form
+    // of g = 64, where clearing and scalar promotes came out ahead (ten fast-AR steps and one slow, batch 8: 1527 us, else 1546; batch 1 step 1122 and 1130).
+    constexpr bool kTwoSums = GM != 64 || MT == 1, kPairs = GM != 64 || MT > 1;
+    int P[NR][MT][4], Q[NR][MT][4];
+    float acc[NR][MT][4];
 #pragma unroll
-    for (int nt = 0; nt < MT; ++nt)
+    for (int h = 0; h < NR; ++h)
 #pragma unroll
-        for (int r = 0; r < 4; ++r) { P[nt][r] = 0; Q[nt][r] = 0; acc[nt][r] = 0.0f; }
+        for (int nt = 0; nt < MT; ++nt)
+#pragma unroll
+            for (int r = 0; r < 4; ++r) { P[h][nt][r] = 0; Q[h][nt][r] = 0; acc[h][nt][r] = 0.0f; }
 
     // Stores a finished 16-row tile held in fragment layout: rows gr / gr+8, tokens 2c / 2c+1.
     auto store_tile = [&](int rt, const float (&v)[MT][4]) {
@@ -707,50 +770,64 @@ __device__ __forceinline__ void gemv_body(const GemvPackedParams& p, const CUten
     };
 
     // Slot 1, a warp's part of the tile its run ends in, lies in the warp's own ring: it is written after the run's last block.
-    static_assert(MT * 4 * 32 * sizeof(float) <= kRingBytes, "a partial tile fits a warp's ring");
+    static_assert(NR * MT * 4 * 32 * sizeof(float) <= kRingBytes, "partial tiles fit a warp's ring");
     float* const ring0 = reinterpret_cast<float*>(smem_raw + (ring - warp * kRingBytes - ptx::smem_u32(smem_raw)));
     auto slot1 = [&](int w) { return ring0 + w * (kRingBytes / 4); };
     // Called when the warp has added its last unit of row tile rt into acc. A tile that lies inside the warp's run is stored;
     // of a cut tile the fp32 partial goes to the warp's slot in shared memory (0: the tile its run begins in, 1: the tile it
     // ends in) and is added up when the whole CTA has streamed its blocks (below).
-    auto finish_tile = [&](int rt) {
-        const unsigned t_lo = static_cast<unsigned>(rt) * p.upt, t_hi = t_lo + p.upt;  // [t_lo, t_hi)
-        if ((u0 <= t_lo && t_hi <= u1) || W8A8_ABLATED(8)) {
-            store_tile(rt, acc);
-        } else {
-            float* mine = u0 < t_hi && u0 >= t_lo ? red_s[warp] : slot1(warp);
+    auto finish_tile = [&](int rt0) {  // rt0: the unit's first tile
+        const unsigned t_lo = (NR == 1 ? static_cast<unsigned>(rt0) : (static_cast<unsigned>(rt0) - ct0) / NR) * p.upt, t_hi = t_lo + p.upt;  // [t_lo, t_hi)
+        const bool whole = (u0 <= t_lo && t_hi <= u1) || W8A8_ABLATED(8);
+        float* mine = u0 < t_hi && u0 >= t_lo ? red_s[warp] : slot1(warp);
+#pragma unroll
+        for (int h = 0; h < NR; ++h) {
+            if (whole) {
+                const int rt = rt0 + h;
+                if (NR == 1 || rt < static_cast<int>(ct1)) store_tile(rt, acc[h]);
+            } else {
+#pragma unroll
+                for (int nt = 0; nt < MT; ++nt)
+#pragma unroll
+                    for (int r = 0; r < 4; ++r) mine[((h * MT + nt) * 4 + r) * 32 + lane] = acc[h][nt][r];
+            }
 #pragma unroll
             for (int nt = 0; nt < MT; ++nt)
 #pragma unroll
-                for (int r = 0; r < 4; ++r) mine[(nt * 4 + r) * 32 + lane] = acc[nt][r];
+                for (int r = 0; r < 4; ++r) acc[h][nt][r] = 0.0f;
         }
-#pragma unroll
-        for (int nt = 0; nt < MT; ++nt)
-#pragma unroll
-            for (int r = 0; r < 4; ++r) acc[nt][r] = 0.0f;
     };
 
-    auto promote = [&](int rt, int j, __half hsa, __half hsb, const float (&xsv)[MT][2]) {
+    auto promote = [&](int h, int rt, int j, __half hsa, __half hsb, const float (&xsv)[MT][2]) {
         const float fa = __half2float(hsa), fb = __half2float(hsb);
 #pragma unroll
         for (int nt = 0; nt < MT; ++nt) {
-            const float x0 = xsv[nt][0], x1 = xsv[nt][1];
+            if constexpr (kTwoSums) {
 #pragma unroll
-            for (int r = 0; r < 4; ++r) { P[nt][r] += Q[nt][r]; Q[nt][r] = 0; }
+                for (int r = 0; r < 4; ++r) P[h][nt][r] += Q[h][nt][r];
+            }
             if (EXTRA && a.dump) {
                 const int t0 = nt * 8 + 2 * c, rA = rt * 16 + gr;
                 const size_t NG = static_cast<size_t>(a.N) * a.G;
 #pragma unroll
                 for (int r = 0; r < 4; ++r) {
                     const int row = rA + 8 * (r >> 1), tok = t0 + (r & 1);
-                    if (row < a.N && tok < a.M) a.dump[tok * NG + static_cast<size_t>(row) * a.G + j] = P[nt][r];
+                    if (row < a.N && tok < a.M) a.dump[tok * NG + static_cast<size_t>(row) * a.G + j] = P[h][nt][r];
                 }
             }
-            acc[nt][0] = __fmaf_rn(__fmul_rn(static_cast<float>(P[nt][0]), fa), x0, acc[nt][0]);
-            acc[nt][1] = __fmaf_rn(__fmul_rn(static_cast<float>(P[nt][1]), fa), x1, acc[nt][1]);
-            acc[nt][2] = __fmaf_rn(__fmul_rn(static_cast<float>(P[nt][2]), fb), x0, acc[nt][2]);
-            acc[nt][3] = __fmaf_rn(__fmul_rn(static_cast<float>(P[nt][3]), fb), x1, acc[nt][3]);
-            P[nt][0] = P[nt][1] = P[nt][2] = P[nt][3] = 0;
+            if constexpr (kPairs) {
+                const uint64_t x2 = pack2(xsv[nt][0], xsv[nt][1]);
+                promote2(acc[h][nt][0], acc[h][nt][1], P[h][nt][0], P[h][nt][1], pack2(fa, fa), x2);
+                promote2(acc[h][nt][2], acc[h][nt][3], P[h][nt][2], P[h][nt][3], pack2(fb, fb), x2);
+            } else {
+#pragma unroll
+                for (int r = 0; r < 4; ++r)
+                    acc[h][nt][r] = __fmaf_rn(__fmul_rn(static_cast<float>(P[h][nt][r]), r < 2 ? fa : fb), xsv[nt][r & 1], acc[h][nt][r]);
+            }
+            if constexpr (GM == 256 || !kPairs) {
+#pragma unroll
+                for (int r = 0; r < 4; ++r) P[h][nt][r] = Q[h][nt][r] = 0;
+            }
         }
     };
 
@@ -762,9 +839,9 @@ __device__ __forceinline__ void gemv_body(const GemvPackedParams& p, const CUten
     // two CTAs share an SM (w2 at M = 16, g = 256: 11.3 -> 9.4 us; at g = 64 the second CTA gains less than the
     // later request costs; at M <= 8 two CTAs fit either way, and a run is often just two blocks long).
     int si = 0;
-    int ub = static_cast<int>(u0 % p.upt), rt = static_cast<int>(u0 / p.upt);
+    int ub = static_cast<int>(u0 % p.upt), rt0 = first_tile(u0), taken = 0;  // the unit's first tile; blocks consumed
     bool ok = true;
-    constexpr bool kInPlace = (in_place(MT, GM) && !FUSED) || QUANT;
+    constexpr bool kInPlace = (in_place(MT, GM, NR) && !FUSED) || QUANT;
     constexpr int NX = kInPlace ? 1 : 2;
     uint4 x[NX][4][MT];
     float xs[NX][GPU][MT][2];
@@ -867,7 +944,6 @@ __device__ __forceinline__ void gemv_body(const GemvPackedParams& p, const CUten
         load_xs_unit(ub, 0);
     }
     for (int t = 0; t < T; ++t) {
-        const int slot = t % kStages;
         // position of the next block (the same row tile or the next one: K restarts at 0)
         int nsi = si + 1, nub = ub;
         if (nsi == p.bpu) { nsi = 0; if (++nub == p.upt) nub = 0; }
@@ -881,77 +957,93 @@ __device__ __forceinline__ void gemv_body(const GemvPackedParams& p, const CUten
             for (int ch = 0; ch < 4; ++ch) load_x(nkb, ch, NX - 1);
             if (nsi == 0) load_xs_unit(nub, NX - 1);
         }
-        if (!ptx::mbar_wait_bounded(&bar[slot], (t / kStages) & 1)) {
-            if (lane == 0) atomicExch(p.status, 600 + slot);
-            ok = false;
-            break;
-        }
-        const uint32_t st = ring + slot * kPitch;
-        // this block's weight scales ride behind its weights: [16 rows][GPU] fp16 (ROWS: in registers since the unit before)
-        __half sa[GPU], sb[GPU];
+        __half sa[NR][GPU], sb[NR][GPU];
 #pragma unroll
-        for (int q = 0; q < GPU; ++q) {
+        for (int h = 0; h < NR; ++h) {
+            if (NR > 1 && h > 0 && rt0 + h >= static_cast<int>(ct1)) break;  // (a lone last tile)
+            const int rt = rt0 + h, nth = NR == 1 ? t : taken, slot = nth % kStages;
+            if (!ptx::mbar_wait_bounded(&bar[slot], (nth / kStages) & 1)) {
+                if (lane == 0) atomicExch(p.status, 600 + slot);
+                ok = false;
+                break;
+            }
+            if constexpr (NR > 1) ++taken;
+            const uint32_t st = ring + slot * kPitch;
+            // this block's weight scales ride behind its weights: [16 rows][GPU] fp16 (ROWS: in registers since the unit before)
             if constexpr (ROWS) {
-                sa[q] = wsn[0][q];
-                sb[q] = wsn[1][q];
-            } else {
-                sa[q] = __ushort_as_half(static_cast<unsigned short>(lds16(st + kBlockW + (gq * GPU + q) * 2)));
-                sb[q] = __ushort_as_half(static_cast<unsigned short>(lds16(st + kBlockW + ((gq + 8) * GPU + q) * 2)));
-            }
-        }
-        if constexpr (ROWS) {
-            if (nsi == 0 && t + 1 < T) load_ws(nub == 0 ? rt + 1 : rt, nub);
-        }
 #pragma unroll
-        for (int ch = 0; ch < 4; ++ch) {  // 64-byte K chunks
-            uint32_t fa, fb;
-            if constexpr (ROWS) {  // box lines are ordered [row][K block]; the 16-byte piece is XOR-ed with the line's low three bits
-                const uint32_t line = static_cast<uint32_t>(gr * 2 + (ch >> 1));
-                fa = st + line * 128 + ((static_cast<uint32_t>((ch & 1) * 4 + c) ^ (line & 7u)) << 4);
-                fb = fa + 16 * 128;
+                for (int q = 0; q < GPU; ++q) {
+                    sa[h][q] = wsn[h][0][q];
+                    sb[h][q] = wsn[h][1][q];
+                }
+                if (h == NR - 1 || rt + 1 >= static_cast<int>(ct1)) {
+                    if (nsi == 0 && t + 1 < T) load_ws(nub == 0 ? rt0 + NR : rt0, nub);
+                }
             } else {
-                fa = st + ch * 1024 + lane * 16;
-                fb = fa + 512;
+                lds_scales<GPU>(st + kBlockW + gq * GPU * 2, sa[h]);
+                lds_scales<GPU>(st + kBlockW + (gq + 8) * GPU * 2, sb[h]);
             }
-            const uint4 wa = lds128(fa), wb = lds128(fb);
 #pragma unroll
-            for (int nt = 0; nt < MT; ++nt) {
-                mma_s8(P[nt], wa.x, wb.x, wa.y, wb.y, x[0][ch][nt].x, x[0][ch][nt].y);
-                mma_s8(Q[nt], wa.z, wb.z, wa.w, wb.w, x[0][ch][nt].z, x[0][ch][nt].w);
+            for (int ch = 0; ch < 4; ++ch) {  // 64-byte K chunks
+                uint32_t fa, fb;
+                if constexpr (ROWS) {  // box lines are ordered [row][K block]; the 16-byte piece is XOR-ed with the line's low three bits
+                    const uint32_t line = static_cast<uint32_t>(gr * 2 + (ch >> 1));
+                    fa = st + line * 128 + ((static_cast<uint32_t>((ch & 1) * 4 + c) ^ (line & 7u)) << 4);
+                    fb = fa + 16 * 128;
+                } else {
+                    fa = st + ch * 1024 + lane * 16;
+                    fb = fa + 512;
+                }
+                const uint4 wa = lds128(fa), wb = lds128(fb);
+                const bool opens = kPairs && (GM == 64 || (GM == 128 && (ch & 1) == 0));  // a group
+#pragma unroll
+                for (int nt = 0; nt < MT; ++nt) {
+                    const uint4 xv = x[0][ch][nt];
+                    if (opens) mma_s8_first(P[h][nt], wa.x, wb.x, wa.y, wb.y, xv.x, xv.y);
+                    else mma_s8(P[h][nt], wa.x, wb.x, wa.y, wb.y, xv.x, xv.y);
+                }
+#pragma unroll
+                for (int nt = 0; nt < MT; ++nt) {
+                    const uint4 xv = x[0][ch][nt];
+                    if (!kTwoSums) mma_s8(P[h][nt], wa.z, wb.z, wa.w, wb.w, xv.z, xv.w);
+                    else if (opens) mma_s8_first(Q[h][nt], wa.z, wb.z, wa.w, wb.w, xv.z, xv.w);
+                    else mma_s8(Q[h][nt], wa.z, wb.z, wa.w, wb.w, xv.z, xv.w);
+                }
+                const bool last_use = h == NR - 1 || rt + 1 >= static_cast<int>(ct1);
+                if (kInPlace && !QUANT && last_use) load_x(nkb, ch, 0);  // (after the range's last block: a block of the same rows, read for nothing)
+                if (GM == 64) {
+                    promote(h, rt, ub * 4 + ch, sa[h][ch % GPU], sb[h][ch % GPU], xs[0][ch % GPU]);
+                    if (kInPlace && !QUANT && last_use) load_xs(nub, ch % GPU, 0);
+                }
+                if (GM == 128 && (ch & 1)) {
+                    promote(h, rt, ub * 2 + (ch >> 1), sa[h][(ch >> 1) % GPU], sb[h][(ch >> 1) % GPU], xs[0][(ch >> 1) % GPU]);
+                    if (kInPlace && !QUANT && last_use) load_xs(nub, (ch >> 1) % GPU, 0);
+                }
             }
-            if (kInPlace && !QUANT) load_x(nkb, ch, 0);  // (after the range's last block: a block of the same rows, read for nothing)
-            if (GM == 64) {
-                promote(rt, ub * 4 + ch, sa[ch % GPU], sb[ch % GPU], xs[0][ch % GPU]);
-                if (kInPlace && !QUANT) load_xs(nub, ch % GPU, 0);
+            // The block's bytes are in registers: the slot may be refilled.
+            __syncwarp();
+            // The fence orders the reads of the slot before the copy that overwrites it. Without it the compiler may sink the
+            // scales' loads down to their use in the promote, past the copy: it did in the M = 9..16 form (128 registers), and
+            // a group's promote then took the next block's scales now and then.
+            if (lane == 0 && pt < blocks) {
+                ptx::fence_proxy_async();
+                issue();
             }
-            if (GM == 128 && (ch & 1)) {
-                promote(rt, ub * 2 + (ch >> 1), sa[(ch >> 1) % GPU], sb[(ch >> 1) % GPU], xs[0][(ch >> 1) % GPU]);
-                if (kInPlace && !QUANT) load_xs(nub, (ch >> 1) % GPU, 0);
-            }
+            if (GM == 256 && NR > 1 && si + 1 == p.bpu) promote(h, rt, ub, sa[h][0], sb[h][0], xs[0][0]);
         }
-        // The block's bytes are in registers: the slot may be refilled.
-        __syncwarp();
-        // The fence orders the reads of the slot before the copy that overwrites it. Without it the compiler may sink the
-        // scales' loads down to their use in the promote, past the copy: it did in the M = 9..16 form (128 registers), and
-        // a group's promote then took the next block's scales now and then.
-        if (lane == 0 && pt < T) {
-            ptx::fence_proxy_async();
-            issue();
-        }
+        if (!ok) break;
 #ifdef W8A8_TAIL_TIMELINE
         if (t == 0) W8A8_STAMP(6);
 #endif
         if (++si == p.bpu) {
             si = 0;
-            if (GM == 256) {
-                promote(rt, ub, sa[0], sb[0], xs[0][0]);
-                if (kInPlace && !QUANT) load_xs(nub, 0, 0);
-            }
+            if (GM == 256 && NR == 1) promote(0, rt0, ub, sa[0][0], sb[0][0], xs[0][0]);
+            if (GM == 256 && kInPlace && !QUANT) load_xs(nub, 0, 0);
             // one call site for the tile end: the row tile is complete, or the range ends inside it
             ++ub;
             if (ub == p.upt || t + 1 == T) {
-                finish_tile(rt);
-                if (ub == p.upt) { ub = 0; ++rt; }
+                finish_tile(rt0);
+                if (ub == p.upt) { ub = 0; rt0 += NR; }
             }
             if (!kInPlace) {
 #pragma unroll
@@ -977,15 +1069,17 @@ __device__ __forceinline__ void gemv_body(const GemvPackedParams& p, const CUten
     // ---- cut tiles: all warps add the partials up, in ascending-K order, a token's pair of rows per item ----
     __syncthreads();
 #pragma unroll 1
-    for (int i = threadIdx.x; i < (kWarps - 1) * MT * 64; i += kThreads) {
-        const int w = i / (MT * 64), rt_cut = cut_s[w][0];
-        if (rt_cut < 0) continue;
-        const int f = i % (MT * 64), nt = f >> 6, e = (f >> 5) & 1, fl = f & 31, last = cut_s[w][2];
-        const float* src = (cut_s[w][1] ? slot1(w) : red_s[w]) + (nt * 4 + e) * 32 + fl;
+    for (int i = threadIdx.x; i < (kWarps - 1) * NR * MT * 64; i += kThreads) {
+        const int w = i / (NR * MT * 64), rg_cut = cut_s[w][0];
+        if (rg_cut < 0) continue;
+        const int f = i % (NR * MT * 64), hn = f >> 6, e = (f >> 5) & 1, fl = f & 31, last = cut_s[w][2];  // hn: tile x token tile
+        const int nt = hn % MT, rt_cut = NR == 1 ? rg_cut : static_cast<int>(ct0) + rg_cut * NR + hn / MT;
+        if (NR > 1 && rt_cut >= static_cast<int>(ct1)) continue;
+        const float* src = (cut_s[w][1] ? slot1(w) : red_s[w]) + (hn * 4 + e) * 32 + fl;
         float v[2] = {0.0f + src[0], 0.0f + src[64]};
 #pragma unroll 1
         for (int ww = w + 1; ww <= last; ++ww) {
-            const float* more = red_s[ww] + (nt * 4 + e) * 32 + fl;
+            const float* more = red_s[ww] + (hn * 4 + e) * 32 + fl;
             v[0] += more[0];
             v[1] += more[64];
         }
@@ -1040,7 +1134,7 @@ __device__ __forceinline__ void gemv_body(const GemvPackedParams& p, const CUten
 
 // How a linear is cut over CTAs and warps.
 struct Plan {
-    int MT, GM, upt, bpu, block_bytes, tiles, ctas, pro;
+    int MT, GM, NR, upt, bpu, block_bytes, tiles, ctas, pro;
     long long U;
 };
 bool make_plan(const LinearArgs& a, Plan& pl, bool rows);

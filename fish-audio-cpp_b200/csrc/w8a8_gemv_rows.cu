@@ -9,13 +9,13 @@ namespace w8a8 {
 namespace {
 using namespace gemv;
 
-template <int MT, int GM, int PRO, bool EXTRA>
-__global__ void __launch_bounds__(kThreads, two_per_sm(MT, GM) ? 2 : 1)
+template <int MT, int GM, int NR, int PRO, bool EXTRA>
+__global__ void __launch_bounds__(kThreads, two_per_sm(MT, GM, NR) ? 2 : 1)
 gemv_rows_kernel(const __grid_constant__ CUtensorMap map, const __grid_constant__ GemvPackedParams p) {
-    gemv_body<MT, GM, PRO, 3, 1, -1, EXTRA, true>(p, &map);
+    gemv_body<MT, GM, NR, PRO, 3, 1, -1, EXTRA, true>(p, &map);
 }
 
-template <int MT, int GM, int PRO, bool EXTRA>
+template <int MT, int GM, int NR, int PRO, bool EXTRA>
 int launch_variant(const LinearArgs& a, const Plan& pl, int* status, cudaStream_t stream) {
     CUtensorMap map;
     // W seen as [N rows][K/128 blocks][128 bytes]; one box = 16 rows x 2 blocks, 128-byte swizzle
@@ -24,7 +24,7 @@ int launch_variant(const LinearArgs& a, const Plan& pl, int* status, cudaStream_
     if (rc) return rc;
     GemvPackedParams p;
     fill_params(a, pl, status, p);
-    auto kern = gemv_rows_kernel<MT, GM, PRO, EXTRA>;
+    auto kern = gemv_rows_kernel<MT, GM, NR, PRO, EXTRA>;
     const size_t smem = static_cast<size_t>(kWarps) * 3 * kBlockW + 1024;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(pl.ctas, 1, 1);
@@ -42,14 +42,18 @@ int launch_variant(const LinearArgs& a, const Plan& pl, int* status, cudaStream_
     return W8A8_OK;
 }
 
+template <int GM, bool EXTRA>
+int launch_codes(const LinearArgs& a, const Plan& pl, int* status, cudaStream_t s) {
+    if (pl.MT == 1) return launch_variant<1, GM, 1, kProCodes, EXTRA>(a, pl, status, s);
+    if (pl.NR == 1)
+        return pl.MT == 2 ? launch_variant<2, GM, 1, kProCodes, EXTRA>(a, pl, status, s) : launch_variant<4, GM, 1, kProCodes, EXTRA>(a, pl, status, s);
+    return pl.MT == 2 ? launch_variant<2, GM, 2, kProCodes, EXTRA>(a, pl, status, s) : launch_variant<4, GM, 2, kProCodes, EXTRA>(a, pl, status, s);
+}
+
 template <int GM>
 int launch_gm(const LinearArgs& a, const Plan& pl, int* status, cudaStream_t s) {
-    if (pl.pro == kProQuant) return launch_variant<1, GM, kProQuant, false>(a, pl, status, s);
-    if (!plain_instance(a))
-        return pl.MT == 1 ? launch_variant<1, GM, kProCodes, true>(a, pl, status, s)
-               : pl.MT == 2 ? launch_variant<2, GM, kProCodes, true>(a, pl, status, s) : launch_variant<4, GM, kProCodes, true>(a, pl, status, s);
-    return pl.MT == 1 ? launch_variant<1, GM, kProCodes, false>(a, pl, status, s)
-           : pl.MT == 2 ? launch_variant<2, GM, kProCodes, false>(a, pl, status, s) : launch_variant<4, GM, kProCodes, false>(a, pl, status, s);
+    if (pl.pro == kProQuant) return launch_variant<1, GM, 1, kProQuant, false>(a, pl, status, s);
+    return plain_instance(a) ? launch_codes<GM, false>(a, pl, status, s) : launch_codes<GM, true>(a, pl, status, s);
 }
 
 }  // namespace

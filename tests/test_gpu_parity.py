@@ -1001,6 +1001,37 @@ def test_fused_swiglu_of_gates_that_round_to_zero(ctx, oracle, pkg):
         assert np.array_equal(dY.cpu().numpy().view(np.uint16), np.repeat(want.view(np.uint16)[:, None], 8, axis=1))
 
 
+@pytest.mark.parametrize("M,N,K,g", [(9, 2560, 9728, 64), (13, 5690, 5632, 128), (16, 5690, 5632, 64), (16, 2560, 9728, 256), (17, 5690, 5632, 64),
+                                     (25, 2560, 9728, 128), (32, 5690, 5632, 256), (16, 2400, 16896, 512), (31, 7168, 4096, 64)])
+def test_decode_linear_of_two_tiles_at_once(ctx, oracle, pkg, M, N, K, g):
+    """Long runs at more than eight rows go through a K block two row tiles at a time: CTAs of one, two and three tiles (a lone last one),
+    tiles and runs cut between warps, rows that end inside a tile, a group of two blocks; packed and row-major weights alike, and with
+    the group sums asked for."""
+    X, W, ws = synth.linear_case(M + N + K, M, N, K, g)
+    Xq, Xs = oracle.quantize(X, g)
+    dW, dS, dXq, dXs = dev(W), dev(ws), dev(Xq), dev(Xs)
+    P = torch.empty((ctx.packed_weight_bytes(N, K, g),), dtype=torch.uint8, device="cuda")
+    ctx.pack_weight(dW, dS, N, K, g, P)
+    ctx.register_packed_weight(dW, P, N, K, g)
+    try:
+        buf, dY = guarded((M, N), torch.float16, 99.0)
+        ctx.linear_q(dW, dS, g, dXq, dXs, dY, M, N, K, kernel=pkg.KERNEL_GEMV_PACKED)
+        dump = torch.full((M, N, K // g), -7, dtype=torch.int32, device="cuda")
+        again = torch.empty_like(dY)
+        ctx.linear_q(dW, dS, g, dXq, dXs, again, M, N, K, kernel=pkg.KERNEL_GEMV_PACKED, dump=dump)
+        buf_r, dR = guarded((M, N), torch.float16, 99.0)
+        ctx.linear_q(dW, dS, g, dXq, dXs, dR, M, N, K, kernel=pkg.KERNEL_GEMV_TMA)
+        torch.cuda.synchronize()
+        ctx.check_device_status()
+    finally:
+        ctx.register_packed_weight(dW, None)
+    assert guards_intact(buf, 99.0) and guards_intact(buf_r, 99.0)
+    assert torch.equal(dY.view(torch.int16), dR.view(torch.int16)) and torch.equal(dY.view(torch.int16), again.view(torch.int16))
+    sums = oracle.group_sums(W, Xq, g)
+    assert np.array_equal(dump.cpu().numpy(), sums)
+    assert_close_fp16(oracle, dY.cpu().numpy(), oracle.linear_q(W, ws, Xq, Xs, g), "two tiles at once", abs_terms=abs_term_sum(sums, ws, Xs))
+
+
 @pytest.mark.parametrize("packed", [True, False])
 @pytest.mark.parametrize("M,g", [(3, 64), (16, 64), (8, 128)])
 def test_decode_linear_scales_at_any_address(ctx, oracle, pkg, M, g, packed):
