@@ -89,7 +89,7 @@ constexpr int kBiasByte = 184, kBias = kBiasByte * kBiasByte * 32, kConstBytes =
 static_assert(kBias > 128 * 128 * 64 && kBias + 128 * 128 * 64 < (1 << 23) && kBias % (1 << 11) == 0 && (kBias >> 11) < (1 << 13),
               "sums above zero and below 2^23; 11 bits of a weight scale times the bias are exact in fp32");
 
-template <int BT, bool PAIR, int GM>
+template <int BT, bool PAIR, int GM, bool SPLIT>
 struct Config {
     static constexpr bool kBiased = GM == 64 && BT >= 96;  // (narrower tiles are a chain, and the MMA would lengthen it: 1.05)
     static constexpr int kRowsB = PAIR ? BT / 2 : BT;                 // token rows this CTA loads
@@ -101,8 +101,11 @@ struct Config {
     // back to back: 4096 x 19456 x 2560 g = 64, 256 wide 395 and now 387, 192 wide 429 and 421, g = 128, 256 wide 281 and 275; 2048 x 6144 x
     // 2560 g = 64, 96 wide 86.8 and 82.9; 150 x 19456 x 2560 g = 64, 32 wide 40.2 and 37.8. (Sixteen in two chunks of eight have room in every form; chunks
     // of sixteen in the narrower ones lose stages of operands for them: 613 x 2560 x 9728 g = 256, 64 wide 29.2 and 42.7.)
-    static constexpr int kScGroups = 8, kScRing = 2;
-    static constexpr int kScSlot = kScGroups * (BT + BR) * 4;         // activation scales [8][BT], weight scales [8][128]
+    // Narrow tiles at g = 256 take four at a time after all: they start when a chunk's scales are there, and a chunk of eight is most of a short K
+    // (us, eight and four: 64 wide, 33 x 9728 x 2560 8.19 and 8.05, 150 x 6144 x 2560 7.35 and 7.14; 32 wide, 100 x 19456 x 2560 18.1 and 17.9). Wider tiles at g = 256 lose
+    // by it, 192 and 256 wide up to 2 %.
+    static constexpr int kScGroups = GM == 256 && BT <= 64 ? 4 : 8, kScRing = 16 / kScGroups;
+    static constexpr int kScSlot = kScGroups * (BT + BR) * 4;         // activation scales [kScGroups][BT], weight scales [kScGroups][128]
     static constexpr int kScBytes = kScRing * kScSlot;
     static constexpr int kConst = kBiased ? kConstBytes : 0;
     static constexpr int kRoom = 226 * 1024 - 1024 - kOutBytes - kScBytes - kConst;
@@ -121,8 +124,9 @@ struct Config {
     // Registers per thread of the form that moves some: at launch, in warpgroup 0, in the others.
     static constexpr int kLaunchRegs = kParts == 2 ? 168 : 96, kLowRegs = kParts == 2 ? 40 : 56, kHighRegs = kParts == 2 ? 232 : 104;
     static_assert(128 * (kLaunchRegs - kLowRegs) >= kEpiWarps * 32 * (kHighRegs - kLaunchRegs), "setmaxnreg sums must balance");
-    // K-groups per unit (see above), the stages that a unit takes, units per turn of the epilogue's loop.
-    static constexpr int kUnit = GM == 64 ? (BT == 32 ? 8 : BT == 64 ? 4 : BT <= 128 ? 2 : 1) : GM == 128 ? (BT <= 64 ? 4 : BT <= 128 ? 2 : 1) : GM == 256 && BT <= 64 ? 2 : 1;
+    // K-groups per unit (see above), the stages that a unit takes, units per turn of the epilogue's loop. A split at g = 256 takes one: two pad a run of
+    // nineteen groups (33 x 2560 x 9728, 32 wide, two CTAs 11.08 us, with one 10.91).
+    static constexpr int kUnit = GM == 64 ? (BT == 32 ? 8 : BT == 64 ? 4 : BT <= 128 ? 2 : 1) : GM == 128 ? (BT <= 64 ? 4 : BT <= 128 ? 2 : 1) : GM == 256 && BT <= 64 && !SPLIT ? 2 : 1;
     static constexpr int kUnitKb = kUnit * GM > BK ? kUnit * GM / BK : 1;
     static constexpr int kUnroll = GM == 64 ? (BT >= 192 || BT == 32 ? 1 : BT == 64 ? 2 : 4) : GM == 128 ? (BT >= 192 || BT == 64 ? 1 : BT == 96 ? 4 : 2) : 1;
     // No more of them than a turn of the ring fills, so that the issuer knows each at compile time.
@@ -354,10 +358,10 @@ __device__ __forceinline__ void infinite_rows(const LinearArgs& a, const uint32_
 // ROWS_FIRST: which side of the tiles is walked first (see walk_rows_first). An instance of its own: chosen in the kernel, by a parameter, it
 // cost the pairs of 192 tokens at g = 64 up to 3 % wherever it was not taken (code placement: 4001 x 6144 x 2560 121.7 and 126.6 us).
 template <int BT, bool PAIR, int GM, bool SPLIT, bool ROWS_FIRST>
-__global__ void __launch_bounds__(Config<BT, PAIR, GM>::kThreads, 1)
+__global__ void __launch_bounds__(Config<BT, PAIR, GM, SPLIT>::kThreads, 1)
 gemm_i8_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_x,
                const __grid_constant__ CUtensorMap map_y, const GemmParams p) {
-    using C = Config<BT, PAIR, GM>;
+    using C = Config<BT, PAIR, GM, SPLIT>;
     constexpr int S = C::kStages, kEpiWarps = C::kEpiWarps, kEpiThreads = kEpiWarps * 32, kScGroups = C::kScGroups;
     extern __shared__ unsigned char smem_raw[];
     __shared__ __align__(8) uint64_t full_bar[S], empty_bar[S], acc_full[C::kSlots], acc_empty[C::kSlots], sc_full[C::kScRing], sc_empty[C::kScRing];
@@ -549,7 +553,7 @@ gemm_i8_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
                 if (code && leader) atomicExch(p.status, code);
             }
         } else {
-            // ---------------- scales, a chunk at a time: activation scales [8][BT], weight scales [8][128], fp32 ----------------
+            // ---------------- scales, a chunk at a time: activation scales [kScGroups][BT], weight scales [kScGroups][128], fp32 ----------------
             const int t64 = threadIdx.x - 64;
             constexpr float kScale = C::kBiased ? 0x1p111f : 1.0f;  // (see promote2)
             int slot = 0;
@@ -944,7 +948,7 @@ template <int BT, bool PAIR, int GM, bool SPLIT>
 inline FormState form_state[2];
 template <int BT, bool PAIR, int GM, bool SPLIT = false>
 Form form(float stage_ns, float group_ns, float tile_ns) {
-    using C = Config<BT, PAIR, GM>;
+    using C = Config<BT, PAIR, GM, SPLIT>;
     Kernel rows_first = nullptr;
     if constexpr (BT >= 128 && !SPLIT && GM != 0) rows_first = gemm_i8_kernel<BT, PAIR, GM, SPLIT, true>;  // (a long prompt's forms)
     return Form{BT, PAIR, SPLIT, {gemm_i8_kernel<BT, PAIR, GM, SPLIT, false>, rows_first}, C::kThreads, C::kSmem, C::kMoveRegs ? C::kLaunchRegs : 0,
