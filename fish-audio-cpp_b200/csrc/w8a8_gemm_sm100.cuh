@@ -91,7 +91,7 @@ static_assert(kBias > 128 * 128 * 64 && kBias + 128 * 128 * 64 < (1 << 23) && kB
 
 template <int BT, bool PAIR, int GM, bool SPLIT>
 struct Config {
-    static constexpr bool kBiased = GM == 64 && BT >= 96;  // (narrower tiles are a chain, and the MMA would lengthen it: 1.05)
+    static constexpr bool kBiased = GM == 64 && BT >= 64;  // (32 wide the MMA lengthens the chain: 2560 x 4096 13.3 and 14.8 us)
     static constexpr int kRowsB = PAIR ? BT / 2 : BT;                 // token rows this CTA loads
     static constexpr int kStageBytes = (BR + kRowsB) * BK;
     static constexpr int kPanelBytes = BT * 128;                      // BT tokens x 64 fp16 columns, 128-byte swizzle
@@ -139,6 +139,13 @@ struct Config {
     // The weight scales a chunk ahead (see the scales' warps): 256 wide, g = 64, 4096 x 19456 x 2560 380 us and 390 without; any group
     // size, 4096 x 19456 x 2560 with one group 267 and 273. Elsewhere it costs what it holds registers for: g = 64, 64 wide, 150 x 6144 x
     // 2560 12.2 and 11.4.
+    // A chunk's scales in reads of 16 or 8 bytes, and activation scales through registers. As reads of two bytes and copies of four, a lane a row, a chunk
+    // takes 1300 to 3000 cycles of the load unit, as long as the tile takes to compute it, and where rows of scales are a power of two
+    // apart (K = 4096) the lines that eight such reads share have left L1 between them. us before and after, g = 64: 150 x 2560 x 4096, 64 wide 18.3 and 13.6;
+    // 150 x 19456 x 2560, 96 wide 30.5 and 28.9; 613 x 2560 x 9728, 96 wide 37.7 and 33.4; 4001 x 2560 x 9728, 192 wide 205 and 194; g = 128 2048 x
+    // 2560 x 4096, 128 wide 40.8 and 37.5. The widest form: registers are short there (weight scales only, g = 128; at g = 64 a chunk ahead is better,
+    // 4096 x 19456 x 2560 403 us and 410). A split at g = 128 starts its runs off those boundaries; at g = 256, with few scales, 2560 x 9728 in narrow tiles lost 1 to 4 %.
+    static constexpr bool kWideScales = GM == 64 ? BT <= 192 : GM == 128 && !SPLIT, kWideX = kWideScales && BT <= 192;
     static constexpr bool kScalesAhead = GM == 0 || (GM == 64 && BT == 256);
     static constexpr int kBatch = GM == 64 && BT <= 64 ? 2 : 1;  // steps whose sums are requested together
     static constexpr int kTmemCols = kAcc * BT <= 128 ? 128 : kAcc * BT <= 256 ? 256 : 512;
@@ -575,6 +582,43 @@ gemm_i8_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
                 const int n0 = tile_n0(tile);
                 load_w(w_row(n0), w_row(n0 + 64), j0);
             };
+            // kWideScales: by 16 or 8 bytes where the address, the row's length and the run's start are multiples of that.
+            uint32_t wv[2][kScGroups / 2];
+            constexpr int XQ = BT == 32 ? kScGroups / 2 : kScGroups, XT = (BT + 63) / 64;  // activation scales per thread and token (32 tokens: half of them), tokens per thread
+            float xv[XT][XQ];
+            const int xt = BT == 32 ? t64 % 32 : t64, xq0 = BT == 32 ? t64 / 32 * XQ : 0;
+            const unsigned w_at = static_cast<unsigned>(reinterpret_cast<unsigned long long>(a.w_scale)) | (2u * G) | (2u * g_first);
+            const unsigned x_at = static_cast<unsigned>(reinterpret_cast<unsigned long long>(a.Xs)) | (4u * G) | (4u * g_first);
+            const bool w16 = (w_at & 15) == 0, w8 = (w_at & 7) == 0, x16 = C::kWideX && (x_at & 15) == 0;
+            auto load_wide = [&](const __half* ws0, const __half* ws1, int m0, int j0) {
+#pragma unroll
+                for (int h = 0; h < 2; ++h) {
+                    const __half* row = h ? ws1 : ws0;
+                    if (w16) {
+                        const uint4 v = *reinterpret_cast<const uint4*>(row + j0);
+                        wv[h][0] = v.x; wv[h][1] = v.y; wv[h][2] = v.z; wv[h][3] = v.w;
+                    } else if (w8) {
+                        const uint2 v = *reinterpret_cast<const uint2*>(row + j0), u = *reinterpret_cast<const uint2*>(row + min(j0 + 4, G - 4));
+                        wv[h][0] = v.x; wv[h][1] = v.y; wv[h][2] = u.x; wv[h][3] = u.y;
+                    } else {
+                        const unsigned short* r = reinterpret_cast<const unsigned short*>(row);
+#pragma unroll
+                        for (int i = 0; i < kScGroups / 2; ++i)
+                            wv[h][i] = r[min(j0 + 2 * i, G - 1)] | static_cast<uint32_t>(r[min(j0 + 2 * i + 1, G - 1)]) << 16;
+                    }
+                }
+                if (x16) {
+#pragma unroll
+                    for (int k = 0; k < XT; ++k) {
+                        const float* xs = a.Xs + static_cast<size_t>(min(m0 + xt + 64 * k, a.M - 1)) * G;
+#pragma unroll
+                        for (int i = 0; i < XQ; i += 4) {
+                            const float4 v = *reinterpret_cast<const float4*>(xs + min(j0 + xq0 + i, G - 4));
+                            xv[k][i] = v.x; xv[k][i + 1] = v.y; xv[k][i + 2] = v.z; xv[k][i + 3] = v.w;
+                        }
+                    }
+                }
+            };
             if constexpr (C::kScalesAhead) load_w_ahead(walker, g_first);
             int ith = 0;
             for (int tile = walker; tile < p.tiles_total && ok; tile += walkers, ++ith) {
@@ -591,14 +635,24 @@ gemm_i8_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
                 const __half* ws1 = w_row(n0 + 64);
                 for (int j0 = g_first; j0 < g_pad; j0 += kScGroups) {
                     const int nj = min(kScGroups, g_end - j0);
-                    if constexpr (!C::kScalesAhead) load_w(ws0, ws1, j0);  // on their way while the slot is waited for
+                    if constexpr (C::kWideScales) load_wide(ws0, ws1, m0, j0);
+                    else if constexpr (!C::kScalesAhead) load_w(ws0, ws1, j0);  // on their way while the slot is waited for
                     if (!wait(&sc_empty[slot], parity)) {
                         atomicExch(p.status, 600 + slot);
                         ok = false;
                         break;
                     }
                     const uint32_t dst = sc_ring + slot * C::kScSlot;
-                    for (int t = t64; t < BT; t += 64) {
+                    if (x16) {
+#pragma unroll
+                        for (int k = 0; k < XT; ++k) {
+                            if (BT % 64 != 0 && BT > 64 && xt + 64 * k >= BT) break;
+#pragma unroll
+                            for (int q = 0; q < XQ; ++q)
+                                asm volatile("st.shared.f32 [%0], %1;" ::"r"(dst + ((xq0 + q) * BT + xs_slot(xt + 64 * k)) * 4), "f"(xq0 + q < nj ? xv[k][q] : 0.0f) : "memory");
+                        }
+                    }
+                    for (int t = x16 ? BT : t64; t < BT; t += 64) {
                         const float* src = a.Xs + static_cast<size_t>(min(m0 + t, a.M - 1)) * G + j0;
 #pragma unroll
                         for (int q = 0; q < kScGroups; ++q) {
@@ -611,6 +665,10 @@ gemm_i8_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
 #pragma unroll
                     for (int q = 0; q < kScGroups; ++q) {
                         const bool real = C::kUnit == 1 || q < nj;
+                        if constexpr (C::kWideScales) {
+                            w[0][q] = __ushort_as_half(static_cast<unsigned short>(wv[0][q >> 1] >> (16 * (q & 1))));
+                            w[1][q] = __ushort_as_half(static_cast<unsigned short>(wv[1][q >> 1] >> (16 * (q & 1))));
+                        }
                         const float w0 = real ? __half2float(w[0][q]) : 0.0f, w1 = real ? __half2float(w[1][q]) : 0.0f;
                         if (C::kBiased && (isinf(w0) || isinf(w1))) infinite_s[ith % kMarks] = ith + 1;
                         asm volatile("st.shared.f32 [%0], %1;" ::"r"(dst + (kScGroups * BT + q * BR + ws_slot(t64)) * 4), "f"(w0 * kScale) : "memory");
@@ -957,8 +1015,8 @@ Form form(float stage_ns, float group_ns, float tile_ns) {
 template <int GM>
 const Form* all_forms(int* count) {
     // per stage at groups of 64, 128 and 256, and per tile, for token widths 32, 64, 96, 128, 192, 256
-    constexpr float kStage[3][6] = {{235, 380, 441, 563, 825, 1142}, {151, 245, 298, 339, 508, 670}, {141, 170, 286, 288, 321, 383}};
-    constexpr float kTile[3][6] = {{110, 260, 610, 920, 1930, 2590}, {440, 390, 720, 1150, 2220, 2550}, {290, 740, 90, 500, 2190, 2730}};
+    constexpr float kStage[3][6] = {{204, 309, 391, 499, 740, 1150}, {152, 207, 294, 321, 483, 665}, {141, 170, 286, 288, 321, 383}};
+    constexpr float kTile[3][6] = {{750, 580, 1150, 1550, 2670, 2830}, {110, 740, 900, 1310, 2820, 2460}, {290, 740, 90, 500, 2190, 2730}};
     constexpr int q = GM == 64 ? 0 : GM == 128 ? 1 : 2;
     static const Form table[] = {form<32, false, GM>(kStage[q][0], 0, kTile[q][0]),       form<64, false, GM>(kStage[q][1], 0, kTile[q][1]),
                                  form<96, false, GM>(kStage[q][2], 0, kTile[q][2]),       form<128, false, GM>(kStage[q][3], 0, kTile[q][3]),

@@ -778,6 +778,29 @@ def test_gemm_tcgen05_k_that_ends_inside_a_unit(gemm_form, oracle, pkg, K, g, bt
                           oracle.linear_q(np.ascontiguousarray(W[rows]), np.ascontiguousarray(ws[rows]), Xq, Xs, g).view(np.uint16))
 
 
+@pytest.mark.parametrize("K,g", [(2560, 64), (2304, 64), (2432, 64), (2560, 128), (2816, 128), (1152, 128), (1280, 256)])
+@pytest.mark.parametrize("bt", [32, 64, 96, 128, 192, 256])
+@pytest.mark.parametrize("off", [0, 1, 4])
+def test_gemm_tcgen05_scales_at_any_address(gemm_form, oracle, pkg, K, g, bt, off):
+    """Scales are read 16 or 8 bytes at a time where a row's address and length allow it: rows of 40, 36, 38, 20, 22, 9 and 5 groups, arrays
+    that begin on such a boundary, one scale and four scales behind it, ragged tokens and rows, and a last chunk that is not full.
+    Bit for bit the oracle's."""
+    M, N = 203, 300
+    ctx = gemm_form(bt, 1)
+    X, W, ws = synth.linear_case(K + bt + off, M, N, K, g)
+    Xq, Xs = oracle.quantize(X, g)
+    dS = torch.empty((N * (K // g) + off,), dtype=torch.float16, device="cuda")[off:].view(N, K // g)
+    dXs = torch.empty((M * (K // g) + off,), dtype=torch.float32, device="cuda")[off:].view(M, K // g)
+    dS.copy_(dev(ws))
+    dXs.copy_(dev(Xs))
+    buf, dY = guarded((M, N), torch.float16, 99.0)
+    ctx.linear_q(dev(W), dS, g, dev(Xq), dXs, dY, M, N, K)
+    torch.cuda.synchronize()
+    ctx.check_device_status()
+    assert guards_intact(buf, 99.0)
+    assert np.array_equal(dY.cpu().numpy().view(np.uint16), oracle.linear_q(W, ws, Xq, Xs, g).view(np.uint16))
+
+
 @pytest.mark.parametrize("g", [64, 128, 256])
 @pytest.mark.parametrize("splits", [2, 4])
 @pytest.mark.parametrize("bt", [32, 64, 96, 128])
