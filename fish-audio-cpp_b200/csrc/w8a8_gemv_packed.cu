@@ -101,7 +101,10 @@ bool gemv::make_plan(const LinearArgs& a, Plan& pl, bool rows) {
     // Decode step, batch 16: g = 64 1790 and 1733, g = 128 1662 and 1610.
     const int sms = device_sms();
     const int most = (pl.tiles + sms - 1) / sms * (a.K / 256);  // blocks of the CTA that holds most, a CTA per SM
-    pl.NR = pl.MT > 1 && most > 8 * kWarps && (pl.MT == 4 || pl.GM == 64 || a.M > 12) ? 2 : 1;
+    // g >= 256 at 9..16 rows fits an SM twice and promotes little: only the longest runs (M = 16 155776 x 2560 65.3 and 62.2; 20000 x 2560 12.6 and 12.5; the
+    // step at batch 16, context 200 1599 and 1613, at batch 14, context 900 1826 and 1842).
+    const bool two = pl.MT == 4 || pl.GM == 64 || (pl.GM == 128 ? a.M > 12 : most > 32 * kWarps);
+    pl.NR = pl.MT > 1 && most > 8 * kWarps && two ? 2 : 1;
     pl.ctas = gemv_packed_ctas(pl.tiles, sms, two_per_sm(pl.MT, pl.GM, pl.NR));
     if ((pl.U + 1) * static_cast<long long>(pl.ctas) * kWarps >= (1ll << 32)) return false;  // 32-bit range math
     return true;

@@ -1025,7 +1025,8 @@ def test_fused_swiglu_of_gates_that_round_to_zero(ctx, oracle, pkg):
 
 
 @pytest.mark.parametrize("M,N,K,g", [(9, 2560, 9728, 64), (13, 5690, 5632, 128), (16, 5690, 5632, 64), (16, 2560, 9728, 256), (17, 5690, 5632, 64),
-                                     (25, 2560, 9728, 128), (32, 5690, 5632, 256), (16, 2400, 16896, 512), (31, 7168, 4096, 64)])
+                                     (25, 2560, 9728, 128), (32, 5690, 5632, 256), (16, 2400, 16896, 512), (31, 7168, 4096, 64),
+                                     (16, 5690, 22528, 256), (13, 5690, 22528, 512)])
 def test_decode_linear_of_two_tiles_at_once(ctx, oracle, pkg, M, N, K, g):
     """Long runs at more than eight rows go through a K block two row tiles at a time: CTAs of one, two and three tiles (a lone last one),
     tiles and runs cut between warps, rows that end inside a tile, a group of two blocks; packed and row-major weights alike, and with
