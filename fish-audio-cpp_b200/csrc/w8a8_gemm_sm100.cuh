@@ -13,7 +13,7 @@
 //                row-major with K contiguous, i.e. already the K-major operand; TMA applies the 128-byte swizzle)
 //   warp 1       MMA issuer: four tcgen05.mma (K = 32) per stage; every K-group accumulates into its own BT-column slice
 //                of tensor memory (two to sixteen), starting with "overwrite" or, at g = 64, with a bias (below)
-//   warps 2, 3   stage the scales of eight K-groups at a time in a ring of their own
+//   warps 2, 3   stage the scales of eight (four) K-groups at a time in a ring of their own
 //   warps 4 ...  epilogue, eight to sixteen warps, each 32 weight rows x a part of the tokens. For every K-group
 //                acc = fma(float(P) * ws, xs, acc), groups ascending -- the arithmetic and order of
 //                accumulate_group_kernel (int8_gemm.cu:213-234) -- in fp32 registers, then the fp16 store
@@ -31,7 +31,7 @@
 // latency, and descriptors computed in divergent code are moved to uniform registers one by one): the tensor pipe ran at
 // 0.6 of its rate. Hence: the whole warp runs the loop and one elected lane issues; the loop is unrolled over the stages
 // so that stage, accumulator slice and descriptor offsets are immediates; group sizes 64 / 128 / 256 are template cases.
-// The promote is the other side, and the bound in most forms: stamps of the clock in an epilogue warp (which cost some 10 % themselves;
+// The promote is the other side, and the bound in most forms: stamps of the clock in an epilogue warp, taken before the units (they cost some 10 % themselves;
 // profiles/gemm_i8_kernel_epilogue_clock_stamps.md) show 1216, 1424 and 1451 clocks per K-group of a 128 x 256 tile at groups of 64, 128
 // and 256, of which 224-358 are waits for the MMAs, against 384 (with the bias), 512 and 1024 of MMAs. In trial programs of sixteen such
 // warps alone, clocks per warp and scheduler for two sums (the programs are not kept):
@@ -57,7 +57,7 @@
 // 0 to sums that are never -0. (700 x 2560 x 2816, g = 256, 64 wide: 11 groups as 12, 11.0 us and 11.7.)
 //
 // Measured back to back in turn, us, without the bias, the units, the 16-byte scale reads and the cheaper SwiGLU, and with them
-// (M x N x K; the long ones under the power cap):
+// (M x N x K; the long ones under the power cap; before units of more than two groups and wide reads of scales, for which see kUnit and kWideScales):
 //   8192 x 19456 x 2560, g = 64   967 -> 787 (844 -> 1037 TOPS); g = 128 617 -> 568; g = 256 447 -> 393 (1827 -> 2076 TOPS)
 //   2048 x  2560 x 9728, g = 64   154 -> 120;  613 x 2560 x 9728  52.8 -> 42.1;  150 x 19456 x 2560  52.6 -> 36.0
 //   4001 x  6144 x 2560, g = 128  95.2 -> 95.2; g = 256 66.9 -> 66.9 (no SwiGLU, pairs of 192 tokens)
