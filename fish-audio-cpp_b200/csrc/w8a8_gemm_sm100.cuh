@@ -990,8 +990,8 @@ struct FormState {
 // K, per K-group and for itself (the start of its chain, conversion, store). Fitted to 4100 times, no cost below zero, then moved by up
 // to 6 % each towards the choices that lose least: seven shapes (the four projections, 9728 x 2560, 4096 x 9728, 1000 x 1024) x 31 token
 // counts from 33 to 8192 x every form that takes them, for each group size. What it does not hold: a chip that is not full, and what
-// several sweeps over a long prompt's codes miss L2 for. Judged by its choice, the rule loses 0.5, 0.4 and 0.3 % against the best form on
-// average (groups of 64, 128, 256), and 0.8, 0.6 and 0.4 % over eight other shapes x eleven token counts.
+// several sweeps over a long prompt's codes miss L2 for. Judged by its choice, the rule loses 0.3, 0.4 and 0.4 % against the best form on
+// average (groups of 64, 128, 256), and 0.3, 0.4 and 0.5 % over eight other shapes x eleven token counts.
 struct Form {
     int bt;
     bool pair, split;
