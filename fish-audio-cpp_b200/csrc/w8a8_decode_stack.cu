@@ -982,8 +982,14 @@ Scratch layout(const w8a8_decode_stack& d, int S) {
     return sc;
 }
 
-int slices_for(const w8a8_decode_stack& d, int sms) {  // as the stand-alone attention launch has them
-    return attention_slices(d.batch * d.n_kv_heads, d.max_blocks_per_seq, sms);
+// Context slices per (sequence, kv head): as many as the CTAs, all resident here, have room for. The stand-alone launch takes fewer for
+// short contexts, for reasons that do not hold here: there is no ring that may hold a whole context (a warp keeps two blocks on their way),
+// no CTA starts later than another, and the merge is a phase of its own at any count. us of a layer, 2560 wide, with its count and with
+// this: context 350, batch 1 70.2 and 64.2, batch 4 71.8 and 67.7, batch 8 74.4 and 71.8. Not only powers of two: context 1937, batch 3 with
+// four 75.8 and with six 72.7, batch 5 with two 84.7 and with three 79.6. Nor may it follow the table's width, or the scratch of a step would.
+int slices_for(const w8a8_decode_stack& d, int sms) {
+    const int want = sms / (d.batch * d.n_kv_heads);
+    return want > 8 ? 8 : want > 1 ? want : 1;
 }
 
 const char* check(const w8a8_decode_stack& d) {

@@ -195,7 +195,8 @@ def test_fast_ar_frame_matches_oracle_chain(pkg, oracle):
 
 @pytest.mark.parametrize("group,dim,n_kv,inter,layers,B,context", [
     (256, 512, 1, 512, 2, 3, 37), (64, 1024, 2, 768, 3, 8, 100), (128, 2560, 8, 1024, 2, 8, 530), (256, 2560, 8, 9728, 2, 5, 1024),
-    (256, 2560, 8, 9728, 1, 8, 1024)])
+    (256, 2560, 8, 9728, 1, 8, 1024), (64, 1024, 8, 1024, 1, 3, 290),
+    (128, 1024, 8, 1024, 1, 4, 290)])
 def test_one_launch_step_matches_the_chain_of_launches(ctx, group, dim, n_kv, inter, layers, B, context):
     """w8a8_decode_stack_step (one persistent cooperative kernel) against decode_step (eight launches per
     layer) from the same state, two steps. Both run the same arithmetic; the one difference is how many CTAs

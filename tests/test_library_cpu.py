@@ -69,6 +69,24 @@ def test_null_context_is_rejected(pkg):
     assert lib.w8a8_destroy(None) == 0
 
 
+@pytest.mark.parametrize("n_kv", [1, 2, 8])
+@pytest.mark.parametrize("batch", [1, 2, 3, 5, 8])
+def test_one_launch_step_fills_the_gpu_whatever_the_tables_width(pkg, batch, n_kv):
+    """The one-launch step's scratch, and with it the number of context slices, is the same for a short block table as for a long one."""
+    from fish_audio_cpp_b200 import capi
+
+    lib = pkg.load_library()
+    d = capi.DecodeStack()
+    d.n_layers, d.batch, d.dim, d.n_q_heads, d.n_kv_heads, d.head_dim, d.inter, d.group_size = 2, batch, 512, 4 * n_kv, n_kv, 128, 512, 64
+    for f in ("layers", "final_norm", "rope_freqs", "positions", "seq_lens", "block_table", "k_cache", "v_cache", "x", "out"):
+        setattr(d, f, 1 << 20)  # (never read: the answer is arithmetic)
+    sizes = set()
+    for blocks in (1, 17, 25, 26, 44, 128, 2048):
+        d.max_blocks_per_seq = blocks
+        sizes.add(lib.w8a8_decode_stack_workspace_bytes(ctypes.byref(d)))
+    assert len(sizes) == 1 and sizes.pop() > 0
+
+
 def test_gemm_form_follows_what_is_asked_for(pkg):
     """The rule that picks the tcgen05 GEMM's form, on the host: a width or split that is asked for is taken or refused, never
     replaced; one CTA per tile and pairs keep to their widths."""
