@@ -24,6 +24,7 @@ from .capi import (  # noqa: F401
     TAIL_ROWNORM,
     Context,
     W8A8Error,
+    debug_attention_slices,
     debug_gemm_form,
     library_path,
     linear_static_scratch,

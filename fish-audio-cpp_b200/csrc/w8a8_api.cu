@@ -617,6 +617,11 @@ int w8a8_debug_gemm_form(int M, int N, int K, int group_size, int sms, int kerne
     return rc ? fail(rc, "no tile form of the tcgen05 GEMM for this shape") : W8A8_OK;
 }
 
+int w8a8_debug_attention_slices(int batch, int n_kv_heads, int max_blocks_per_seq, int sms, const int* room9) {
+    if (batch < 1 || n_kv_heads < 1 || max_blocks_per_seq < 0 || sms < 1 || !room9) return 0;
+    return attention_slices(batch, n_kv_heads, max_blocks_per_seq, sms, room9);
+}
+
 size_t w8a8_packed_weight_bytes(int N, int K, int group_size) { return packed_weight_bytes(N, K, group_size); }
 
 int w8a8_pack_weight(w8a8_ctx* ctx, const void* W, const void* w_scale, int N, int K, int group_size,

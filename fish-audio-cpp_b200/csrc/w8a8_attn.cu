@@ -663,25 +663,64 @@ int launch_qknorm_rope_kvwrite(const __half* qkv, const __half* q_norm_w, const 
     return W8A8_OK;
 }
 
-// Context slices per (sequence, kv head) pair, for the longest sequence the table can hold. us of a decode layer at 8 kv heads.
-// At most as many as run at once, a cluster's CTAs lying in one GPC: sixteen clusters of eight do not fit (36 blocks 40.8, with three 35.8), nor
-// 24 of six (40.5, with four 36.3) nor 48 of three (42.1, with two 37.7); 40 of three and 32 of four do.
-// One, as long as its ring holds the whole context: every further CTA starts later (it finds no SM that the projection ahead has
-// left free) and has a state to merge. 17 blocks, batch 1 34.1 with eight and 32.9 with one, batch 5 36.6 with two and 34.1, batch 8 37.4 and 36.4; 25 blocks,
-// batch 4 36.0 and 34.8; 30 blocks, batch 8, 37.7 with two and 38.2 with one.
-// Then a slice per twelve blocks: 45 blocks, batch 1 34.4 with eight and 34.0 with three, batch 2 39.9 and 35.9; 128 blocks, batch 2 41.2 with
-// eight, 38.3 with four and 37.6 with six, batch 5 45.9 with two and 41.8 with three. Two where three fit, and 72 CTAs in three, are worse than
-// their neighbours: batch 4, 45 blocks 37.2 with two, 36.5 with three; batch 3 37.2, 37.1 and, with four, 36.3.
-int attention_slices(int pairs, int blocks, int sms) {
-    const int most = pairs * 8 <= sms / 2 ? 8 : pairs * 6 <= sms * 2 / 3 ? 6 : pairs * 4 <= sms * 7 / 8 ? 4 : pairs * 3 <= sms * 5 / 6 ? 3 : pairs * 2 <= sms ? 2 : 1;
-    if (blocks <= kRing + 1 || most == 1) return 1;
-    const int want = blocks / 12 < most ? blocks / 12 : most;
-    if (want == 2 && most >= 3 && pairs > 8) return pairs * 3 >= 64 && pairs * 3 < 90 ? 4 : 3;
-    if (want == 3 && pairs * 3 >= 64 && pairs * 3 < 90) return 4;
-    return want >= 8 ? 8 : want >= 6 ? 6 : want >= 4 ? 4 : want;
+// Context slices per (sequence, kv head) pair: the count that costs least for the longest sequence the block table can hold (the host knows
+// the table's width, not the lengths: a wide table gets the slices of a long context). In 10 ns, fitted to a decode layer's time over 8, 4, 2
+// and 1 kv heads, batches of 1 to 16 and 8 to 128 blocks, by the choices it makes:
+//   15 a block of the slice           70 a round of its eight warps      300 if there is a second slice, whose state has to be merged
+//   38 a slice                        160 if not all CTAs find a free SM while the projection ahead, of 48 row tiles a kv head, still runs
+// Only counts whose clusters run at once, each in one GPC (room[S] of them): sixteen clusters of eight take two rounds (36 blocks 40.4 us, with three 35.8).
+// It loses 0.2, 0.3, 0.7 and 0.7 % of a layer against the best count at 8, 4, 2 and 1 kv heads, 4 % at most (table widths just past a
+// round). us a layer: 8 kv heads, 17 blocks, batch 1 34.3 with eight and 32.6 with one, batch 5 37.0 with two and 34.6; 45 blocks, batch 1 34.9 with
+// eight and 33.0 with three, batch 3 36.9 with three and 36.6 with four; 128 blocks, batch 5 46.0 with two and 41.8 with three; 2 kv heads,
+// batch 1, 25 blocks 24.7 with one and 23.4 with four.
+int attention_slices(int batch, int n_kv, int blocks, int sms, const int* room) {
+    const int pairs = batch * n_kv, free_sms = sms - 48 * n_kv > sms / 6 ? sms - 48 * n_kv : sms / 6;
+    int best = 1;
+    long best_cost = 0;
+    for (int S = 1; S <= kMaxSlices; ++S) {
+        if (S == 5 || S == 7 || (S > 1 && pairs > room[S])) continue;
+        const long mine = (blocks + S - 1) / S, rounds = (mine + kAttnWarps - 1) / kAttnWarps;
+        const long cost = 15 * mine + 70 * rounds + (S > 1 ? 300 : 0) + 38 * S + (pairs * S > free_sms ? 160 : 0);
+        if (S == 1 || cost < best_cost) { best = S; best_cost = cost; }
+    }
+    return best;
 }
 
 namespace {
+constexpr int kAttnSmem = kRing * kStageBytes + 1024;
+SmemAttribute attn_attribute[2];
+
+// Clusters of 2 .. 8 CTAs of the attention that the current device runs at once; asked for once per device.
+void cluster_room(int (&room)[kMaxSlices + 1]) {
+    static std::atomic<int> known[64][kMaxSlices + 1];  // plus one
+    int dev = 0;
+    const bool named = cudaGetDevice(&dev) == cudaSuccess && dev < 64;
+    for (int S = 2; S <= kMaxSlices; ++S) {
+        int n = named ? known[dev][S].load(std::memory_order_relaxed) - 1 : -1;
+        if (n < 0) {
+            cudaLaunchConfig_t cfg = {};
+            cfg.gridDim = dim3(S, 1, 1);
+            cfg.blockDim = dim3(kAttnThreads, 1, 1);
+            cfg.dynamicSmemBytes = kAttnSmem;
+            cudaLaunchAttribute attr[1];
+            attr[0].id = cudaLaunchAttributeClusterDimension;
+            attr[0].val.clusterDim.x = S;
+            attr[0].val.clusterDim.y = 1;
+            attr[0].val.clusterDim.z = 1;
+            cfg.attrs = attr;
+            cfg.numAttrs = 1;
+            if (attn_attribute[1](reinterpret_cast<const void*>(paged_attention_decode_kernel<true>), kAttnSmem) != cudaSuccess ||
+                cudaOccupancyMaxActiveClusters(&n, paged_attention_decode_kernel<true>, &cfg) != cudaSuccess) {
+                cudaGetLastError();
+                n = 0;
+            } else if (named) {
+                known[dev][S].store(n + 1, std::memory_order_relaxed);
+            }
+        }
+        room[S] = n;
+    }
+}
+
 int launch_attention(const AttnParams& base, int B, int splits, cudaStream_t stream);
 }
 
@@ -722,7 +761,11 @@ int launch_attention(const AttnParams& base, int B, int splits, cudaStream_t str
         return fail(W8A8_ERR_UNSUPPORTED, "paged attention here handles 4 query heads per kv head (got %d / %d)", n_q, n_kv);
     if (Xq && (g <= 0 || (kQPerKv * kHeadDim) % g != 0))
         return fail(W8A8_ERR_UNSUPPORTED, "fused output quantisation needs a group size dividing 512 (got %d)", g);
-    if (splits <= 0) splits = attention_slices(B * n_kv, base.max_blocks, device_sms());
+    if (splits <= 0) {
+        int room[kMaxSlices + 1];
+        cluster_room(room);
+        splits = attention_slices(B, n_kv, base.max_blocks, device_sms(), room);
+    }
     if (splits > kMaxSlices) splits = kMaxSlices;
     AttnParams p = base;
     p.S = splits;
@@ -733,11 +776,10 @@ int launch_attention(const AttnParams& base, int B, int splits, cudaStream_t str
     if (rc) return rc;
     rc = make_tensor_map_2d_u8(&map_v, p.v_cache, kHeadDim * 2, uint64_t(1) << 30, kHeadDim * 2, 128, kBlockTokens, 1);
     if (rc) return rc;
-    const size_t smem = static_cast<size_t>(kRing) * kStageBytes + 1024;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(splits, n_kv, B);
     cfg.blockDim = dim3(kAttnThreads, 1, 1);
-    cfg.dynamicSmemBytes = smem;
+    cfg.dynamicSmemBytes = kAttnSmem;
     cfg.stream = stream;
     cudaLaunchAttribute attr[2];
     attr[0].id = cudaLaunchAttributeClusterDimension;
@@ -748,10 +790,8 @@ int launch_attention(const AttnParams& base, int B, int splits, cudaStream_t str
     attr[1].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
     cfg.numAttrs = pdl_enabled(kPdlAttn) ? 2 : 1;
-    static SmemAttribute attribute[2];
-    const int most = static_cast<int>(smem);
-    const cudaError_t e = p.qkv ? launch_with_smem(attribute[1], most, cfg, paged_attention_decode_kernel<true>, map_k, map_v, p)
-                                : launch_with_smem(attribute[0], most, cfg, paged_attention_decode_kernel<false>, map_k, map_v, p);
+    const cudaError_t e = p.qkv ? launch_with_smem(attn_attribute[1], kAttnSmem, cfg, paged_attention_decode_kernel<true>, map_k, map_v, p)
+                                : launch_with_smem(attn_attribute[0], kAttnSmem, cfg, paged_attention_decode_kernel<false>, map_k, map_v, p);
     if (e != cudaSuccess) return fail(W8A8_ERR_CUDA, "paged_attention_decode launch: %s", cudaGetErrorString(e));
     return W8A8_OK;
 }

@@ -145,7 +145,6 @@ int launch_linear_gemv_rows(const LinearArgs& a, int* device_status, cudaStream_
 // w8a8_gemv_packed.cu : M <= 32 over pre-packed weights (linear byte stream, 1-D bulk copies).
 size_t packed_weight_bytes(int N, int K, int g);
 int launch_pack_weight(const int8_t* W, const __half* S, int N, int K, int g, void* out, cudaStream_t s);
-int attention_slices(int pairs, int max_blocks, int sms);  // CTAs that share a (sequence, kv head) pair's context
 int gemv_packed_ctas(int tiles, int sms, bool two_per_sm);  // CTAs that share a linear's row tiles
 bool gemv_packed_supports(const LinearArgs& a);  // also answers for the prologue and tail forms (fields of a set)
 bool quant_form_wins(const LinearArgs& a);       // whether fp16 rows (X set, Xq null) should be quantised inside the linear
@@ -159,6 +158,8 @@ int launch_paged_attention_decode(const __half* q, const __half* k_cache, const 
                                   const int* block_table, const int* seq_lens, int B, int n_q, int n_kv,
                                   int max_blocks, float sm_scale, int layer, int n_layers, __half* out, int g,
                                   int8_t* Xq, float* Xs, int splits, int* status, cudaStream_t stream);
+// CTAs that share a (sequence, kv head) pair's context; room[S]: clusters of S that run at once, S = 2 .. 8.
+int attention_slices(int batch, int n_kv, int max_blocks, int sms, const int* room);
 int launch_qkv_attention_decode(const __half* qkv, const __half* q_norm_w, const __half* k_norm_w, float eps,
                                 const float* freqs, const int* positions, __half* k_cache, __half* v_cache,
                                 const int* block_table, const int* seq_lens, int B, int n_q, int n_kv, int max_blocks,

@@ -98,7 +98,7 @@ def test_paged_attention_decode(ctx, oracle, B, lens, splits):
 
 
 # One to eight slices as the launch chooses them (the table's width and the batch decide), the longest sequence filling the table.
-@pytest.mark.parametrize("B,max_blocks", [(8, 25), (1, 26), (8, 26), (1, 44), (5, 45), (3, 40), (4, 128), (2, 128), (1, 128), (10, 128)])
+@pytest.mark.parametrize("B,max_blocks", [(8, 25), (1, 26), (8, 26), (1, 44), (5, 45), (3, 40), (4, 128), (2, 128), (1, 128), (10, 128), (8, 60)])
 def test_paged_attention_decode_with_chosen_slices(ctx, oracle, B, max_blocks):
     rng = np.random.default_rng(B + max_blocks)
     layer = 1

@@ -87,6 +87,27 @@ def test_one_launch_step_fills_the_gpu_whatever_the_tables_width(pkg, batch, n_k
     assert len(sizes) == 1 and sizes.pop() > 0
 
 
+ROOM_148 = {2: 74, 3: 45, 4: 33, 5: 26, 6: 22, 7: 15, 8: 15}  # what the occupancy query answers on 148 SMs
+
+
+@pytest.mark.parametrize("sms,room", [(148, ROOM_148), (132, {2: 66, 3: 40, 4: 28, 6: 18, 8: 14}), (148, {})])
+def test_attention_slices_run_at_once(pkg, sms, room):
+    """More slices than one only where all their clusters run at once, for any batch, kv heads and table width; one for the shortest tables."""
+    for n_kv in (1, 2, 4, 8):
+        for batch in range(1, 33):
+            for blocks in (0, 1, 8, 17, 25, 26, 36, 45, 60, 96, 128, 2048):
+                s = pkg.debug_attention_slices(batch, n_kv, blocks, sms, room)
+                assert s == 1 or batch * n_kv <= room.get(s, 0), (batch, n_kv, blocks, s)
+                assert s == 1 or blocks > 8
+
+
+@pytest.mark.parametrize("batch,n_kv,blocks,want", [(8, 8, 25, 1), (1, 8, 45, 3), (5, 8, 45, 3), (3, 8, 60, 4), (2, 8, 128, 6), (1, 8, 128, 8),
+                                                    (12, 1, 128, 8), (8, 8, 128, 2), (10, 8, 128, 1), (1, 2, 25, 4)])
+def test_attention_slices_that_were_measured_fastest(pkg, batch, n_kv, blocks, want):
+    """Within 1 % of a decode layer of the fastest count."""
+    assert pkg.debug_attention_slices(batch, n_kv, blocks, 148, ROOM_148) == want
+
+
 def test_gemm_form_follows_what_is_asked_for(pkg):
     """The rule that picks the tcgen05 GEMM's form, on the host: a width or split that is asked for is taken or refused, never
     replaced; one CTA per tile and pairs keep to their widths."""
