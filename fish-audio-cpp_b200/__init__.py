@@ -26,6 +26,7 @@ from .capi import (  # noqa: F401
     W8A8Error,
     debug_attention_slices,
     debug_gemm_form,
+    debug_gemv_form,
     library_path,
     linear_static_scratch,
     load_library,

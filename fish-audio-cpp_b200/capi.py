@@ -91,6 +91,7 @@ def load_library() -> C.CDLL:
         "w8a8_debug_tail_counters": (I, [P, P, I, P]),
         "w8a8_debug_force_gemm_form": (I, [P, I, I]),
         "w8a8_debug_gemm_form": (I, [I, I, I, I, I, I, I, I, I, P]),
+        "w8a8_debug_gemv_form": (I, [I, I, I, I, I, I, P]),
         "w8a8_debug_attention_slices": (I, [I, I, I, I, P]),
         "w8a8_pack_gate_up": (I, [P, P, P, P, P, I, I, I, P, P, P]),
         "w8a8_decode_stack_workspace_bytes": (Z, [C.POINTER(DecodeStack)]),
@@ -128,7 +129,7 @@ EXPORTS = [
     "w8a8_ctx_workspace_bytes", "w8a8_check_device_status", "w8a8_quantize", "w8a8_rms_norm",
     "w8a8_rmsnorm_quantize", "w8a8_silu", "w8a8_mul", "w8a8_residual_add", "w8a8_linear", "w8a8_linear_q",
     "w8a8_rmsnorm_linear", "w8a8_linear_q_tail", "w8a8_debug_tail_counters", "w8a8_debug_force_gemm_form", "w8a8_debug_gemm_form",
-    "w8a8_debug_attention_slices",
+    "w8a8_debug_attention_slices", "w8a8_debug_gemv_form",
     "w8a8_decode_stack_workspace_bytes", "w8a8_decode_stack_step",
     "w8a8_decode_stack_timeline",
     "w8a8_pack_gate_up", "w8a8_qknorm_rope_kvwrite", "w8a8_paged_attention_decode", "w8a8_qkv_attention_decode",
@@ -221,6 +222,13 @@ def debug_gemm_form(M, N, K, group_size, sms=148, kernel=KERNEL_GEMM, token_widt
     """(tokens per tile, CTAs per tile's rows, CTAs along its K) of the tcgen05 GEMM, or None where no form takes the shape."""
     out = (C.c_int * 3)()
     rc = load_library().w8a8_debug_gemm_form(M, N, K, group_size, sms, kernel, token_width, splits, int(moved_registers), out)
+    return None if rc else tuple(out)
+
+
+def debug_gemv_form(M, N, K, group_size, sms=148, kernel=KERNEL_GEMV_PACKED):
+    """(token rows, row tiles at once, CTAs) of the decode linear, or None where it does not take the shape."""
+    out = (C.c_int * 3)()
+    rc = load_library().w8a8_debug_gemv_form(M, N, K, group_size, sms, kernel, out)
     return None if rc else tuple(out)
 
 

@@ -617,6 +617,12 @@ int w8a8_debug_gemm_form(int M, int N, int K, int group_size, int sms, int kerne
     return rc ? fail(rc, "no tile form of the tcgen05 GEMM for this shape") : W8A8_OK;
 }
 
+int w8a8_debug_gemv_form(int M, int N, int K, int group_size, int sms, int kernel, int* form_out3) {
+    if (!form_out3 || (kernel != W8A8_KERNEL_GEMV_PACKED && kernel != W8A8_KERNEL_GEMV_TMA)) return fail(W8A8_ERR_INVALID_ARG, "debug_gemv_form: bad arguments");
+    const int rc = gemv_form(M, N, K, norm_group(K, group_size), sms, kernel == W8A8_KERNEL_GEMV_PACKED, form_out3);
+    return rc ? fail(rc, "the decode linear does not take this shape") : W8A8_OK;
+}
+
 int w8a8_debug_attention_slices(int batch, int n_kv_heads, int max_blocks_per_seq, int sms, const int* room9) {
     if (batch < 1 || n_kv_heads < 1 || max_blocks_per_seq < 0 || sms < 1 || !room9) return 0;
     return attention_slices(batch, n_kv_heads, max_blocks_per_seq, sms, room9);

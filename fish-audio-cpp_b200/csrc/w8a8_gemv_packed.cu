@@ -28,7 +28,7 @@ size_t fused_smem_bytes(int K, int G) {  // norm weight + padded code rows + sca
 
 }  // namespace
 
-bool gemv::make_plan(const LinearArgs& a, Plan& pl, bool rows) {
+bool gemv::make_plan(const LinearArgs& a, Plan& pl, bool rows, int sms) {
     const bool fused = a.norm_weight != nullptr, quant = !fused && a.X && !a.Xq;
     if (a.M < 1 || a.M > 32) return false;
     if (rows) {  // TMA wants W 16-byte aligned; the scales of a unit are read as one word; whole-row prologues are the packed form's
@@ -94,17 +94,25 @@ bool gemv::make_plan(const LinearArgs& a, Plan& pl, bool rows) {
     pl.tiles = (a.N + 15) / 16;
     pl.U = static_cast<long long>(pl.tiles) * pl.upt;
     // Up to two CTAs per SM where their registers and shared memory fit twice, never more CTAs than row tiles.
-    // Two row tiles at once where the CTA that holds most has more than eight blocks per warp: half the reads of activations, twice the code,
-    // which runs cold, and a longer first step. us, one tile and two: M = 16, g = 64 2560 x 9728 12.6 and 10.5, 20000 x 2560 15.2 and 13.3,
-    // 155776 x 2560 82 and 65; g = 128 11.2 and 9.9, 14.5 and 12.8, 72 and 64; M = 32, g = 64 12000 x 9728 45.5 and 40.0, g = 256 155776 x 2560 98 and 76; but
-    // 6144 x 2560 at M = 32 11.1 and 12.3, and at g >= 128 and M = 9, where the other form fits an SM twice, 2560 x 9728 9.4 and 9.7.
-    // Decode step, batch 16: g = 64 1790 and 1733, g = 128 1662 and 1610.
-    const int sms = device_sms();
-    const int most = (pl.tiles + sms - 1) / sms * (a.K / 256);  // blocks of the CTA that holds most, a CTA per SM
+    // Two row tiles at once where the CTA that holds most has two at least and more than eight blocks per warp: half the reads of activations,
+    // twice the code, which runs cold, and a longer first step. us, one tile and two: M = 16, g = 64 2560 x 9728 10.7 and 9.1, 19456 x 2560
+    // 12.8 and 11.7, 155776 x 2560 77 and 64; g = 128 9728 x 11008 28.0 and 23.8; M = 32, g = 256 155776 x 2560 98 and 76 (with its quantiser); but
+    // 6144 x 2560 at M = 32 11.1 and 12.3, at g >= 128 and M = 9, where the other form fits an SM twice, 2560 x 9728 9.4 and 9.7, and where no CTA
+    // has two tiles, M = 32, g = 64 2048 x 16640, 13.0 and 17.4. Decode step, batch 16: g = 64 1790 and 1733, g = 128 1662 and 1610.
+    // A lone last tile counts in the split over the warps as two do (its steps cost little less), so an odd number of tiles streams as long as
+    // the next even one: M = 32, g = 64 6144 x 9728, three tiles, 21.5 and 23.6, row-major 21.9 and 26.2; M = 19, 19456 x 9728, nine, 50.1 and 54.2.
+    // Dealing blocks out evenly instead is faster there but slower at M = 16 (19456 x 2560 11.5 and 12.2). So odd numbers only from where one
+    // tile more is little against the gain, earlier while a run is short of what memory gives: M = 16, g = 64 9728 x 4096, five, 12.0 and 11.5, but
+    // 9728 x 9728 21.1 and 21.3, row-major 22.6 and 23.3; M = 16, g = 256 9728 x 22784, five, 49.8 and 45.1.
+    // (Packed and row-major weights take the same, so that they give the same bits; row-major alone, M > 16 at g = 128 would be better off with one tile:
+    // 2560 x 9728 15.3 and 15.8, 8448 x 9728 24.9 and 27.0; packed 13.7 and 13.6, 22.1 and 22.4.)
+    const int held = (pl.tiles + sms - 1) / sms, most = held * (a.K / 256);  // row tiles and blocks of the CTA that holds most, a CTA per SM
+    const bool short_run = most <= 20 * kWarps;
+    const int odd_from = pl.MT == 2 ? (pl.GM > 64 ? 3 : short_run ? 5 : 9) : pl.GM == 256 && short_run ? 9 : 15;
     // g >= 256 at 9..16 rows fits an SM twice and promotes little: only the longest runs (M = 16 155776 x 2560 65.3 and 62.2; 20000 x 2560 12.6 and 12.5; the
     // step at batch 16, context 200 1599 and 1613, at batch 14, context 900 1826 and 1842).
     const bool two = pl.MT == 4 || pl.GM == 64 || (pl.GM == 128 ? a.M > 12 : most > 32 * kWarps);
-    pl.NR = pl.MT > 1 && most > 8 * kWarps && two ? 2 : 1;
+    pl.NR = pl.MT > 1 && most > 8 * kWarps && two && held >= 2 && (held % 2 == 0 || held >= odd_from) ? 2 : 1;
     pl.ctas = gemv_packed_ctas(pl.tiles, sms, two_per_sm(pl.MT, pl.GM, pl.NR));
     if ((pl.U + 1) * static_cast<long long>(pl.ctas) * kWarps >= (1ll << 32)) return false;  // 32-bit range math
     return true;
@@ -249,12 +257,29 @@ bool quant_form_wins(const LinearArgs& a) {
 
 bool gemv_packed_supports(const LinearArgs& a) {
     Plan pl;
-    return make_plan(a, pl, false);
+    return make_plan(a, pl, false, device_sms());
+}
+
+int gemv_form(int M, int N, int K, int g, int sms, bool packed, int* out3) {
+    alignas(16) static const unsigned char there[16] = {};  // (never read)
+    LinearArgs a = {};
+    a.M = M; a.N = N; a.K = K; a.g = g; a.G = num_groups(K, g);
+    a.Xq = a.W = reinterpret_cast<const int8_t*>(there);
+    a.Xs = reinterpret_cast<const float*>(there);
+    a.w_scale = reinterpret_cast<const __half*>(there);
+    a.packed = there;
+    a.Y = reinterpret_cast<__half*>(const_cast<unsigned char*>(there));
+    Plan pl;
+    if (N < 1 || K < 1 || sms < 1 || !make_plan(a, pl, !packed, sms)) return W8A8_ERR_UNSUPPORTED;
+    out3[0] = 8 * pl.MT;
+    out3[1] = pl.NR;
+    out3[2] = pl.ctas;
+    return W8A8_OK;
 }
 
 int launch_linear_gemv_packed(const LinearArgs& a, int* device_status, cudaStream_t s) {
     Plan pl;
-    if (!make_plan(a, pl, false)) return fail(W8A8_ERR_UNSUPPORTED, "packed gemv kernel does not take this shape");
+    if (!make_plan(a, pl, false, device_sms())) return fail(W8A8_ERR_UNSUPPORTED, "packed gemv kernel does not take this shape");
     if (pl.MT == 1) return launch_gm<1, 1>(a, pl, device_status, s);
     if (pl.NR == 1) return pl.MT == 2 ? launch_gm<2, 1>(a, pl, device_status, s) : launch_gm<4, 1>(a, pl, device_status, s);
     return pl.MT == 2 ? launch_gm<2, 2>(a, pl, device_status, s) : launch_gm<4, 2>(a, pl, device_status, s);

@@ -1137,7 +1137,7 @@ struct Plan {
     int MT, GM, NR, upt, bpu, block_bytes, tiles, ctas, pro;
     long long U;
 };
-bool make_plan(const LinearArgs& a, Plan& pl, bool rows);
+bool make_plan(const LinearArgs& a, Plan& pl, bool rows, int sms);
 // The plain instances read the activation scales of a unit as one word; a call whose scales are not aligned for that runs EXTRA.
 inline bool plain_instance(const LinearArgs& a) {
     return !a.dump && a.tail_kind == kTailNone && a.tp.world == 0 && (reinterpret_cast<uintptr_t>(a.Xs) & (a.g == 64 ? 15u : a.g == 128 ? 7u : 3u)) == 0;

@@ -60,12 +60,12 @@ int launch_gm(const LinearArgs& a, const Plan& pl, int* status, cudaStream_t s) 
 
 bool gemv_rows_supports(const LinearArgs& a) {
     Plan pl;
-    return make_plan(a, pl, true);
+    return make_plan(a, pl, true, device_sms());
 }
 
 int launch_linear_gemv_rows(const LinearArgs& a, int* device_status, cudaStream_t s) {
     Plan pl;
-    if (!make_plan(a, pl, true)) return fail(W8A8_ERR_UNSUPPORTED, "TMA gemv kernel does not take this shape");
+    if (!make_plan(a, pl, true, device_sms())) return fail(W8A8_ERR_UNSUPPORTED, "TMA gemv kernel does not take this shape");
     switch (pl.GM) {
         case 64: return launch_gm<64>(a, pl, device_status, s);
         case 128: return launch_gm<128>(a, pl, device_status, s);

@@ -146,6 +146,7 @@ int launch_linear_gemv_rows(const LinearArgs& a, int* device_status, cudaStream_
 size_t packed_weight_bytes(int N, int K, int g);
 int launch_pack_weight(const int8_t* W, const __half* S, int N, int K, int g, void* out, cudaStream_t s);
 int gemv_packed_ctas(int tiles, int sms, bool two_per_sm);  // CTAs that share a linear's row tiles
+int gemv_form(int M, int N, int K, int g, int sms, bool packed, int* out3);  // {tokens per warp, row tiles at once, CTAs}, or not supported
 bool gemv_packed_supports(const LinearArgs& a);  // also answers for the prologue and tail forms (fields of a set)
 bool quant_form_wins(const LinearArgs& a);       // whether fp16 rows (X set, Xq null) should be quantised inside the linear
 int launch_linear_gemv_packed(const LinearArgs& a, int* device_status, cudaStream_t s);

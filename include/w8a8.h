@@ -214,6 +214,9 @@ W8A8_API int w8a8_debug_force_gemm_form(w8a8_ctx* ctx, int token_width, int spli
 W8A8_API int w8a8_debug_gemm_form(int M, int N, int K, int group_size, int sms, int kernel, int token_width, int splits,
                                   int moved_registers, int* form_out3);
 
+/* Diagnostic, host only: how the decode linear over quantised activations (W8A8_KERNEL_GEMV_PACKED, or _GEMV_TMA over the row-major matrix) goes
+ * through a weight on a GPU of `sms` SMs: {token rows it is compiled for (8, 16 or 32), row tiles that a warp takes at once, CTAs}. */
+W8A8_API int w8a8_debug_gemv_form(int M, int N, int K, int group_size, int sms, int kernel, int* form_out3);
 /* Diagnostic, host only: the context slices that the paged attention takes where the caller asks for none, on a GPU of `sms` SMs that runs
  * room9[S] clusters of S CTAs of it at once (S = 2 .. 8; entries 0 and 1 are not read). 0: bad arguments. */
 W8A8_API int w8a8_debug_attention_slices(int batch, int n_kv_heads, int max_blocks_per_seq, int sms, const int* room9);

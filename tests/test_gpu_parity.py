@@ -1024,13 +1024,19 @@ def test_fused_swiglu_of_gates_that_round_to_zero(ctx, oracle, pkg):
         assert np.array_equal(dY.cpu().numpy().view(np.uint16), np.repeat(want.view(np.uint16)[:, None], 8, axis=1))
 
 
-@pytest.mark.parametrize("M,N,K,g", [(9, 2560, 9728, 64), (13, 5690, 5632, 128), (16, 5690, 5632, 64), (16, 2560, 9728, 256), (17, 5690, 5632, 64),
-                                     (25, 2560, 9728, 128), (32, 5690, 5632, 256), (16, 2400, 16896, 512), (31, 7168, 4096, 64),
-                                     (16, 5690, 22528, 256), (13, 5690, 22528, 512)])
-def test_decode_linear_of_two_tiles_at_once(ctx, oracle, pkg, M, N, K, g):
-    """Long runs at more than eight rows go through a K block two row tiles at a time: CTAs of one, two and three tiles (a lone last one),
-    tiles and runs cut between warps, rows that end inside a tile, a group of two blocks; packed and row-major weights alike, and with
-    the group sums asked for."""
+@pytest.mark.parametrize("M,N,K,g,tiles", [
+    (9, 2560, 9728, 64, 2), (13, 5690, 5632, 128, 2), (16, 5690, 5632, 64, 1), (16, 2560, 9728, 256, 1), (17, 5690, 5632, 64, 1),
+    (25, 2560, 9728, 128, 2), (32, 5690, 5632, 256, 1), (16, 2400, 16896, 512, 1), (31, 7168, 4096, 64, 1),
+    (16, 5690, 22528, 256, 2), (13, 5690, 22528, 512, 2),
+    (16, 19000, 2048, 64, 2), (16, 2400, 33024, 256, 2), (13, 2391, 33280, 512, 2), (17, 7197, 4352, 64, 2), (31, 7200, 4352, 256, 2),
+    (32, 7200, 4608, 512, 2), (25, 33168, 1280, 128, 2)])
+def test_decode_linear_of_two_tiles_at_once(ctx, oracle, pkg, M, N, K, g, tiles):
+    """Long runs at more than eight rows go through a K block two row tiles at a time: CTAs of one, two, three, eight and nine tiles (a lone last
+    one), tiles and runs cut between warps, rows that end inside a tile, a group of two blocks; packed and row-major weights alike, and with
+    the group sums asked for. tiles: row tiles at once on 148 SMs; shapes beside the rule's edges keep to one."""
+    if torch.cuda.get_device_properties(0).multi_processor_count == 148:
+        for kernel in (pkg.KERNEL_GEMV_PACKED, pkg.KERNEL_GEMV_TMA):
+            assert pkg.debug_gemv_form(M, N, K, g, kernel=kernel)[1] == tiles
     X, W, ws = synth.linear_case(M + N + K, M, N, K, g)
     Xq, Xs = oracle.quantize(X, g)
     dW, dS, dXq, dXs = dev(W), dev(ws), dev(Xq), dev(Xs)
@@ -1054,6 +1060,47 @@ def test_decode_linear_of_two_tiles_at_once(ctx, oracle, pkg, M, N, K, g):
     sums = oracle.group_sums(W, Xq, g)
     assert np.array_equal(dump.cpu().numpy(), sums)
     assert_close_fp16(oracle, dY.cpu().numpy(), oracle.linear_q(W, ws, Xq, Xs, g), "two tiles at once", abs_terms=abs_term_sum(sums, ws, Xs))
+
+
+@pytest.mark.parametrize("M,N,K,g", [(16, 2560, 9728, 64), (13, 4752, 5632, 128), (16, 2400, 33024, 256), (20, 2560, 9728, 64), (32, 7200, 4352, 256),
+                                     (25, 2416, 9728, 128)])
+@pytest.mark.parametrize("kernel_name", ["KERNEL_GEMV_PACKED", "KERNEL_GEMV_TMA"])
+def test_epilogues_of_two_tiles_at_once(ctx, pkg, kernel_name, M, N, K, g):
+    """SwiGLU and residual add in the form that takes two row tiles at once: the bits of its plain output put through the separate kernels
+    (silu, mul; a residual add). Whole, cut and lone last tiles."""
+    kernel = getattr(pkg, kernel_name)
+    if torch.cuda.get_device_properties(0).multi_processor_count == 148:
+        assert pkg.debug_gemv_form(M, N, K, g, kernel=kernel)[1] == 2
+    gen = torch.Generator(device="cuda").manual_seed(M + K)
+    W = torch.randint(-127, 128, (N, K), dtype=torch.int8, device="cuda", generator=gen)
+    ws = torch.empty((N, K // g), device="cuda").uniform_(1e-3, 5e-3, generator=gen).half()
+    Xq = torch.randint(-127, 128, (M, K), dtype=torch.int8, device="cuda", generator=gen)
+    Xs = torch.empty((M, K // g), device="cuda").uniform_(1e-4, 1e-3, generator=gen)  # (outputs of order one: gates that matter)
+    R = torch.randn((M, N), device="cuda", generator=gen).half()
+    P = torch.empty((ctx.packed_weight_bytes(N, K, g),), dtype=torch.uint8, device="cuda")
+    ctx.pack_weight(W, ws, N, K, g, P)
+    ctx.register_packed_weight(W, P, N, K, g)
+    try:
+        plain = torch.empty((M, N), dtype=torch.float16, device="cuda")
+        buf, dR = guarded((M, N), torch.float16, 99.0)
+        buf_a, dA = guarded((M, N // 2), torch.float16, 99.0)
+        ctx.linear_q(W, ws, g, Xq, Xs, plain, M, N, K, kernel=kernel)
+        ctx.linear_q(W, ws, g, Xq, Xs, dR, M, N, K, kernel=kernel, epilogue=pkg.EPI_RESIDUAL, residual=R)
+        ctx.linear_q(W, ws, g, Xq, Xs, dA, M, N, K, kernel=kernel, epilogue=pkg.EPI_SWIGLU)
+        blocks = plain.view(M, N // 16, 2, 8)
+        gate, up = blocks[:, :, 0].reshape(M, N // 2).contiguous(), blocks[:, :, 1].reshape(M, N // 2).contiguous()
+        ctx.silu(gate, M * N // 2)
+        ctx.mul(gate, up, M * N // 2)
+        added = R.clone()
+        ctx.residual_add(added, plain, M * N)
+        torch.cuda.synchronize()
+        ctx.check_device_status()
+    finally:
+        ctx.register_packed_weight(W, None)
+    assert guards_intact(buf, 99.0) and guards_intact(buf_a, 99.0)
+    assert torch.isfinite(plain).all() and (plain.float().abs() > 0.1).any()
+    assert torch.equal(dR.view(torch.int16), added.view(torch.int16))
+    assert torch.equal(dA.view(torch.int16), gate.view(torch.int16))
 
 
 @pytest.mark.parametrize("packed", [True, False])

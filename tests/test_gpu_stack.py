@@ -46,11 +46,12 @@ def oracle_step(oracle, st, x_in, k_cache, v_cache, bt, positions, jitter=None):
     return oracle.rms_norm(x, cpu(st.final_norm), c.eps)
 
 
-@pytest.mark.parametrize("group,dim,qk_norm,context", [(64, 512, True, 37), (256, 512, True, 37), (256, 1024, True, 37),
-                                                        (64, 1024, False, 3)])  # the last: the fast AR's form
-def test_stack_matches_oracle_chain(ctx, oracle, group, dim, qk_norm, context):
-    cfg = S.SlowARConfig(n_layer=2, dim=dim, n_head=4, n_kv=1, inter=512, group=group, qk_norm=qk_norm)
-    B = 3
+# the fourth: the fast AR's form; the last: a full batch, w1|w3 and w2 two row tiles at once
+@pytest.mark.parametrize("group,dim,qk_norm,context,B,inter", [(64, 512, True, 37, 3, 512), (256, 512, True, 37, 3, 512),
+                                                               (256, 1024, True, 37, 3, 512), (64, 1024, False, 3, 3, 512),
+                                                               (64, 2560, True, 37, 16, 9728)])
+def test_stack_matches_oracle_chain(ctx, oracle, group, dim, qk_norm, context, B, inter):
+    cfg = S.SlowARConfig(n_layer=2 if dim < 2560 else 1, dim=dim, n_head=4, n_kv=1, inter=inter, group=group, qk_norm=qk_norm)
     st = S.SlowARStack(torch, ctx, cfg, B, context, max_new=8, seed=5)
     rng = np.random.default_rng(group)
     x_in = rng.standard_normal((B, cfg.dim)).astype(np.float16)

@@ -108,6 +108,25 @@ def test_attention_slices_that_were_measured_fastest(pkg, batch, n_kv, blocks, w
     assert pkg.debug_attention_slices(batch, n_kv, blocks, 148, ROOM_148) == want
 
 
+@pytest.mark.parametrize("M,N,K,g,tiles", [
+    (16, 2560, 9728, 64, 2), (16, 19456, 2560, 64, 2), (32, 2560, 9728, 64, 2), (16, 9728, 8704, 128, 2), (32, 155776, 2560, 256, 2),
+    (16, 9728, 4096, 64, 2), (16, 9728, 22784, 256, 2), (29, 19456, 4096, 256, 2),
+    (32, 2048, 16640, 64, 1), (16, 2290, 22784, 64, 1),   # no CTA has two tiles to share activations
+    (32, 6144, 9728, 64, 1), (29, 6144, 14848, 64, 1), (20, 9728, 9728, 256, 1), (16, 9728, 9728, 64, 1),  # a lone third, fifth tile
+    (19, 19456, 9728, 64, 1), (18, 19456, 2560, 128, 1),  # a lone ninth, more than 16 rows
+    (16, 6144, 2560, 64, 1), (8, 2560, 9728, 64, 1), (12, 2560, 9728, 128, 1), (16, 2560, 9728, 256, 1)])
+def test_decode_linear_takes_two_tiles_only_where_that_is_faster(pkg, M, N, K, g, tiles):
+    """Packed and row-major weights alike, so that they give the same bits."""
+    for kernel in (pkg.KERNEL_GEMV_PACKED, pkg.KERNEL_GEMV_TMA):
+        form = pkg.debug_gemv_form(M, N, K, g, kernel=kernel)
+        assert form[:2] == (8 if M <= 8 else 16 if M <= 16 else 32, tiles)
+
+
+def test_decode_linear_form_refuses_what_the_kernels_refuse(pkg):
+    assert pkg.debug_gemv_form(33, 2560, 2560, 64) is None and pkg.debug_gemv_form(8, 2560, 2432, 64) is None
+    assert pkg.debug_gemv_form(8, 2560, 2560, 96) is None and pkg.debug_gemv_form(0, 2560, 2560, 64) is None
+
+
 def test_gemm_form_follows_what_is_asked_for(pkg):
     """The rule that picks the tcgen05 GEMM's form, on the host: a width or split that is asked for is taken or refused, never
     replaced; one CTA per tile and pairs keep to their widths."""
