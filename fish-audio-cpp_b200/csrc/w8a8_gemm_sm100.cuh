@@ -117,6 +117,11 @@ struct Config {
     // 192 wide, 4001 x 2560 x 9728: four 124.6, three 130, two 136. g = 256, 256 wide, 4096 x 19456 x 2560: two 160, four 165; 128 wide, 2048 x
     // 6144 x 2560: two, in steps of 32, 35.4, four 36.7.
     static constexpr int kParts = GM == 64 ? (BT == 192 ? 4 : BT == 96 ? 3 : 2) : GM == 128 ? (BT >= 192 ? 4 : 2) : GM == 256 ? (BT == 192 ? 4 : 2) : 4;
+    // With two parts at 128 and 256 tokens a thread stores twice as much as with four: all reads of a residual tile at once, and rows that leave element
+    // by element eight or sixteen tokens at a time. us, one read after another and now: g = 256, 256 wide 5299 x 1836 x 9728 with a residual
+    // 247 and 124, 7730 x 9728 x 1280 with a residual 155 and 137, 7071 x 7721 x 9984 615 and 562; g = 128, 128 wide 943 x 19456 x 896 with a
+    // residual 47.8 and 41.9. (The narrower tiles as they are: unrolled, they lose more by code placement than that store is.)
+    static constexpr bool kFewStore = kParts == 2 && BT >= 128 && GM >= 128;
     static constexpr int kStep = (GM == 64 && BT == 256) || (GM >= 128 && BT == 128) ? 32 : 16;  // tokens per step of the promote
     static constexpr int kEpiWarps = 4 * kParts, kThreads = 128 + kEpiWarps * 32;
     // The widest tile needs more registers in its epilogue warps than all threads can have: warpgroup 0 gives some up.
@@ -918,10 +923,10 @@ gemm_i8_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
                 if (p.tma_store) {  // residual: 16-byte pieces, sixteen threads per token row
                     const int piece = et & 15, rt = et >> 4;
                     if (piece * 8 < width) {
-                        // Up to four rows at a time: their reads are memory latencies, one after the other eight to a tile of 256
-                        // tokens. (All of them at once, or four in the forms for any group size, spill registers in the loop above.)
+                        // Several rows at a time: their reads are memory latencies. (All of them at once with four parts, or four in the forms
+                        // for any group size, spill registers in the loop above.)
                         constexpr int kRowStep = kEpiThreads / 16;
-                        constexpr int kRows = GM == 0 ? 2 : BT % (4 * kRowStep) == 0 ? 4 : BT % (3 * kRowStep) == 0 ? 3 : 2;
+                        constexpr int kRows = GM == 0 ? 2 : C::kFewStore ? BT / kRowStep : BT % (4 * kRowStep) == 0 ? 4 : BT % (3 * kRowStep) == 0 ? 3 : 2;
                         static_assert(BT % (kRows * kRowStep) == 0, "whole rounds");
                         const size_t o0 = static_cast<size_t>(m0) * ycols + y0 + piece * 8;
 #pragma unroll 1
@@ -952,13 +957,39 @@ gemm_i8_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
                     }
                 } else {  // any row pitch: element by element
                     const int col = et & 127;
-                    if (col < width) {
+                    auto staged = [&](int t) {
+                        uint16_t b;
+                        asm volatile("ld.shared.u16 %0, [%1];" : "=h"(b)
+                                     : "r"(out_stage + (col >> 6) * C::kPanelBytes + t * 128 + ((((col & 63) >> 3) ^ (t & 7)) << 4) + (col & 7) * 2));
+                        return __ushort_as_half(b);
+                    };
+                    if constexpr (C::kFewStore) {
+                        constexpr int kTok = BT / 16;  // (256 wide, 7071 x 7721 x 9984 592 us with eight, 562 with sixteen; 128 wide eight)
+                        static_assert(BT % (kTok * C::kParts) == 0, "whole rounds");
+                        if (col < width) {
+#pragma unroll 1
+                            for (int t0 = et >> 7; t0 < tokens; t0 += kTok * C::kParts) {
+                                const size_t o0 = static_cast<size_t>(m0) * ycols + y0 + col;
+                                __half y[kTok], r[kTok];
+#pragma unroll
+                                for (int i = 0; i < kTok; ++i) {
+                                    const int t = t0 + i * C::kParts < tokens ? t0 + i * C::kParts : t0;
+                                    y[i] = staged(t);
+                                    r[i] = a.epilogue == W8A8_EPI_RESIDUAL ? a.residual[o0 + static_cast<size_t>(t) * ycols] : __float2half(0.0f);
+                                }
+#pragma unroll
+                                for (int i = 0; i < kTok; ++i) {
+                                    const int t = t0 + i * C::kParts;
+                                    if (t >= tokens) break;
+                                    if (a.epilogue == W8A8_EPI_RESIDUAL) y[i] = __float2half(__half2float(y[i]) + __half2float(r[i]));
+                                    a.Y[o0 + static_cast<size_t>(t) * ycols] = y[i];
+                                }
+                            }
+                        }
+                    } else if (col < width) {
                         for (int t = et >> 7; t < tokens; t += C::kParts) {
                             const size_t o = static_cast<size_t>(m0 + t) * ycols + y0 + col;
-                            uint16_t b;
-                            asm volatile("ld.shared.u16 %0, [%1];" : "=h"(b)
-                                         : "r"(out_stage + (col >> 6) * C::kPanelBytes + t * 128 + ((((col & 63) >> 3) ^ (t & 7)) << 4) + (col & 7) * 2));
-                            __half y = __ushort_as_half(b);
+                            __half y = staged(t);
                             if (a.epilogue == W8A8_EPI_RESIDUAL) y = __float2half(__half2float(y) + __half2float(a.residual[o]));
                             a.Y[o] = y;
                         }
