@@ -1,13 +1,15 @@
 // Chooses and launches the tcgen05 GEMM (kernel and its reasons: w8a8_gemm_sm100.cuh).
 #include "w8a8_gemm_sm100.cuh"
 
+#include <algorithm>
+
 namespace w8a8 {
 namespace gemm {
 
 // Group sizes without a case of their own, and calls that want the group sums. (Costs fitted at groups of 32, 320, 512 and K, 40 to 4001
 // tokens, within 15 %. Nowhere there was the pair the faster one: 5-15 % slower.)
 const Form* forms_any(int* count) {
-    static const Form table[] = {form<128, false, 0>(332, 332, 1250), form<128, true, 0>(345, 355, 1840)};
+    static const Form table[] = {form<128, false, 0>({332, 332, 1250, 0, 1760, 0, 3500}), form<128, true, 0>({345, 355, 1840, 0, 1760, 0, 3500})};
     *count = static_cast<int>(sizeof(table) / sizeof(table[0]));
     return table;
 }
@@ -59,18 +61,17 @@ struct Choice {
     int splits;
 };
 
-// The tile form that ends first: whole waves of tiles over the SMs (or pairs), each tile at its measured cost. A width
-// that leaves the last wave nearly empty loses to one that fills it; narrow tiles win where there are few tokens.
+// The tile form that ends first: whole waves of tiles over the SMs (or pairs), each wave at its tiles' cost or at the time in which memory brings
+// the weights that it is the first to read (6 TB/s), whichever is longer, and a quarter of the other: 19456 rows by 64 tokens are 152 tiles, a
+// wave that memory bounds and four tiles more. A width that leaves the last wave nearly empty loses to one that fills it; narrow tiles win
+// where there are few tokens.
 // A tile's K is split over two or four CTAs where all of them fit the chip at once (a cluster of four leaves some SMs of a
-// GPC over: 128 of 148 taken as usable); meeting and adding up came out of the fit as 2.6-2.9 us for two and 5-5.6 for four. A split adds
-// the groups in another order than the other kernels do, so it has to save 10 % at least, with which 2.3 and 4.5 us choose best, and K = 2560
-// never splits.
-// Rows that are no multiple of eight leave element by element: 55 ns per token of a thread's part (measured at 4097 rows), which
-// the 256-token pairs at g = 64, with half the threads, lose by (4001 x 4097 x 2560 148 us, 192 wide 134).
+// GPC over: 128 of 148 taken as usable); 1.9 and 3.4 us for meeting and adding up choose best, 1.4 and 2.9 at g = 64. A split adds the groups in
+// another order than the other kernels do, so it has to save 6 % at least, and K = 2560 never splits.
 // table_g: the group size whose forms are looked at (0: those of any group size). pair: -1 either, 0 one CTA per tile, 1 a pair.
 // only_bt, only_splits: 0, or the token width and the split (1: none) to take; no form where they do not fit the shape.
 template <class Usable>
-Choice choose(int M, int N, int K, int table_g, int g, int sms, int pair, int only_bt, int only_splits, Usable usable) {
+Choice choose(int M, int N, int K, int table_g, int g, bool residual, int sms, int pair, int only_bt, int only_splits, Usable usable) {
     int count = 0;
     const Form* table = forms(table_g, &count);
     Choice best = {nullptr, 1};
@@ -80,15 +81,20 @@ Choice choose(int M, int N, int K, int table_g, int g, int sms, int pair, int on
         if (pair >= 0 && (f.pair != (pair != 0) || f.split)) continue;
         if (only_bt && f.bt != only_bt) continue;
         const int rows = f.pair ? 2 * BR : BR, walkers = f.pair ? sms / 2 : sms, kb_total = K / BK;
-        const double tile_ns = f.tile_ns + (N % 8 == 0 ? 0.0 : 55.0 * f.bt / f.parts);
-        const long tiles = static_cast<long>((M + f.bt - 1) / f.bt) * ((N + rows - 1) / rows);
+        const Cost& c = f.cost;
+        const double tile_ns = c.tile + (N % 8 == 0 ? (residual ? c.residual : 0.0f) : residual ? c.odd_residual : c.odd);
+        const long tiles_m = (M + f.bt - 1) / f.bt, tiles = tiles_m * ((N + rows - 1) / rows);
         for (int splits = f.split ? 2 : 1; splits <= (f.split ? 4 : 1); splits *= 2) {
             if (only_splits && splits != only_splits) continue;
             if (f.split && (tiles * splits > (splits == 2 ? sms / 2 * 2 : sms * 7 / 8 - 1) || (splits - 1) * split_kb(K, g, splits) >= kb_total))
                 continue;
             const double kb = padded_kb(f, f.split ? split_kb(K, g, splits) : kb_total);
-            double ns = ((tiles * splits + walkers - 1) / walkers) * (kb * f.stage_ns + kb * BK / g * f.group_ns + tile_ns);
-            if (f.split) ns = (ns + (splits == 2 ? 2300 : 4500)) / 0.9;
+            const double wave_ns = kb * c.stage + kb * BK / g * c.group + tile_ns;
+            const double memory_ns = static_cast<double>(rows) * K / tiles_m / splits / 6000;  // a tile's share of the weights it is the first to read
+            const long waves = (tiles * splits + walkers - 1) / walkers, last = tiles * splits - (waves - 1) * walkers;
+            auto both = [](double x, double y) { return std::max(x, y) + 0.25 * std::min(x, y); };
+            double ns = c.start + (waves - 1) * both(wave_ns, walkers * memory_ns) + both(wave_ns, last * memory_ns);
+            if (f.split) ns = (ns + (splits == 2 ? 1900 : 3400) - (g == 64 ? 500 : 0)) / 0.94;
             if ((!best.form || ns < best_ns) && usable(f)) { best = {&f, splits}; best_ns = ns; }
         }
     }
@@ -111,7 +117,7 @@ bool gemm_supports(const LinearArgs& a) {
 int gemm_form(int M, int N, int K, int g, int sms, int form, int only_bt, int only_splits, bool moved_registers, int* out3) {
     using namespace gemm;
     if (M < 1 || N < 1 || K < 1 || sms < 2 || K % BK != 0 || g % 32 != 0 || K % g != 0) return W8A8_ERR_UNSUPPORTED;
-    const Choice c = choose(M, N, K, g, g, sms, form, only_bt, only_splits, [&](const Form& f) { return moved_registers || f.launch_regs == 0; });
+    const Choice c = choose(M, N, K, g, g, false, sms, form, only_bt, only_splits, [&](const Form& f) { return moved_registers || f.launch_regs == 0; });
     if (!c.form) return W8A8_ERR_UNSUPPORTED;
     out3[0] = c.form->bt;
     out3[1] = c.form->pair ? 2 : 1;
@@ -124,7 +130,7 @@ int launch_linear_gemm(const LinearArgs& a, int* device_status, cudaStream_t str
     if (!gemm_supports(a)) return fail(W8A8_ERR_UNSUPPORTED, "tcgen05 GEMM does not take this shape");
     const int sms = device_sms();
 
-    const Choice choice = choose(a.M, a.N, a.K, a.dump ? 0 : a.g, a.g, sms, form, a.gemm_bt, a.gemm_splits, balanced);
+    const Choice choice = choose(a.M, a.N, a.K, a.dump ? 0 : a.g, a.g, a.epilogue == W8A8_EPI_RESIDUAL, sms, form, a.gemm_bt, a.gemm_splits, balanced);
     const Form* best = choice.form;
     const int best_splits = choice.splits;
     if (!best) return fail(W8A8_ERR_UNSUPPORTED, "no tile form of the tcgen05 GEMM for this shape (token width %d, splits %d asked for)",

@@ -1017,43 +1017,53 @@ struct FormState {
     SmemAttribute attribute;
     std::atomic<int> registers{0};  // per thread, as compiled (0: not asked for yet)
 };
-// A tile form: its kernel and what the launch needs to know about it. stage_ns, group_ns, tile_ns: what a tile takes per 128 bytes of
-// K, per K-group and for itself (the start of its chain, conversion, store). Fitted to 4100 times, no cost below zero, then moved by up
-// to 6 % each towards the choices that lose least: seven shapes (the four projections, 9728 x 2560, 4096 x 9728, 1000 x 1024) x 31 token
-// counts from 33 to 8192 x every form that takes them, for each group size. What it does not hold: a chip that is not full, and what
-// several sweeps over a long prompt's codes miss L2 for. Judged by its choice, the rule loses 0.3, 0.4 and 0.4 % against the best form on
-// average (groups of 64, 128, 256), and 0.3, 0.4 and 0.5 % over eight other shapes x eleven token counts.
+// What a form's tiles take, ns: per 128 bytes of K, per K-group, per tile (conversion, TMA store), once per launch (the launch itself, the first
+// operands, the end of a chain that nothing overlaps); and per tile on top, for rows that leave element by element, for a residual, for
+// both. Least squares over 15,000 times of one of the forms under the model in choose(): the four projections and 9728 x 2560 at 30 token counts from
+// 33 to 8192, 890 drawn shapes (33 to 8192 tokens, 128 to 24,000 rows, K from 128 to 12,800, every epilogue, odd rows) and 420 of up to 420
+// tokens; the model's count three times. No cost is moved after the fit. Judged by its choice against the best form, groups of 64, 128 and 256, the
+// rule loses on average 0.4, 0.6 and 1.0 % over 299 other drawn shapes, 0.6, 0.8 and 1.0 % over the drawn ones it was fitted to, 0.0, 0.2 and 0.2 %
+// over the model's. (Costs per stage and tile alone, moved towards the choices that lose least over the model's shapes: 1.6, 2.1 and 2.3; 1.4, 2.2 and
+// 2.7; 0.4 each.)
+struct Cost {
+    float stage, group, tile, start, odd, residual, odd_residual;
+};
+// A tile form: its kernel and what the launch needs to know about it.
 struct Form {
     int bt;
     bool pair, split;
     Kernel kernel[2];  // tokens walked first, rows walked first (or none)
     int threads, smem;
     int launch_regs;  // per thread, if the form moves some between its warpgroups; else 0
-    float stage_ns, group_ns, tile_ns;
-    int parts, unit_kb;  // Config::kParts, Config::kUnitKb
+    Cost cost;
+    int unit_kb;  // Config::kUnitKb
     FormState* state;  // [2]
 };
 template <int BT, bool PAIR, int GM, bool SPLIT>
 inline FormState form_state[2];
 template <int BT, bool PAIR, int GM, bool SPLIT = false>
-Form form(float stage_ns, float group_ns, float tile_ns) {
+Form form(const Cost& cost) {
     using C = Config<BT, PAIR, GM, SPLIT>;
     Kernel rows_first = nullptr;
     if constexpr (BT >= 128 && !SPLIT && GM != 0) rows_first = gemm_i8_kernel<BT, PAIR, GM, SPLIT, true>;  // (a long prompt's forms)
     return Form{BT, PAIR, SPLIT, {gemm_i8_kernel<BT, PAIR, GM, SPLIT, false>, rows_first}, C::kThreads, C::kSmem, C::kMoveRegs ? C::kLaunchRegs : 0,
-                stage_ns, group_ns, tile_ns, C::kParts, C::kUnitKb, form_state<BT, PAIR, GM, SPLIT>};
+                cost, C::kUnitKb, form_state<BT, PAIR, GM, SPLIT>};
 }
 template <int GM>
 const Form* all_forms(int* count) {
-    // per stage at groups of 64, 128 and 256, and per tile, for token widths 32, 64, 96, 128, 192, 256
-    constexpr float kStage[3][6] = {{204, 309, 391, 499, 740, 1150}, {152, 207, 294, 321, 483, 665}, {141, 170, 286, 288, 321, 383}};
-    constexpr float kTile[3][6] = {{750, 580, 1150, 1550, 2670, 2830}, {110, 740, 900, 1310, 2820, 2460}, {290, 740, 90, 500, 2190, 2730}};
-    constexpr int q = GM == 64 ? 0 : GM == 128 ? 1 : 2;
-    static const Form table[] = {form<32, false, GM>(kStage[q][0], 0, kTile[q][0]),       form<64, false, GM>(kStage[q][1], 0, kTile[q][1]),
-                                 form<96, false, GM>(kStage[q][2], 0, kTile[q][2]),       form<128, false, GM>(kStage[q][3], 0, kTile[q][3]),
-                                 form<192, true, GM>(kStage[q][4], 0, kTile[q][4]),       form<256, true, GM>(kStage[q][5], 0, kTile[q][5]),
-                                 form<32, false, GM, true>(kStage[q][0], 0, kTile[q][0]), form<64, false, GM, true>(kStage[q][1], 0, kTile[q][1]),
-                                 form<96, false, GM, true>(kStage[q][2], 0, kTile[q][2]), form<128, false, GM, true>(kStage[q][3], 0, kTile[q][3])};
+    // groups of 64, 128 and 256; token widths 32, 64, 96, 128, 192, 256
+    static constexpr Cost kCost[3][6] = {
+        {{188, 0, 489, 2990, 1330, 296, 1890}, {286, 0, 788, 3080, 2430, 611, 4200}, {363, 0, 1100, 2940, 2340, 770, 3830},
+         {488, 0, 1190, 2970, 4210, 1200, 6100}, {729, 0, 1740, 4120, 3410, 1610, 8360}, {1080, 0, 1260, 4970, 7930, 4070, 14500}},
+        {{136, 0, 298, 3050, 1260, 315, 2110}, {186, 0, 622, 3100, 2470, 519, 4350}, {260, 0, 861, 2730, 3120, 576, 6180},
+         {303, 0, 1060, 2540, 3000, 702, 1470}, {466, 0, 1510, 3630, 3680, 1270, 5070}, {616, 0, 1610, 3760, 4740, 2060, 6100}},
+        {{122, 0, 227, 2880, 1110, 221, 2150}, {142, 0, 573, 3020, 2280, 401, 4400}, {232, 0, 731, 2160, 2610, 448, 6620},
+         {249, 0, 776, 2370, 2430, 518, 1960}, {297, 0, 1580, 3410, 3390, 1010, 6260}, {362, 0, 1950, 3010, 5940, 1660, 3410}}};
+    const Cost* c = kCost[GM == 64 ? 0 : GM == 128 ? 1 : 2];
+    static const Form table[] = {form<32, false, GM>(c[0]),       form<64, false, GM>(c[1]),       form<96, false, GM>(c[2]),
+                                 form<128, false, GM>(c[3]),      form<192, true, GM>(c[4]),       form<256, true, GM>(c[5]),
+                                 form<32, false, GM, true>(c[0]), form<64, false, GM, true>(c[1]), form<96, false, GM, true>(c[2]),
+                                 form<128, false, GM, true>(c[3])};
     *count = static_cast<int>(sizeof(table) / sizeof(table[0]));
     return table;
 }
