@@ -157,6 +157,10 @@ def test_gemm_form_follows_what_is_asked_for(pkg):
     (2048, 2560, 9728, 256, (192, 2, 1)),  # 62 us; tiles of 96 tokens 74
     (150, 2560, 9728, 256, (64, 1, 2)),    # 12.9 us; tiles of 32, not split, 14.3
     (4001, 4097, 2560, 64, (192, 2, 1)),   # rows that leave element by element: 134 us; 256 wide 148
+    (1441, 9728, 512, 128, (128, 1, 1)),  # a short K: 16.5 us; 32 wide 27.3
+    (4438, 6144, 512, 256, (256, 2, 1)),  # 19.5 us; 96 wide 30.0
+    (186, 19456, 3328, 256, (64, 1, 1)),  # a second wave of few tiles: 22.4 us; one wave of pairs of 192 25.0
+    (64, 19456, 2560, 64, (32, 1, 1)),  # a wave that memory bounds: 17.0 us; 64 wide 18.3
 ])
 def test_gemm_form_that_was_measured_fastest(pkg, M, N, K, g, want):
     assert pkg.debug_gemm_form(M, N, K, g) == want
