@@ -826,8 +826,36 @@ def test_gemm_tcgen05_split_k(gemm_form, oracle, pkg, M, N, K, bt, splits, g):
                       abs_terms=abs_term_sum(oracle.group_sums(W, Xq, g), ws, Xs))
 
 
+@pytest.mark.parametrize("K,g", [(2560, 64), (1408, 64), (2816, 128), (2560, 256)])
+@pytest.mark.parametrize("bt,splits", [(32, 2), (64, 2), (64, 4), (96, 2), (96, 4), (128, 2), (128, 4)])
+@pytest.mark.parametrize("off", [0, 1, 4])
+def test_gemm_tcgen05_split_scales_at_any_address(gemm_form, oracle, pkg, K, g, bt, splits, off):
+    """Scales in a split form, where a run may begin off the boundary that its array begins on: runs of 20, 12, 11, 10, 6, 5 and 3 groups, arrays on a
+    16-byte boundary, one scale and four scales behind it. Aligned arrays give the same bits, so the form's aligned output, held to the
+    split's bar, stands for the others."""
+    M, N = 101, 300
+    ctx = gemm_form(bt, splits)
+    X, W, ws = synth.linear_case(K + bt + splits, M, N, K, g)
+    Xq, Xs = oracle.quantize(X, g)
+    dW, dXq, outs = dev(W), dev(Xq), []
+    for o in (0, off):
+        dS = torch.empty((N * (K // g) + o,), dtype=torch.float16, device="cuda")[o:].view(N, K // g)
+        dXs = torch.empty((M * (K // g) + o,), dtype=torch.float32, device="cuda")[o:].view(M, K // g)
+        dS.copy_(dev(ws))
+        dXs.copy_(dev(Xs))
+        buf, dY = guarded((M, N), torch.float16, 99.0)
+        ctx.linear_q(dW, dS, g, dXq, dXs, dY, M, N, K)
+        torch.cuda.synchronize()
+        ctx.check_device_status()
+        assert guards_intact(buf, 99.0)
+        outs.append(dY)
+    assert torch.equal(outs[0].view(torch.int16), outs[-1].view(torch.int16))
+    assert_close_fp16(oracle, outs[0].cpu().numpy(), oracle.linear_q(W, ws, Xq, Xs, g), "split K, scales at any address",
+                      abs_terms=abs_term_sum(oracle.group_sums(W, Xq, g), ws, Xs))
+
+
 @pytest.mark.parametrize("epilogue", ["NONE", "RESIDUAL", "SWIGLU"])
-@pytest.mark.parametrize("bt,splits", [(64, 1), (96, 1), (96, 2), (128, 1), (128, 4), (192, 1), (256, 1)])
+@pytest.mark.parametrize("bt,splits", [(64, 1), (64, 2), (64, 4), (96, 1), (96, 2), (128, 1), (128, 4), (192, 1), (256, 1)])
 def test_gemm_tcgen05_infinite_weight_scales(gemm_form, oracle, pkg, bt, splits, epilogue):
     """Group size 64, where the wide forms' sums carry a bias: rows with an infinite weight scale still give what float(P) * scale
     gives, signed infinities, and NaN where a group sum is zero; every other row is the oracle's."""
@@ -892,7 +920,7 @@ def test_gemm_tcgen05_many_tiles_per_cta(gemm_form, oracle, pkg, bt, form, g, K)
 
 @pytest.mark.parametrize("wval,qval", [(-128, -128), (-128, 127), (127, 127), (127, -128)])
 @pytest.mark.parametrize("g", [64, 128, 256])
-@pytest.mark.parametrize("bt,splits", [(32, 1), (64, 1), (96, 1), (128, 1), (192, 1), (256, 1), (96, 2), (128, 2)])
+@pytest.mark.parametrize("bt,splits", [(32, 1), (64, 1), (96, 1), (128, 1), (192, 1), (256, 1), (64, 2), (96, 2), (128, 2)])
 def test_gemm_tcgen05_largest_sums_without_dump(gemm_form, oracle, pkg, bt, splits, g, wval, qval):
     """The forms that a call without group sums takes, at the largest sums of a group, 128 * 128 * g of either sign (at g = 64 the
     wide forms add a bias that has to keep such a sum positive and inside 23 bits), -128 among the activation codes too. Bit for
@@ -922,13 +950,14 @@ def test_gemm_tcgen05_largest_sums_without_dump(gemm_form, oracle, pkg, bt, spli
 
 
 @pytest.mark.parametrize("epilogue", ["NONE", "RESIDUAL"])
-@pytest.mark.parametrize("g", [64, 256])
+@pytest.mark.parametrize("g", [64, 128, 256])
 @pytest.mark.parametrize("bt,form", WIDTHS)
-@pytest.mark.parametrize("N", [133, 4097])
+@pytest.mark.parametrize("N", [133, 136, 4097])
 def test_gemm_tcgen05_rows_that_are_no_multiple_of_eight(gemm_form, oracle, pkg, N, bt, form, g, epilogue):
-    """Output rows of any pitch leave element by element, by as many threads per token as the form has parts. A vocabulary of 4097
+    """Output rows of any pitch leave element by element, by as many threads per token as the form has parts; a residual's rows that
+    are multiples of eight (136) in pieces of 16 bytes. A last tile of few tokens. A vocabulary of 4097
     sampled rows is such a weight. Bit for bit the oracle's."""
-    M, K = (bt + 37, 512) if N == 133 else (33, 256)
+    M, K = (33, 256) if N == 4097 else (bt + 37, 512)
     ctx = gemm_form(bt, 1)
     X, W, ws = synth.linear_case(N + bt, M, N, K, g)
     Xq, Xs = oracle.quantize(X, g)
@@ -945,7 +974,7 @@ def test_gemm_tcgen05_rows_that_are_no_multiple_of_eight(gemm_form, oracle, pkg,
     assert np.array_equal(dY.cpu().numpy().view(np.uint16), want.view(np.uint16))
 
 
-@pytest.mark.parametrize("bt,form", [(96, "SINGLE"), (128, "SINGLE"), (192, "PAIR"), (256, "PAIR")])
+@pytest.mark.parametrize("bt,form", [(64, "SINGLE"), (96, "SINGLE"), (128, "SINGLE"), (192, "PAIR"), (256, "PAIR")])
 def test_gemm_tcgen05_infinite_weight_scales_over_many_tiles(gemm_form, oracle, pkg, bt, form):
     """Tiles with an infinite weight scale and tiles without one in turn on one CTA, one chunk of scales per tile, so that the
     scales are staged up to three tiles ahead of the tile that is being written."""
