@@ -959,7 +959,7 @@ struct Scratch {
     size_t qkv, xq, xs, aq, as_, act, actq, acts, delta, attn_part, barrier, timeline, total;
 };
 
-Scratch layout(const w8a8_decode_stack& d, int S) {
+Scratch layout(const w8a8_decode_stack& d, int sms) {
     Scratch sc;
     const size_t B = d.batch, g = d.group_size;
     const size_t qkv_n = static_cast<size_t>(d.n_q_heads + 2 * d.n_kv_heads) * kHeadDim;
@@ -975,7 +975,9 @@ Scratch layout(const w8a8_decode_stack& d, int S) {
     sc.actq = take(B * d.inter);
     sc.acts = take(B * (d.inter / g) * 4);
     sc.delta = take(B * d.dim * 2);
-    sc.attn_part = take(B * d.n_kv_heads * S * kQPerKv * kPartStride * 4);
+    // what slices_for() asks for at this batch or any smaller one, so that scratch for a batch serves the smaller ones too
+    const size_t pairs = B * d.n_kv_heads, most = pairs > static_cast<size_t>(sms) ? pairs : static_cast<size_t>(sms);
+    sc.attn_part = take((8 * pairs < most ? 8 * pairs : most) * kQPerKv * kPartStride * 4);
     sc.barrier = take(256);
     sc.timeline = take(static_cast<size_t>(18 * d.n_layers + 2) * 8);
     sc.total = off;
@@ -1009,13 +1011,13 @@ const char* check(const w8a8_decode_stack& d) {
 
 size_t decode_stack_workspace_bytes(const w8a8_decode_stack& d) {
     if (check(d)) return 0;
-    return layout(d, slices_for(d, device_sms())).total;
+    return layout(d, device_sms()).total;
 }
 
 int decode_stack_timeline(const w8a8_decode_stack& d, const unsigned char* workspace, unsigned long long* out, int capacity,
                           cudaStream_t stream) {
     if (const char* why = check(d)) return fail(W8A8_ERR_UNSUPPORTED, "decode stack: %s", why);
-    const Scratch sc = layout(d, slices_for(d, device_sms()));
+    const Scratch sc = layout(d, device_sms());
     const int n = 18 * d.n_layers + 2;
     if (capacity < n) return fail(W8A8_ERR_INVALID_ARG, "timeline needs room for %d stamps", n);
     cudaError_t e = cudaMemcpyAsync(out, workspace + sc.timeline, static_cast<size_t>(n) * 8, cudaMemcpyDeviceToHost, stream);
@@ -1029,7 +1031,7 @@ int launch_decode_stack(const w8a8_decode_stack& d, unsigned char* workspace, si
     const int sms = device_sms();
     StackParams p = {};
     p.S = slices_for(d, sms);
-    const Scratch sc = layout(d, p.S);
+    const Scratch sc = layout(d, sms);
     if (sc.total > workspace_bytes)
         return fail(W8A8_ERR_WORKSPACE, "decode stack needs %zu bytes of scratch, context has %zu", sc.total, workspace_bytes);
     p.layers = d.layers;

@@ -87,6 +87,21 @@ def test_one_launch_step_fills_the_gpu_whatever_the_tables_width(pkg, batch, n_k
     assert len(sizes) == 1 and sizes.pop() > 0
 
 
+@pytest.mark.parametrize("n_kv", [1, 2, 4, 8])
+def test_one_launch_scratch_for_a_batch_serves_smaller_ones(pkg, n_kv):
+    from fish_audio_cpp_b200 import capi
+
+    lib = pkg.load_library()
+    d = capi.DecodeStack()
+    d.n_layers, d.dim, d.n_q_heads, d.n_kv_heads, d.head_dim, d.inter, d.group_size, d.max_blocks_per_seq = 1, 256, 4 * n_kv, n_kv, 128, 256, 64, 64
+    for f in ("layers", "final_norm", "rope_freqs", "positions", "seq_lens", "block_table", "k_cache", "v_cache", "x", "out"):
+        setattr(d, f, 1 << 20)  # (never read: the answer is arithmetic)
+    sizes = []
+    for d.batch in range(1, 9):
+        sizes.append(lib.w8a8_decode_stack_workspace_bytes(ctypes.byref(d)))
+    assert sizes == sorted(sizes)
+
+
 ROOM_148 = {2: 74, 3: 45, 4: 33, 5: 26, 6: 22, 7: 15, 8: 15}  # what the occupancy query answers on 148 SMs
 
 
