@@ -31,10 +31,11 @@
 // latency, and descriptors computed in divergent code are moved to uniform registers one by one): the tensor pipe ran at
 // 0.6 of its rate. Hence: the whole warp runs the loop and one elected lane issues; the loop is unrolled over the stages
 // so that stage, accumulator slice and descriptor offsets are immediates; group sizes 64 / 128 / 256 are template cases.
-// The promote is the other side, and the bound in most forms: stamps of the clock in an epilogue warp, taken before the units (they cost some 10 % themselves;
-// profiles/gemm_i8_kernel_epilogue_clock_stamps.md) show 1216, 1424 and 1451 clocks per K-group of a 128 x 256 tile at groups of 64, 128
-// and 256, of which 224-358 are waits for the MMAs, against 384 (with the bias), 512 and 1024 of MMAs. In trial programs of sixteen such
-// warps alone, clocks per warp and scheduler for two sums (the programs are not kept):
+// The promote is the other side, and the bound in most forms. Stamps of the clock in an epilogue warp, taken before the units, the chunks of eight
+// groups and the wide reads of scales (they cost some 10 % themselves, and have not been taken again), showed 1216, 1424 and 1451 clocks per
+// K-group of a 128 x 256 tile at groups of 64, 128 and 256, of which 224-358 were waits for the MMAs, against 384 (with the bias), 512 and 1024
+// of MMAs. The counters of the present forms at 2048 x 19456 x 2560: tensor pipe 59 % busy at g = 256 (256 wide), 35 % at g = 64 (128 wide), a
+// third of that the bias; issue slots 53 and 50 %. In trial programs of sixteen such warps alone, clocks per warp and scheduler for two sums (the programs are not kept):
 //   * two conversions, a packed multiply and a packed FMA 4.3 by themselves, 6.9-7.2 with the tensor-memory and shared-memory reads around
 //     them, as if conversions and those reads shared a way into the registers; two packed FMAs without conversions 5.1-5.6 with the
 //     reads. Hence the BIAS at g = 64 (promote2): each group's accumulator starts from a constant, made by one more MMA of a
@@ -54,13 +55,13 @@
 // 32 wide 20.9 -> 20.2 (96 and 128 wide lose a sixth by units of two: there the MMAs of a unit take longer than its promote hides).
 // A tile's K, or its run of a split, is padded to whole units, so that slots and columns stay immediates of the issuer: loads past
 // K bring zeros, those past a run the next run's operands, and the scales of the groups that only fill a unit are zero, which adds
-// 0 to sums that are never -0. (700 x 2560 x 2816, g = 256, 64 wide: 11 groups as 12, 11.0 us and 11.7.)
+// 0 to sums that are never -0. (700 x 2560 x 2816, g = 256, 64 wide: 11 groups as 12, 11.0 us and 11.7. A short K pays most: 150 x 2560 x 1280,
+// g = 128, ten groups as twelve, 5.1 us with single groups and 5.5; 267 x 3680 x 384, g = 64, six as eight, 4.9 and 5.9.)
 //
-// Measured back to back in turn, us, without the bias, the units, the 16-byte scale reads and the cheaper SwiGLU, and with them
-// (M x N x K; the long ones under the power cap; before units of more than two groups and wide reads of scales, for which see kUnit and kWideScales):
-//   8192 x 19456 x 2560, g = 64   967 -> 787 (844 -> 1037 TOPS); g = 128 617 -> 568; g = 256 447 -> 393 (1827 -> 2076 TOPS)
-//   2048 x  2560 x 9728, g = 64   154 -> 120;  613 x 2560 x 9728  52.8 -> 42.1;  150 x 19456 x 2560  52.6 -> 36.0
-//   4001 x  6144 x 2560, g = 128  95.2 -> 95.2; g = 256 66.9 -> 66.9 (no SwiGLU, pairs of 192 tokens)
+// Back to back, us, without the bias, the units, the 16-byte scale reads and the cheaper SwiGLU, and as it is (M x N x K; the long ones under the power cap):
+//   8192 x 19456 x 2560 with SwiGLU, g = 64 967 -> 799 (844 -> 1021 TOPS); g = 128 617 -> 531; g = 256 447 -> 369 (1827 -> 2211 TOPS)
+//   g = 64 2048 x 2560 x 9728 154 -> 90;  613 x 2560 x 9728 52.8 -> 32.8;  150 x 19456 x 2560 with SwiGLU 52.6 -> 29.4
+//   4001 x 6144 x 2560, g = 128 95.2 -> 77.8; g = 256 66.9 -> 55.6
 //
 // Every mbarrier wait is bounded; a wait that runs out records an error word, and the CTA still frees its tensor memory
 // before it returns.
@@ -317,7 +318,7 @@ __device__ __forceinline__ uint64_t smem_desc(uint32_t saddr) {
 // With the bias (promote2), an infinite weight scale gives infinity less infinity. The output columns of such weight rows, in the
 // tile that lies in shared memory, are formed anew, from the operands: signed infinities and NaN as float(P) * ws has them. Slow, and
 // only run for a tile that has met an infinite scale (one such row: 4001 x 6144 x 2560 997 us with a search of every row by every
-// thread in every tile that followed, 190 now, 161 without such a row). First which rows those are, a thread per row, into rows[4]:
+// thread in every tile that followed, 171 now, 116 without such a row). First which rows those are, a thread per row, into rows[4]:
 __device__ __forceinline__ void find_infinite_rows(const LinearArgs& a, uint32_t* rows, int n0, int et) {
     bool any = false;
     if (et < BR && n0 + et < a.N)

@@ -668,7 +668,7 @@ PREFILL_CASES = [(name, g, 2048) for name in ("qkv", "o", "gate_up", "down") for
 
 @pytest.mark.parametrize("name,g,M", PREFILL_CASES)
 def test_prefill_shapes_full_size(ctx, oracle, pkg, name, g, M):
-    """configs[2], all sixteen cases (four projections x g in {256, 64} x M in {2048, 8192}): the whole GEMM
+    """Prefill, sixteen cases (four projections x g in {256, 64} x M in {2048, 8192}): the whole GEMM
     runs on the GPU; a random 48-token x 192-row sub-problem is recomputed by the oracle (each output
     depends only on its own token row and weight row) and must agree bit for bit; a second run of the full
     problem, through the form of the kernel that the default did NOT pick (a CTA pair per tile where it takes one CTA, and the
@@ -1496,7 +1496,7 @@ def test_gemm_tcgen05_extreme_codes(ctx, oracle, pkg, g, wval, qval, form):
 
 # ---------------------------------------------------------------- headline shapes at full size
 DECODE_CASES = [(name, g, M) for name in ("qkv", "o", "gate_up", "down") for g in (256, 64) for M in (1, 4, 16)] + \
-    [("gate", 256, 16)]  # configs[0]: the un-fused gate projection, M = 16, K = 2560, N = 9728, g = 256
+    [("gate", 256, 16)]  # the un-fused gate projection, M = 16, K = 2560, N = 9728, g = 256
 
 
 @pytest.mark.parametrize("name,g,M", DECODE_CASES)
